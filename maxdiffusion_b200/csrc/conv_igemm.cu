@@ -41,9 +41,8 @@ constexpr int MAX_TAPS = 36;      // 27 (3x3x3) or 4 classes x 9
 constexpr int MAX_CLASSES = 4;
 // TMEM columns per accumulator: 256 (two accumulators = all 512 columns, one CTA per SM) for wide tiles, 128 for
 // tiles of at most 128 output channels, which run TWO CTAs per SM (256 columns and half the shared memory each).
-// One thread can issue a tcgen05.mma only every ~100 ns whatever its width, so with narrow tiles a single issuing
-// lane leaves the tensor pipe half idle; two co-resident CTAs are two issuing lanes, each tile still accumulated
-// by one thread in a fixed order (bitwise reproducible).
+// A narrow tile holds little tensor work per pipeline stage; two co-resident CTAs overlap one's waits and epilogue with
+// the other's products, each tile still accumulated by one thread in a fixed order (bitwise reproducible).
 
 struct Tap {
   int o0;              // added to the channel coordinate (parity * C in the stride-2 view, else 0)
@@ -142,7 +141,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int issued = 0;
@@ -191,7 +190,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(BM, p.BN, false, false);
       int stage = 0;
       uint32_t phase = 0;

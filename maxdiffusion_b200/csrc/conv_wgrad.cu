@@ -101,7 +101,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int issued = 0;
@@ -160,7 +160,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(BM, p.BN, true, true);
       int stage = 0;
       uint32_t phase = 0;

@@ -30,6 +30,15 @@ constexpr int Y_CHUNK_BYTES = BY * 128;         // 8 KiB
 constexpr int MAX_SEGMENTS = 8;
 constexpr int EW_GROUPS = 4;                    // elementwise warp groups, 16 of the 64 columns each
 constexpr int NUM_THREADS = 128 + EW_GROUPS * 128;  // warp 0 TMA, warp 1 score MMAs, warp 2 accumulating MMAs, warps 4.. elementwise
+// The lane of a role warp that issues its products. head_dim 128: the lane elected by `elect.sync` (see ptx.cuh; dQ pass
+// at 32760^2 x 8 heads 5.88 -> 5.43 ms, dK/dV 7.13 -> 6.94 ms). head_dim 64 keeps lane 0: its steps are half as long, and
+// products that arrive faster only make the elementwise warps collide (4 x 4096^2 x 10 heads: 553 / 373 us with lane 0
+// against 590 / 398 us elected).
+template <int HD>
+__device__ __forceinline__ bool issuing_lane(int lane) {
+  if (HD == 128) return elect_one();
+  return lane == 0;
+}
 template <int HD>
 constexpr int smem_bytes() {
   return 2 * (HD / 64) * X_CHUNK_BYTES + Y_STAGES * 2 * (HD / 64) * Y_CHUNK_BYTES + Y_STAGES * 128 * 4 + 1024 + 256;
@@ -199,7 +208,7 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
     // Three lanes in different warps feed the tensor pipe: a step's waits, commits and MMA instructions cost an
     // issuing lane more cycles than the products take to execute. Warp 1 issues X1 Y1^T (S), warp 3 issues
     // X2 Y2^T (dP), warp 2 the accumulating products. Every dependency between them is an mbarrier.
-    if (lane == 0 && total_steps > 0) {
+    if (total_steps > 0 && issuing_lane<HD>(lane)) {
       constexpr uint32_t idesc_t = make_idesc_bf16(128, BY, false, false);   // score tiles, N = 64
       const bool second = warp == 3;
       bool ok = mbar_wait(x_full, 0, abort_flag, p.status, 80);
@@ -232,7 +241,7 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
     }
   } else if (warp == 2) {
     // ------------------------------ issuing lane B: accumulating products --------
-    if (lane == 0 && total_steps > 0) {
+    if (total_steps > 0 && issuing_lane<HD>(lane)) {
       constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, false, true); // B operand MN-major
       const uint64_t ym0 = make_smem_desc(smem_u32(sy), Y_CHUNK_BYTES, 1024);
       constexpr uint32_t STAGE_STEP = (2 * Y_TILE_BYTES) >> 4, TILE_STEP = Y_TILE_BYTES >> 4;

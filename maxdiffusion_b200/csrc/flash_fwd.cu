@@ -302,7 +302,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0 && total_blocks > 0) {
+    if (total_blocks > 0 && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       unsigned long long seen = 0;  // (segment, head group) flags that have been observed
@@ -351,7 +351,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
   } else if (warp == 1 || warp == 3) {
     // ------------------------------ issuing lanes: S_t = Q_t K_j^T --------------
-    if (lane == 0 && total_blocks > 0) {
+    if (total_blocks > 0 && elect_one()) {
       const int t = warp >> 1;  // warp 1 -> tile 0, warp 3 -> tile 1
       constexpr uint32_t idesc_s = make_idesc_bf16(128, BKV, false, false);
       // descriptors are built once; the address field (units of 16 bytes) advances by addition
@@ -397,7 +397,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     }
   } else if (warp == 2 || warp == 4) {
     // ------------------------------ issuing lanes: O_t += P_t V_j ----------------
-    if (lane == 0 && total_blocks > 0) {
+    if (total_blocks > 0 && elect_one()) {
       const int t = (warp >> 1) - 1;  // warp 2 -> tile 0, warp 4 -> tile 1
       constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, false, true);
       const uint64_t vd0 = make_smem_desc(smem_u32(sv), KV_CHUNK_BYTES, 1024);

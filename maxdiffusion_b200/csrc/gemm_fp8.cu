@@ -93,7 +93,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   const uint32_t tmem_base = *tmem_ptr_smem;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int issued = 0;
@@ -121,7 +121,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = p.int8 ? make_idesc_i8(BM, BN) : make_idesc_f8(BM, BN, p.a_e5m2, p.b_e5m2);
       int stage = 0;
       uint32_t phase = 0;
