@@ -1,15 +1,20 @@
 // Persistent, warp-specialised bf16 GEMM for sm_100a:
 //     D[M,N] = epilogue( A[M,K] * B[N,K]^T )
-// Operands come through (non-multicast) TMA into 128-byte-swizzled shared memory, the product is
-// issued by one thread with tcgen05.mma (128 x 256 x 16 per instruction), fp32 accumulators sit in
-// TMEM and are double buffered (2 x 256 columns) so that the epilogue of tile i overlaps the main
-// loop of tile i+1.
+// Operands come through (non-multicast) TMA into 128-byte-swizzled shared memory, products are issued by one thread with
+// tcgen05.mma, fp32 accumulators sit in TMEM and are double buffered (2 x 256 columns) so that the epilogue of tile i
+// overlaps the main loop of tile i+1.
+//
+// What bounds it is the operand feed from L2: every shape ran at about 57 bytes per clock and SM, which a 128 x 256 tile
+// of one CTA (48 KB per 512 tensor clocks) turns into 60 % of the tensor rate. So tiles of more than 128 rows are
+// computed by a PAIR of CTAs (`cta_group::2`): 256 x BN, each CTA fetching its own 128 rows of A and half of B (32 KB per
+// 512 clocks at BN = 256) and draining its own 128 accumulator rows. One CTA / a pair: 65520 x 5120 x 5120 2566 / 2278 us
+// (1508 TFLOP/s), 4608 x 12288 x 3072 285 / 230 us.
 //
 // Either operand may be "MN-major" (stored transposed, i.e. A as [K,M] or B as [K,N]); this is what
 // lets dgrad (dX = dY * W) and wgrad (dW = dY^T * X) run on the same kernel without transposes.
 //
-// Roles:  warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2..5 and 6..9 = two epilogue groups, each
-// taking one column half of every tile (own staging slab, named barrier and TMA-store issuing thread).
+// Roles:  warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer (of a pair: in the even CTA), warps 2..5 and 6..9 = two
+// epilogue groups that take the tile's 128-byte-wide slabs in turn.
 // Covers the reference's XLA:GPU / cuBLAS matmuls behind every Dense layer
 // (src/maxdiffusion/models/attention_flax.py:2471-2525, models/wan/transformers/transformer_wan.py:220-330)
 // together with the elementwise fusions XLA places after them (bias, GELU-tanh, gated residual).
@@ -18,24 +23,26 @@
 namespace mdb {
 
 namespace gemm {
-constexpr int BM = 128;
+constexpr int BM = 128;  // rows of one CTA; a pair's tile has 256
 constexpr int BK = 64;
 constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
-constexpr int NUM_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2..5 and 6..9: two epilogue groups (one column half each)
-constexpr int GROUP_M = 8;
-// The tile is 128 x BN with BN = 256 (the default) or 128 (on request). The narrower tile fills the waves of the
-// 148 persistent CTAs better at small M, but it moves a third more operand bytes per FLOP from L2 into shared
-// memory and measured 1.3-1.5x SLOWER on every shape of an 8-way sequence split (4095 x 5120 x 5120: 0.228 ms
-// against 0.173 ms), so the launcher never picks it by itself: operand traffic, not wave fill, is the limit.
-__host__ __device__ constexpr int stages_for(int bn) { return bn == 256 ? 4 : 6; }                    // 4 x 48 KiB or 6 x 32 KiB
-__host__ __device__ constexpr int stage_bytes(int bn) { return A_BYTES + bn * BK * 2; }
-// Output staging of the epilogue: one 128-row x 128-byte slab (64 bf16 or 32 fp32 columns) per epilogue group in the
-// 128-byte swizzle, written by the group's warps and drained by its TMA stores.
-constexpr int SLAB_BYTES = BM * 128;
-constexpr int STAGING_BYTES = 2 * SLAB_BYTES;
-constexpr int BIAS_BYTES = 256 * 4;  // the tile's bias columns as fp32
-__host__ __device__ constexpr int smem_bytes(int bn) {
-  return stages_for(bn) * stage_bytes(bn) + STAGING_BYTES + BIAS_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int NUM_THREADS = 320;  // warp 0 TMA, warp 1 MMA, warps 2..5 and 6..9: two epilogue groups
+constexpr int EPI_WARPS = 8;
+constexpr int MAX_STAGES = 8;
+constexpr int ACC_COLS = 256;     // TMEM columns of one accumulator
+// Output staging of the epilogue: a slab of 32 rows x 128 bytes (64 bf16 or 32 fp32 columns) per epilogue warp, in which
+// the accumulator rows that a thread owns become the 128-byte lines that 8 lanes store together. Everything a warp stages
+// stays within the warp: no CTA barrier and no wait for an earlier store.
+constexpr int SLAB_BYTES = 32 * 128;
+constexpr int STAGING_BYTES = EPI_WARPS * SLAB_BYTES;
+constexpr int BIAS_BYTES = 2 * 256 * 4;  // the tile's bias columns as fp32, for two tiles in turn
+constexpr int FIXED_BYTES = STAGING_BYTES + BIAS_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int SMEM_LIMIT = 227 * 1024;
+// One stage holds a k-block of A (128 rows) and of this CTA's share of B; a multiple of 1024 bytes.
+__host__ __device__ constexpr int stage_bytes(int bn, int cg) { return A_BYTES + bn / cg * BK * 2; }
+__host__ constexpr int stages_for(int bn, int cg) {
+  const int n = (SMEM_LIMIT - FIXED_BYTES) / stage_bytes(bn, cg);
+  return n < MAX_STAGES ? n : MAX_STAGES;
 }
 
 enum Epilogue : int {
@@ -44,6 +51,17 @@ enum Epilogue : int {
   kEpiGatedRes = 2,   // out = residual + gate[batch(row), col] * (acc*alpha + bias)
   kEpiSilu = 3,       // out = silu(acc*alpha + bias)
   kEpiAddRes = 4,     // out = residual + acc*alpha + bias
+};
+
+// Epilogues are compiled one by one: a kernel that carries all of them does not fit the instruction cache, and a short
+// product then spends its time on fetching code (128 x 256 x 64: 7.5 us with one kernel for all, 6.2 us so; 8192 x 2560 x
+// 64, five rounds of tiles: 23.1 and 13.3 us).
+enum EpilogueKind : int {
+  kPlain = 0,    // bf16 out, bias or none
+  kAct = 1,      // bf16 out, bias, GELU-tanh or SiLU
+  kRes = 2,      // bf16 out, bias, (gated) residual
+  kPlainF32 = 3, // fp32 out or split-K partials, bias or none
+  kDirect = 4,   // anything, 16-byte stores from one thread per row
 };
 
 struct Params {
@@ -66,12 +84,11 @@ struct Params {
   int splits;
   int kb_per_split;
   float* partial;
-  int partial_rows;  // rows per split in `partial` (M rounded up to the tile height when TMA stores write it)
-  // 1: the epilogue stages 128-byte-wide slabs in shared memory and writes them with TMA stores (full lines, clipped
-  // at the edges of the tensor) instead of 16-byte stores from one thread per row
-  int tma_store;
+  int bn;      // columns of a tile: 64, 128, 192 or 256
+  int stages;  // pipeline depth
 };
 
+template <int GROUP_M>
 __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int& m_idx, int& n_idx) {
   // Grouped rasterisation: GROUP_M row-blocks share each sweep over the column-blocks so that
   // concurrently running CTAs reuse both operands out of L2.
@@ -84,54 +101,63 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
   n_idx = local / rows;
 }
 
-template <bool A_MN, bool B_MN, int BN>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+template <bool A_MN, bool B_MN, int CG, int EK>
+__global__ void __cluster_dims__(CG, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-            const __grid_constant__ CUtensorMap tmap_c, const Params p) {
-  constexpr int STAGES = stages_for(BN);
-  constexpr int STAGE_BYTES = stage_bytes(BN);
-  constexpr int TMEM_COLS = 2 * BN;  // two accumulators
+            const Params p) {
+  constexpr int TILE_M = CG * BM;
+  constexpr int GROUP_M = 8;
+  constexpr int TMEM_COLS = 2 * ACC_COLS;   // two accumulators
+  const int STAGES = p.stages, BN = p.bn, BN_CTA = BN / CG;
+  const int STAGE_BYTES = A_BYTES + BN_CTA * BK * 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + STAGES * STAGE_BYTES;  // 1024-byte aligned: every stage is a multiple of 1024 bytes
   float* bias_s = reinterpret_cast<float*>(staging + STAGING_BYTES);
   uint64_t* bars = reinterpret_cast<uint64_t*>(staging + STAGING_BYTES + BIAS_BYTES);
-  uint64_t* full_bar = bars;                    // [STAGES]
-  uint64_t* empty_bar = bars + STAGES;          // [STAGES]
-  uint64_t* tmem_full = bars + 2 * STAGES;      // [2]
-  uint64_t* tmem_empty = bars + 2 * STAGES + 2; // [2]
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint64_t* full_bar = bars;                        // [MAX_STAGES]; of a pair: only the even CTA's are used
+  uint64_t* empty_bar = bars + MAX_STAGES;          // [MAX_STAGES]
+  uint64_t* tmem_full = bars + 2 * MAX_STAGES;      // [2]
+  uint64_t* tmem_empty = bars + 2 * MAX_STAGES + 2; // [2]; of a pair: only the even CTA's are used
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_m = (p.M + BM - 1) / BM;
+  const int rank = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int group_id = static_cast<int>(blockIdx.x) / CG, num_groups = static_cast<int>(gridDim.x) / CG;
+  const int num_m = (p.M + TILE_M - 1) / TILE_M;
   const int num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
   const int num_work = num_tiles * p.splits;
 
   if (threadIdx.x == 0) {
+    prefetch_tensormap(&tmap_a);
+    prefetch_tensormap(&tmap_b);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 256);  // both epilogue groups have read the accumulator
+      mbar_init(&tmem_empty[a], CG * EPI_WARPS);  // every epilogue warp (of both CTAs) has read the accumulator
     }
     *abort_flag = 0;
     fence_mbar_init();
-    prefetch_tensormap(&tmap_a);
-    prefetch_tensormap(&tmap_b);
-    if (p.tma_store) prefetch_tensormap(&tmap_c);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_ptr_smem, TMEM_COLS);
-    tmem_relinquish();
+    if (CG == 2) {
+      tmem_alloc_pair(tmem_ptr_smem, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_ptr_smem, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (CG == 2) cluster_sync();  // the partner's barriers are initialised and its TMEM is allocated
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
@@ -142,58 +168,76 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       uint32_t phase = 0;
       int issued = 0;
       bool ok = true;
-      for (int work = blockIdx.x; work < num_work && ok; work += gridDim.x) {
+      for (int work = group_id; work < num_work && ok; work += num_groups) {
         int m_idx, n_idx;
         const int split = work / num_tiles;
-        tile_coords(work - split * num_tiles, num_m, num_n, m_idx, n_idx);
-        const int m0 = m_idx * BM, n0 = n_idx * BN;
+        tile_coords<GROUP_M>(work - split * num_tiles, num_m, num_n, m_idx, n_idx);
+        const int m0 = m_idx * TILE_M + rank * BM, n0 = n_idx * BN + rank * BN_CTA;
         const int kb_begin = split * p.kb_per_split, kb_end = min(num_kb, kb_begin + p.kb_per_split);
         for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 10)) { ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           uint8_t* sb = sa + A_BYTES;
-          mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
           const int k0 = kb * BK;
-          if (A_MN) {
+          if (CG == 2) {
+            // both CTAs' copies complete on the even CTA's barrier, which expects the bytes of both
+            if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
+            const uint32_t bar = cluster_map(&full_bar[stage], 0);
+            if (A_MN) {
 #pragma unroll
-            for (int c = 0; c < BM / 64; ++c) tma_load_2d(sa + c * (BK * 128), &tmap_a, &full_bar[stage], m0 + c * 64, k0);
+              for (int c = 0; c < BM / 64; ++c) tma_load_2d_pair(sa + c * (BK * 128), &tmap_a, bar, m0 + c * 64, k0);
+            } else {
+              tma_load_2d_pair(sa, &tmap_a, bar, k0, m0);
+            }
+            if (B_MN) {
+              for (int c = 0; c < BN_CTA / 64; ++c) tma_load_2d_pair(sb + c * (BK * 128), &tmap_b, bar, n0 + c * 64, k0);
+            } else {
+              tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);
+            }
           } else {
-            tma_load_2d(sa, &tmap_a, &full_bar[stage], k0, m0);
-          }
-          if (B_MN) {
+            mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
+            if (A_MN) {
 #pragma unroll
-            for (int c = 0; c < BN / 64; ++c) tma_load_2d(sb + c * (BK * 128), &tmap_b, &full_bar[stage], n0 + c * 64, k0);
-          } else {
-            tma_load_2d(sb, &tmap_b, &full_bar[stage], k0, n0);
+              for (int c = 0; c < BM / 64; ++c) tma_load_2d(sa + c * (BK * 128), &tmap_a, &full_bar[stage], m0 + c * 64, k0);
+            } else {
+              tma_load_2d(sa, &tmap_a, &full_bar[stage], k0, m0);
+            }
+            if (B_MN) {
+              for (int c = 0; c < BN_CTA / 64; ++c) tma_load_2d(sb + c * (BK * 128), &tmap_b, &full_bar[stage], n0 + c * 64, k0);
+            } else {
+              tma_load_2d(sb, &tmap_b, &full_bar[stage], k0, n0);
+            }
           }
           ++issued;
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
       if (!ok) {
-        // Give the copies already in flight a bounded chance to land before the CTA exits.
+        // Give the copies already in flight a bounded chance to land before the CTA exits. The odd CTA of a pair has no
+        // barrier of its own to look at: it gives its copies a fixed time.
         const int pending = issued < STAGES ? issued : STAGES;
-        for (int i = 0; i < pending; ++i) {
+        for (int i = 0; i < pending && rank == 0; ++i) {
           int s = (stage - 1 - i + 2 * STAGES) % STAGES;
           uint32_t ph = (i < stage) ? phase : (phase ^ 1u);
           for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(&full_bar[s], ph); ++spin) {}
         }
+        for (int i = 0; i < 100 && CG == 2; ++i) __nanosleep(10000);
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+    if (rank == 0 && elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(TILE_M, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int work = blockIdx.x; work < num_work && ok; work += gridDim.x, ++it) {
+      for (int work = group_id; work < num_work && ok; work += num_groups, ++it) {
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1u;
         if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 20)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
         const int kb_begin = (work / num_tiles) * p.kb_per_split, kb_end = min(num_kb, kb_begin + p.kb_per_split);
         for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, 21)) { ok = false; break; }
@@ -206,113 +250,122 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
                                      : make_smem_desc(sa + k * 32, 16, 1024);
             const uint64_t db = B_MN ? make_smem_desc(sb + k * 2048, BK * 128, 1024)
                                      : make_smem_desc(sb + k * 32, 16, 1024);
-            umma_ss(d_tmem, da, db, idesc, (kb > kb_begin || k > 0) ? 1u : 0u);
+            const uint32_t accumulate = (kb > kb_begin || k > 0) ? 1u : 0u;
+            if (CG == 2) umma_ss_pair(d_tmem, da, db, idesc, accumulate);
+            else umma_ss(d_tmem, da, db, idesc, accumulate);
           }
-          umma_commit(&empty_bar[stage]);
+          if (CG == 2) umma_commit_pair(&empty_bar[stage]);
+          else umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&tmem_full[acc]);
+        if (ok) {
+          if (CG == 2) umma_commit_pair(&tmem_full[acc]);
+          else umma_commit(&tmem_full[acc]);
+        }
       }
     }
   } else {
     // ------------------------------ Epilogue ----------------------------------
-    // Two groups of four warps share a tile: group g takes the columns [g BN/2, (g + 1) BN/2). With short
-    // contractions (10-20 K blocks) a tile's epilogue lasts as long as its main loop; two groups halve it. Each group
-    // has its own staging slab, named barrier and store-issuing thread.
+    // Two groups of four warps share a tile and take its slabs (64 bf16 or 32 fp32 columns) in turn. With short
+    // contractions (10-20 K blocks) a tile's epilogue lasts as long as its main loop; two groups halve it.
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31 are reachable from this warp
     const int row_in_tile = quarter * 32 + lane;
     const int egroup = (warp - 2) >> 2;
     const int group_thread = static_cast<int>(threadIdx.x) - 64 - egroup * 128;
-    const int col_begin = egroup * (BN / 2), col_end = col_begin + BN / 2;
+    constexpr bool f32 = EK == kPlainF32;
+    constexpr int slab_cols = f32 ? 32 : 64;
+    const bool use_bias = p.bias != nullptr && p.splits == 1;
     int it = 0;
     bool ok = true;
-    for (int work = blockIdx.x; work < num_work && ok; work += gridDim.x, ++it) {
+    for (int work = group_id; work < num_work && ok; work += num_groups, ++it) {
       int m_idx, n_idx;
       const int split = work / num_tiles;
-      tile_coords(work - split * num_tiles, num_m, num_n, m_idx, n_idx);
+      tile_coords<GROUP_M>(work - split * num_tiles, num_m, num_n, m_idx, n_idx);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
+      float* bias_t = bias_s + acc * 256;
+      if (EK != kDirect && use_bias) {
+        // the tile's bias columns once, as fp32, while the products run; a warp that still reads the previous tile's is
+        // one barrier behind and reads the other buffer
+        for (int c = group_thread; c < BN; c += 128) {
+          const int col = n_idx * BN + c;
+          if (((c / slab_cols) & 1) == egroup) bias_t[c] = col < p.N ? __bfloat162float(p.bias[col]) : 0.0f;
+        }
+        named_bar_sync(1 + egroup, 128);
+      }
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status, 30)) { ok = false; break; }
       tc_fence_after_sync();
-      const long long row = static_cast<long long>(m_idx) * BM + row_in_tile;
+      const long long row0 = static_cast<long long>(m_idx) * TILE_M + rank * BM;  // may lie beyond M in the odd CTA
+      const long long row = row0 + row_in_tile;
       const bool row_ok = row < p.M;
       const int batch = (p.rows_per_batch > 0) ? static_cast<int>(row / p.rows_per_batch) : 0;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
-      if (p.tma_store) {
-        // ---- staged epilogue: 128 bytes of every row per slab, swizzled, one TMA store per slab ----
-        const bool f32 = p.out_f32 || p.splits > 1;
-        const int slab_cols = f32 ? 32 : 64;
-        const bool leader = group_thread == 0;  // the group's first thread issues and tracks its stores
-        const long long out_row0 = (p.splits > 1 ? static_cast<long long>(split) * p.partial_rows : 0) +
-                                   static_cast<long long>(m_idx) * BM;
-        const int sw = row_in_tile & 7;
-        const bool use_bias = p.bias != nullptr && p.splits == 1;
-        const bool res_epi = (p.epi == kEpiGatedRes || p.epi == kEpiAddRes) && p.splits == 1;
-        // bf16 output: the residual slab is fetched by coalesced loads (8 lanes per 128-byte row) and handed to the
-        // row-owning threads through the staging slab; a warp touches only its own 32 rows, so a warp sync suffices
-        const bool res_staged = res_epi && !f32;
-        if (use_bias) {
-          // the tile's bias columns once, as fp32 (the previous tile's readers passed its last slab barrier)
-          for (int c = col_begin + group_thread; c < col_end; c += 128) {
-            const int col = n_idx * BN + c;
-            bias_s[c] = col < p.N ? __bfloat162float(p.bias[col]) : 0.0f;
-          }
-        }
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * ACC_COLS;
+      if constexpr (EK != kDirect) {
+        // ---- staged epilogue: 128 bytes of 32 rows per warp and slab, swizzled ----
+        const int sw = lane & 7;
+        uint8_t* slab = staging + (warp - 2) * SLAB_BYTES;
+        uint8_t* my_row = slab + lane * 128;
+        const long long warp_row0 = row0 + quarter * 32;
+        const int rows_valid = warp_row0 < p.M ? static_cast<int>(min(32ll, p.M - warp_row0)) : 0;
+        // the lines: lane l moves 16 bytes (chunk l & 7) of the rows (l >> 3) + 4 i
+        const int line_row = lane >> 3, line_chunk = lane & 7;
+        constexpr int esz = f32 ? 4 : 2;
+        uint8_t* out_base = p.splits > 1
+            ? reinterpret_cast<uint8_t*>(p.partial) + (static_cast<long long>(split) * p.M + warp_row0) * p.N * 4
+            : reinterpret_cast<uint8_t*>(p.out) + warp_row0 * p.ldo * esz;
+        const long long out_pitch = (p.splits > 1 ? static_cast<long long>(p.N) : p.ldo) * esz;
 #pragma unroll 1
-        for (int c0 = col_begin; c0 < col_end; c0 += slab_cols) {
+        for (int c0 = egroup * slab_cols; c0 < BN; c0 += 2 * slab_cols) {
           const int col0 = n_idx * BN + c0;
-          if (col0 >= p.N) break;  // uniform across the group
-          uint8_t* slab = staging + egroup * SLAB_BYTES;
-          uint4 rv[8];
-          if (res_staged) {  // issued before the barrier: their latency overlaps the wait for the slab
+          if (col0 >= p.N || rows_valid <= 0) break;  // uniform across the warp
+          const int line_col = col0 + line_chunk * (16 / esz);
+          uint32_t r[2][32];
+          tmem_ld_x32(taddr + c0, r[0]);
+          if (!f32) tmem_ld_x32(taddr + c0 + 32, r[1]);  // bf16: two 32-column loads per slab; fp32: one
+          if constexpr (EK == kRes) {  // the residual passes through the slab
+            uint4 rv[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const int rl = quarter * 32 + i * 4 + (lane >> 3);
-              const long long grow = static_cast<long long>(m_idx) * BM + rl;
-              const int gcol = col0 + (lane & 7) * 8;
-              rv[i] = (grow < p.M && gcol < p.N) ? *reinterpret_cast<const uint4*>(p.residual + grow * p.ldr + gcol)
-                                                 : make_uint4(0u, 0u, 0u, 0u);
+              const int rl = line_row + 4 * i;
+              rv[i] = (rl < rows_valid && line_col < p.N)
+                          ? *reinterpret_cast<const uint4*>(p.residual + (warp_row0 + rl) * p.ldr + line_col)
+                          : make_uint4(0u, 0u, 0u, 0u);
             }
-          }
-          if (leader) tma_store_wait_read<0>();  // the group's previous store is done reading the slab
-          named_bar_sync(1 + egroup, 128);
-          if (res_staged) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const int rl = quarter * 32 + i * 4 + (lane >> 3);
-              *reinterpret_cast<uint4*>(slab + rl * 128 + ((((lane & 7) ^ (rl & 7))) << 4)) = rv[i];
+              const int rl = line_row + 4 * i;
+              *reinterpret_cast<uint4*>(slab + rl * 128 + ((line_chunk ^ (rl & 7)) << 4)) = rv[i];
             }
             __syncwarp();
           }
-          uint8_t* my_row = slab + row_in_tile * 128;
+          tmem_wait_ld();
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {  // bf16: two 32-column loads per slab; fp32: one
+          for (int h = 0; h < 2; ++h) {
             if (f32 && h == 1) break;
-            uint32_t r[32];
-            tmem_ld_x32(taddr + c0 + h * 32, r);
-            tmem_wait_ld();
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
               const int col = col0 + h * 32 + v * 8;
               float x[8];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(r[v * 8 + j]) * p.alpha;
-              if (p.splits == 1 && col < p.N) {
-                if (use_bias) {
-                  const float4 b0 = *reinterpret_cast<const float4*>(bias_s + c0 + h * 32 + v * 8);
-                  const float4 b1 = *reinterpret_cast<const float4*>(bias_s + c0 + h * 32 + v * 8 + 4);
-                  x[0] += b0.x; x[1] += b0.y; x[2] += b0.z; x[3] += b0.w;
-                  x[4] += b1.x; x[5] += b1.y; x[6] += b1.z; x[7] += b1.w;
-                }
+              for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(r[h][v * 8 + j]) * p.alpha;
+              if (use_bias) {  // zeros beyond N
+                const float4 b0 = *reinterpret_cast<const float4*>(bias_t + c0 + h * 32 + v * 8);
+                const float4 b1 = *reinterpret_cast<const float4*>(bias_t + c0 + h * 32 + v * 8 + 4);
+                x[0] += b0.x; x[1] += b0.y; x[2] += b0.z; x[3] += b0.w;
+                x[4] += b1.x; x[5] += b1.y; x[6] += b1.z; x[7] += b1.w;
+              }
+              if constexpr (EK == kAct) {
                 if (p.epi == kEpiGeluTanh) {
 #pragma unroll
                   for (int j = 0; j < 8; ++j) x[j] = gelu_tanh(x[j]);
-                } else if (p.epi == kEpiSilu) {
+                } else {
 #pragma unroll
                   for (int j = 0; j < 8; ++j) x[j] = x[j] / (1.0f + __expf(-x[j]));
-                } else if (res_epi && row_ok) {
-                  const uint4 rres = res_staged ? *reinterpret_cast<const uint4*>(my_row + (((h * 4 + v) ^ sw) << 4))
-                                                : *reinterpret_cast<const uint4*>(p.residual + row * p.ldr + col);
+                }
+              }
+              if constexpr (EK == kRes) {
+                if (row_ok && col < p.N) {
+                  const uint4 rres = *reinterpret_cast<const uint4*>(my_row + (((h * 4 + v) ^ sw) << 4));
                   const uint32_t rw[4] = {rres.x, rres.y, rres.z, rres.w};
                   float g[8];
                   if (p.epi == kEpiGatedRes) {
@@ -347,21 +400,23 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               }
             }
           }
-          fence_proxy_async_smem();
-          named_bar_sync(1 + egroup, 128);
-          if (leader) {
-            tma_store_2d(&tmap_c, slab, col0, static_cast<int>(out_row0));
-            tma_store_commit();
+          __syncwarp();
+          if (line_col < p.N) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int rl = line_row + 4 * i;
+              const uint4 ov = *reinterpret_cast<const uint4*>(slab + rl * 128 + ((line_chunk ^ (rl & 7)) << 4));
+              if (rl < rows_valid)
+                *reinterpret_cast<uint4*>(out_base + rl * out_pitch + static_cast<long long>(line_col) * esz) = ov;
+            }
           }
+          __syncwarp();  // the lines have been read before the next slab (or tile) overwrites them
         }
-        tc_fence_before_sync();
-        mbar_arrive(&tmem_empty[acc]);
-        continue;
-      }
+      } else {
 #pragma unroll 1
-      for (int c = egroup * (BN / 64); c < (egroup + 1) * (BN / 64); ++c) {
+      for (int c = egroup; c < BN / 32; c += 2) {
         const int col0 = n_idx * BN + c * 32;
-        if (col0 >= p.N) break;  // uniform across the group
+        if (col0 >= p.N || row0 >= p.M) break;  // uniform across the group
         uint32_t r[32];
         tmem_ld_x32(taddr + c * 32, r);
         tmem_wait_ld();
@@ -374,7 +429,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(r[v * 8 + j]) * p.alpha;
             if (p.splits > 1) {
-              float* o = p.partial + (static_cast<long long>(split) * p.partial_rows + row) * p.N + col;
+              float* o = p.partial + (static_cast<long long>(split) * p.M + row) * p.N + col;
               *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
               *reinterpret_cast<float4*>(o + 4) = make_float4(x[4], x[5], x[6], x[7]);
               continue;
@@ -431,76 +486,122 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
         }
       }
+      }
       tc_fence_before_sync();
-      mbar_arrive(&tmem_empty[acc]);
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_cluster(cluster_map(&tmem_empty[acc], 0));
+        else mbar_arrive(&tmem_empty[acc]);
+      }
     }
-    if (p.tma_store && group_thread == 0) tma_store_wait_read<0>();  // shared memory stays valid until the stores have read it
   }
 
   tc_fence_before_sync();
   __syncthreads();
+  if (CG == 2) cluster_sync();  // neither CTA leaves while the other's products or arrivals still reach into it
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if (CG == 2) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
-// out[i] = sum over splits of partial[s][i], in split order; n8 = M * N / 8 vectors of 8 values.
-__global__ void splitk_fold_kernel(const float* __restrict__ partial, void* __restrict__ out, long long ldo, int M, int N,
-                                   int splits, int out_f32, int partial_rows) {
-  const long long n8 = static_cast<long long>(M) * N / 8;
-  const long long split_stride = static_cast<long long>(partial_rows) * N;
-  const int n_vec = N / 8;
+// out = epilogue(sum over splits of partial[s], in split order); one thread per 8 columns.
+__global__ void splitk_fold_kernel(const __grid_constant__ Params p) {
+  const int n_vec = p.N / 8;
+  const long long n8 = static_cast<long long>(p.M) * n_vec;
+  const long long split_stride = static_cast<long long>(p.M) * p.N;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n8;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < splits; ++s) {
-      const float4* src = reinterpret_cast<const float4*>(partial + s * split_stride + i * 8);
+    float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int s = 0; s < p.splits; ++s) {
+      const float4* src = reinterpret_cast<const float4*>(p.partial + s * split_stride + i * 8);
       const float4 a = src[0], b = src[1];
-      acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-      acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+      x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
+      x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
     }
     const long long row = i / n_vec;
     const int col = static_cast<int>(i - row * n_vec) * 8;
-    if (out_f32) {
-      float* o = reinterpret_cast<float*>(out) + row * ldo + col;
-      *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-      *reinterpret_cast<float4*>(o + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    if (p.bias) {
+      const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
+      const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(bw[j]);
+        x[2 * j] += f.x;
+        x[2 * j + 1] += f.y;
+      }
+    }
+    if (p.epi == kEpiGeluTanh) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = gelu_tanh(x[j]);
+    } else if (p.epi == kEpiSilu) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = x[j] / (1.0f + __expf(-x[j]));
+    } else if (p.epi == kEpiGatedRes || p.epi == kEpiAddRes) {
+      const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + row * p.ldr + col);
+      const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+      const float* g = p.epi == kEpiGatedRes
+                           ? p.gate + (p.rows_per_batch > 0 ? row / p.rows_per_batch : 0) * p.gate_ld + col
+                           : nullptr;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(rw[j]);
+        x[2 * j] = f.x + (g ? g[2 * j] : 1.0f) * x[2 * j];
+        x[2 * j + 1] = f.y + (g ? g[2 * j + 1] : 1.0f) * x[2 * j + 1];
+      }
+    }
+    if (p.out_f32) {
+      float* o = reinterpret_cast<float*>(p.out) + row * p.ldo + col;
+      *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
+      *reinterpret_cast<float4*>(o + 4) = make_float4(x[4], x[5], x[6], x[7]);
     } else {
       uint4 ov;
-      ov.x = pack_bf16x2(acc[0], acc[1]);
-      ov.y = pack_bf16x2(acc[2], acc[3]);
-      ov.z = pack_bf16x2(acc[4], acc[5]);
-      ov.w = pack_bf16x2(acc[6], acc[7]);
-      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + row * ldo + col) = ov;
+      ov.x = pack_bf16x2(x[0], x[1]);
+      ov.y = pack_bf16x2(x[2], x[3]);
+      ov.z = pack_bf16x2(x[4], x[5]);
+      ov.w = pack_bf16x2(x[6], x[7]);
+      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + row * p.ldo + col) = ov;
     }
   }
 }
 
-template <bool A_MN, bool B_MN, int BN>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p, cudaStream_t stream) {
-  auto kern = gemm_kernel<A_MN, B_MN, BN>;
+template <bool A_MN, bool B_MN, int CG, int EK>
+int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, cudaStream_t stream) {
+  auto kern = gemm_kernel<A_MN, B_MN, CG, EK>;
   static bool configured = false;
   if (!configured) {
-    MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(BN)));
+    MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
     configured = true;
   }
-  const int num_work = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.splits;
-  const int grid = num_work < sm_count() ? num_work : sm_count();
-  kern<<<grid, NUM_THREADS, smem_bytes(BN), stream>>>(ta, tb, tc, p);
+  const int num_work = ((p.M + CG * BM - 1) / (CG * BM)) * ((p.N + p.bn - 1) / p.bn) * p.splits;
+  const int slots = sm_count() / CG;
+  const int grid = (num_work < slots ? num_work : slots) * CG;
+  kern<<<grid, NUM_THREADS, p.stages * stage_bytes(p.bn, CG) + FIXED_BYTES, stream>>>(ta, tb, p);
   if (p.splits > 1) {
     const long long n8 = static_cast<long long>(p.M) * p.N / 8;
-    const int blocks = static_cast<int>(n8 / 256 + 1 < sm_count() * 4 ? n8 / 256 + 1 : sm_count() * 4);
-    splitk_fold_kernel<<<blocks, 256, 0, stream>>>(p.partial, p.out, p.ldo, p.M, p.N, p.splits, p.out_f32, p.partial_rows);
+    const int blocks = static_cast<int>(n8 / 128 + 1 < sm_count() * 16 ? n8 / 128 + 1 : sm_count() * 16);
+    splitk_fold_kernel<<<blocks, 128, 0, stream>>>(p);
   }
   return static_cast<int>(cudaGetLastError());
+}
+
+template <bool A_MN, bool B_MN, int CG>
+int launch_kind(int kind, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, cudaStream_t stream) {
+  switch (kind) {
+    case kPlain: return launch<A_MN, B_MN, CG, kPlain>(ta, tb, p, stream);
+    case kAct: return launch<A_MN, B_MN, CG, kAct>(ta, tb, p, stream);
+    case kRes: return launch<A_MN, B_MN, CG, kRes>(ta, tb, p, stream);
+    case kPlainF32: return launch<A_MN, B_MN, CG, kPlainF32>(ta, tb, p, stream);
+    default: return launch<A_MN, B_MN, CG, kDirect>(ta, tb, p, stream);
+  }
 }
 
 }  // namespace gemm
 }  // namespace mdb
 
-static int g_force_tile_n = 0;
-static int g_epilogue_mode = 0;  // 0: TMA-store epilogue where the output allows it; 1: always direct stores
+static int g_epilogue_mode = 0;  // 0: staged epilogue; 1: direct stores
 
 // Tile search / benchmarks: 1 pins the direct-store epilogue (one thread per row, 16-byte stores), 0 restores the default.
 extern "C" int mdb_gemm_epilogue_mode(int mode) {
@@ -512,41 +613,26 @@ extern "C" int mdb_gemm_epilogue_mode(int mode) {
 // C entry point. A is [M,K] with leading dimension lda (a_mn_major = 0) or [K,M] (a_mn_major = 1);
 // B is [N,K] (b_mn_major = 0) or [K,N] (b_mn_major = 1). All leading dimensions are in elements and
 // must be multiples of 8; N must be a multiple of 8. Returns 0 or a CUDA / encoder error code.
-static int gemm_impl(const void* A, const void* B, void* out, const void* bias, const void* residual, const void* gate,
-                     int M, int N, int K, long long lda, long long ldb, long long ldo, long long ldr, long long gate_ld,
-                     int rows_per_batch, int a_mn_major, int b_mn_major, int epi, int out_f32, float alpha,
-                     float* partial, int splits, void* stream_ptr);
-
+//
+// The launch shape is the caller's (`ops/kernels.py: gemm_plan`): `ctas` per tile (1 or 2), tile width `bn` (64, 128, 192
+// or 256; a transposed B needs a multiple of 64 columns per CTA), and `splits` of the contraction, which run as separate
+// work items with fp32 partials (`partial`: splits * M * N values) and are summed in split order by a second kernel that
+// also applies the epilogue (for products with fewer tiles than the GPU has SMs).
 extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void* bias, const void* residual,
                              const void* gate, int M, int N, int K, long long lda, long long ldb, long long ldo,
                              long long ldr, long long gate_ld, int rows_per_batch, int a_mn_major, int b_mn_major,
-                             int epi, int out_f32, float alpha, void* stream_ptr) {
-  return gemm_impl(A, B, out, bias, residual, gate, M, N, K, lda, ldb, ldo, ldr, gate_ld, rows_per_batch, a_mn_major,
-                   b_mn_major, epi, out_f32, alpha, nullptr, 1, stream_ptr);
-}
-
-// Split-K form: out = alpha * A B^T with the contraction cut into `splits` ranges that run as separate work items
-// (for products whose output has fewer tiles than the GPU has SMs: weight gradients). `partial` is a caller-provided
-// fp32 workspace of splits * M * N values; no bias / epilogue. The sum over splits runs in split order.
-extern "C" int mdb_gemm_bf16_splitk(const void* A, const void* B, void* out, int M, int N, int K, long long lda,
-                                    long long ldb, long long ldo, int a_mn_major, int b_mn_major, int out_f32,
-                                    float alpha, void* partial, int splits, void* stream_ptr) {
-  if (splits < 1 || splits > 64 || (splits > 1 && partial == nullptr)) return 3005;
-  return gemm_impl(A, B, out, nullptr, nullptr, nullptr, M, N, K, lda, ldb, ldo, 0, 0, 0, a_mn_major, b_mn_major, 0,
-                   out_f32, alpha, static_cast<float*>(partial), splits, stream_ptr);
-}
-
-static int gemm_impl(const void* A, const void* B, void* out, const void* bias, const void* residual, const void* gate,
-                     int M, int N, int K, long long lda, long long ldb, long long ldo, long long ldr, long long gate_ld,
-                     int rows_per_batch, int a_mn_major, int b_mn_major, int epi, int out_f32, float alpha,
-                     float* partial, int splits, void* stream_ptr) {
+                             int epi, int out_f32, float alpha, int ctas, int bn, int splits, void* partial,
+                             void* stream_ptr) {
   using namespace mdb;
   using namespace mdb::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int BN = g_force_tile_n ? g_force_tile_n : 256;
   if ((N & 7) || (lda & 7) || (ldb & 7) || (ldo & 3) || (!out_f32 && (ldo & 7))) return 3001;
   if ((epi == kEpiGatedRes || epi == kEpiAddRes) && (!residual || (ldr & 7))) return 3002;
   if (epi == kEpiGatedRes && (!gate || (gate_ld & 3))) return 3003;
+  if ((ctas != 1 && ctas != 2) || (bn != 64 && bn != 128 && bn != 192 && bn != 256)) return 3004;
+  if (splits < 1 || splits > 64 || (splits > 1 && partial == nullptr)) return 3005;
+  const int bn_cta = bn / ctas;
+  if (b_mn_major && bn_cta % 64) return 3004;
   CUtensorMap ta, tb;
   int rc;
   if (a_mn_major) {
@@ -569,7 +655,7 @@ static int gemm_impl(const void* A, const void* B, void* out, const void* bias, 
   } else {
     uint64_t dims[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(N)};
     uint64_t str[1] = {static_cast<uint64_t>(ldb) * 2};
-    uint32_t box[2] = {BK, static_cast<uint32_t>(BN)};
+    uint32_t box[2] = {BK, static_cast<uint32_t>(bn_cta)};
     rc = encode_tmap_bf16(&tb, B, 2, dims, str, box);
   }
   if (rc) return rc;
@@ -585,6 +671,8 @@ static int gemm_impl(const void* A, const void* B, void* out, const void* bias, 
   p.epi = epi;
   p.out_f32 = out_f32;
   p.alpha = alpha;
+  p.bn = bn;
+  p.stages = stages_for(bn, ctas);
   p.status = status_buffer();
   {
     // every split gets at least one k-block: the count is recomputed from the rounded-up range
@@ -593,48 +681,21 @@ static int gemm_impl(const void* A, const void* B, void* out, const void* bias, 
     if (per < 1) per = 1;
     p.kb_per_split = per;
     p.splits = (num_kb + per - 1) / per;
-    p.partial = partial;
+    p.partial = static_cast<float*>(partial);
     if (p.splits <= 1) { p.splits = 1; p.kb_per_split = num_kb; }
   }
-  // Output map for the TMA-store epilogue: [N (inner), rows], 128-byte-wide boxes of 128 rows. With split-K it
-  // covers the fp32 partials, whose splits are `partial_rows` = M rounded up to the tile height apart, so that a
-  // tile's rows beyond M fall into padding instead of the next split.
-  CUtensorMap tc;
-  p.partial_rows = (M + BM - 1) / BM * BM;
-  {
-    const bool f32 = out_f32 || p.splits > 1;
-    const void* base = p.splits > 1 ? static_cast<const void*>(partial) : out;
-    const long long ld = p.splits > 1 ? N : ldo;
-    const uint64_t rows = p.splits > 1 ? static_cast<uint64_t>(p.splits) * p.partial_rows : static_cast<uint64_t>(M);
-    const int esz = f32 ? 4 : 2;
-    p.tma_store = g_epilogue_mode == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0 && ((ld * esz) & 15) == 0;
-    if (p.tma_store) {
-      uint64_t dims[2] = {static_cast<uint64_t>(N), rows};
-      uint64_t str[1] = {static_cast<uint64_t>(ld) * esz};
-      uint32_t box[2] = {static_cast<uint32_t>(128 / esz), BM};
-      rc = f32 ? encode_tmap_f32(&tc, base, 2, dims, str, box, 1) : encode_tmap_bf16(&tc, base, 2, dims, str, box);
-      if (rc) return rc;
-    } else {
-      tc = ta;  // unused by the kernel; any valid map
-      if (p.splits > 1) p.partial_rows = M;
-    }
+  const bool f32 = out_f32 || p.splits > 1;
+  const bool act = epi == kEpiGeluTanh || epi == kEpiSilu, res = epi == kEpiGatedRes || epi == kEpiAddRes;
+  int kind = kDirect;
+  if (g_epilogue_mode == 0) {
+    if (f32) kind = p.splits > 1 || epi == kEpiNone ? kPlainF32 : kDirect;
+    else kind = act ? kAct : (res ? kRes : kPlain);
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  if (BN == 256) {
-    if (a_mn_major) {
-      return b_mn_major ? launch<true, true, 256>(ta, tb, tc, p, stream) : launch<true, false, 256>(ta, tb, tc, p, stream);
-    }
-    return b_mn_major ? launch<false, true, 256>(ta, tb, tc, p, stream) : launch<false, false, 256>(ta, tb, tc, p, stream);
+  if (ctas == 2) {
+    if (a_mn_major) return b_mn_major ? launch_kind<true, true, 2>(kind, ta, tb, p, stream) : launch_kind<true, false, 2>(kind, ta, tb, p, stream);
+    return b_mn_major ? launch_kind<false, true, 2>(kind, ta, tb, p, stream) : launch_kind<false, false, 2>(kind, ta, tb, p, stream);
   }
-  if (a_mn_major) {
-    return b_mn_major ? launch<true, true, 128>(ta, tb, tc, p, stream) : launch<true, false, 128>(ta, tb, tc, p, stream);
-  }
-  return b_mn_major ? launch<false, true, 128>(ta, tb, tc, p, stream) : launch<false, false, 128>(ta, tb, tc, p, stream);
-}
-
-// 0: the default width (256); 128 or 256: use that tile width (tile search, benchmarks, tests).
-extern "C" int mdb_gemm_force_tile_n(int bn) {
-  if (bn != 0 && bn != 128 && bn != 256) return 3004;
-  g_force_tile_n = bn;
-  return 0;
+  if (a_mn_major) return b_mn_major ? launch_kind<true, true, 1>(kind, ta, tb, p, stream) : launch_kind<true, false, 1>(kind, ta, tb, p, stream);
+  return b_mn_major ? launch_kind<false, true, 1>(kind, ta, tb, p, stream) : launch_kind<false, false, 1>(kind, ta, tb, p, stream);
 }

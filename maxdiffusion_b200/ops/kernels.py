@@ -7,6 +7,7 @@ on top of these.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from typing import Sequence
 
@@ -29,33 +30,54 @@ def _rowmajor(t: torch.Tensor) -> torch.Tensor:
 _SM_COUNT = 148
 
 
-def split_k_for(M: int, N: int, K: int, sms: int = _SM_COUNT) -> int:
-  """How many ranges to cut the contraction into (1 = no split). A product whose output has fewer 128 x 256 tiles
-  than the GPU has SMs leaves SMs idle for the whole contraction (weight gradients: K is the token count); splitting
-  K makes more work items at the price of fp32 partials that a fold kernel sums. The model: waves of work items
-  times k-blocks per item (about 0.4 us per k-block), plus the write and read of every partial at HBM speed."""
-  tiles = -(-M // 128) * -(-N // 256)
+# Microseconds of one 64-deep k-block per (CTAs per tile, tile width): the larger of the operand feed into an SM (about 122
+# bytes a nanosecond) and the products. Fitted on a B200 to 33 shapes of 128 .. 65 520 rows x 4 widths x 1 / 2 CTAs.
+_KB_US = {(1, 64): 0.19, (1, 128): 0.25, (1, 192): 0.30, (1, 256): 0.39, (2, 64): 0.17, (2, 128): 0.20, (2, 192): 0.235, (2, 256): 0.27}
+
+
+@functools.lru_cache(maxsize=4096)
+def gemm_plan(M: int, N: int, K: int, b_mn: bool = False, splittable: bool = True, sms: int = _SM_COUNT, tile_n: int = 0,
+              ctas: int = 0) -> tuple:
+  """(CTAs per tile, tile width, splits of the contraction) with the least modelled time. A wave of work items takes as
+  long as its k-blocks or as the epilogue of a tile, whichever is longer; the last epilogue is exposed. Where the output has
+  fewer tiles than the GPU has SMs (few tokens; weight gradients, whose contraction is the token count), cutting the
+  contraction makes more work items at the price of fp32 partials and a second kernel (3 us + their traffic): 384 x 3072 x
+  15360 takes 51 us whole and 33 us in three parts. `tile_n` / `ctas` restrict the choice."""
+  best, best_cost = (1, 256, 1), None
   num_kb = -(-K // 64)
-  if tiles * 2 > sms or num_kb < 16:
-    return 1
-  fold_us = M * N * 8 / 5e6  # one partial written and read, in microseconds at 5 TB/s
-  best, best_cost = 1, -(-tiles // sms) * num_kb * 0.41
-  for s in range(2, 33):
-    per = -(-num_kb // s)
-    if per < 4:
-      break
-    s_eff = -(-num_kb // per)
-    cost = -(-tiles * s_eff // sms) * per * 0.41 + s_eff * fold_us + 2.0
-    if cost < best_cost * 0.9:
-      best, best_cost = s_eff, cost
+  for (cg, bn), kb_us in _KB_US.items():
+    if (ctas and cg != ctas) or (tile_n and bn != tile_n) or (b_mn and (bn // cg) % 64) or (cg == 2 and M <= 128 and not ctas):
+      continue
+    tiles = -(-M // (128 * cg)) * -(-N // bn)
+    slots = sms // cg
+    epi_us = 0.4 + 0.0065 * bn if cg == 1 else 0.8 + 0.009 * bn
+    for s in range(1, 33 if splittable and tiles * 2 <= slots and num_kb >= 16 else 2):
+      per = -(-num_kb // s)
+      if per < 4 and s > 1:
+        break
+      s_eff = -(-num_kb // per)
+      cost = -(-tiles * s_eff // slots) * max(per * kb_us, epi_us) + epi_us
+      if s_eff > 1:
+        cost = cost * 1.05 + 3.0 + s_eff * M * N * 8 / 6e6
+      if best_cost is None or cost < best_cost - 1e-9:
+        best, best_cost = (cg, bn, s_eff), cost
   return best
+
+
+def split_k_for(M: int, N: int, K: int, sms: int = _SM_COUNT) -> int:
+  """How many ranges `gemm` cuts the contraction of a plain product into (1 = no split)."""
+  return gemm_plan(M, N, K, sms=sms)[2]
+
+
+_FORCE_TILE_N = 0
+_FORCE_CTAS = 0
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, epi: str = "none",
          residual=None, gate=None, rows_per_batch: int = 0, out=None, out_dtype=torch.bfloat16, alpha: float = 1.0,
          split_k: int = 0):
   """D[M,N] = epi(alpha * A·Bᵀ + bias) on the tcgen05 GEMM. A: [M,K] (or [K,M] if a_mn); B: [N,K] (or [K,N]).
-  `split_k`: 0 = chosen by `split_k_for` for plain products (no bias / epilogue), 1 = never, n = that many ranges."""
+  `split_k`: 0 = chosen by `gemm_plan`, 1 = never, n = that many ranges (plain products: no bias / epilogue)."""
   assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
   a, b = _rowmajor(a), _rowmajor(b)
   K, M = (a.shape if a_mn else a.shape[::-1])
@@ -72,19 +94,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
   if bias is not None:
     assert bias.dtype == torch.bfloat16 and bias.is_contiguous()
   plain = bias is None and epi == "none" and residual is None and gate is None
-  splits = (split_k_for(M, N, K) if split_k == 0 else split_k) if plain else 1
-  if splits > 1:
-    partial = torch.empty((splits, -(-M // 128) * 128, N), device=a.device, dtype=torch.float32)  # splits a whole tile apart
-    rc = _lib.lib().mdb_gemm_bf16_splitk(_lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, a.stride(0), b.stride(0),
-                                         out.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32), float(alpha),
-                                         _lib.ptr(partial), splits, _lib.stream())
-    _lib.check(rc, "mdb_gemm_bf16_splitk")
-    return out
+  ctas, bn, splits = gemm_plan(M, N, K, b_mn, split_k == 0, _SM_COUNT, _FORCE_TILE_N, _FORCE_CTAS)
+  if split_k > 0:
+    splits = split_k if plain else 1
+  partial = torch.empty((splits, M, N), device=a.device, dtype=torch.float32) if splits > 1 else None
   rc = _lib.lib().mdb_gemm_bf16(
       _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(bias), _lib.ptr(residual), _lib.ptr(gate), M, N, K,
       a.stride(0), b.stride(0), out.stride(0), residual.stride(0) if residual is not None else 0,
       gate.stride(0) if gate is not None and gate.dim() == 2 else 0, rows_per_batch, int(a_mn), int(b_mn), _EPI[epi],
-      int(out.dtype == torch.float32), float(alpha), _lib.stream())
+      int(out.dtype == torch.float32), float(alpha), ctas, bn, splits, _lib.ptr(partial), _lib.stream())
   _lib.check(rc, "mdb_gemm_bf16")
   return out
 
@@ -96,8 +114,19 @@ def gemm_epilogue_mode(direct: bool = False) -> None:
 
 
 def gemm_force_tile_n(bn: int = 0) -> None:
-  """Tile width of the bf16 GEMM: 0 is the default (256), 128 / 256 pin it (tile search, benchmarks, tests)."""
-  _lib.check(_lib.lib().mdb_gemm_force_tile_n(int(bn)), "mdb_gemm_force_tile_n")
+  """Tile width of the bf16 GEMM: 0 is the rule's choice, 64 / 128 / 192 / 256 pin it (tile search, benchmarks, tests)."""
+  global _FORCE_TILE_N
+  if bn not in (0, 64, 128, 192, 256):
+    raise _lib.KernelError(f"no GEMM tile is {bn} wide")
+  _FORCE_TILE_N = int(bn)
+
+
+def gemm_force_ctas(ctas: int = 0) -> None:
+  """CTAs that share a tile of the bf16 GEMM: 0 is the rule's choice, 1 or 2 (a pair, 256 rows) pin it."""
+  global _FORCE_CTAS
+  if ctas not in (0, 1, 2):
+    raise _lib.KernelError(f"a GEMM tile is shared by 1 or 2 CTAs, not {ctas}")
+  _FORCE_CTAS = int(ctas)
 
 
 FLASH_HEAD_DIMS = (64, 128)
