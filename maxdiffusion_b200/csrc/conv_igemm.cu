@@ -16,8 +16,14 @@
 //     parity * C + channel) and the box stays dense;
 //   * nearest-2x upsample + 3x3 conv: four output-parity classes, each a 2x2 convolution of the LOW resolution
 //     input with pre-summed weights (2.25x fewer FLOPs than up-sampling first), written with stride 2.
-// Roles per CTA (persistent, one per SM): warp 0 TMA producer, warp 1 TMEM owner + MMA issuer, warps 2..5 epilogue
+// Roles per CTA (persistent): warp 0 TMA producer, warp 1 TMEM owner + MMA issuer, warps 2..5 epilogue
 // (bias, SiLU, residual add, ragged-edge masking). Accumulators are double buffered in TMEM.
+//
+// What bounds it is the operand feed from L2 (about 57 bytes per clock and SM on every shape): a 128 x 96 tile of one CTA
+// needs 28 KB per 192 tensor clocks. So two neighbouring M-tiles are computed by a PAIR of CTAs (`cta_group::2`), each
+// fetching its own box of positions and half of the weights, and draining its own 128 accumulator rows.
+// A product with too few tiles for the chip (the low-resolution stages of a UNet) is cut along the contraction into
+// `splits` work items with fp32 partials, which a second kernel sums in order and finishes (bias, SiLU, residual).
 // Channel counts that are not multiples of 64 (96, 192, 320) cost no tensor work: the last channel block is
 // fetched with zero fill and only its valid 16-wide K steps are issued.
 // The lane that issues the MMAs pays a fixed price per pipeline stage (barrier wait, fence, commit: several hundred
@@ -71,38 +77,92 @@ struct Params {
   const __nv_bfloat16* bias;      // [N] or nullptr
   const __nv_bfloat16* residual;  // addressed like out, or nullptr
   int epi;
+  int splits;                     // > 1: fp32 partials [splits][class, M-tile, 128 positions][N] instead of the output
+  float* partial;
   DeviceStatus* status;
 };
 
 struct TileCoord {
   int cls, n_idx, m1, m2, m3, m4;
+  int mt;         // M-tile within the class
+  bool in_range;  // false: the second half of a pair that covers the class's odd last M-tile
 };
 
-__device__ __forceinline__ TileCoord decode_tile(int tile, const Params& p, int nt1, int nt2, int nt3, int num_n) {
+// First (tap, channel block) unit of work item `split`: the units are cut into ranges that differ by at most one.
+__device__ __forceinline__ int unit_cut(int split, int splits, int units) {
+  return static_cast<int>(static_cast<long long>(units) * split / splits);
+}
+
+// Epilogue of 8 channels of one output position: bias, SiLU, residual, store.
+__device__ __forceinline__ void finish8(float (&x)[8], const Params& p, long long off, int col) {
+  if (p.bias) {
+    const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
+    const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float2 f = unpack_bf16x2(bw[j]);
+      x[2 * j] += f.x;
+      x[2 * j + 1] += f.y;
+    }
+  }
+  if (p.epi == kEpiSilu) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = x[j] / (1.0f + __expf(-x[j]));
+  }
+  if (p.residual) {
+    const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + off + col);
+    const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float2 f = unpack_bf16x2(rw[j]);
+      x[2 * j] += f.x;
+      x[2 * j + 1] += f.y;
+    }
+  }
+  uint4 ov;
+  ov.x = pack_bf16x2(x[0], x[1]);
+  ov.y = pack_bf16x2(x[2], x[3]);
+  ov.z = pack_bf16x2(x[4], x[5]);
+  ov.w = pack_bf16x2(x[6], x[7]);
+  *reinterpret_cast<uint4*>(p.out + off + col) = ov;
+}
+
+// M-tiles of a class, in coordinates.
+__device__ __forceinline__ void decode_m(int mt, const Params& p, int nt1, int nt2, int nt3, TileCoord& c) {
+  c.mt = mt;
+  c.m1 = (mt % nt1) * p.box1; mt /= nt1;
+  c.m2 = (mt % nt2) * p.box2; mt /= nt2;
+  c.m3 = (mt % nt3) * p.box3; mt /= nt3;
+  c.m4 = mt;  // == ext4 for the tile after the last: its boxes lie outside the tensor and are filled with zeros
+}
+
+template <int CG>
+__device__ __forceinline__ TileCoord decode_tile(int tile, int rank, const Params& p, int nt1, int nt2, int nt3, int num_mt,
+                                                 int num_n) {
   TileCoord c;
+  const int num_mp = (num_mt + CG - 1) / CG;
   c.n_idx = tile % num_n; tile /= num_n;
-  c.m1 = (tile % nt1) * p.box1; tile /= nt1;
-  c.m2 = (tile % nt2) * p.box2; tile /= nt2;
-  c.m3 = (tile % nt3) * p.box3; tile /= nt3;
-  c.m4 = tile % p.ext4; tile /= p.ext4;
-  c.cls = tile;
+  c.cls = tile / num_mp;
+  decode_m((tile - c.cls * num_mp) * CG + rank, p, nt1, nt2, nt3, c);
+  c.in_range = c.mt < num_mt;
   return c;
 }
 
-__global__ void __launch_bounds__(NUM_THREADS, 2)
+template <int CG>
+__global__ void __cluster_dims__(CG, 1, 1) __launch_bounds__(NUM_THREADS, 2)
 conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_alt,
                   const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int STAGES = p.stages;
-  const int B_BYTES = p.BN * BK * 2;
-  const int UNIT_BYTES = A_BYTES + B_BYTES;   // a multiple of 1024: BN is a multiple of 16
+  const int B_BYTES = p.BN / CG * BK * 2;     // this CTA's share of the weights
+  const int UNIT_BYTES = A_BYTES + B_BYTES;   // a multiple of 1024: BN / CG is a multiple of 8
   const int STAGE_BYTES = p.ups * UNIT_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
-  uint64_t* full_bar = bars;                          // [MAX_STAGES]
+  uint64_t* full_bar = bars;                          // [MAX_STAGES]; of a pair: only the even CTA's are used
   uint64_t* empty_bar = bars + MAX_STAGES;            // [MAX_STAGES]
   uint64_t* tmem_full = bars + 2 * MAX_STAGES;        // [2]
-  uint64_t* tmem_empty = bars + 2 * MAX_STAGES + 2;   // [2]
+  uint64_t* tmem_empty = bars + 2 * MAX_STAGES + 2;   // [2]; of a pair: only the even CTA's are used
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
@@ -112,8 +172,12 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   const int nt2 = (p.ext2 + p.box2 - 1) / p.box2;
   const int nt3 = (p.ext3 + p.box3 - 1) / p.box3;
   const int num_n = (p.N + p.BN - 1) / p.BN;
-  const int num_tiles = p.n_classes * p.ext4 * nt3 * nt2 * nt1 * num_n;
+  const int num_mt = p.ext4 * nt3 * nt2 * nt1;
+  const int num_tiles = p.n_classes * ((num_mt + CG - 1) / CG) * num_n;
+  const int num_work = num_tiles * p.splits;
   const int num_kb = (p.C + BK - 1) / BK;
+  const int rank = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int group_id = static_cast<int>(blockIdx.x) / CG, num_groups = static_cast<int>(gridDim.x) / CG;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -122,7 +186,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 128);
+      mbar_init(&tmem_empty[a], CG * 4);  // the epilogue warps (of both CTAs)
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -131,11 +195,17 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   }
   const int ACC_COLS = p.acc_cols;
   if (warp == 1) {
-    tmem_alloc(tmem_ptr_smem, 2 * ACC_COLS);
-    tmem_relinquish();
+    if (CG == 2) {
+      tmem_alloc_pair(tmem_ptr_smem, 2 * ACC_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_ptr_smem, 2 * ACC_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (CG == 2) cluster_sync();  // the partner's barriers are initialised and its TMEM is allocated
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
@@ -146,17 +216,21 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       uint32_t phase = 0;
       int issued = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TileCoord tc = decode_tile(tile, p, nt1, nt2, nt3, num_n);
-        const int n0 = tc.n_idx * p.BN;
+      for (int work = group_id; work < num_work && ok; work += num_groups) {
+        const int split = work / num_tiles;
+        const TileCoord tc = decode_tile<CG>(work - split * num_tiles, rank, p, nt1, nt2, nt3, num_mt, num_n);
+        const int n0 = tc.n_idx * p.BN + rank * (p.BN / CG);
         const int t0 = p.tap_begin[tc.cls];
-        const int n_units = (p.tap_begin[tc.cls + 1] - t0) * num_kb;
-        int ti = t0, kb = 0;
-        Tap tap = p.taps[ti];
-        for (int u0 = 0; u0 < n_units && ok; u0 += p.ups) {
+        const int all_units = (p.tap_begin[tc.cls + 1] - t0) * num_kb;
+        const int u_begin = unit_cut(split, p.splits, all_units), n_units = unit_cut(split + 1, p.splits, all_units);
+        int ti = t0 + u_begin / num_kb, kb = u_begin % num_kb;
+        Tap tap = p.taps[min(ti, MAX_TAPS - 1)];
+        for (int u0 = u_begin; u0 < n_units && ok; u0 += p.ups) {
           const int nu = min(p.ups, n_units - u0);
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 110)) { ok = false; break; }
-          mbar_expect_tx(&full_bar[stage], nu * UNIT_BYTES);
+          // both CTAs' copies complete on the even CTA's barrier, which expects the bytes of both
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], CG * nu * UNIT_BYTES);
+          const uint32_t pair_bar = CG == 2 ? cluster_map(&full_bar[stage], 0) : 0u;
           uint8_t* sa = smem + stage * STAGE_BYTES;
           for (int j = 0; j < nu; ++j, sa += UNIT_BYTES) {
             int c1 = tc.m1 + tap.o1, c2 = tc.m2 + tap.o2, c3 = tc.m3 + tap.o3, c4 = tc.m4 + tap.o4;
@@ -166,8 +240,13 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
               if (p.alt_dim == 3 && c3 < 0) { c3 += p.alt_shift; map = &tmap_alt; }
               else if (p.alt_dim == 2 && c2 < 0) { c2 += p.alt_shift; map = &tmap_alt; }
             }
-            tma_load_5d(sa, map, &full_bar[stage], tap.o0 + kb * BK, c1, c2, c3, c4);
-            tma_load_2d(sa + A_BYTES, &tmap_w, &full_bar[stage], tap.koff + kb * BK, n0);
+            if (CG == 2) {
+              tma_load_5d_pair(sa, map, pair_bar, tap.o0 + kb * BK, c1, c2, c3, c4);
+              tma_load_2d_pair(sa + A_BYTES, &tmap_w, pair_bar, tap.koff + kb * BK, n0);
+            } else {
+              tma_load_5d(sa, map, &full_bar[stage], tap.o0 + kb * BK, c1, c2, c3, c4);
+              tma_load_2d(sa + A_BYTES, &tmap_w, &full_bar[stage], tap.koff + kb * BK, n0);
+            }
             if (++kb == num_kb) {
               kb = 0;
               ++ti;
@@ -179,25 +258,28 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         }
       }
       if (!ok) {
-        // Give the copies already in flight a bounded chance to land before the CTA exits.
+        // Give the copies already in flight a bounded chance to land before the CTA exits. The odd CTA of a pair has no
+        // barrier of its own to look at: it gives its copies a fixed time.
         const int pending = issued < STAGES ? issued : STAGES;
-        for (int i = 0; i < pending; ++i) {
+        for (int i = 0; i < pending && rank == 0; ++i) {
           int s = (stage - 1 - i + 2 * STAGES) % STAGES;
           uint32_t ph = (i < stage) ? phase : (phase ^ 1u);
           for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(&full_bar[s], ph); ++spin) {}
         }
+        for (int i = 0; i < 100 && CG == 2; ++i) __nanosleep(10000);
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer --------------------------------
-    if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(BM, p.BN, false, false);
+    // ------------------------------ MMA issuer (of a pair: in the even CTA) ----
+    if (rank == 0 && elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(CG * BM, p.BN, false, false);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
-        const int cls = tile / (num_tiles / p.n_classes);
+      for (int work = group_id; work < num_work && ok; work += num_groups, ++it) {
+        const int split = work / num_tiles;
+        const int cls = (work - split * num_tiles) / (num_tiles / p.n_classes);
         const int n_taps = p.tap_begin[cls + 1] - p.tap_begin[cls];
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1u;
@@ -205,11 +287,11 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
         uint32_t accumulate = 0;
-        const int n_units = n_taps * num_kb;
+        const int u_begin = unit_cut(split, p.splits, n_taps * num_kb), n_units = unit_cut(split + 1, p.splits, n_taps * num_kb);
         // this lane is the critical resource of the kernel: no divisions, descriptors advance by addition
         const int last_ksteps = (p.C - (num_kb - 1) * BK + 15) / 16;
-        int kb = 0;
-        for (int u0 = 0; u0 < n_units; u0 += p.ups) {
+        int kb = u_begin % num_kb;
+        for (int u0 = u_begin; u0 < n_units; u0 += p.ups) {
           const int nu = min(p.ups, n_units - u0);
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, 121)) { ok = false; break; }
           tc_fence_after_sync();
@@ -218,8 +300,17 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             const uint64_t da = make_smem_desc(sa, 16, 1024);
             const uint64_t db = make_smem_desc(sa + A_BYTES, 16, 1024);
             const bool last = (kb + 1 == num_kb);
-            if (!last || last_ksteps == BK / 16) {
-              // one K step (16 bf16 = 32 bytes) advances the descriptors' address field (units of 16 bytes) by 2
+            // one K step (16 bf16 = 32 bytes) advances the descriptors' address field (units of 16 bytes) by 2
+            if (CG == 2) {
+              if (!last || last_ksteps == BK / 16) {
+                umma_ss_pair(d_tmem, da, db, idesc, accumulate);
+                umma_ss_pair(d_tmem, da + 2, db + 2, idesc, 1u);
+                umma_ss_pair(d_tmem, da + 4, db + 4, idesc, 1u);
+                umma_ss_pair(d_tmem, da + 6, db + 6, idesc, 1u);
+              } else {
+                for (int k = 0; k < last_ksteps; ++k) umma_ss_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, k ? 1u : accumulate);
+              }
+            } else if (!last || last_ksteps == BK / 16) {
               umma_ss(d_tmem, da, db, idesc, accumulate);
               umma_ss(d_tmem, da + 2, db + 2, idesc, 1u);
               umma_ss(d_tmem, da + 4, db + 4, idesc, 1u);
@@ -230,10 +321,14 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             accumulate = 1u;
             kb = last ? 0 : kb + 1;
           }
-          umma_commit(&empty_bar[stage]);
+          if (CG == 2) umma_commit_pair(&empty_bar[stage]);
+          else umma_commit(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit(&tmem_full[acc]);
+        if (ok) {
+          if (CG == 2) umma_commit_pair(&tmem_full[acc]);
+          else umma_commit(&tmem_full[acc]);
+        }
       }
     }
   } else {
@@ -245,14 +340,15 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const int r3 = r / (p.box1 * p.box2);
     int it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
-      const TileCoord tc = decode_tile(tile, p, nt1, nt2, nt3, num_n);
+    for (int work = group_id; work < num_work && ok; work += num_groups, ++it) {
+      const int split = work / num_tiles;
+      const TileCoord tc = decode_tile<CG>(work - split * num_tiles, rank, p, nt1, nt2, nt3, num_mt, num_n);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
       if (!mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status, 130)) { ok = false; break; }
       tc_fence_after_sync();
       const int p1 = tc.m1 + r1, p2 = tc.m2 + r2, p3 = tc.m3 + r3;
-      const bool row_ok = p1 < p.ext1 && p2 < p.ext2 && p3 < p.ext3;
+      const bool row_ok = tc.in_range && p1 < p.ext1 && p2 < p.ext2 && p3 < p.ext3;
       const long long off = tc.m4 * p.os4 + p3 * p.os3 + p2 * p.os2 + p1 * p.os1 + p.class_off[tc.cls];
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * ACC_COLS;
       const int n0 = tc.n_idx * p.BN;
@@ -271,58 +367,71 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             float x[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[h * 8 + j]);
-            if (p.bias) {
-              const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
-              const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float2 f = unpack_bf16x2(bw[j]);
-                x[2 * j] += f.x;
-                x[2 * j + 1] += f.y;
-              }
+            if (p.splits > 1) {
+              float* o = p.partial +
+                         ((static_cast<long long>(split) * p.n_classes + tc.cls) * num_mt + tc.mt) * BM * p.N +
+                         static_cast<long long>(r) * p.N + col;
+              *reinterpret_cast<float4*>(o) = make_float4(x[0], x[1], x[2], x[3]);
+              *reinterpret_cast<float4*>(o + 4) = make_float4(x[4], x[5], x[6], x[7]);
+            } else {
+              finish8(x, p, off, col);
             }
-            if (p.epi == kEpiSilu) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) x[j] = x[j] / (1.0f + __expf(-x[j]));
-            }
-            if (p.residual) {
-              const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + off + col);
-              const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float2 f = unpack_bf16x2(rw[j]);
-                x[2 * j] += f.x;
-                x[2 * j + 1] += f.y;
-              }
-            }
-            uint4 ov;
-            ov.x = pack_bf16x2(x[0], x[1]);
-            ov.y = pack_bf16x2(x[2], x[3]);
-            ov.z = pack_bf16x2(x[4], x[5]);
-            ov.w = pack_bf16x2(x[6], x[7]);
-            *reinterpret_cast<uint4*>(p.out + off + col) = ov;
           }
         }
       }
       tc_fence_before_sync();
-      mbar_arrive(&tmem_empty[acc]);
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_cluster(cluster_map(&tmem_empty[acc], 0));
+        else mbar_arrive(&tmem_empty[acc]);
+      }
     }
   }
 
   tc_fence_before_sync();
   __syncthreads();
+  if (CG == 2) cluster_sync();  // neither CTA leaves while the other's products or arrivals still reach into it
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 2 * ACC_COLS);
+    if (CG == 2) tmem_dealloc_pair(tmem_base, 2 * ACC_COLS);
+    else tmem_dealloc(tmem_base, 2 * ACC_COLS);
   }
 }
 
-// Tile width for N output channels: the multiple of 16 (<= 256) that wastes the fewest padded columns, the widest
-// among equals (a wider tile moves fewer operand bytes per FLOP).
-static int pick_bn(int N) {
-  int best = 16;
+// Sum of the partials of a split contraction, in split order, and the epilogue. One thread per 8 channels of a position.
+__global__ void conv_fold_kernel(const __grid_constant__ Params p) {
+  const int nt1 = (p.ext1 + p.box1 - 1) / p.box1, nt2 = (p.ext2 + p.box2 - 1) / p.box2, nt3 = (p.ext3 + p.box3 - 1) / p.box3;
+  const int num_mt = p.ext4 * nt3 * nt2 * nt1;
+  const int n_vec = p.N / 8;
+  const long long rows = static_cast<long long>(p.n_classes) * num_mt * BM;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < rows * n_vec;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long row = i / n_vec;
+    const int col = static_cast<int>(i - row * n_vec) * 8;
+    const int r = static_cast<int>(row % BM);
+    TileCoord tc;
+    tc.cls = static_cast<int>(row / BM / num_mt);
+    decode_m(static_cast<int>(row / BM % num_mt), p, nt1, nt2, nt3, tc);
+    const int p1 = tc.m1 + r % p.box1, p2 = tc.m2 + (r / p.box1) % p.box2, p3 = tc.m3 + r / (p.box1 * p.box2);
+    if (p1 >= p.ext1 || p2 >= p.ext2 || p3 >= p.ext3) continue;
+    float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int s = 0; s < p.splits; ++s) {
+      const float4* src = reinterpret_cast<const float4*>(p.partial + (s * rows + row) * p.N + col);
+      const float4 a = src[0], b = src[1];
+      x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
+      x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
+    }
+    finish8(x, p, tc.m4 * p.os4 + p3 * p.os3 + p2 * p.os2 + p1 * p.os1 + p.class_off[tc.cls], col);
+  }
+}
+
+// Tile width for N output channels: the multiple of `step` (16; 32 for a pair) up to `most` that wastes the fewest padded
+// columns, the widest among equals (a wider tile moves fewer operand bytes per FLOP).
+static int pick_bn(int N, int most, int step) {
+  int best = step;
   long long best_cost = -1;
-  for (int bn = 16; bn <= 256; bn += 16) {
+  for (int bn = step; bn <= most; bn += step) {
     const long long cost = static_cast<long long>((N + bn - 1) / bn) * bn;
     if (best_cost < 0 || cost < best_cost || (cost == best_cost && bn > best)) {
       best = bn;
@@ -354,13 +463,15 @@ extern "C" int mdb_conv_igemm_tune(int ups, int stages, int ctas_per_sm) {
 //   box       : tile extents along dims 1..3 (product 128);  ext: output positions along dims 1..4
 //   taps      : n_taps_total x 6 ints (o0, o1, o2, o3, o4, koff);  tap_begin: n_classes + 1 ints
 //   out_strides (dims 1..4, elements), class_off (n_classes): where output position (p1..p4) of a class goes
+//   ctas_per_tile (1 / 2), max_bn (widest tile), splits: the launch shape (`ops/conv.py: conv_plan`); with splits > 1
+//   `partial` holds splits * n_classes * M-tiles * 128 * N fp32 values
 // All channel counts and strides must keep 16-byte alignment (multiples of 8 elements); C a multiple of 16.
 extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, void* out, const void* bias,
                               const void* residual, const long long* dims, const long long* strides,
                               const long long* alt_dims, const long long* alt_strides, const int* box, const int* ext,
                               int C, int N, long long k_total, int n_classes, const int* tap_begin, const int* taps,
                               int alt_dim, int alt_shift, const long long* out_strides, const long long* class_off,
-                              int epi, void* stream_ptr) {
+                              int epi, int ctas_per_tile, int max_bn, int splits, void* partial, void* stream_ptr) {
   using namespace mdb;
   using namespace mdb::conv;
   if (n_classes < 1 || n_classes > MAX_CLASSES) return 3601;
@@ -395,8 +506,15 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
   p.box1 = box[0]; p.box2 = box[1]; p.box3 = box[2];
   p.ext1 = ext[0]; p.ext2 = ext[1]; p.ext3 = ext[2]; p.ext4 = ext[3];
   p.C = C; p.N = N;
-  p.BN = pick_bn(N);
-  const int unit_bytes = A_BYTES + p.BN * BK * 2;
+  const int cg = ctas_per_tile == 2 ? 2 : 1;
+  if (max_bn < 16 * cg || max_bn > 256 || splits < 1 || (splits > 1 && partial == nullptr)) return 3608;
+  p.BN = pick_bn(N, max_bn, 16 * cg);
+  p.splits = splits;
+  p.partial = static_cast<float*>(partial);
+  for (int c = 0; c < n_classes; ++c) {
+    if (splits > (tap_begin[c + 1] - tap_begin[c]) * ((C + BK - 1) / BK)) return 3608;  // every split has a unit
+  }
+  const int unit_bytes = A_BYTES + p.BN / cg * BK * 2;
   int ctas_per_sm = p.BN <= 128 ? 2 : 1;
   if (g_tune_ctas > 0) ctas_per_sm = (g_tune_ctas == 2 && p.BN <= 128) ? 2 : 1;
   p.acc_cols = ctas_per_sm == 2 ? 128 : 256;
@@ -434,7 +552,7 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
     }
     uint64_t wd[2] = {static_cast<uint64_t>(k_total), static_cast<uint64_t>(N)};
     uint64_t ws[1] = {static_cast<uint64_t>(k_total) * 2};
-    uint32_t wb[2] = {BK, static_cast<uint32_t>(p.BN)};
+    uint32_t wb[2] = {BK, static_cast<uint32_t>(p.BN / cg)};
     rc = encode_tmap_bf16(&tw, w, 2, wd, ws, wb);
     if (rc) return rc;
   }
@@ -444,15 +562,22 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
   if (ctas_per_sm == 2 && smem < 80 * 1024) smem = 80 * 1024;
   static bool configured = false;
   if (!configured) {
-    MDB_CHECK_CUDA(cudaFuncSetAttribute(conv_igemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    MDB_CHECK_CUDA(cudaFuncSetAttribute(conv_igemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    MDB_CHECK_CUDA(cudaFuncSetAttribute(conv_igemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured = true;
   }
   const auto cdiv = [](long long a, long long b) { return (a + b - 1) / b; };
-  const long long tiles = static_cast<long long>(n_classes) * ext[3] * cdiv(ext[2], box[2]) * cdiv(ext[1], box[1]) *
-                          cdiv(ext[0], box[0]) * cdiv(N, p.BN);
-  if (tiles >= (1ll << 31)) return 3607;
-  const long long slots = static_cast<long long>(sm_count()) * ctas_per_sm;
-  const int grid = tiles < slots ? static_cast<int>(tiles) : static_cast<int>(slots);
-  conv_igemm_kernel<<<grid, NUM_THREADS, smem, static_cast<cudaStream_t>(stream_ptr)>>>(tx, talt, tw, p);
+  const long long m_tiles = static_cast<long long>(ext[3]) * cdiv(ext[2], box[2]) * cdiv(ext[1], box[1]) * cdiv(ext[0], box[0]);
+  const long long work = static_cast<long long>(n_classes) * cdiv(m_tiles, cg) * cdiv(N, p.BN) * splits;
+  if (work >= (1ll << 30)) return 3607;
+  const long long slots = static_cast<long long>(sm_count()) * ctas_per_sm / cg;
+  const int grid = static_cast<int>(work < slots ? work : slots) * cg;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  if (cg == 2) conv_igemm_kernel<2><<<grid, NUM_THREADS, smem, stream>>>(tx, talt, tw, p);
+  else conv_igemm_kernel<1><<<grid, NUM_THREADS, smem, stream>>>(tx, talt, tw, p);
+  if (splits > 1) {
+    const long long vecs = n_classes * m_tiles * BM * (N / 8);
+    conv_fold_kernel<<<static_cast<int>(cdiv(vecs, 128)), 128, 0, stream>>>(p);
+  }
   return static_cast<int>(cudaGetLastError());
 }

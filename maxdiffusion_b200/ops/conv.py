@@ -19,6 +19,7 @@ CPU tensors and fp32 run the PyTorch reference (`F.conv3d` / `F.conv2d`), which 
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -32,7 +33,7 @@ def _declare(L):
   c_void_p, c_int, c_ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
   llp, ip = ctypes.POINTER(c_ll), ctypes.POINTER(c_int)
   L.mdb_conv_igemm.argtypes = [c_void_p] * 6 + [llp] * 4 + [ip, ip, c_int, c_int, c_ll, c_int, ip, ip, c_int, c_int,
-                                                           llp, llp, c_int, c_void_p]
+                                                           llp, llp, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
   L.mdb_conv_igemm.restype = c_int
   L.mdb_rms_act_cl.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int, ctypes.c_float, c_int,
                                c_int, c_int, c_void_p]
@@ -221,16 +222,72 @@ def _pick_box(e1: int, e2: int, e3: int, allow3: bool):
   return best
 
 
+_PLAN = None  # a launch shape (CTAs per tile, widest tile, splits) instead of `conv_plan`'s: benchmarks, tests
+
+
+def _tile_width(n: int, most: int, step: int) -> int:
+  """The kernel's choice (`pick_bn`): the multiple of `step` that wastes the fewest columns, the widest among equals."""
+  return min(range(step, most + 1, step), key=lambda bn: (-(-n // bn) * bn, -bn))
+
+
+@functools.lru_cache(maxsize=4096)
+def conv_plan(m_tiles: int, n_classes: int, n: int, units: int, sms: int = 148) -> tuple:
+  """(CTAs per tile, widest tile, splits) with the least modelled time of an implicit-GEMM convolution: `m_tiles` boxes of
+  128 positions per class, `n` output channels, `units` (tap, 64-channel block) steps per tile.
+
+  A step costs its operand feed: 16 KB of positions and 128 bytes per output channel, the latter shared by a pair. Measured
+  on a B200, one CTA against a pair: 96 -> 96 channels at 4 x 480 x 832 1021 / 918 us, 384 -> 384 at 2 x 120 x 208 338 / 277
+  us; tiles of fewer than 24 steps gain less than the pair's hand-over costs (up-sampling 192 -> 96: 315 / 359 us). Few
+  tiles leave SMs idle: cutting the contraction pays for its fp32 partials (2 x 8 x 8 x 1280 -> 1280: 61 us whole, 18 us in
+  12 parts; 2 x 16 x 16 x 2560 -> 1280: 135 / 38 us in 6)."""
+  best, best_cost = (1, 256, 1), None
+  for cg in (1, 2):
+    if cg == 2 and (m_tiles < 2 or units < 24):
+      continue
+    seen = set()
+    for most in (256, 128, 64):
+      bn = _tile_width(n, most, 16 * cg)
+      if bn in seen:
+        continue
+      seen.add(bn)
+      one = (0.23 + 0.00055 * bn) if cg == 1 else (0.19 + 0.00058 * bn)  # microseconds per step, one CTA on the SM
+      two = (0.26 + 0.002 * bn) if cg == 1 else (0.30 + 0.001 * bn)      # of each of two CTAs that share the SM
+      tiles = n_classes * -(-m_tiles // cg) * -(-n // bn)
+      slots = sms // cg
+      for s in range(1, 25 if tiles * 2 <= slots * 2 else 2):
+        if s > 1 and units // s < 8:
+          break
+        items, per = tiles * s, -(-units // s)
+        if bn <= 128:
+          rounds, rest = divmod(items, 2 * slots)
+          cost = per * (rounds * two + (0 if rest == 0 else one if rest <= slots else two))
+        else:
+          cost = per * -(-items // slots) * one
+        cost += 5.0
+        if s > 1:
+          cost = cost * 1.03 + 4.0 + s * n_classes * m_tiles * 128 * n * 8 / 4e6
+        if best_cost is None or cost < best_cost - 1e-9:
+          best, best_cost = (cg, most, s), cost
+  return best
+
+
 def _launch(x, x_alt, pk: PackedConv, dims, strides, alt_dims, alt_strides, box, ext, out, out_strides, class_off,
             residual, silu, alt_dim=-1, alt_shift=0, tap_shift1=0):
   taps, begin, n_classes = pk.tap_arrays(tap_shift1)
   LL, I = ctypes.c_longlong, ctypes.c_int
   arr = lambda T, v: (T * len(v))(*[int(i) for i in v])
+  m_tiles = ext[3]
+  for e, b in zip(ext[:3], box):
+    m_tiles *= -(-e // b)
+  ctas, max_bn, splits = _PLAN or conv_plan(m_tiles, n_classes, pk.n_pad, -(-pk.c_in // 64) * min(len(c) for c in pk.taps))
+  partial = None
+  if splits > 1:
+    partial = torch.empty(splits * n_classes * m_tiles * 128 * pk.n_pad, device=out.device, dtype=torch.float32)
   rc = _lib.lib().mdb_conv_igemm(
       _lib.ptr(x), _lib.ptr(x_alt), _lib.ptr(pk.w), _lib.ptr(out), _lib.ptr(pk.bias), _lib.ptr(residual),
       arr(LL, dims), arr(LL, strides), arr(LL, alt_dims if alt_dims else dims), arr(LL, alt_strides if alt_strides else strides),
       arr(I, box), arr(I, ext), pk.c_in, pk.n_pad, pk.w.shape[1], n_classes, begin, taps, alt_dim, alt_shift,
-      arr(LL, out_strides), arr(LL, class_off), 1 if silu else 0, _lib.stream())
+      arr(LL, out_strides), arr(LL, class_off), 1 if silu else 0, ctas, max_bn, splits, _lib.ptr(partial), _lib.stream())
   _lib.check(rc, "mdb_conv_igemm")
   return out
 
