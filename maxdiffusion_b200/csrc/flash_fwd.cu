@@ -228,6 +228,32 @@ __device__ __forceinline__ void copy_cta(const CopyPlan& cp, int ci, DeviceStatu
   }
 }
 
+// exp2(s * scale - m) of 64 scores of a row, packed as bf16; returns the fp32 sums over even and odd keys. A ragged
+// tail (FULL = false) is a function of its own: the tests on every score would cost the common case as much as the rest.
+template <bool FULL>
+__device__ __forceinline__ uint64_t exp_half(const uint32_t (&s)[2][32], uint32_t (&pk)[32], float scale, float m, int valid) {
+  const uint64_t scale2 = pack_f32x2(scale, scale), neg_m2 = pack_f32x2(-m, -m);
+  uint64_t rs = 0;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float p0, p1;
+      unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][2 * i]), __uint_as_float(s[c][2 * i + 1])), scale2, neg_m2), p0, p1);
+      p0 = fast_exp2(p0);
+      p1 = fast_exp2(p1);
+      if (!FULL) {
+        const int col = c * 32 + 2 * i;
+        if (col >= valid) p0 = 0.0f;
+        if (col + 1 >= valid) p1 = 0.0f;
+      }
+      rs = add_f32x2(rs, pack_f32x2(p0, p1));
+      pk[c * 16 + i] = pack_bf16x2(p0, p1);
+    }
+  }
+  return rs;
+}
+
 template <int HD, int KV_STAGES>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ KVMaps maps, const Params p,
@@ -471,9 +497,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             float mx0 = -INFINITY, mx1 = -INFINITY;  // two chains
             if (valid == BKV) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                mx0 = fmaxf(mx0, __uint_as_float(sv2[0][i]));
-                mx1 = fmaxf(mx1, __uint_as_float(sv2[1][i]));
+              for (int i = 0; i < 32; i += 2) {
+                mx0 = max3(mx0, __uint_as_float(sv2[0][i]), __uint_as_float(sv2[0][i + 1]));
+                mx1 = max3(mx1, __uint_as_float(sv2[1][i]), __uint_as_float(sv2[1][i + 1]));
               }
             } else {
 #pragma unroll
@@ -509,24 +535,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
           }
           // probabilities, written over S as packed bf16 (32 columns)
-          float rs0 = 0.0f, rs1 = 0.0f;
           uint32_t pk[32];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              float p0 = fast_exp2(__uint_as_float(sv2[c][2 * i]) * p.scale_log2 - m);
-              float p1 = fast_exp2(__uint_as_float(sv2[c][2 * i + 1]) * p.scale_log2 - m);
-              if (valid != BKV) {
-                const int col = c * 32 + 2 * i;
-                if (col >= valid) p0 = 0.0f;
-                if (col + 1 >= valid) p1 = 0.0f;
-              }
-              rs0 += p0;
-              rs1 += p1;
-              pk[c * 16 + i] = pack_bf16x2(p0, p1);
-            }
-          }
+          const uint64_t rs = valid == BKV ? exp_half<true>(sv2, pk, p.scale_log2, m, valid)
+                                           : exp_half<false>(sv2, pk, p.scale_log2, m, valid);
+          float rs0, rs1;
+          unpack_f32x2(rs, rs0, rs1);
           tmem_st_x32(s_addr, pk);
           l += rs0 + rs1;
           tmem_wait_st();
