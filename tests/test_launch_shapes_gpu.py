@@ -1,0 +1,100 @@
+"""Launch shapes of the tensor-core kernels at the edges of their tiles: GEMM tiles of one CTA or a pair, cut contractions
+with an epilogue in the fold, convolutions by pairs and in parts. Oracle: float64 PyTorch.
+
+Tolerances: fp32 accumulation of bf16 products and one rounding to bf16 (2^-9 relative to a value) give 1.7e-3 in the
+2-norm; 4e-3 leaves room for a second rounding (the residual)."""
+import pytest
+import torch
+
+from maxdiffusion_b200.ops import conv as C
+from maxdiffusion_b200.ops import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def _randn(*shape, scale=1.0):
+  return (torch.randn(shape, device="cuda") * scale).to(torch.bfloat16)
+
+
+def _rel(got, want):
+  return ((got.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("ctas,bn", [(1, 64), (1, 192), (1, 256), (2, 64), (2, 128), (2, 192), (2, 256)])
+@pytest.mark.parametrize("M,N,Kd", [(8, 8, 8), (128, 64, 64), (129, 200, 136), (257, 264, 72), (640, 520, 1032)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_gemm_tiles(ctas, bn, M, N, Kd, a_mn, b_mn):
+  if b_mn and (bn // ctas) % 64:
+    pytest.skip("a transposed B needs a multiple of 64 columns per CTA")
+  torch.manual_seed(0)
+  M -= M % 8 if a_mn else 0
+  a, b, bias = _randn(*((Kd, M) if a_mn else (M, Kd))), _randn(*((Kd, N) if b_mn else (N, Kd))), _randn(N)
+  want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t()) + bias.double()
+  guard = torch.full((M + 2, N), 7.0, device="cuda", dtype=torch.bfloat16)
+  K.gemm_force_ctas(ctas)
+  K.gemm_force_tile_n(bn)
+  try:
+    assert K.gemm_plan(M, N, Kd, b_mn, True, 148, bn, ctas)[:2] == (ctas, bn)
+    K.gemm(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, out=guard[1:-1])
+  finally:
+    K.gemm_force_ctas(0)
+    K.gemm_force_tile_n(0)
+  assert _rel(guard[1:-1], want) < 4e-3
+  assert bool((guard[0] == 7).all()) and bool((guard[-1] == 7).all())
+
+
+@pytest.mark.parametrize("epi", ["none", "gelu_tanh", "silu", "add_res", "gated_res"])
+@pytest.mark.parametrize("M,N,Kd", [(136, 328, 4104), (384, 512, 8192)])
+def test_gemm_cut_contraction_with_epilogue(epi, M, N, Kd):
+  """Few tiles and a long contraction: the fold kernel applies the epilogue."""
+  torch.manual_seed(1)
+  a, b, bias, res = _randn(M, Kd), _randn(N, Kd, scale=0.05), _randn(N), _randn(M, N)
+  rows = M // 2
+  gate = torch.randn((2, N), device="cuda")
+  assert K.gemm_plan(M, N, Kd)[2] > 1
+  got = K.gemm(a, b, bias=bias, epi=epi, residual=res if "res" in epi else None, gate=gate if epi == "gated_res" else None,
+               rows_per_batch=rows if epi == "gated_res" else 0)
+  want = a.double() @ b.double().t() + bias.double()
+  if epi == "gelu_tanh":
+    want = torch.nn.functional.gelu(want, approximate="tanh")
+  elif epi == "silu":
+    want = torch.nn.functional.silu(want)
+  elif epi == "add_res":
+    want = want + res.double()
+  elif epi == "gated_res":
+    want = res.double() + gate.double().repeat_interleave(rows, 0) * want
+  assert _rel(got, want) < 4e-3
+
+
+@pytest.mark.parametrize("plan", [(1, 64, 3), (2, 256, 1), (2, 64, 2), (1, 256, 7), (2, 32, 1)])
+@pytest.mark.parametrize("B,H,W,Ci,Co", [(1, 8, 16, 64, 64), (2, 17, 23, 64, 328), (1, 33, 40, 96, 96), (3, 9, 70, 192, 24)])
+def test_conv_launch_shapes(plan, B, H, W, Ci, Co):
+  """An odd number of M-tiles (the pair's second half lies outside), ragged edges, parts of the contraction."""
+  torch.manual_seed(2)
+  x, w, b, res = _randn(B, H, W, Ci), _randn(Co, Ci, 3, 3, scale=0.05), _randn(Co), _randn(B, H, W, Co)
+  nchw = x.permute(0, 3, 1, 2).double()
+  want = torch.nn.functional.conv2d(nchw, w.double(), b.double(), padding=1).permute(0, 2, 3, 1)
+  up = torch.nn.functional.conv2d(torch.nn.functional.interpolate(nchw, scale_factor=2, mode="nearest"), w.double(), b.double(),
+                                  padding=1).permute(0, 2, 3, 1)
+  pk, pu = C.pack_conv2d(w, b), C.pack_upsample_conv2d(w, b)
+  C._PLAN = plan
+  try:
+    got, fused = C.conv2d(x, pk), C.conv2d(x, pk, residual=res, silu=True)
+    got_up = C.upsample2x_conv2d(x, pu) if plan[2] <= 4 * (-(-Ci // 64)) else None
+  finally:
+    C._PLAN = None
+  assert _rel(got, want) < 4e-3
+  assert _rel(fused, torch.nn.functional.silu(want) + res.double()) < 4e-3
+  if got_up is not None:
+    assert _rel(got_up, up) < 6e-3  # the parity weights are sums, rounded to bf16 once more
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Sk", [(1, 1), (127, 63), (129, 65), (300, 128), (257, 191)])
+def test_attention_ragged_tails(D, Sq, Sk):
+  torch.manual_seed(3)
+  q, k, v = _randn(2, Sq, 3, D), _randn(2, Sk, 3, D), _randn(2, Sk, 3, D)
+  out, lse = K.flash_fwd(q, [k], [v])
+  s = torch.einsum("bshd,bthd->bhst", q.double(), k.double()) / D ** 0.5
+  assert _rel(out, torch.einsum("bhst,bthd->bshd", s.softmax(-1), v.double())) < 5e-3  # P is rounded to bf16 too
+  assert (lse.double() * 0.6931471805599453 - s.logsumexp(-1)).abs().max() < 1e-4
