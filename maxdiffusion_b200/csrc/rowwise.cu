@@ -372,7 +372,7 @@ ln_rows_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                    const __nv_bfloat16* __restrict__ gamma, int rows_per_batch, int C, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ partial) {
-  extern __shared__ float fold[];  // [2][C]: the CTA's column sums, added warp by warp in warp order
+  extern __shared__ float fold[];  // [warps][2][C]: every warp's column sums
   const Strip s = my_strip(rows_per_batch);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = C >> 3;
   const float inv_c = 1.0f / C;
@@ -435,25 +435,25 @@ ln_rows_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
     }
   }
   if (partial) {
-    for (int w = 0; w < THREADS / 32; ++w) {
-      if (warp == w) {
+    // all warps store at once and every thread adds a few columns over the warps, in warp order. (Adding warp by warp into
+    // one row serialised eight bank-conflicting passes of a CTA that holds only a few rows per warp.)
+    float* mine = fold + static_cast<size_t>(warp) * 2 * C;
 #pragma unroll
-        for (int k = 0; k < VPL; ++k) {
-          const int vi = lane + k * 32;
-          if (vi < nvec) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int c = vi * 8 + j;
-              fold[c] = (w == 0 ? 0.0f : fold[c]) + acc0[k][j];
-              fold[C + c] = (w == 0 ? 0.0f : fold[C + c]) + acc1[k][j];
-            }
-          }
-        }
+    for (int k = 0; k < VPL; ++k) {
+      const int vi = lane + k * 32;
+      if (vi < nvec) {
+        storef8(mine + vi * 8, acc0[k]);
+        storef8(mine + C + vi * 8, acc1[k]);
       }
-      __syncthreads();
     }
+    __syncthreads();
     const long long cta = static_cast<long long>(blockIdx.y) * gridDim.x + blockIdx.x;
-    for (int i = threadIdx.x; i < 2 * C; i += THREADS) partial[cta * 2 * C + i] = fold[i];
+    for (int i = threadIdx.x; i < 2 * C; i += THREADS) {
+      float t = fold[i];
+#pragma unroll
+      for (int w = 1; w < THREADS / 32; ++w) t += fold[static_cast<size_t>(w) * 2 * C + i];
+      partial[cta * 2 * C + i] = t;
+    }
   }
 }
 
@@ -727,24 +727,36 @@ gated_res_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16
 }
 
 // Column sums of a bf16 matrix (bias gradient): partial[cta][0][c] = sum_rows x
+// grid = (tiles of 256 columns, row chunks): the eight warps of a CTA take the chunk's rows in turn, 16 bytes per lane, and
+// add up through shared memory; partial[chunk][C]. (One CTA per chunk over all columns left most threads without a column
+// at C <= 1280 and wrote four times as many partials.)
 __global__ void __launch_bounds__(THREADS)
-colsum_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int rows_per_batch, int C,
-              float* __restrict__ partial) {
-  const Strip s = my_strip(rows_per_batch);
-  const int nvec = C >> 3;
-  const long long cta = static_cast<long long>(blockIdx.y) * gridDim.x + blockIdx.x;
-  for (int vi = threadIdx.x; vi < nvec; vi += THREADS) {
-    float acc[8];
+colsum_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int rows, int C, float* __restrict__ partial) {
+  __shared__ float red[THREADS / 32][256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = (rows + gridDim.y - 1) / gridDim.y;
+  const int begin = min(rows, static_cast<int>(blockIdx.y) * per), end = min(rows, begin + per);
+  const int col = blockIdx.x * 256 + lane * 8;
+  float acc[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+  for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+  if (col < C) {
 #pragma unroll 4
-    for (long long row = s.begin; row < s.end; ++row) {
+    for (int row = begin + warp; row < end; row += THREADS / 32) {
       float v[8];
-      load8(x + row * ldx + vi * 8, v);
+      load8(x + row * ldx + col, v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += v[j];
     }
-    storef8(partial + cta * C + vi * 8, acc);
+  }
+  storef8(&red[warp][lane * 8], acc);
+  __syncthreads();
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c < C) {
+    float t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) t += red[w][threadIdx.x];
+    partial[static_cast<long long>(blockIdx.y) * C + c] = t;
   }
 }
 
@@ -882,17 +894,21 @@ extern "C" int mdb_ln_bwd(const void* dy, const void* x, const float* mean, cons
   dim3 grid(ctas_per_batch, num_batches);
   if (scale == nullptr && C <= 2048) {  // plain affine, short rows: a warp per row
     const int vpl = ((C >> 3) + 31) / 32;
-    const size_t smem = out_sums ? 2 * static_cast<size_t>(C) * sizeof(float) : 0;
+    const size_t smem = out_sums ? (THREADS / 32) * 2 * static_cast<size_t>(C) * sizeof(float) : 0;  // at most 128 KB
 #define MDB_LN_ROWS_BWD(V)                                                                                        \
+  if (smem > 48 * 1024)                                                                                           \
+    MDB_CHECK_CUDA(cudaFuncSetAttribute(ln_rows_bwd_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+                                        (THREADS / 32) * 2 * 2048 * 4));                                          \
   ln_rows_bwd_kernel<V><<<grid, THREADS, smem, st>>>(static_cast<const __nv_bfloat16*>(dy),                       \
                                                      static_cast<const __nv_bfloat16*>(x), mean, rstd,             \
                                                      static_cast<const __nv_bfloat16*>(gamma), rows_per_batch, C,  \
                                                      static_cast<__nv_bfloat16*>(dx), out_sums ? scratch : nullptr)
-    if (vpl <= 1) MDB_LN_ROWS_BWD(1);
-    else if (vpl == 2) MDB_LN_ROWS_BWD(2);
-    else if (vpl <= 4) MDB_LN_ROWS_BWD(4);
-    else if (vpl <= 5) MDB_LN_ROWS_BWD(5);
-    else MDB_LN_ROWS_BWD(8);
+    if (vpl <= 1) { MDB_LN_ROWS_BWD(1); }
+    else if (vpl == 2) { MDB_LN_ROWS_BWD(2); }
+    else if (vpl == 3) { MDB_LN_ROWS_BWD(3); }
+    else if (vpl <= 4) { MDB_LN_ROWS_BWD(4); }
+    else if (vpl <= 5) { MDB_LN_ROWS_BWD(5); }
+    else { MDB_LN_ROWS_BWD(8); }
 #undef MDB_LN_ROWS_BWD
     if (out_sums) {
       dim3 g2((2 * C + 31) / 32, num_batches);
@@ -1035,7 +1051,8 @@ extern "C" int mdb_colsum(const void* x, long long ldx, int rows, int C, float* 
   if (C <= 0 || (C & 7)) return 3201;
   if (rows <= 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  dim3 grid(ctas, 1);
+  if (ctas < 1 || ctas > 65535) return 3203;
+  dim3 grid((C + 255) / 256, ctas);
   colsum_kernel<<<grid, THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(x), ldx, rows, C, scratch);
   dim3 g2((C + 31) / 32, 1);
   fold_partials_kernel<<<g2, 256, 0, st>>>(scratch, out, ctas, 1, C, 0);
@@ -1127,7 +1144,7 @@ extern "C" int mdb_colsum_noalloc(const void* x, long long ldx, int rows, int co
     g_colsum_scratch_addr[dev] = scratch;
   }
   const int ctas = rows < MDB_COLSUM_NOALLOC_CTAS ? rows : MDB_COLSUM_NOALLOC_CTAS;
-  colsum_kernel<<<dim3(ctas, 1), THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(x), ldx, rows, cols, scratch);
+  colsum_kernel<<<dim3((cols + 255) / 256, ctas), THREADS, 0, st>>>(static_cast<const __nv_bfloat16*>(x), ldx, rows, cols, scratch);
   const cudaError_t first = cudaGetLastError();  // each launch is checked: the second must not hide the first
   if (first != cudaSuccess) return static_cast<int>(first);
   fold_partials_kernel<<<dim3((cols + 31) / 32, 1), 256, 0, st>>>(scratch, out, ctas, 1, cols, 0);

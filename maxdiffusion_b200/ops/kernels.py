@@ -379,6 +379,8 @@ def ln_bwd(dy, x, mean, rstd, gamma=None, scale=None, need_sums=True):
   B, S, C = x.shape
   dx = torch.empty_like(x)
   cpb = _ctas_per_batch(B, S)
+  if scale is None and C <= 2048:  # a warp per row: four rows per warp, or the partial sums cost more than the rows
+    cpb = min(cpb, -(-S // 32))
   sums = scratch = None
   if need_sums:
     sums = torch.empty((B, 2, C), device=x.device, dtype=torch.float32)
@@ -456,7 +458,8 @@ def colsum(x2d):
   """fp32 column sums of a bf16 [rows, C] matrix (bias gradient)."""
   assert x2d.dim() == 2 and x2d.stride(-1) == 1 and x2d.dtype == torch.bfloat16
   rows, C = x2d.shape
-  ctas = max(1, min(rows, _TARGET_CTAS))
+  # row chunks: enough CTAs over all column tiles for the chip, and at least 32 rows (four per warp) each
+  ctas = max(1, min(-(-rows // 32), _TARGET_CTAS // -(-C // 256)))
   out = torch.empty((C,), device=x2d.device, dtype=torch.float32)
   scratch = torch.empty((ctas * C,), device=x2d.device, dtype=torch.float32)
   rc = _lib.lib().mdb_colsum(_lib.ptr(x2d), x2d.stride(0), rows, C, _lib.ptr(out), _lib.ptr(scratch), ctas,
