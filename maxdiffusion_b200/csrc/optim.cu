@@ -101,16 +101,8 @@ __global__ void __launch_bounds__(256) adamw_bf16x8_kernel(uint4* __restrict__ p
   }
 }
 
-// partial[block] = {sum x^2, max |x|}
-template <typename T>
-__global__ void sumsq_maxabs_kernel(const T* __restrict__ x, long long n, float2* __restrict__ partial) {
-  float s = 0.0f, mx = 0.0f;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float v = to_f<T>(x[i]);
-    s += v * v;
-    mx = fmaxf(mx, fabsf(v));
-  }
+// Block sums of (sum, max) pairs; thread 0 has the result.
+__device__ __forceinline__ float2 block_sum_max(float s, float mx) {
   __shared__ float ss[32], sm[32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -119,18 +111,50 @@ __global__ void sumsq_maxabs_kernel(const T* __restrict__ x, long long n, float2
   }
   if ((threadIdx.x & 31) == 0) { ss[threadIdx.x >> 5] = s; sm[threadIdx.x >> 5] = mx; }
   __syncthreads();
+  float ts = 0.0f, tm = 0.0f;
   if (threadIdx.x == 0) {
-    float ts = 0.0f, tm = 0.0f;
     for (int i = 0; i < (blockDim.x >> 5); ++i) { ts += ss[i]; tm = fmaxf(tm, sm[i]); }
-    partial[blockIdx.x] = make_float2(ts, tm);
   }
+  return make_float2(ts, tm);
 }
-// out[0] += sum, out[1] = max(out[1], max)  -- single thread block, fixed order
+
+// partial[block] = {sum x^2, max |x|}. 16 bytes per load where x starts on a 16-byte boundary, single values for the rest.
+// (With 2-byte loads and a fold by one thread, 4608 x 15360 values took 45 + 28 us.)
+template <typename T>
+__global__ void sumsq_maxabs_kernel(const T* __restrict__ x, long long n, float2* __restrict__ partial) {
+  constexpr int PER = 16 / sizeof(T);
+  float s = 0.0f, mx = 0.0f;
+  const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long step = static_cast<long long>(gridDim.x) * blockDim.x;
+  const long long nvec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / PER : 0;
+#pragma unroll 4
+  for (long long i = tid; i < nvec; i += step) {
+    const uint4 u = reinterpret_cast<const uint4*>(x)[i];
+    const T* e = reinterpret_cast<const T*>(&u);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const float v = to_f<T>(e[j]);
+      s += v * v;
+      mx = fmaxf(mx, fabsf(v));
+    }
+  }
+  for (long long i = nvec * PER + tid; i < n; i += step) {
+    const float v = to_f<T>(x[i]);
+    s += v * v;
+    mx = fmaxf(mx, fabsf(v));
+  }
+  const float2 t = block_sum_max(s, mx);
+  if (threadIdx.x == 0) partial[blockIdx.x] = t;
+}
 __global__ void fold_sumsq_kernel(const float2* __restrict__ partial, int n, float* __restrict__ out, int accumulate) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float ts = 0.0f, tm = 0.0f;
-    for (int i = 0; i < n; ++i) { ts += partial[i].x; tm = fmaxf(tm, partial[i].y); }
-    if (accumulate) { out[0] += ts; out[1] = fmaxf(out[1], tm); } else { out[0] = ts; out[1] = tm; }
+  float s = 0.0f, mx = 0.0f;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    s += partial[i].x;
+    mx = fmaxf(mx, partial[i].y);
+  }
+  const float2 t = block_sum_max(s, mx);
+  if (threadIdx.x == 0) {
+    if (accumulate) { out[0] += t.x; out[1] = fmaxf(out[1], t.y); } else { out[0] = t.x; out[1] = t.y; }
   }
 }
 
@@ -192,6 +216,6 @@ extern "C" int mdb_sumsq_maxabs(const void* x, long long n, int is_f32, float* o
     sumsq_maxabs_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(x), n, part);
   else
     sumsq_maxabs_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), n, part);
-  fold_sumsq_kernel<<<1, 32, 0, st>>>(part, blocks, out, accumulate);
+  fold_sumsq_kernel<<<1, 256, 0, st>>>(part, blocks, out, accumulate);
   return static_cast<int>(cudaGetLastError());
 }

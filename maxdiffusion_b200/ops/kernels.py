@@ -515,8 +515,9 @@ def adamw(p, g, m, v, *, lr, b1, b2, eps, wd, step, grad_scale=1.0, clip_value=0
 def sumsq_maxabs(x, out=None, accumulate=False):
   """out (fp32 [2]) = {sum x², max |x|}; with accumulate the result is folded into `out`."""
   assert x.is_contiguous()
-  if out is None:
-    out = torch.zeros((2,), device=x.device, dtype=torch.float32)
+  if out is None:  # the kernel writes both values unless it adds to them or there is nothing to read
+    make = torch.zeros if accumulate or x.numel() == 0 else torch.empty
+    out = make((2,), device=x.device, dtype=torch.float32)
   scratch = torch.empty((2048,), device=x.device, dtype=torch.float32)
   rc = _lib.lib().mdb_sumsq_maxabs(_lib.ptr(x), x.numel(), int(x.dtype == torch.float32), _lib.ptr(out),
                                    _lib.ptr(scratch), int(accumulate), _lib.stream())
