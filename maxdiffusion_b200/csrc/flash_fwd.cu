@@ -84,6 +84,7 @@ struct CopyPlan {
 
 struct Params {
   int B, H, q_len;
+  int d;  // channels of a head, a multiple of 8 up to the built head_dim; TMA fills the rest of a tile with zeros
   int num_segments;
   int kv_len[MAX_SEGMENTS];
   __nv_bfloat16* out;
@@ -572,6 +573,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         if (row_ok) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
+            if (c * 32 + v * 8 >= p.d) break;
             uint4 ov;
             ov.x = pack_bf16x2(__uint_as_float(r[v * 8 + 0]) * inv, __uint_as_float(r[v * 8 + 1]) * inv);
             ov.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]) * inv, __uint_as_float(r[v * 8 + 3]) * inv);
@@ -676,27 +678,29 @@ static int flash_fwd_launch(const void* q, const void* const* k_ptrs, const void
                             long long o_ss, long long o_sh, float softmax_scale, const unsigned int* seg_flags,
                             unsigned int flag_target, const MdbCopyPlan* plan, void* stream_ptr,
                             const float* m_fixed = nullptr, const int* fixed_heads = nullptr,
-                            const MdbOutScatter* scatter = nullptr) {
+                            const MdbOutScatter* scatter = nullptr, int head_dim = HD) {
   using namespace mdb;
   using namespace mdb::fa;
+  if (head_dim <= HD - 64 || head_dim > HD || (head_dim & 7)) return 3110;
   if (B <= 0 || H <= 0 || q_len <= 0) return 0;
   if (num_segments < 1 || num_segments > MAX_SEGMENTS) return 3101;
   if ((q_sb | q_ss | q_sh | k_sb | k_ss | k_sh | v_sb | v_ss | v_sh | o_sb | o_ss | o_sh) & 7) return 3102;
   CUtensorMap tq;
   KVMaps maps;
   Params p;
-  int rc = make_map(&tq, q, HD, B, q_len, H, q_sb, q_ss, q_sh, BQ);
+  int rc = make_map(&tq, q, head_dim, B, q_len, H, q_sb, q_ss, q_sh, BQ);
   if (rc) return rc;
   for (int s = 0; s < MAX_SEGMENTS; ++s) {
     const int src = s < num_segments ? s : 0;
     p.kv_len[s] = s < num_segments ? kv_lens[s] : 0;
     const int len = kv_lens[src] > 0 ? kv_lens[src] : 1;
-    rc = make_map(&maps.k[s], k_ptrs[src], HD, B, len, H, k_sb, k_ss, k_sh, BKV);
+    rc = make_map(&maps.k[s], k_ptrs[src], head_dim, B, len, H, k_sb, k_ss, k_sh, BKV);
     if (rc) return rc;
-    rc = make_map(&maps.v[s], v_ptrs[src], HD, B, len, H, v_sb, v_ss, v_sh, BKV);
+    rc = make_map(&maps.v[s], v_ptrs[src], head_dim, B, len, H, v_sb, v_ss, v_sh, BKV);
     if (rc) return rc;
   }
   p.B = B; p.H = H; p.q_len = q_len;
+  p.d = head_dim;
   p.num_segments = num_segments;
   p.out = static_cast<__nv_bfloat16*>(out);
   p.o_stride_b = o_sb; p.o_stride_s = o_ss; p.o_stride_h = o_sh;
@@ -818,6 +822,22 @@ extern "C" int mdb_flash_fwd_scatter(const void* q, const void* const* k_ptrs, c
   return flash_fwd_launch<128>(q, k_ptrs, v_ptrs, nullptr, nullptr, B, H, q_len, num_segments, kv_lens, q_sb, q_ss, q_sh, k_sb,
                                k_ss, k_sh, v_sb, v_ss, v_sh, o_sb, o_ss, o_sh, softmax_scale, seg_flags, flag_target,
                                plan, stream_ptr, nullptr, nullptr, scatter);
+}
+
+// Any head_dim that is a multiple of 8 up to 128 (Stable Diffusion 1.x: 40 and 80), on the kernel of the next built size: the
+// tensor maps end at head_dim, so the missing channels of a tile arrive as zeros and the epilogue stores only real ones.
+extern "C" int mdb_flash_fwd_narrow(const void* q, const void* const* k_ptrs, const void* const* v_ptrs, void* out,
+                                    float* lse, int B, int H, int q_len, int num_segments, const int* kv_lens,
+                                    long long q_sb, long long q_ss, long long q_sh, long long k_sb, long long k_ss,
+                                    long long k_sh, long long v_sb, long long v_ss, long long v_sh, long long o_sb,
+                                    long long o_ss, long long o_sh, float softmax_scale, int head_dim, void* stream_ptr) {
+  if (head_dim <= 64)
+    return flash_fwd_launch<64>(q, k_ptrs, v_ptrs, out, lse, B, H, q_len, num_segments, kv_lens, q_sb, q_ss, q_sh, k_sb, k_ss,
+                                k_sh, v_sb, v_ss, v_sh, o_sb, o_ss, o_sh, softmax_scale, nullptr, 0, nullptr, stream_ptr,
+                                nullptr, nullptr, nullptr, head_dim);
+  return flash_fwd_launch<128>(q, k_ptrs, v_ptrs, out, lse, B, H, q_len, num_segments, kv_lens, q_sb, q_ss, q_sh, k_sb, k_ss,
+                               k_sh, v_sb, v_ss, v_sh, o_sb, o_ss, o_sh, softmax_scale, nullptr, 0, nullptr, stream_ptr,
+                               nullptr, nullptr, nullptr, head_dim);
 }
 
 // Same for head_dim 64 (Stable Diffusion / SDXL / LTX-Video heads).

@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(256) fold_partials_kernel(const float* __restr
 template <int NV>
 __global__ void __launch_bounds__(THREADS, 4)
 rms_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_bfloat16* __restrict__ y, long long ldy,
-                    const __nv_bfloat16* __restrict__ w, int w_per_head, const float* __restrict__ cos_t,
+                    long long y_batch, const __nv_bfloat16* __restrict__ w, int w_per_head, const float* __restrict__ cos_t,
                     const float* __restrict__ sin_t, int rows_per_batch, int C, int group, float eps,
                     float* __restrict__ rstd_out, const HeadScatter sc) {
   __shared__ float2 red[2][THREADS / 32];
@@ -569,7 +569,7 @@ rms_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_bfl
           const long long drow = (static_cast<long long>(s.batch) * sc.n + sc.me) * rows_per_batch + pos;
           store8(sc.base[r] + (drow * sc.hn + (head - r * sc.hn)) * 128 + (vi & 15) * 8, o);
         } else {
-          store8(y + row * ldy + vi * 8, o);
+          store8(y + s.batch * y_batch + pos * ldy + vi * 8, o);
         }
       }
     }
@@ -936,14 +936,14 @@ extern "C" int mdb_ln_bwd(const void* dy, const void* x, const float* mean, cons
   return static_cast<int>(cudaGetLastError());
 }
 
-static int launch_rms_rope_fwd(const void* x, long long ldx, void* y, long long ldy, const void* w, int w_per_head,
+static int launch_rms_rope_fwd(const void* x, long long ldx, void* y, long long ldy, long long y_batch, const void* w, int w_per_head,
                                const float* cos_t, const float* sin_t, int num_batches, int rows_per_batch, int C, int group,
                                float eps, float* rstd_out, const mdb::rw::HeadScatter& sc, int ctas_per_batch, void* stream) {
   using namespace mdb::rw;
   dim3 grid(ctas_per_batch, num_batches);
 #define MDB_RMS_FWD(NV)                                                                                 \
   rms_rope_fwd_kernel<NV><<<grid, THREADS, 0, static_cast<cudaStream_t>(stream)>>>(                     \
-      static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy,                   \
+      static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy, y_batch,          \
       static_cast<const __nv_bfloat16*>(w), w_per_head, cos_t, sin_t, rows_per_batch, C, group, eps, rstd_out, sc)
   switch (vectors_per_thread(C)) {
     case 1: MDB_RMS_FWD(1); break;
@@ -955,7 +955,8 @@ static int launch_rms_rope_fwd(const void* x, long long ldx, void* y, long long 
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int mdb_rms_rope_fwd(const void* x, long long ldx, void* y, long long ldy, const void* w, int w_per_head,
+// y: row pitch ldy, batch pitch y_batch (elements), so that the result may be a part of a longer sequence's buffer.
+extern "C" int mdb_rms_rope_fwd(const void* x, long long ldx, void* y, long long ldy, long long y_batch, const void* w, int w_per_head,
                                 const float* cos_t, const float* sin_t, int num_batches, int rows_per_batch, int C,
                                 int group, float eps, float* rstd_out, int ctas_per_batch, void* stream) {
   if (int rc = check_c(C)) return rc;
@@ -964,7 +965,8 @@ extern "C" int mdb_rms_rope_fwd(const void* x, long long ldx, void* y, long long
   HeadScatter sc;
   sc.n = 0; sc.me = 0; sc.hn = 1;
   for (int i = 0; i < 8; ++i) sc.base[i] = nullptr;
-  return launch_rms_rope_fwd(x, ldx, y, ldy, w, w_per_head, cos_t, sin_t, num_batches, rows_per_batch, C, group, eps, rstd_out,
+  if ((ldy | y_batch) & 7) return 3204;
+  return launch_rms_rope_fwd(x, ldx, y, ldy, y_batch, w, w_per_head, cos_t, sin_t, num_batches, rows_per_batch, C, group, eps, rstd_out,
                              sc, ctas_per_batch, stream);
 }
 
@@ -983,7 +985,7 @@ extern "C" int mdb_rms_rope_fwd_scatter(const void* x, long long ldx, const void
   HeadScatter sc;
   sc.n = n; sc.me = me; sc.hn = heads / n;
   for (int i = 0; i < 8; ++i) sc.base[i] = i < n ? reinterpret_cast<__nv_bfloat16*>(peer_ptrs[i]) : nullptr;
-  return launch_rms_rope_fwd(x, ldx, nullptr, 0, w, w_per_head, cos_t, sin_t, num_batches, rows_per_batch, C, group, eps,
+  return launch_rms_rope_fwd(x, ldx, nullptr, 0, 0, w, w_per_head, cos_t, sin_t, num_batches, rows_per_batch, C, group, eps,
                              nullptr, sc, ctas_per_batch, stream);
 }
 

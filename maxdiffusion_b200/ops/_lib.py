@@ -130,6 +130,8 @@ def _declare(L: ctypes.CDLL) -> None:
   L.mdb_flash_fwd.restype = c_int
   L.mdb_flash_fwd_d64.argtypes = L.mdb_flash_fwd.argtypes
   L.mdb_flash_fwd_d64.restype = c_int
+  L.mdb_flash_fwd_narrow.argtypes = L.mdb_flash_fwd.argtypes[:-4] + [c_int, c_void_p]
+  L.mdb_flash_fwd_narrow.restype = c_int
   for name in ("mdb_flash_fwd_fixed_m", "mdb_flash_fwd_fixed_m_d64"):
     getattr(L, name).argtypes = L.mdb_flash_fwd.argtypes + [c_void_p, c_void_p]
     getattr(L, name).restype = c_int
@@ -148,7 +150,7 @@ def _declare(L: ctypes.CDLL) -> None:
   L.mdb_ln_fwd.restype = c_int
   L.mdb_ln_bwd.argtypes = [c_void_p] * 6 + [c_ll, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
   L.mdb_ln_bwd.restype = c_int
-  L.mdb_rms_rope_fwd.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
+  L.mdb_rms_rope_fwd.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
                                  c_int, c_int, c_float, c_void_p, c_int, c_void_p]
   L.mdb_rms_rope_fwd.restype = c_int
   L.mdb_rms_rope_bwd.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,

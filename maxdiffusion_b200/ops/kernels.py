@@ -225,6 +225,34 @@ def flash_fwd(q: torch.Tensor, k_list: Sequence[torch.Tensor], v_list: Sequence[
   return (out, lse) if return_lse else out
 
 
+def flash_narrow_ok(*tensors) -> bool:
+  """Whether `flash_fwd_narrow` can read these [B,S,H,D] tensors where they are: D a multiple of 8 up to 128, unit inner
+  stride, 16-byte aligned start and strides (what a projection's output has)."""
+  for t in tensors:
+    if t.shape[-1] % 8 or t.shape[-1] > 128 or t.stride(-1) != 1 or t.data_ptr() % 16 or any(st % 8 for st in t.stride()[:-1]):
+      return False
+  return True
+
+
+def flash_fwd_narrow(q, k_list, v_list, scale: float):
+  """Attention forward for a head_dim between the built sizes (Stable Diffusion 1.x: 40, 80) without padded copies: the
+  tensor maps end at D and the kernel of the next size gets zeros beyond. No log-sum-exp (inference)."""
+  B, Sq, H, D = q.shape
+  k0, v0 = k_list[0], v_list[0]
+  assert q.dtype == torch.bfloat16 and flash_narrow_ok(q, *k_list, *v_list)
+  assert all(k.dtype == torch.bfloat16 and k.stride() == k0.stride() for k in k_list)
+  assert all(v.dtype == torch.bfloat16 and v.stride() == v0.stride() for v in v_list)
+  n = len(k_list)
+  out = torch.empty((B, Sq, H, D), device=q.device, dtype=torch.bfloat16)
+  rc = _lib.lib().mdb_flash_fwd_narrow(
+      _lib.ptr(q), (ctypes.c_void_p * n)(*[k.data_ptr() for k in k_list]), (ctypes.c_void_p * n)(*[v.data_ptr() for v in v_list]),
+      _lib.ptr(out), 0, B, H, Sq, n, (ctypes.c_int * n)(*[k.shape[1] for k in k_list]), q.stride(0), q.stride(1), q.stride(2),
+      k0.stride(0), k0.stride(1), k0.stride(2), v0.stride(0), v0.stride(1), v0.stride(2), out.stride(0), out.stride(1),
+      out.stride(2), float(scale), D, _lib.stream())
+  _lib.check(rc, "mdb_flash_fwd_narrow")
+  return out
+
+
 def flash_fwd_scatter(q, k_list, v_list, peer_out_ptrs, rows_per_rank: int, heads_total: int, head_off: int,
                       scale: float | None = None, seg_flags=None, flag_target: int = 0, plan=None) -> None:
   """Attention forward (head_dim 128) whose epilogue stores the output rows straight into the ranks that own them:
@@ -392,18 +420,20 @@ def ln_bwd(dy, x, mean, rstd, gamma=None, scale=None, need_sums=True):
   return dx, sums
 
 
-def rms_rope_fwd(x, w=None, cos=None, sin=None, heads=1, per_head=False, eps=1e-6, save_stats=False):
-  """x: [B,S,C] bf16 (row stride arbitrary, e.g. a slice of a fused QKV output) -> [B,S,H,D] contiguous."""
+def rms_rope_fwd(x, w=None, cos=None, sin=None, heads=1, per_head=False, eps=1e-6, save_stats=False, out=None):
+  """x: [B,S,C] bf16 (row stride arbitrary, e.g. a slice of a fused QKV output) -> [B,S,H,D] contiguous. `out` [B,S,C]
+  may be a part of a longer sequence's buffer (unit inner stride, pitches multiples of 8)."""
   B, S, C = x.shape
   assert x.dtype == torch.bfloat16 and x.stride(-1) == 1 and x.stride(0) == S * x.stride(1)
-  y = torch.empty((B, S, C), device=x.device, dtype=torch.bfloat16)
+  y = torch.empty((B, S, C), device=x.device, dtype=torch.bfloat16) if out is None else out
+  assert y.shape == (B, S, C) and y.dtype == torch.bfloat16 and y.stride(-1) == 1 and y.data_ptr() % 16 == 0
   group = 128 if per_head else C
   rstd = None
   if save_stats:
     rstd = torch.empty((B, S, heads) if per_head else (B, S), device=x.device, dtype=torch.float32)
   if cos is not None:
     assert cos.dtype == torch.float32 and cos.shape == (S, 64) and cos.is_contiguous() and sin.is_contiguous()
-  rc = _lib.lib().mdb_rms_rope_fwd(_lib.ptr(x), x.stride(1), _lib.ptr(y), C, _lib.ptr(w), int(per_head),
+  rc = _lib.lib().mdb_rms_rope_fwd(_lib.ptr(x), x.stride(1), _lib.ptr(y), y.stride(1), y.stride(0), _lib.ptr(w), int(per_head),
                                    _lib.ptr(cos), _lib.ptr(sin), B, S, C, group, float(eps), _lib.ptr(rstd),
                                    _ctas_per_batch(B, S), _lib.stream())
   _lib.check(rc, "mdb_rms_rope_fwd")
