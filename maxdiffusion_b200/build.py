@@ -18,6 +18,7 @@ PKG_DIR = Path(__file__).resolve().parent
 SRC_DIR = PKG_DIR / "csrc"
 OBJ_DIR = PKG_DIR / "csrc" / "build"
 LIB_PATH = PKG_DIR / "_kernels.so"
+HOST_PATH = PKG_DIR / "_host_ops.so"  # CPython extension over the kernel library (csrc/host_ops.cpp)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -81,7 +82,33 @@ def build(verbose: bool = True, force: bool = False) -> Path:
       raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
     if verbose:
       print(f"[build] linked {LIB_PATH}")
+  _build_host_ops(verbose, force)
   return LIB_PATH
+
+
+def _build_host_ops(verbose: bool, force: bool) -> None:
+  """Compiles csrc/host_ops.cpp against the installed PyTorch and links it to `_kernels.so` beside it."""
+  import sysconfig
+
+  import torch
+
+  root = Path(torch.__file__).resolve().parent
+  cuda = Path(_nvcc()).resolve().parent.parent
+  src, obj, stamp = SRC_DIR / "host_ops.cpp", OBJ_DIR / "host_ops.o", OBJ_DIR / "host_ops.sha"
+  flags = ["-std=c++17", "-O2", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+  digest = hashlib.sha256(" ".join([torch.__version__, sys.version, *flags]).encode() + src.read_bytes()).hexdigest()
+  if force or not HOST_PATH.exists() or not stamp.exists() or stamp.read_text() != digest:
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda / "include"]
+    libs = ["-L", str(PKG_DIR), "-l:_kernels.so", "-Wl,-rpath,$ORIGIN", "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu",
+            "-ltorch", "-lc10_cuda", "-lc10"]  # PyTorch's libraries are loaded before this one: no run path to them
+    for cmd in (["g++", *flags, *[f"-I{i}" for i in inc], "-c", str(src), "-o", str(obj)],
+                ["g++", "-shared", str(obj), "-o", str(HOST_PATH), *libs]):
+      res = subprocess.run(cmd, capture_output=True, text=True)
+      if res.returncode != 0:
+        raise RuntimeError(f"{src.name}: {' '.join(cmd[:2])} failed:\n{res.stdout}\n{res.stderr}")
+    stamp.write_text(digest)
+    if verbose:
+      print(f"[build] linked {HOST_PATH}")
 
 
 if __name__ == "__main__":

@@ -14,6 +14,7 @@ from pathlib import Path
 import torch
 
 _LIB = None
+_HOST = None
 _LOCK = threading.Lock()
 LIB_PATH = Path(__file__).resolve().parent.parent / "_kernels.so"
 
@@ -62,6 +63,30 @@ def lib() -> ctypes.CDLL:
   return _LIB
 
 
+def host_ops():
+  """The CPython extension over the kernel library (`csrc/host_ops.cpp`), or None where there is no GPU."""
+  global _HOST
+  if _HOST is None:
+    if not torch.cuda.is_available():
+      return None
+    lib()
+    with _LOCK:
+      if _HOST is None:
+        import importlib.util
+
+        from . import kernels
+
+        path = LIB_PATH.with_name("_host_ops.so")
+        if not path.exists():
+          raise KernelError(f"{path} is missing; run `python -m maxdiffusion_b200.build`")
+        spec = importlib.util.spec_from_file_location("_host_ops", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.setup(KernelError, kernels.gemm_plan)
+        _HOST = mod
+  return _HOST
+
+
 def available() -> bool:
   """True when CUDA tensors can be served by the kernel library."""
   return torch.cuda.is_available()
@@ -73,12 +98,14 @@ def use_kernels(*tensors: torch.Tensor) -> bool:
   return t.is_cuda
 
 
-def stream() -> ctypes.c_void_p:
-  return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def stream() -> int:
+  """The current stream of the current device, as the integer the entry points take. (Building `torch.cuda.Stream` and
+  `c_void_p` objects for every launch cost as much host time as the launch: a UNet step of 840 launches was bound by it.)"""
+  return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-  return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def ptr(t: torch.Tensor | None) -> int:
+  return 0 if t is None else t.data_ptr()
 
 
 def check(rc: int, what: str) -> None:
@@ -89,7 +116,7 @@ def check(rc: int, what: str) -> None:
 
 
 def launch_count() -> int:
-  return _launches
+  return _launches + (0 if _HOST is None else _HOST.launches())
 
 
 def read_status(clear: bool = True) -> tuple[int, int, int, int]:

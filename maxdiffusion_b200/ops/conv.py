@@ -20,7 +20,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import Optional, Sequence
 
 import torch
@@ -88,16 +88,22 @@ class PackedConv:
   kind: str
   src: tuple = ()                 # (weight, bias, stride, pad_top_left) as given: what the PyTorch reference path runs
 
+  _tap_cache: dict = field(default_factory=dict, repr=False)
+
   def tap_arrays(self, shift1: int = 0):
     """ctypes arrays of the tap table; `shift1` is added to every tap's offset along dim 1 (the width): an input
     that carries `shift1` halo columns on each side produces outputs for its interior columns only."""
+    hit = self._tap_cache.get(shift1)
+    if hit is not None:
+      return hit
     flat, begin, k = [], [0], 0
     for cls in self.taps:
       for t in cls:
         flat.extend([t[0], t[1] + shift1, t[2], t[3], t[4], k * self.c_pad])
         k += 1
       begin.append(k)
-    return (ctypes.c_int * len(flat))(*flat), (ctypes.c_int * len(begin))(*begin), len(self.taps)
+    self._tap_cache[shift1] = (ctypes.c_int * len(flat))(*flat), (ctypes.c_int * len(begin))(*begin), len(self.taps)
+    return self._tap_cache[shift1]
 
 
 def _pack(w_taps: torch.Tensor, bias, taps, kind: str) -> PackedConv:
@@ -205,6 +211,7 @@ def pack_conv2d_dgrad(weight: torch.Tensor, stride: int = 1, pad_top_left: Optio
   return pk
 
 
+@functools.lru_cache(maxsize=4096)
 def _pick_box(e1: int, e2: int, e3: int, allow3: bool):
   """Tile (b1, b2, b3) with b1 * b2 * b3 = 128 that covers the e1 x e2 x e3 output positions with the least padding;
   among equals the widest along the fastest axis."""
@@ -271,15 +278,30 @@ def conv_plan(m_tiles: int, n_classes: int, n: int, units: int, sms: int = 148) 
   return best
 
 
+@functools.lru_cache(maxsize=8192)
+def _carray(T, values: tuple):
+  """ctypes array of the given integers (read only: the entry points copy what they need)."""
+  return (T * len(values))(*[int(v) for v in values])
+
+
 def _launch(x, x_alt, pk: PackedConv, dims, strides, alt_dims, alt_strides, box, ext, out, out_strides, class_off,
             residual, silu, alt_dim=-1, alt_shift=0, tap_shift1=0):
   taps, begin, n_classes = pk.tap_arrays(tap_shift1)
   LL, I = ctypes.c_longlong, ctypes.c_int
-  arr = lambda T, v: (T * len(v))(*[int(i) for i in v])
+  arr = lambda T, v: _carray(T, tuple(v))
   m_tiles = ext[3]
   for e, b in zip(ext[:3], box):
     m_tiles *= -(-e // b)
   ctas, max_bn, splits = _PLAN or conv_plan(m_tiles, n_classes, pk.n_pad, -(-pk.c_in // 64) * min(len(c) for c in pk.taps))
+  host = _lib.host_ops()
+  if host is not None:
+    dims, strides, box, ext = tuple(dims), tuple(strides), tuple(box), tuple(ext)
+    r = host.conv(x, x_alt, pk.w, out, pk.bias, residual, dims, strides, tuple(alt_dims) if alt_dims else dims,
+                  tuple(alt_strides) if alt_strides else strides, box, ext, pk.c_in, pk.n_pad, ctypes.addressof(taps),
+                  ctypes.addressof(begin), alt_dim, alt_shift, tuple(out_strides), tuple(class_off), 1 if silu else 0, ctas,
+                  max_bn, splits, m_tiles)
+    if r is not NotImplemented:
+      return out
   partial = None
   if splits > 1:
     partial = torch.empty(splits * n_classes * m_tiles * 128 * pk.n_pad, device=out.device, dtype=torch.float32)

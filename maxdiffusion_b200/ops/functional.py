@@ -18,8 +18,11 @@ import threading
 from typing import Sequence
 
 import torch
+import torch._C as _C
+import torch.autograd.forward_ad as _fwd_ad
 import torch.nn.functional as F
 
+from . import _lib
 from . import conv as OC
 from . import kernels as K
 from . import ref
@@ -44,6 +47,23 @@ def _fast(t: torch.Tensor) -> bool:
   return t.is_cuda and t.dtype == torch.bfloat16 and not _LIBRARY_MODE
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter, type(None))
+
+
+def _direct(*tensors) -> bool:
+  """True when an op may call its kernel without its `torch.autograd.Function`: autograd is off, and nothing that works
+  through the Function is at work (a functorch transform, forward-mode duals, a tensor subclass, a graph tracer), nor a
+  pass that is run again with autograd on (a rematerialised block: both passes must round alike). The Function's
+  bookkeeping is most of an op's host time."""
+  if (torch.is_grad_enabled() or _remat.rerun or _C._are_functorch_transforms_active() or _fwd_ad._current_level >= 0 or
+      _C._get_tracing_state() is not None or _C._len_torch_dispatch_stack() > 0 or torch.compiler.is_compiling()):
+    return False
+  for t in tensors:
+    if type(t) not in _PLAIN:
+      return False
+  return True
+
+
 # ---------------------------------------------------------------------------------------------
 # remat bookkeeping for attention outputs
 # ---------------------------------------------------------------------------------------------
@@ -53,6 +73,7 @@ class _RematState(threading.local):
     self.mode = None  # None | "record" | "replay"
     self.store = None
     self.cursor = 0
+    self.rerun = False  # inside the first pass of a block whose backward runs it again
 
 
 _remat = _RematState()
@@ -136,6 +157,22 @@ def linear(x, weight, bias=None, activation: str | None = None, residual=None):
       weight = weight.to(torch.bfloat16)
     if bias is not None and bias.dtype != torch.bfloat16:
       bias = bias.to(torch.bfloat16)
+    if _direct(x, weight, bias, residual) and activation in (None, "gelu_tanh", "silu"):
+      if activation is None or residual is None:
+        r = _lib.host_ops().linear(x, weight, bias, K._EPI["add_res" if residual is not None else activation or "none"], residual,
+                                   K._FORCE_TILE_N, K._FORCE_CTAS)
+        if r is not NotImplemented:
+          return r
+      n = weight.shape[0]
+      x2 = x.reshape(-1, x.shape[-1])
+      if residual is None:
+        y = K.gemm(x2, weight, bias=bias, epi=activation or "none")
+      elif activation is None and residual.dtype == torch.bfloat16:
+        r2 = residual.reshape(-1, n)
+        y = K.gemm(x2, weight, bias=bias, epi="add_res", residual=r2 if r2.is_contiguous() else r2.contiguous())
+      else:
+        return residual + K.gemm(x2, weight, bias=bias, epi=activation or "none").view(*x.shape[:-1], n)
+      return y.view(*x.shape[:-1], n)
     if residual is not None and (activation is not None or residual.dtype != torch.bfloat16):
       return residual + _LinearFn.apply(x, weight, bias, activation)
     return _LinearFn.apply(x, weight, bias, activation, residual)
@@ -237,7 +274,15 @@ def attention(q, k, v, scale: float | None = None, fixed_m=None, keep_mask=None)
   vs = list(v) if isinstance(v, (list, tuple)) else [v]
   D = q.shape[-1]
   scale = scale if scale is not None else 1.0 / math.sqrt(D)
+  if (len(ks) == 1 and fixed_m is None and keep_mask is None and _fast(q) and _remat.mode is None and not K._FLASH_TUNED and
+      _direct(q, ks[0], vs[0])):
+    r = _lib.host_ops().attention(q, ks[0], vs[0], scale)
+    if r is not NotImplemented:
+      return r
   if _fast(q) and D not in K.FLASH_HEAD_DIMS and D < max(K.FLASH_HEAD_DIMS) and D % 8 == 0:
+    if (keep_mask is None and _remat.mode is None and _direct(q, *ks, *vs) and K.flash_narrow_ok(q, *ks, *vs) and
+        all(t.stride() == ks[0].stride() for t in ks) and all(t.stride() == vs[0].stride() for t in vs)):
+      return K.flash_fwd_narrow(q, ks, vs, scale)
     # other head sizes (Stable Diffusion 1.x / 2.x: 40, 80) ride the next built size: zero channels add nothing to
     # q.k and produce zero output channels, which are cut off again; the scale stays that of the true size
     Dp = min(d for d in K.FLASH_HEAD_DIMS if d > D)
@@ -263,6 +308,8 @@ def attention(q, k, v, scale: float | None = None, fixed_m=None, keep_mask=None)
                                        vc[b:b + 1].index_select(1, idx)))
     return rows[0] if len(rows) == 1 else torch.cat(rows, dim=0)
   if fast:
+    if _remat.mode is None and _direct(q, *ks, *vs):
+      return K.flash_fwd(q, ks, vs, scale, return_lse=False, fixed_m=fixed_m)
     return _AttentionFn.apply(q, scale, len(ks), fixed_m, *ks, *vs)
   kc = torch.cat(ks, dim=1) if len(ks) > 1 else ks[0]
   vc = torch.cat(vs, dim=1) if len(vs) > 1 else vs[0]
@@ -313,6 +360,9 @@ def layer_norm_mod(x, gamma=None, beta=None, scale=None, shift=None, eps: float 
       shift = shift.float() if shift.dtype != torch.float32 else shift
       if scale.stride(-1) != 1 or shift.stride(-1) != 1 or scale.stride(0) != shift.stride(0):
         scale, shift = scale.contiguous(), shift.contiguous()
+    if _direct(x, gamma, beta, scale, shift):
+      r = _lib.host_ops().layer_norm(x, gamma, beta, scale, shift, eps)
+      return r if r is not NotImplemented else K.ln_fwd(x, gamma, beta, scale, shift, eps)
     return _LayerNormModFn.apply(x, gamma, beta, scale, shift, eps)
   return ref.layer_norm_mod(x, gamma, beta, scale, shift, eps)
 
@@ -333,6 +383,10 @@ class _GegluFn(torch.autograd.Function):
 def geglu(u: torch.Tensor) -> torch.Tensor:
   """u [..., 2 * inner] = (h | gate) -> h * gelu(gate), exact GELU; one kernel forward, one backward."""
   if _fast(u) and u.shape[-1] % 16 == 0:
+    if _direct(u):
+      u = u if u.is_contiguous() else u.contiguous()
+      r = _lib.host_ops().geglu(u)
+      return r if r is not NotImplemented else K.geglu_fwd(u)
     return _GegluFn.apply(u if u.is_contiguous() else u.contiguous())
   h, gate = u.chunk(2, dim=-1)
   return h * torch.nn.functional.gelu(gate)
@@ -368,8 +422,28 @@ def rms_norm_rope(x, weight=None, cos=None, sin=None, heads: int = 1, per_head: 
     if cos is not None:
       cos = cos.float().contiguous() if (cos.dtype != torch.float32 or not cos.is_contiguous()) else cos
       sin = sin.float().contiguous() if (sin.dtype != torch.float32 or not sin.is_contiguous()) else sin
+    if _direct(x, weight, cos, sin):
+      r = _lib.host_ops().rms_rope(x, weight, cos, sin, heads, per_head, eps)
+      return r if r is not NotImplemented else K.rms_rope_fwd(x, weight, cos, sin, heads, per_head, eps)
     return _RmsRopeFn.apply(x, weight, cos, sin, heads, per_head, eps)
   return ref.rms_norm_rope(x, weight, cos, sin, heads, per_head, eps)
+
+
+def joint_norm_rope(parts, heads: int, eps: float = 1e-6):
+  """Per-head RMSNorm + RoPE of several streams, concatenated along the sequence: parts = [(x [B,S_i,C], weight, cos, sin),
+  ...] -> [B, sum S_i, H, D]. Without autograd every stream is written where it belongs in the joint buffer."""
+  x0 = parts[0][0]
+  B, C = x0.shape[0], x0.shape[-1]
+  if all(_fast(x) and x.shape[-1] == C and C // heads == 128 and C % 128 == 0 and C <= 8192 and x.stride(-1) == 1 and
+         x.stride(0) == x.shape[1] * x.stride(1) and cos.dtype == sin.dtype == torch.float32 and cos.is_contiguous() and
+         sin.is_contiguous() and _direct(x, w, cos, sin) for x, w, cos, sin in parts):
+    joint = torch.empty((B, sum(x.shape[1] for x, *_ in parts), C), device=x0.device, dtype=x0.dtype)
+    at = 0
+    for x, w, cos, sin in parts:
+      K.rms_rope_fwd(x, w, cos, sin, heads, True, eps, out=joint[:, at:at + x.shape[1]])
+      at += x.shape[1]
+    return joint.view(B, at, heads, C // heads)
+  return torch.cat([rms_norm_rope(x, w, cos, sin, heads=heads, per_head=True, eps=eps) for x, w, cos, sin in parts], dim=1)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -403,6 +477,8 @@ def gated_residual(res, y, gate=None):
     y = y if y.is_contiguous() else y.contiguous()
     if gate is not None and (gate.dtype != torch.float32 or gate.stride(-1) != 1):
       gate = gate.float().contiguous()
+    if _direct(res, y, gate):
+      return K.gated_res_fwd(res, y, gate)
     return _GatedResFn.apply(res, y, gate)
   return ref.gated_residual(res, y, gate)
 
@@ -432,12 +508,16 @@ class _CheckpointFn(torch.autograd.Function):
       ctx.offload_event.record()
       tensors = (None,) + tuple(tensors[1:])
     ctx.save_for_backward(*tensors)
-    with torch.no_grad():
-      if ctx.store is not None:
-        with remat.record(ctx.store):
+    outer, _remat.rerun = _remat.rerun, True
+    try:
+      with torch.no_grad():
+        if ctx.store is not None:
+          with remat.record(ctx.store):
+            out = fn(*args)
+        else:
           out = fn(*args)
-      else:
-        out = fn(*args)
+    finally:
+      _remat.rerun = outer
     return out
 
   @staticmethod
@@ -569,6 +649,13 @@ def group_norm(x, groups: int, gamma=None, beta=None, eps: float = 1e-6, act: bo
   """GroupNorm over a channels-first tensor [N, C, *spatial] with optional fused SiLU. A 4-D bf16 tensor in
   channels-last memory (what `conv2d` produces) stays in that layout."""
   if _fast(x) and _is_channels_last(x) and x.shape[1] % 8 == 0 and x.shape[1] <= 2048:
+    if _direct(x, gamma, beta):
+      r = _lib.host_ops().group_norm_cl(x, groups, gamma, beta, eps, act)
+      if r is not NotImplemented:
+        return r
+      N, C, H, W = x.shape
+      y3 = OC.group_norm_cl_fwd(x.permute(0, 2, 3, 1).view(N, H * W, C), groups, gamma, beta, eps, act)[0]
+      return y3.view(N, H, W, C).permute(0, 3, 1, 2)
     return _GroupNormCLFn.apply(x, gamma, beta, groups, eps, act)
   if x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and not _LIBRARY_MODE:
     x = x if x.is_contiguous() else x.contiguous()
@@ -597,24 +684,29 @@ def _packed(weight: torch.Tensor, bias, kind: str, make):
   return hit[1]
 
 
+def _conv2d_fwd(x, weight, bias, stride, pad, upsample):
+  """(output NCHW in channels-last memory, the input as a dense [N, H, W, C])."""
+  xc = x.contiguous(memory_format=torch.channels_last).permute(0, 2, 3, 1)
+  if upsample:
+    pk = _packed(weight, bias, "up", lambda: OC.pack_upsample_conv2d(weight.detach(), None if bias is None else bias.detach()))
+    y = OC.upsample2x_conv2d(OC.pad_channels(xc, pk.c_in), pk)
+  else:
+    pk = _packed(weight, bias, f"s{stride}p{pad}", lambda: OC.pack_conv2d(weight.detach(), None if bias is None else bias.detach(),
+                                                                         stride=stride, pad_top_left=pad))
+    y = OC.conv2d(OC.pad_channels(xc, pk.c_in), pk)
+  return y.permute(0, 3, 1, 2), xc
+
+
 class _Conv2dFn(torch.autograd.Function):
   """3x3 convolution, stride 1 or 2, optionally preceded by a nearest-2x up-sampling (fused), on channels-last memory.
   Forward and input gradient run on the implicit-GEMM kernel; the weight gradient on `ops.conv.conv2d_wgrad`."""
 
   @staticmethod
   def forward(ctx, x, weight, bias, stride, pad, upsample):
-    N, C, H, W = x.shape
-    xc = x.contiguous(memory_format=torch.channels_last).permute(0, 2, 3, 1)  # [N, H, W, C], dense
-    if upsample:
-      pk = _packed(weight, bias, "up", lambda: OC.pack_upsample_conv2d(weight.detach(), None if bias is None else bias.detach()))
-      y = OC.upsample2x_conv2d(OC.pad_channels(xc, pk.c_in), pk)
-    else:
-      pk = _packed(weight, bias, f"s{stride}p{pad}", lambda: OC.pack_conv2d(weight.detach(), None if bias is None else bias.detach(),
-                                                                           stride=stride, pad_top_left=pad))
-      y = OC.conv2d(OC.pad_channels(xc, pk.c_in), pk)
+    y, xc = _conv2d_fwd(x, weight, bias, stride, pad, upsample)
     ctx.save_for_backward(xc, weight)
     ctx.cfg = (stride, pad, upsample, bias is not None)
-    return y.permute(0, 3, 1, 2)
+    return y
 
   @staticmethod
   def backward(ctx, dy):
@@ -663,6 +755,8 @@ def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = Fa
       ((stride == 1 and pad_tl == 1) or (stride == 2 and pad_tl in (0, 1)))):
     if weight.dtype != torch.bfloat16:
       weight = weight.to(torch.bfloat16)
+    if _direct(x, weight, bias):
+      return _conv2d_fwd(x, weight, bias, stride, pad_tl, upsample)[0]
     return _Conv2dFn.apply(x, weight, bias, stride, pad_tl, upsample)
   if upsample:
     x = F.interpolate(x, scale_factor=2.0, mode="nearest")

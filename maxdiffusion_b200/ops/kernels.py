@@ -78,6 +78,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          split_k: int = 0):
   """D[M,N] = epi(alpha * A·Bᵀ + bias) on the tcgen05 GEMM. A: [M,K] (or [K,M] if a_mn); B: [N,K] (or [K,N]).
   `split_k`: 0 = chosen by `gemm_plan`, 1 = never, n = that many ranges (plain products: no bias / epilogue)."""
+  host = _lib.host_ops()
+  if host is not None and out_dtype in (torch.bfloat16, torch.float32):
+    r = host.gemm(a, b, bool(a_mn), bool(b_mn), bias, _EPI[epi], residual, gate, rows_per_batch, out, out_dtype is torch.float32, alpha,
+                  split_k, _FORCE_TILE_N, _FORCE_CTAS)
+    if r is not NotImplemented:
+      return r
   assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
   a, b = _rowmajor(a), _rowmajor(b)
   K, M = (a.shape if a_mn else a.shape[::-1])
