@@ -16,6 +16,10 @@
 //     parity * C + channel) and the box stays dense;
 //   * nearest-2x upsample + 3x3 conv: four output-parity classes, each a 2x2 convolution of the LOW resolution
 //     input with pre-summed weights (2.25x fewer FLOPs than up-sampling first), written with stride 2.
+// Neighbouring taps along the width read almost the same positions. When a tile is 128 positions of one row (`group` taps
+// wide), the row is fetched once with the spare columns of all of them, and tap j's operand starts j rows (128 bytes each)
+// further in shared memory: the fetched positions of a 3x3 kernel fall to a third. 96 -> 96 channels at 4 x 480 x 832: 22 KB
+// per 192 tensor clocks become 11.7 KB, 943 us become 678 us.
 // Roles per CTA (persistent): warp 0 TMA producer, warp 1 TMEM owner + MMA issuer, warps 2..5 epilogue
 // (bias, SiLU, residual add, ragged-edge masking). Accumulators are double buffered in TMEM.
 //
@@ -40,7 +44,6 @@ namespace conv {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
 constexpr int NUM_THREADS = 192;
 constexpr int MAX_STAGES = 6;
 constexpr int MAX_TAPS = 36;      // 27 (3x3x3) or 4 classes x 9
@@ -68,7 +71,9 @@ struct Params {
   int N;                         // output channels, multiple of 8
   int BN;                        // tile width: multiple of 16, <= 256
   int stages;
-  int ups;                       // (tap, channel block) units per pipeline stage: 1 or 2
+  int ups;                       // (tap group, channel block) units per pipeline stage: 1 or 2
+  int group;                     // taps that share a fetched row: 1, 2 or 3 (more than 1 only with boxes of one row)
+  int a_bytes;                   // shared memory of a unit's positions: (128 + group - 1) rows, a multiple of 1024
   int acc_cols;                  // TMEM columns per accumulator: 128 or 256
   int alt_dim, alt_shift, has_alt;  // a tap whose coordinate along alt_dim is negative reads the second map at +alt_shift
   long long os1, os2, os3, os4;  // output strides (elements) along dims 1..4
@@ -77,6 +82,7 @@ struct Params {
   const __nv_bfloat16* bias;      // [N] or nullptr
   const __nv_bfloat16* residual;  // addressed like out, or nullptr
   int epi;
+  int tap_step;                   // K index distance of the taps of a group
   int splits;                     // > 1: fp32 partials [splits][class, M-tile, 128 positions][N] instead of the output
   float* partial;
   DeviceStatus* status;
@@ -156,7 +162,9 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int STAGES = p.stages;
   const int B_BYTES = p.BN / CG * BK * 2;     // this CTA's share of the weights
-  const int UNIT_BYTES = A_BYTES + B_BYTES;   // a multiple of 1024: BN / CG is a multiple of 8
+  const int GROUP = p.group;
+  const int UNIT_BYTES = p.a_bytes + GROUP * B_BYTES;  // a multiple of 1024: BN / CG is a multiple of 8
+  const int UNIT_TX = (BM + GROUP - 1) * 128 + GROUP * B_BYTES;  // bytes that a unit's copies deliver
   const int STAGE_BYTES = p.ups * UNIT_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* full_bar = bars;                          // [MAX_STAGES]; of a pair: only the even CTA's are used
@@ -221,15 +229,15 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const TileCoord tc = decode_tile<CG>(work - split * num_tiles, rank, p, nt1, nt2, nt3, num_mt, num_n);
         const int n0 = tc.n_idx * p.BN + rank * (p.BN / CG);
         const int t0 = p.tap_begin[tc.cls];
-        const int all_units = (p.tap_begin[tc.cls + 1] - t0) * num_kb;
+        const int all_units = (p.tap_begin[tc.cls + 1] - t0) / GROUP * num_kb;
         const int u_begin = unit_cut(split, p.splits, all_units), n_units = unit_cut(split + 1, p.splits, all_units);
-        int ti = t0 + u_begin / num_kb, kb = u_begin % num_kb;
+        int ti = t0 + u_begin / num_kb * GROUP, kb = u_begin % num_kb;
         Tap tap = p.taps[min(ti, MAX_TAPS - 1)];
         for (int u0 = u_begin; u0 < n_units && ok; u0 += p.ups) {
           const int nu = min(p.ups, n_units - u0);
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, p.status, 110)) { ok = false; break; }
           // both CTAs' copies complete on the even CTA's barrier, which expects the bytes of both
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], CG * nu * UNIT_BYTES);
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], CG * nu * UNIT_TX);
           const uint32_t pair_bar = CG == 2 ? cluster_map(&full_bar[stage], 0) : 0u;
           uint8_t* sa = smem + stage * STAGE_BYTES;
           for (int j = 0; j < nu; ++j, sa += UNIT_BYTES) {
@@ -242,14 +250,16 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             }
             if (CG == 2) {
               tma_load_5d_pair(sa, map, pair_bar, tap.o0 + kb * BK, c1, c2, c3, c4);
-              tma_load_2d_pair(sa + A_BYTES, &tmap_w, pair_bar, tap.koff + kb * BK, n0);
+              for (int g = 0; g < GROUP; ++g)
+                tma_load_2d_pair(sa + p.a_bytes + g * B_BYTES, &tmap_w, pair_bar, tap.koff + g * p.tap_step + kb * BK, n0);
             } else {
               tma_load_5d(sa, map, &full_bar[stage], tap.o0 + kb * BK, c1, c2, c3, c4);
-              tma_load_2d(sa + A_BYTES, &tmap_w, &full_bar[stage], tap.koff + kb * BK, n0);
+              for (int g = 0; g < GROUP; ++g)
+                tma_load_2d(sa + p.a_bytes + g * B_BYTES, &tmap_w, &full_bar[stage], tap.koff + g * p.tap_step + kb * BK, n0);
             }
             if (++kb == num_kb) {
               kb = 0;
-              ++ti;
+              ti += GROUP;
               if (ti < p.tap_begin[tc.cls + 1]) tap = p.taps[ti];
             }
           }
@@ -280,7 +290,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       for (int work = group_id; work < num_work && ok; work += num_groups, ++it) {
         const int split = work / num_tiles;
         const int cls = (work - split * num_tiles) / (num_tiles / p.n_classes);
-        const int n_taps = p.tap_begin[cls + 1] - p.tap_begin[cls];
+        const int n_taps = (p.tap_begin[cls + 1] - p.tap_begin[cls]) / GROUP;
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1u;
         if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 120)) { ok = false; break; }
@@ -297,28 +307,31 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
           tc_fence_after_sync();
           uint32_t sa = smem_u32(smem + stage * STAGE_BYTES);
           for (int j = 0; j < nu; ++j, sa += UNIT_BYTES) {
-            const uint64_t da = make_smem_desc(sa, 16, 1024);
-            const uint64_t db = make_smem_desc(sa + A_BYTES, 16, 1024);
             const bool last = (kb + 1 == num_kb);
-            // one K step (16 bf16 = 32 bytes) advances the descriptors' address field (units of 16 bytes) by 2
-            if (CG == 2) {
-              if (!last || last_ksteps == BK / 16) {
-                umma_ss_pair(d_tmem, da, db, idesc, accumulate);
-                umma_ss_pair(d_tmem, da + 2, db + 2, idesc, 1u);
-                umma_ss_pair(d_tmem, da + 4, db + 4, idesc, 1u);
-                umma_ss_pair(d_tmem, da + 6, db + 6, idesc, 1u);
+            for (int g = 0; g < GROUP; ++g) {
+              // the 128-byte swizzle follows the address, so an operand may start at any row of the fetched tile
+              const uint64_t da = make_smem_desc(sa + g * 128, 16, 1024);
+              const uint64_t db = make_smem_desc(sa + p.a_bytes + g * B_BYTES, 16, 1024);
+              // one K step (16 bf16 = 32 bytes) advances the descriptors' address field (units of 16 bytes) by 2
+              if (CG == 2) {
+                if (!last || last_ksteps == BK / 16) {
+                  umma_ss_pair(d_tmem, da, db, idesc, accumulate);
+                  umma_ss_pair(d_tmem, da + 2, db + 2, idesc, 1u);
+                  umma_ss_pair(d_tmem, da + 4, db + 4, idesc, 1u);
+                  umma_ss_pair(d_tmem, da + 6, db + 6, idesc, 1u);
+                } else {
+                  for (int k = 0; k < last_ksteps; ++k) umma_ss_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, k ? 1u : accumulate);
+                }
+              } else if (!last || last_ksteps == BK / 16) {
+                umma_ss(d_tmem, da, db, idesc, accumulate);
+                umma_ss(d_tmem, da + 2, db + 2, idesc, 1u);
+                umma_ss(d_tmem, da + 4, db + 4, idesc, 1u);
+                umma_ss(d_tmem, da + 6, db + 6, idesc, 1u);
               } else {
-                for (int k = 0; k < last_ksteps; ++k) umma_ss_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, k ? 1u : accumulate);
+                for (int k = 0; k < last_ksteps; ++k) umma_ss(d_tmem, da + 2 * k, db + 2 * k, idesc, k ? 1u : accumulate);
               }
-            } else if (!last || last_ksteps == BK / 16) {
-              umma_ss(d_tmem, da, db, idesc, accumulate);
-              umma_ss(d_tmem, da + 2, db + 2, idesc, 1u);
-              umma_ss(d_tmem, da + 4, db + 4, idesc, 1u);
-              umma_ss(d_tmem, da + 6, db + 6, idesc, 1u);
-            } else {
-              for (int k = 0; k < last_ksteps; ++k) umma_ss(d_tmem, da + 2 * k, db + 2 * k, idesc, k ? 1u : accumulate);
+              accumulate = 1u;
             }
-            accumulate = 1u;
             kb = last ? 0 : kb + 1;
           }
           if (CG == 2) umma_commit_pair(&empty_bar[stage]);
@@ -463,6 +476,7 @@ extern "C" int mdb_conv_igemm_tune(int ups, int stages, int ctas_per_sm) {
 //   box       : tile extents along dims 1..3 (product 128);  ext: output positions along dims 1..4
 //   taps      : n_taps_total x 6 ints (o0, o1, o2, o3, o4, koff);  tap_begin: n_classes + 1 ints
 //   out_strides (dims 1..4, elements), class_off (n_classes): where output position (p1..p4) of a class goes
+//   group: taps that share a fetched row (consecutive in the table, one step along dim 1 apart; box[0] = 128)
 //   ctas_per_tile (1 / 2), max_bn (widest tile), splits: the launch shape (`ops/conv.py: conv_plan`); with splits > 1
 //   `partial` holds splits * n_classes * M-tiles * 128 * N fp32 values
 // All channel counts and strides must keep 16-byte alignment (multiples of 8 elements); C a multiple of 16.
@@ -471,7 +485,8 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
                               const long long* alt_dims, const long long* alt_strides, const int* box, const int* ext,
                               int C, int N, long long k_total, int n_classes, const int* tap_begin, const int* taps,
                               int alt_dim, int alt_shift, const long long* out_strides, const long long* class_off,
-                              int epi, int ctas_per_tile, int max_bn, int splits, void* partial, void* stream_ptr) {
+                              int epi, int ctas_per_tile, int max_bn, int splits, void* partial, int group,
+                              void* stream_ptr) {
   using namespace mdb;
   using namespace mdb::conv;
   if (n_classes < 1 || n_classes > MAX_CLASSES) return 3601;
@@ -503,6 +518,18 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
     p.taps[i].koff = t[5];
     if (t[5] & 7) return 3606;
   }
+  if (group < 1 || group > 3 || (group > 1 && (box[0] != BM || n_taps % group))) return 3604;
+  p.group = group;
+  p.tap_step = group > 1 ? taps[6 + 5] - taps[5] : 0;
+  for (int c = 0; c < n_classes; ++c) {
+    if ((tap_begin[c + 1] - tap_begin[c]) % group) return 3604;
+  }
+  for (int i = 0; i < n_taps; ++i) {  // a group: the same position but for one step along dim 1 per tap, K ranges in line
+    const int *t = taps + 6 * i, *f = taps + 6 * (i - i % group);
+    const int g = i % group;
+    if (t[0] != f[0] || t[1] != f[1] + g || t[2] != f[2] || t[3] != f[3] || t[4] != f[4] || t[5] != f[5] + g * p.tap_step) return 3604;
+  }
+  p.a_bytes = ((BM + group - 1) * 128 + 1023) / 1024 * 1024;
   p.box1 = box[0]; p.box2 = box[1]; p.box3 = box[2];
   p.ext1 = ext[0]; p.ext2 = ext[1]; p.ext3 = ext[2]; p.ext4 = ext[3];
   p.C = C; p.N = N;
@@ -512,17 +539,22 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
   p.splits = splits;
   p.partial = static_cast<float*>(partial);
   for (int c = 0; c < n_classes; ++c) {
-    if (splits > (tap_begin[c + 1] - tap_begin[c]) * ((C + BK - 1) / BK)) return 3608;  // every split has a unit
+    if (splits > (tap_begin[c + 1] - tap_begin[c]) / group * ((C + BK - 1) / BK)) return 3608;  // every split has a unit
   }
-  const int unit_bytes = A_BYTES + p.BN / cg * BK * 2;
-  int ctas_per_sm = p.BN <= 128 ? 2 : 1;
-  if (g_tune_ctas > 0) ctas_per_sm = (g_tune_ctas == 2 && p.BN <= 128) ? 2 : 1;
+  const int unit_bytes = p.a_bytes + group * (p.BN / cg * BK * 2);
+  constexpr int kHalfSm = 112 * 1024 - 1024 - 256;
+  int ctas_per_sm = p.BN <= 128 && 2 * unit_bytes <= kHalfSm ? 2 : 1;  // two stages each
+  if (g_tune_ctas > 0) ctas_per_sm = (g_tune_ctas == 2 && p.BN <= 128 && 2 * unit_bytes <= kHalfSm) ? 2 : 1;
   p.acc_cols = ctas_per_sm == 2 ? 128 : 256;
-  const int budget = (ctas_per_sm == 2 ? 112 : 226) * 1024 - 1024 - 256;
-  p.ups = g_tune_ups > 0 ? g_tune_ups : (ctas_per_sm == 2 ? 1 : (p.BN <= 128 ? 2 : 1));
+  const int budget = ctas_per_sm == 2 ? kHalfSm : 226 * 1024 - 1024 - 256;
+  p.ups = g_tune_ups > 0 ? g_tune_ups : (ctas_per_sm == 2 ? 1 : (p.BN <= 128 && group == 1 ? 2 : 1));
   if (p.ups < 1 || p.ups > 2) return 3608;
   p.stages = budget / (p.ups * unit_bytes);
   if (g_tune_stages > 0 && g_tune_stages < p.stages) p.stages = g_tune_stages;
+  if (p.stages < 2 && p.ups == 2) {  // two units a stage were asked for and do not fit twice
+    p.ups = 1;
+    p.stages = budget / unit_bytes;
+  }
   if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
   if (p.stages < 2) return 3608;
   p.alt_dim = alt_dim; p.alt_shift = alt_shift; p.has_alt = (x_alt != nullptr && alt_dim >= 2 && alt_dim <= 3) ? 1 : 0;
@@ -536,7 +568,7 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
   CUtensorMap tx, talt, tw;
   {
     uint64_t d[5], s[4];
-    uint32_t b[5] = {BK, static_cast<uint32_t>(box[0]), static_cast<uint32_t>(box[1]), static_cast<uint32_t>(box[2]), 1};
+    uint32_t b[5] = {BK, static_cast<uint32_t>(box[0] + group - 1), static_cast<uint32_t>(box[1]), static_cast<uint32_t>(box[2]), 1};
     for (int i = 0; i < 5; ++i) d[i] = static_cast<uint64_t>(dims[i]);
     for (int i = 0; i < 4; ++i) s[i] = static_cast<uint64_t>(strides[i]) * 2;
     int rc = encode_tmap_bf16(&tx, x, 5, d, s, b);

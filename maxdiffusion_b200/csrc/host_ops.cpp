@@ -41,7 +41,7 @@ int mdb_gn_cl_apply(const void*, const void*, void*, const float*, const float*,
                     int, int, int, void*);
 int mdb_conv_igemm(const void*, const void*, const void*, void*, const void*, const void*, const long long*, const long long*,
                    const long long*, const long long*, const int*, const int*, int, int, long long, int, const int*, const int*,
-                   int, int, const long long*, const long long*, int, int, int, int, void*, void*);
+                   int, int, const long long*, const long long*, int, int, int, int, void*, int, void*);
 }
 
 namespace {
@@ -378,11 +378,11 @@ bool ints(PyObject* o, T* out, Py_ssize_t n) {
 }
 
 // conv(x, x_alt, w, out, bias, residual, dims, strides, alt_dims, alt_strides, box, ext, c_in, n_pad, taps, begin, alt_dim,
-//      alt_shift, out_strides, class_off, silu, ctas, max_bn, splits, m_tiles): the arguments of `ops.conv._launch`, shapes as
+//      alt_shift, out_strides, class_off, silu, ctas, max_bn, splits, m_tiles, group): the arguments of `ops.conv._launch`, shapes as
 // tuples, taps and begin as the addresses of int arrays. Returns `out`.
 PyObject* py_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 25 || !THPVariable_Check(a[0]) || !THPVariable_Check(a[2]) || !THPVariable_Check(a[3])) return not_implemented();
+  if (n != 26 || !THPVariable_Check(a[0]) || !THPVariable_Check(a[2]) || !THPVariable_Check(a[3])) return not_implemented();
   const Tensor &x = THPVariable_Unpack(a[0]), &w = THPVariable_Unpack(a[2]), &out = THPVariable_Unpack(a[3]);
   const Tensor *alt, *bias, *residual;
   if (!opt_tensor(a[1], alt) || !opt_tensor(a[4], bias) || !opt_tensor(a[5], residual)) return not_implemented();
@@ -400,13 +400,14 @@ PyObject* py_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int silu = static_cast<int>(PyLong_AsLong(a[20])), ctas = static_cast<int>(PyLong_AsLong(a[21]));
   const int max_bn = static_cast<int>(PyLong_AsLong(a[22])), splits = static_cast<int>(PyLong_AsLong(a[23]));
   const int64_t m_tiles = PyLong_AsLongLong(a[24]);
+  const int group = static_cast<int>(PyLong_AsLong(a[25]));
   if (PyErr_Occurred()) return nullptr;
   Tensor partial;
   if (splits > 1) partial = at::empty({splits * static_cast<int64_t>(classes) * m_tiles * 128 * n_pad}, out.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous));
   const int rc = mdb_conv_igemm(x.data_ptr(), data(alt), w.data_ptr(), out.data_ptr(), data(bias), data(residual), dims, strides,
                                 alt_dims, alt_strides, box, ext, c_in, n_pad, w.size(1), static_cast<int>(classes), begin, taps,
                                 alt_dim, alt_shift, os, class_off, silu, ctas, max_bn, splits,
-                                splits > 1 ? partial.data_ptr() : nullptr, stream());
+                                splits > 1 ? partial.data_ptr() : nullptr, group, stream());
   return done(rc, "mdb_conv_igemm", out);
   END_HANDLE_TH_ERRORS
 }

@@ -33,7 +33,7 @@ def _declare(L):
   c_void_p, c_int, c_ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
   llp, ip = ctypes.POINTER(c_ll), ctypes.POINTER(c_int)
   L.mdb_conv_igemm.argtypes = [c_void_p] * 6 + [llp] * 4 + [ip, ip, c_int, c_int, c_ll, c_int, ip, ip, c_int, c_int,
-                                                           llp, llp, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
+                                                           llp, llp, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]
   L.mdb_conv_igemm.restype = c_int
   L.mdb_rms_act_cl.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_ll, c_int, ctypes.c_float, c_int,
                                c_int, c_int, c_void_p]
@@ -89,6 +89,18 @@ class PackedConv:
   src: tuple = ()                 # (weight, bias, stride, pad_top_left) as given: what the PyTorch reference path runs
 
   _tap_cache: dict = field(default_factory=dict, repr=False)
+
+  def row_group(self) -> int:
+    """How many consecutive taps step along the width by one position each (they can share a fetched row): 2, 3 or 1."""
+    hit = self._tap_cache.get("group")
+    if hit is None:
+      hit = 1
+      for g in (3, 2):
+        if all(len(cls) % g == 0 and all((t[0], t[1] - i % g, *t[2:]) == cls[i - i % g] for i, t in enumerate(cls)) for cls in self.taps):
+          hit = g
+          break
+      self._tap_cache["group"] = hit
+    return hit
 
   def tap_arrays(self, shift1: int = 0):
     """ctypes arrays of the tap table; `shift1` is added to every tap's offset along dim 1 (the width): an input
@@ -186,9 +198,9 @@ def pack_conv2d_dgrad(weight: torch.Tensor, stride: int = 1, pad_top_left: Optio
   p = kh // 2 if pad_top_left is None else pad_top_left
   wt = weight.permute(1, 2, 3, 0)  # [Ci, kh, kw, Co]
   if stride == 1:
-    # dX[i] = sum_a dY[i + p - a] W[a]
-    taps = [[(0, p - b, p - a, 0, 0) for a in range(kh) for b in range(kw)]]
-    pk = _pack(wt.reshape(ci, kh * kw, co), None, taps, "conv2d_dgrad_s1")
+    # dX[i] = sum_a dY[i + p - a] W[a], the taps in the order of rising positions (neighbours can share a fetched row)
+    taps = [[(0, b - (kw - 1 - p), a - (kh - 1 - p), 0, 0) for a in range(kh) for b in range(kw)]]
+    pk = _pack(wt.flip(1, 2).reshape(ci, kh * kw, co), None, taps, "conv2d_dgrad_s1")
     pk.src = (weight, None, 1, p)
     return pk
   assert stride == 2
@@ -238,9 +250,10 @@ def _tile_width(n: int, most: int, step: int) -> int:
 
 
 @functools.lru_cache(maxsize=4096)
-def conv_plan(m_tiles: int, n_classes: int, n: int, units: int, sms: int = 148) -> tuple:
+def conv_plan(m_tiles: int, n_classes: int, n: int, units: int, group: int = 1, sms: int = 148) -> tuple:
   """(CTAs per tile, widest tile, splits) with the least modelled time of an implicit-GEMM convolution: `m_tiles` boxes of
-  128 positions per class, `n` output channels, `units` (tap, 64-channel block) steps per tile.
+  128 positions per class, `n` output channels, `units` (tap, 64-channel block) steps per tile, `group` taps that share a
+  fetched row.
 
   A step costs its operand feed: 16 KB of positions and 128 bytes per output channel, the latter shared by a pair. Measured
   on a B200, one CTA against a pair: 96 -> 96 channels at 4 x 480 x 832 1021 / 918 us, 384 -> 384 at 2 x 120 x 208 338 / 277
@@ -248,8 +261,9 @@ def conv_plan(m_tiles: int, n_classes: int, n: int, units: int, sms: int = 148) 
   tiles leave SMs idle: cutting the contraction pays for its fp32 partials (2 x 8 x 8 x 1280 -> 1280: 61 us whole, 18 us in
   12 parts; 2 x 16 x 16 x 2560 -> 1280: 135 / 38 us in 6)."""
   best, best_cost = (1, 256, 1), None
+  units //= group
   for cg in (1, 2):
-    if cg == 2 and (m_tiles < 2 or units < 24):
+    if cg == 2 and (m_tiles < 2 or units * group < 24):
       continue
     seen = set()
     for most in (256, 128, 64):
@@ -257,8 +271,13 @@ def conv_plan(m_tiles: int, n_classes: int, n: int, units: int, sms: int = 148) 
       if bn in seen:
         continue
       seen.add(bn)
+      if group > 1 and 17408 + group * 128 * bn // cg > 112 * 1024:  # two stages do not fit
+        continue
       one = (0.23 + 0.00055 * bn) if cg == 1 else (0.19 + 0.00058 * bn)  # microseconds per step, one CTA on the SM
       two = (0.26 + 0.002 * bn) if cg == 1 else (0.30 + 0.001 * bn)      # of each of two CTAs that share the SM
+      if group > 1:  # of a step of `group` taps: the row once, the weights of every tap; or the products
+        feed, mma = (16640 + group * 128 * bn / cg) / 105e3, group * bn * 0.0014
+        one, two = max(feed, mma) + 0.02, max(1.85 * feed, 2 * mma) + 0.1
       tiles = n_classes * -(-m_tiles // cg) * -(-n // bn)
       slots = sms // cg
       for s in range(1, 25 if tiles * 2 <= slots * 2 else 2):
@@ -284,22 +303,40 @@ def _carray(T, values: tuple):
   return (T * len(values))(*[int(v) for v in values])
 
 
+def _tile_box(pk: PackedConv, e1: int, e2: int, e3: int, allow3: bool) -> tuple:
+  """The box of least padding, or 128 positions of one row, which neighbouring taps can share (`_launch`), where the row's
+  padding costs less than the sharing saves. Measured on a B200 with pairs, box / row: 96 -> 96 channels at 4 x 480 x 832 943
+  / 678 us, 192 -> 192 at 4 x 200 x 360 573 / 373 us, 320 -> 320 at 4 x 128 x 128 139 / 79 us, 96 -> 3 at 4 x 480 x 832 835 /
+  410 us: at least a quarter of the time (an eighth from 256 channels up, whose feed is mostly weights: 384 -> 384 at 208
+  columns 277 / 290 us, at 104 columns 71 / 52 us), a half for a handful of channels. Up-sampling (two taps) saves a tenth."""
+  box, group = _pick_box(e1, e2, e3, allow3), pk.row_group()
+  if group > 1 and _ROWS:
+    cost = _round_up(e1, box[0]) * _round_up(e2, box[1]) * _round_up(e3, box[2])
+    if _round_up(e1, 128) * e2 * e3 <= cost * (1.08 if group == 2 else 1.6 if pk.n_pad <= 32 else 1.25 if pk.n_pad < 256 else 1.16):
+      return 128, 1, 1
+  return box
+
+
+_ROWS = True  # False: never share fetched rows (benchmarks, tests)
+
+
 def _launch(x, x_alt, pk: PackedConv, dims, strides, alt_dims, alt_strides, box, ext, out, out_strides, class_off,
             residual, silu, alt_dim=-1, alt_shift=0, tap_shift1=0):
   taps, begin, n_classes = pk.tap_arrays(tap_shift1)
   LL, I = ctypes.c_longlong, ctypes.c_int
   arr = lambda T, v: _carray(T, tuple(v))
+  group = pk.row_group() if box[0] == 128 and _ROWS else 1  # taps that share a fetched row
   m_tiles = ext[3]
   for e, b in zip(ext[:3], box):
     m_tiles *= -(-e // b)
-  ctas, max_bn, splits = _PLAN or conv_plan(m_tiles, n_classes, pk.n_pad, -(-pk.c_in // 64) * min(len(c) for c in pk.taps))
+  ctas, max_bn, splits = _PLAN or conv_plan(m_tiles, n_classes, pk.n_pad, -(-pk.c_in // 64) * min(len(c) for c in pk.taps), group)
   host = _lib.host_ops()
   if host is not None:
     dims, strides, box, ext = tuple(dims), tuple(strides), tuple(box), tuple(ext)
     r = host.conv(x, x_alt, pk.w, out, pk.bias, residual, dims, strides, tuple(alt_dims) if alt_dims else dims,
                   tuple(alt_strides) if alt_strides else strides, box, ext, pk.c_in, pk.n_pad, ctypes.addressof(taps),
                   ctypes.addressof(begin), alt_dim, alt_shift, tuple(out_strides), tuple(class_off), 1 if silu else 0, ctas,
-                  max_bn, splits, m_tiles)
+                  max_bn, splits, m_tiles, group)
     if r is not NotImplemented:
       return out
   partial = None
@@ -309,7 +346,7 @@ def _launch(x, x_alt, pk: PackedConv, dims, strides, alt_dims, alt_strides, box,
       _lib.ptr(x), _lib.ptr(x_alt), _lib.ptr(pk.w), _lib.ptr(out), _lib.ptr(pk.bias), _lib.ptr(residual),
       arr(LL, dims), arr(LL, strides), arr(LL, alt_dims if alt_dims else dims), arr(LL, alt_strides if alt_strides else strides),
       arr(I, box), arr(I, ext), pk.c_in, pk.n_pad, pk.w.shape[1], n_classes, begin, taps, alt_dim, alt_shift,
-      arr(LL, out_strides), arr(LL, class_off), 1 if silu else 0, ctas, max_bn, splits, _lib.ptr(partial), _lib.stream())
+      arr(LL, out_strides), arr(LL, class_off), 1 if silu else 0, ctas, max_bn, splits, _lib.ptr(partial), group, _lib.stream())
   _lib.check(rc, "mdb_conv_igemm")
   return out
 
@@ -351,7 +388,7 @@ def conv3d_causal(x: torch.Tensor, pk: PackedConv, hist: Optional[torch.Tensor] 
   else:
     assert out.shape == (B, T, H, W, pk.n_pad) and out.stride(-1) == 1 and out.dtype == x.dtype
     assert all(s % 8 == 0 for s in out.stride()[:-1]) and residual is None
-  b1, b2, _ = _pick_box(W, H, 1, False)
+  b1, b2, _ = _tile_box(pk, W, H, 1, False)
   alt_dims = alt_strides = None
   if hist is not None:
     _check_cl(hist, pk.c_in)
@@ -376,7 +413,7 @@ def conv2d(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = N
   n = pk.n_pad
   if pk.kind in ("conv2d", "conv2d_dgrad_s1"):
     out = torch.empty((B, H, W, n), dtype=x.dtype, device=x.device)
-    box = _pick_box(W, H, B, True)
+    box = _tile_box(pk, W, H, B, True)
     dims, strides = [C, W, H, B, 1], [x.stride(2), x.stride(1), x.stride(0), x.stride(0) * B]
     ext, os_ = [W, H, B, 1], [n, W * n, H * W * n, B * H * W * n]
   elif pk.kind == "conv2d_s2":
@@ -404,7 +441,7 @@ def _parity_conv(x, pk, silu=False, halo: int = 0):
   W = Win - 2 * halo
   n = pk.n_pad
   out = torch.empty((B, 2 * H, 2 * W, n), dtype=x.dtype, device=x.device)
-  box = _pick_box(W, H, B, True)
+  box = _tile_box(pk, W, H, B, True)
   class_off = [rh * 2 * W * n + rw * n for rh in (0, 1) for rw in (0, 1)]
   _launch(x, None, pk, [C, Win, H, B, 1], [x.stride(2), x.stride(1), x.stride(0), x.stride(0) * B], None, None, box,
           [W, H, B, 1], out, [2 * n, 4 * W * n, 4 * H * W * n, 4 * B * H * W * n], class_off, None, silu, tap_shift1=halo)

@@ -1,0 +1,120 @@
+"""The CPython extension against the Python wrappers: the same kernels on the same launch shapes, so equal bit for bit, over
+the layouts that a caller can hand in (the extension passes on what it does not take)."""
+import pytest
+import torch
+
+from maxdiffusion_b200.ops import _lib, conv as OC, functional as OF, kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+class _Nothing:
+  """Takes nothing: every call goes on to the Python wrappers."""
+
+  def __getattr__(self, name):
+    return lambda *a: NotImplemented
+
+
+def _both(monkeypatch, fn):
+  with torch.no_grad():
+    before = _lib.host_ops().launches()
+    got = fn()
+    used = _lib.host_ops().launches() > before
+    with monkeypatch.context() as m:
+      m.setattr(_lib, "host_ops", lambda: _Nothing())
+      want = fn()
+  assert torch.equal(got, want) and got.shape == want.shape and got.stride() == want.stride() and got.dtype == want.dtype
+  return used
+
+
+def _randn(*shape):
+  return torch.randn(shape, device="cuda").to(torch.bfloat16)
+
+
+_FORMS = {"dense": lambda: _randn(3, 40, 64), "2d": lambda: _randn(17, 64), "4d": lambda: _randn(2, 3, 5, 64),
+          "slice of channels": lambda: _randn(3, 40, 192)[..., 64:128], "part of a sequence": lambda: _randn(3, 50, 64)[:, 5:45],
+          "transposed": lambda: _randn(40, 3, 64).transpose(0, 1), "every second row": lambda: _randn(3, 80, 64)[:, ::2],
+          "expanded": lambda: _randn(1, 40, 64).expand(3, 40, 64), "one row": lambda: _randn(1, 1, 64),
+          "columns apart": lambda: _randn(3, 40, 128)[..., ::2]}
+
+
+@pytest.mark.parametrize("form", list(_FORMS))
+@pytest.mark.parametrize("act", [None, "gelu_tanh", "silu", "residual"])
+def test_linear(monkeypatch, form, act):
+  torch.manual_seed(0)
+  x, w, b = _FORMS[form](), _randn(72, 64), _randn(72)
+  res = _randn(*x.shape[:-1], 72) if act == "residual" else None
+  used = _both(monkeypatch, lambda: OF.linear(x, w, b, None if res is not None else act, residual=res))
+  assert used or form in ("transposed", "part of a sequence", "expanded", "columns apart")
+  _both(monkeypatch, lambda: OF.linear(x, w[::2], None))  # a strided weight
+  if res is not None:
+    _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.transpose(0, 1).contiguous().transpose(0, 1)))
+    _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.float()))
+
+
+@pytest.mark.parametrize("D", [8, 40, 64, 80, 128])
+def test_attention(monkeypatch, D):
+  torch.manual_seed(1)
+  q, k, v = _randn(2, 70, 3, D), _randn(2, 90, 3, D), _randn(2, 90, 3, D)
+  assert _both(monkeypatch, lambda: OF.attention(q, k, v))
+  fused = _randn(2, 70, 3, 3, D)
+  assert _both(monkeypatch, lambda: OF.attention(fused[:, :, 0], fused[:, :, 1], fused[:, :, 2], scale=0.3))
+  _both(monkeypatch, lambda: OF.attention(q.transpose(1, 2).contiguous().transpose(1, 2), [k, k], [v, v]))
+  if D in K.FLASH_HEAD_DIMS:
+    return  # there the kernel itself refuses strides that TMA cannot take
+  wide = _randn(2, 70, 3, D + 4)
+  _both(monkeypatch, lambda: OF.attention(wide[..., :D], wide[..., :D], wide[..., :D]))  # copied
+
+
+def test_norms_and_gates(monkeypatch):
+  torch.manual_seed(2)
+  for C in (64, 640, 1280, 3072):
+    x, g, b = _randn(2, 33, C), _randn(C), _randn(C)
+    s = torch.randn(2, 3 * C, device="cuda")
+    assert _both(monkeypatch, lambda: OF.layer_norm_mod(x, g, b))
+    assert _both(monkeypatch, lambda: OF.layer_norm_mod(x, scale=s[:, :C], shift=s[:, C:2 * C]))
+    _both(monkeypatch, lambda: OF.layer_norm_mod(x, scale=s[:, :C].to(torch.bfloat16), shift=s[:, C:2 * C]))
+    _both(monkeypatch, lambda: OF.layer_norm_mod(x.transpose(0, 1), g, b))
+    assert _both(monkeypatch, lambda: OF.geglu(x))
+  qkv, w = _randn(2, 33, 3 * 256), _randn(128)
+  cos, sin = torch.randn(33, 64, device="cuda"), torch.randn(33, 64, device="cuda")
+  assert _both(monkeypatch, lambda: OF.rms_norm_rope(qkv[..., 256:512], w, cos, sin, heads=2, per_head=True))
+  assert _both(monkeypatch, lambda: OF.rms_norm_rope(qkv[..., :256], _randn(256) * 0 + 1, heads=2))
+  two = [(qkv[..., :256], w, cos, sin), (_randn(2, 7, 256), w, cos[:7].contiguous(), sin[:7].contiguous())]
+  joint = torch.cat([OF.rms_norm_rope(x, w, c, s, heads=2, per_head=True) for x, w, c, s in two], dim=1)
+  with torch.no_grad():
+    assert torch.equal(OF.joint_norm_rope(two, 2), joint)
+
+
+@pytest.mark.parametrize("shape", [(2, 64, 8, 8), (1, 320, 17, 5), (3, 96, 1, 9)])
+def test_group_norm_and_conv(monkeypatch, shape):
+  torch.manual_seed(3)
+  C = shape[1]
+  x = _randn(*shape).contiguous(memory_format=torch.channels_last)
+  g, b, w, cb = _randn(C), _randn(C), _randn(48, C, 3, 3) * 0.05, _randn(48)
+  for act in (False, True):
+    _both(monkeypatch, lambda: OF.group_norm(x, 32, g, b, 1e-5, act))
+    _both(monkeypatch, lambda: OF.group_norm(x, 32, g.float(), b.float(), 1e-5, act))
+  _both(monkeypatch, lambda: OF.conv2d(x, w, cb))
+  _both(monkeypatch, lambda: OF.conv2d(x.contiguous(), w, None, upsample=True))
+  clip, hist = _randn(1, 3, 6, 10, C), _randn(1, 2, 6, 10, C)
+  pk = OC.pack_conv3d(_randn(40, C, 3, 3, 3) * 0.05, _randn(40))
+  _both(monkeypatch, lambda: OC.conv3d_causal(clip, pk, hist))
+
+
+def test_direct_calls_leave_autograd_alone():
+  """Everything that works through the autograd functions still goes through them."""
+  x, w = _randn(2, 8, 64), torch.nn.Parameter(_randn(72, 64))
+  assert OF.linear(x, w).requires_grad
+  with torch.no_grad():
+    assert OF._direct(x, w) and not OF._direct(torch.nn.Buffer(x).as_subclass(type("T", (torch.Tensor,), {})))
+    import torch.autograd.forward_ad as fwAD
+    with fwAD.dual_level():
+      assert not OF._direct(x)
+    out = []
+    torch.func.vmap(lambda t: (out.append(OF._direct(t)), t)[1])(x)
+    assert out == [False]
+  store = []
+  y = OF.checkpoint_block(lambda t: (store.append(OF._direct(t)), OF.linear(t, w))[1], x.requires_grad_())
+  y.float().sum().backward()
+  assert store == [False, False] and w.grad is not None
