@@ -216,6 +216,8 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
   if (CG == 2) cluster_sync();  // the partner's barriers are initialised and its TMEM is allocated
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  allow_successor();
+  wait_for_predecessor();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -413,6 +415,8 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 
 // Sum of the partials of a split contraction, in split order, and the epilogue. One thread per 8 channels of a position.
 __global__ void conv_fold_kernel(const __grid_constant__ Params p) {
+  allow_successor();
+  wait_for_predecessor();
   const int nt1 = (p.ext1 + p.box1 - 1) / p.box1, nt2 = (p.ext2 + p.box2 - 1) / p.box2, nt3 = (p.ext3 + p.box3 - 1) / p.box3;
   const int num_mt = p.ext4 * nt3 * nt2 * nt1;
   const int n_vec = p.N / 8;
@@ -605,11 +609,11 @@ extern "C" int mdb_conv_igemm(const void* x, const void* x_alt, const void* w, v
   const long long slots = static_cast<long long>(sm_count()) * ctas_per_sm / cg;
   const int grid = static_cast<int>(work < slots ? work : slots) * cg;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  if (cg == 2) conv_igemm_kernel<2><<<grid, NUM_THREADS, smem, stream>>>(tx, talt, tw, p);
-  else conv_igemm_kernel<1><<<grid, NUM_THREADS, smem, stream>>>(tx, talt, tw, p);
+  MDB_CHECK_CUDA(launch_overlapped(cg == 2 ? conv_igemm_kernel<2> : conv_igemm_kernel<1>, grid, NUM_THREADS, smem, stream, tx, talt,
+                                   tw, p));
   if (splits > 1) {
     const long long vecs = n_classes * m_tiles * BM * (N / 8);
-    conv_fold_kernel<<<static_cast<int>(cdiv(vecs, 128)), 128, 0, stream>>>(p);
+    MDB_CHECK_CUDA(launch_overlapped(conv_fold_kernel, static_cast<int>(cdiv(vecs, 128)), 128, 0, stream, p));
   }
   return static_cast<int>(cudaGetLastError());
 }

@@ -262,6 +262,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int n_copy = cp.n_remote > 0 ? cp.n_copy_ctas : 0;
   const int n_compute = static_cast<int>(gridDim.x) - n_copy;
   if (static_cast<int>(blockIdx.x) >= n_compute) {
+    wait_for_predecessor();
     copy_cta(cp, static_cast<int>(blockIdx.x) - n_compute, p.status);
     return;
   }
@@ -325,6 +326,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  if (n_copy == 0 && p.seg_flags == nullptr) allow_successor();  // a launch that waits for peers keeps the SMs to itself
+  wait_for_predecessor();
   // TMEM columns: S(t, b) = t*128 + b*64 (P aliases it as 32 packed columns), O(t) = 256 + t*128.
 
   if (warp == 0) {
@@ -662,8 +665,7 @@ static int launch_variant(dim3 grid, cudaStream_t st, const CUtensorMap& tq, con
                                         smem_bytes<HD, STAGES>()));
     configured = true;
   }
-  flash_fwd_kernel<HD, STAGES><<<grid, NUM_THREADS, smem_bytes<HD, STAGES>(), st>>>(tq, maps, p, cp);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(mdb::launch_overlapped(flash_fwd_kernel<HD, STAGES>, grid, NUM_THREADS, smem_bytes<HD, STAGES>(), st, tq, maps, p, cp));
 }
 
 // q: [B, q_len, H, 128]; k/v segment s: [B, kv_len[s], H, 128]; out like q. Strides are in elements

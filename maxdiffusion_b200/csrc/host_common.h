@@ -27,6 +27,23 @@ int encode_tmap_f32(CUtensorMap* map, const void* base, int rank, const uint64_t
 
 int sm_count();
 
+// Launch of a kernel that begins with `wait_for_predecessor()`: its set-up (barriers, TMEM, descriptor and instruction
+// fetch) overlaps the end of the kernel before it in the stream.
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace mdb
 
 #define MDB_CHECK_CUDA(expr)                      \

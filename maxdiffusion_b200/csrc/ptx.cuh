@@ -433,6 +433,15 @@ __host__ __device__ constexpr uint32_t make_idesc_i8(int m, int n) {
 }
 
 // ----------------------------------------------------------------------------------------
+// Launch overlap (`launch_overlapped` in host_common.h): a kernel launched that way may start while its predecessor in the
+// stream still runs. It does everything that touches no global memory, then waits until the predecessor has finished and
+// its writes are visible; no read of an input and no write of an output comes before that.
+// ----------------------------------------------------------------------------------------
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the successor's CTAs start (they wait as above) once every CTA of this grid has come here.
+__device__ __forceinline__ void allow_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ----------------------------------------------------------------------------------------
 // Small numeric helpers
 // ----------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

@@ -133,6 +133,8 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y
               const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
               const float* __restrict__ scale, const float* __restrict__ shift, long long mod_ld, int rows_per_batch,
               int C, float eps, float* __restrict__ mean_out, float* __restrict__ rstd_out) {
+  allow_successor();
+  wait_for_predecessor();
   __shared__ float2 red[2][THREADS / 32];
   int parity = 0;
   const Strip s = my_strip(rows_per_batch);
@@ -317,6 +319,8 @@ __global__ void __launch_bounds__(THREADS)
 ln_rows_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                    const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta, int rows_per_batch,
                    int C, float eps, float* __restrict__ mean_out, float* __restrict__ rstd_out) {
+  allow_successor();
+  wait_for_predecessor();
   const Strip s = my_strip(rows_per_batch);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = C >> 3;
   const float inv_c = 1.0f / C;
@@ -503,6 +507,8 @@ rms_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_bfl
                     long long y_batch, const __nv_bfloat16* __restrict__ w, int w_per_head, const float* __restrict__ cos_t,
                     const float* __restrict__ sin_t, int rows_per_batch, int C, int group, float eps,
                     float* __restrict__ rstd_out, const HeadScatter sc) {
+  allow_successor();
+  wait_for_predecessor();
   __shared__ float2 red[2][THREADS / 32];
   int parity = 0;
   const Strip s = my_strip(rows_per_batch);
@@ -674,6 +680,8 @@ __global__ void __launch_bounds__(THREADS)
 gated_res_fwd_kernel(const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ y,
                      const float* __restrict__ gate, long long gate_ld, int rows_per_batch, int C,
                      __nv_bfloat16* __restrict__ out) {
+  allow_successor();
+  wait_for_predecessor();
   const Strip s = my_strip(rows_per_batch);
   const int nvec = C >> 3;
   for (int k = 0; k < MAXV; ++k) {
@@ -801,6 +809,8 @@ __device__ __forceinline__ float gelu_erf_grad(float x) {
 }
 __global__ void geglu_fwd_kernel(const __nv_bfloat16* __restrict__ u, __nv_bfloat16* __restrict__ y, long long rows,
                                  int inner_vecs) {
+  allow_successor();
+  wait_for_predecessor();
   const long long total = rows * inner_vecs;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -859,7 +869,7 @@ extern "C" int mdb_ln_fwd(const void* x, void* y, const void* gamma, const void*
   if (scale == nullptr && shift == nullptr && C <= 2048) {  // plain affine, short rows: a warp per row
     const int vpl = ((C >> 3) + 31) / 32;
 #define MDB_LN_ROWS_FWD(V)                                                                                          \
-  ln_rows_fwd_kernel<V><<<grid, THREADS, 0, static_cast<cudaStream_t>(stream)>>>(                                   \
+  launch_overlapped(ln_rows_fwd_kernel<V>, grid, THREADS, 0, static_cast<cudaStream_t>(stream),                     \
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(gamma), \
       static_cast<const __nv_bfloat16*>(beta), rows_per_batch, C, eps, mean_out, rstd_out)
     if (vpl <= 1) MDB_LN_ROWS_FWD(1);
@@ -871,7 +881,7 @@ extern "C" int mdb_ln_fwd(const void* x, void* y, const void* gamma, const void*
     return static_cast<int>(cudaGetLastError());
   }
 #define MDB_LN_FWD(NV)                                                                                          \
-  ln_fwd_kernel<NV><<<grid, THREADS, 0, static_cast<cudaStream_t>(stream)>>>(                                   \
+  launch_overlapped(ln_fwd_kernel<NV>, grid, THREADS, 0, static_cast<cudaStream_t>(stream),                     \
       static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(gamma), \
       static_cast<const __nv_bfloat16*>(beta), scale, shift, mod_ld, rows_per_batch, C, eps, mean_out, rstd_out)
   switch (vectors_per_thread(C)) {
@@ -942,7 +952,7 @@ static int launch_rms_rope_fwd(const void* x, long long ldx, void* y, long long 
   using namespace mdb::rw;
   dim3 grid(ctas_per_batch, num_batches);
 #define MDB_RMS_FWD(NV)                                                                                 \
-  rms_rope_fwd_kernel<NV><<<grid, THREADS, 0, static_cast<cudaStream_t>(stream)>>>(                     \
+  launch_overlapped(rms_rope_fwd_kernel<NV>, grid, THREADS, 0, static_cast<cudaStream_t>(stream),       \
       static_cast<const __nv_bfloat16*>(x), ldx, static_cast<__nv_bfloat16*>(y), ldy, y_batch,          \
       static_cast<const __nv_bfloat16*>(w), w_per_head, cos_t, sin_t, rows_per_batch, C, group, eps, rstd_out, sc)
   switch (vectors_per_thread(C)) {
@@ -1025,7 +1035,7 @@ extern "C" int mdb_gated_res_fwd(const void* res, const void* y, const float* ga
   if (int rc = check_c(C)) return rc;
   if (num_batches <= 0 || rows_per_batch <= 0) return 0;
   dim3 grid(ctas_per_batch, num_batches);
-  gated_res_fwd_kernel<<<grid, THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_overlapped(gated_res_fwd_kernel, grid, THREADS, 0, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(res), static_cast<const __nv_bfloat16*>(y), gate, gate_ld, rows_per_batch, C,
       static_cast<__nv_bfloat16*>(out));
   return static_cast<int>(cudaGetLastError());
@@ -1087,7 +1097,7 @@ extern "C" int mdb_geglu_fwd(const void* u, void* y, long long rows, int inner, 
   if (rows <= 0) return 0;
   const long long total = rows * (inner >> 3);
   const int blocks = static_cast<int>(total / 256 + 1 < 148 * 8 ? total / 256 + 1 : 148 * 8);
-  geglu_fwd_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_overlapped(geglu_fwd_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream),
       static_cast<const __nv_bfloat16*>(u), static_cast<__nv_bfloat16*>(y), rows, inner >> 3);
   return static_cast<int>(cudaGetLastError());
 }

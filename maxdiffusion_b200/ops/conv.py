@@ -669,7 +669,7 @@ def wide_head_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale
 # ---------------------------------------------------------------------------------------------
 def _gn_splits(n: int, hw: int) -> int:
   """Strips of pixels per image so that the sums pass fills the GPU (about 4 CTAs per SM) without tiny strips."""
-  return max(1, min((4 * 148 + n - 1) // n, (hw + 63) // 64))
+  return max(1, min((4 * 148 + n - 1) // n, (hw + 15) // 16))
 
 
 def _gn_partial(x3, dy3=None, act_a=None, act_b=None):
