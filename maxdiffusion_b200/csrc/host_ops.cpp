@@ -20,6 +20,7 @@
 extern "C" {
 int mdb_gemm_bf16(const void*, const void*, void*, const void*, const void*, const void*, int, int, int, long long, long long,
                   long long, long long, long long, int, int, int, int, int, float, int, int, int, void*, void*);
+int mdb_gemm_geglu(const void*, const void*, void*, const void*, int, int, int, long long, long long, long long, void*);
 int mdb_flash_fwd(const void*, const void* const*, const void* const*, void*, float*, int, int, int, int, const int*, long long,
                   long long, long long, long long, long long, long long, long long, long long, long long, long long, long long,
                   long long, float, const unsigned int*, unsigned int, const void*, void*);
@@ -212,6 +213,28 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// geglu_linear(x, weight, bias): [..., K] x [2 N, K]^T -> h * gelu(gate) [..., N]
+PyObject* py_geglu_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 3 || !THPVariable_Check(a[0]) || !THPVariable_Check(a[1])) return not_implemented();
+  const Tensor &x = THPVariable_Unpack(a[0]), &w = THPVariable_Unpack(a[1]);
+  const Tensor* bias;
+  if (!opt_tensor(a[2], bias)) return not_implemented();
+  int64_t M, lda;
+  if (!bf16(x) || !bf16(w) || w.dim() != 2 || w.stride(1) != 1 || !rows_of(x, M, lda)) return not_implemented();
+  const int64_t K = x.size(-1), N = w.size(0) / 2;
+  if (M <= 128) return not_implemented();  // the GEMM and the GEGLU kernel are as fast
+  if (w.size(1) != K || w.size(0) % 16 || N <= 0 || K <= 0 || M > INT_MAX || N > INT_MAX / 2 || K > INT_MAX) return not_implemented();
+  if (bias && (!bf16(*bias) || !bias->is_contiguous() || bias->numel() != 2 * N)) return not_implemented();
+  std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
+  sizes.back() = N;
+  const Tensor out = at::empty(sizes, x.options());
+  const int rc = mdb_gemm_geglu(x.data_ptr(), w.data_ptr(), out.data_ptr(), data(bias), static_cast<int>(M), static_cast<int>(N),
+                                static_cast<int>(K), lda, w.stride(0), N, stream());
+  return done(rc, "mdb_gemm_geglu", out);
+  END_HANDLE_TH_ERRORS
+}
+
 // attention(q, k, v, scale): [B,S,H,D] without a log-sum-exp; D a multiple of 8 up to 128
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -343,7 +366,7 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (groups <= 0 || C % groups || (C & 7) || C > 2048 || N > 65535 || HW > INT_MAX) return not_implemented();
   for (const Tensor* p : {gamma, beta})
     if (p && (!bf16(*p) || !p->is_contiguous() || p->numel() != C)) return not_implemented();
-  const int splits = static_cast<int>(std::max<int64_t>(1, std::min((kCtasTarget + N - 1) / N, (HW + 63) / 64)));
+  const int splits = static_cast<int>(std::max<int64_t>(1, std::min((kCtasTarget + N - 1) / N, (HW + 15) / 16)));
   const auto f = x.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous);
   // one buffer: the strips' sums, then a and b [N, C], mean and rstd [N, groups]
   const int64_t sums = N * splits * C * 2;
@@ -429,7 +452,7 @@ PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
 
 #define MDB_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
-PyMethodDef kMethods[] = {MDB_FAST(gemm), MDB_FAST(linear), MDB_FAST(attention), MDB_FAST(layer_norm), MDB_FAST(geglu),
+PyMethodDef kMethods[] = {MDB_FAST(gemm), MDB_FAST(linear), MDB_FAST(geglu_linear), MDB_FAST(attention), MDB_FAST(layer_norm), MDB_FAST(geglu),
                           MDB_FAST(rms_rope), MDB_FAST(group_norm_cl), MDB_FAST(conv), MDB_FAST(setup),
                           {"launches", py_launches, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

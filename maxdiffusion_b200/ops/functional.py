@@ -392,6 +392,15 @@ def geglu(u: torch.Tensor) -> torch.Tensor:
   return h * torch.nn.functional.gelu(gate)
 
 
+def geglu_linear(x, weight, bias=None):
+  """`geglu` of `linear`. Without autograd one kernel does both and the projection is never written."""
+  if _fast(x) and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and _direct(x, weight, bias):
+    r = _lib.host_ops().geglu_linear(x, weight, bias)
+    if r is not NotImplemented:
+      return r
+  return geglu(linear(x, weight, bias))
+
+
 class _RmsRopeFn(torch.autograd.Function):
 
   @staticmethod

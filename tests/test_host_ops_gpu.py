@@ -52,6 +52,24 @@ def test_linear(monkeypatch, form, act):
     _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.float()))
 
 
+_FORMS["more than a tile"] = lambda: _randn(3, 87, 64)
+
+
+@pytest.mark.parametrize("form", list(_FORMS))
+@pytest.mark.parametrize("N", [8, 136, 320])
+def test_geglu_linear(form, N):
+  """Against float64; the product is not rounded to bf16 in between, so one rounding (2^-9 of a value) is all."""
+  torch.manual_seed(4)
+  x, w, b = _FORMS[form](), _randn(2 * N, 64), _randn(2 * N)
+  with torch.no_grad():
+    for bias in (b, None):
+      u = x.double() @ w.double().t() + (0 if bias is None else bias.double())
+      want = u[..., :N] * torch.nn.functional.gelu(u[..., N:])
+      got = OF.geglu_linear(x, w, bias)
+      assert got.shape == want.shape and (got.double() - want).norm() < 4e-3 * want.norm()
+  assert OF.geglu_linear(x, torch.nn.Parameter(w)).requires_grad
+
+
 @pytest.mark.parametrize("D", [8, 40, 64, 80, 128])
 def test_attention(monkeypatch, D):
   torch.manual_seed(1)
