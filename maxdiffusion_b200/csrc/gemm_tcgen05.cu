@@ -85,8 +85,14 @@ struct Params {
   int splits;
   int kb_per_split;
   float* partial;
+  int mats;    // B matrices of the same shape that share A (1 .. MAX_MATS); matrix i gives columns [i N, (i + 1) N) of out
   int bn;      // columns of a tile: 64, 128, 192 or 256
   int stages;  // pipeline depth
+};
+
+constexpr int MAX_MATS = 3;
+struct BMaps {
+  CUtensorMap m[MAX_MATS];
 };
 
 template <int GROUP_M>
@@ -104,8 +110,7 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 
 template <bool A_MN, bool B_MN, int CG, int EK>
 __global__ void __cluster_dims__(CG, 1, 1) __launch_bounds__(NUM_THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-            const Params p) {
+gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ BMaps maps_b, const Params p) {
   constexpr int TILE_M = CG * BM;
   constexpr int GROUP_M = 8;
   constexpr int TMEM_COLS = 2 * ACC_COLS;   // two accumulators
@@ -130,14 +135,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const int num_m = (p.M + TILE_M - 1) / TILE_M;
   constexpr int HALVES = EK == kGeglu ? 2 : 1;  // GEGLU: half of a tile's columns are gates of the other half
   const int OUT_N = BN / HALVES;                 // output columns of a tile
-  const int num_n = (p.N + OUT_N - 1) / OUT_N;
+  const int mat_n = (p.N + OUT_N - 1) / OUT_N;   // column tiles of one B matrix
+  const int num_n = mat_n * p.mats;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
   const int num_work = num_tiles * p.splits;
 
   if (threadIdx.x == 0) {
     prefetch_tensormap(&tmap_a);
-    prefetch_tensormap(&tmap_b);
+    prefetch_tensormap(&maps_b.m[0]);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
@@ -177,6 +183,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         int m_idx, n_idx;
         const int split = work / num_tiles;
         tile_coords<GROUP_M>(work - split * num_tiles, num_m, num_n, m_idx, n_idx);
+        const int mat = p.mats > 1 ? n_idx / mat_n : 0;
+        n_idx -= mat * mat_n;
+        const CUtensorMap& tmap_b = maps_b.m[mat];
         const int m0 = m_idx * TILE_M + rank * BM;
         // GEGLU (pairs only): the even CTA fetches rows n of B, the odd one rows N + n
         const int n0 = EK == kGeglu ? n_idx * OUT_N + rank * p.N : n_idx * BN + rank * BN_CTA;
@@ -288,6 +297,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       int m_idx, n_idx;
       const int split = work / num_tiles;
       tile_coords<GROUP_M>(work - split * num_tiles, num_m, num_n, m_idx, n_idx);
+      const int mat = p.mats > 1 ? n_idx / mat_n : 0;
+      n_idx -= mat * mat_n;
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
       float* bias_t = bias_s + acc * 256;
@@ -320,7 +331,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         constexpr int esz = f32 ? 4 : 2;
         uint8_t* out_base = p.splits > 1
             ? reinterpret_cast<uint8_t*>(p.partial) + (static_cast<long long>(split) * p.M + warp_row0) * p.N * 4
-            : reinterpret_cast<uint8_t*>(p.out) + warp_row0 * p.ldo * esz;
+            : reinterpret_cast<uint8_t*>(p.out) + (warp_row0 * p.ldo + static_cast<long long>(mat) * p.N) * esz;
         const long long out_pitch = (p.splits > 1 ? static_cast<long long>(p.N) : p.ldo) * esz;
 #pragma unroll 1
         for (int c0 = egroup * slab_cols; c0 < OUT_N; c0 += 2 * slab_cols) {
@@ -608,7 +619,7 @@ __global__ void splitk_fold_kernel(const __grid_constant__ Params p) {
 }
 
 template <bool A_MN, bool B_MN, int CG, int EK>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, cudaStream_t stream) {
+int launch(const CUtensorMap& ta, const BMaps& tb, const Params& p, cudaStream_t stream) {
   auto kern = gemm_kernel<A_MN, B_MN, CG, EK>;
   static bool configured = false;
   if (!configured) {
@@ -616,7 +627,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, cudaSt
     configured = true;
   }
   const int out_n = EK == kGeglu ? p.bn / 2 : p.bn;
-  const int num_work = ((p.M + CG * BM - 1) / (CG * BM)) * ((p.N + out_n - 1) / out_n) * p.splits;
+  const int num_work = ((p.M + CG * BM - 1) / (CG * BM)) * ((p.N + out_n - 1) / out_n) * p.mats * p.splits;
   const int slots = sm_count() / CG;
   const int grid = (num_work < slots ? num_work : slots) * CG;
   MDB_CHECK_CUDA(launch_overlapped(kern, grid, NUM_THREADS, p.stages * stage_bytes(p.bn, CG) + FIXED_BYTES, stream, ta, tb, p));
@@ -629,7 +640,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, cudaSt
 }
 
 template <bool A_MN, bool B_MN, int CG>
-int launch_kind(int kind, const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, cudaStream_t stream) {
+int launch_kind(int kind, const CUtensorMap& ta, const BMaps& tb, const Params& p, cudaStream_t stream) {
   switch (kind) {
     case kPlain: return launch<A_MN, B_MN, CG, kPlain>(ta, tb, p, stream);
     case kAct: return launch<A_MN, B_MN, CG, kAct>(ta, tb, p, stream);
@@ -674,7 +685,8 @@ extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void
   if (splits < 1 || splits > 64 || (splits > 1 && partial == nullptr)) return 3005;
   const int bn_cta = bn / ctas;
   if (b_mn_major && bn_cta % 64) return 3004;
-  CUtensorMap ta, tb;
+  CUtensorMap ta;
+  BMaps tb = {};
   int rc;
   if (a_mn_major) {
     uint64_t dims[2] = {static_cast<uint64_t>(M), static_cast<uint64_t>(K)};
@@ -692,12 +704,12 @@ extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void
     uint64_t dims[2] = {static_cast<uint64_t>(N), static_cast<uint64_t>(K)};
     uint64_t str[1] = {static_cast<uint64_t>(ldb) * 2};
     uint32_t box[2] = {64, BK};
-    rc = encode_tmap_bf16(&tb, B, 2, dims, str, box);
+    rc = encode_tmap_bf16(&tb.m[0], B, 2, dims, str, box);
   } else {
     uint64_t dims[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(N)};
     uint64_t str[1] = {static_cast<uint64_t>(ldb) * 2};
     uint32_t box[2] = {BK, static_cast<uint32_t>(bn_cta)};
-    rc = encode_tmap_bf16(&tb, B, 2, dims, str, box);
+    rc = encode_tmap_bf16(&tb.m[0], B, 2, dims, str, box);
   }
   if (rc) return rc;
   Params p;
@@ -712,6 +724,7 @@ extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void
   p.epi = epi;
   p.out_f32 = out_f32;
   p.alpha = alpha;
+  p.mats = 1;
   p.bn = bn;
   p.stages = stages_for(bn, ctas);
   p.status = status_buffer();
@@ -751,19 +764,21 @@ extern "C" int mdb_gemm_geglu(const void* A, const void* B, void* out, const voi
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((N & 7) || (lda & 7) || (ldb & 7) || (ldo & 7)) return 3001;
   constexpr int bn = 256, ctas = 2;
-  CUtensorMap ta, tb;
+  CUtensorMap ta;
+  BMaps tb = {};
   uint64_t da[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(M)}, db[2] = {static_cast<uint64_t>(K), 2ull * N};
   uint64_t sa[1] = {static_cast<uint64_t>(lda) * 2}, sb[1] = {static_cast<uint64_t>(ldb) * 2};
   uint32_t box_a[2] = {BK, BM}, box_b[2] = {BK, bn / 2};
   int rc = encode_tmap_bf16(&ta, A, 2, da, sa, box_a);
   if (rc) return rc;
-  rc = encode_tmap_bf16(&tb, B, 2, db, sb, box_b);
+  rc = encode_tmap_bf16(&tb.m[0], B, 2, db, sb, box_b);
   if (rc) return rc;
   Params p = {};
   p.M = M; p.N = N; p.K = K;
   p.out = out; p.ldo = ldo;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.alpha = 1.0f;
+  p.mats = 1;
   p.splits = 1;
   p.kb_per_split = (K + BK - 1) / BK;
   p.bn = bn;
@@ -771,4 +786,39 @@ extern "C" int mdb_gemm_geglu(const void* A, const void* B, void* out, const voi
   p.status = status_buffer();
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   return launch<false, false, 2, kGeglu>(ta, tb, p, stream);
+}
+
+// out [M, mats * N] = A [M, K] times each of `mats` matrices B_i [N, K] transposed, side by side: projections of the same
+// rows (q, k, v) in one launch. Apart / together: 2048 x (3 x 1280) x 1280 28.0 / 18.7 us, 154 x (2 x 1280) x 2048 16.5 / 9.1 us.
+extern "C" int mdb_gemm_group(const void* A, const void* const* B, int mats, void* out, int M, int N, int K, long long lda,
+                              long long ldb, long long ldo, int ctas, int bn, void* stream_ptr) {
+  using namespace mdb;
+  using namespace mdb::gemm;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (mats < 1 || mats > MAX_MATS) return 3008;
+  if ((N & 7) || (lda & 7) || (ldb & 7) || (ldo & 7)) return 3001;
+  if ((ctas != 1 && ctas != 2) || (bn != 64 && bn != 128 && bn != 192 && bn != 256)) return 3004;
+  CUtensorMap ta;
+  BMaps tb = {};
+  uint64_t da[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(M)}, db[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(N)};
+  uint64_t sa[1] = {static_cast<uint64_t>(lda) * 2}, sb[1] = {static_cast<uint64_t>(ldb) * 2};
+  uint32_t box_a[2] = {BK, BM}, box_b[2] = {BK, static_cast<uint32_t>(bn / ctas)};
+  int rc = encode_tmap_bf16(&ta, A, 2, da, sa, box_a);
+  if (rc) return rc;
+  for (int i = 0; i < mats; ++i) {
+    rc = encode_tmap_bf16(&tb.m[i], B[i], 2, db, sb, box_b);
+    if (rc) return rc;
+  }
+  Params p = {};
+  p.M = M; p.N = N; p.K = K;
+  p.out = out; p.ldo = ldo;
+  p.alpha = 1.0f;
+  p.mats = mats;
+  p.splits = 1;
+  p.kb_per_split = (K + BK - 1) / BK;
+  p.bn = bn;
+  p.stages = stages_for(bn, ctas);
+  p.status = status_buffer();
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  return ctas == 2 ? launch<false, false, 2, kPlain>(ta, tb, p, stream) : launch<false, false, 1, kPlain>(ta, tb, p, stream);
 }

@@ -21,6 +21,7 @@ extern "C" {
 int mdb_gemm_bf16(const void*, const void*, void*, const void*, const void*, const void*, int, int, int, long long, long long,
                   long long, long long, long long, int, int, int, int, int, float, int, int, int, void*, void*);
 int mdb_gemm_geglu(const void*, const void*, void*, const void*, int, int, int, long long, long long, long long, void*);
+int mdb_gemm_group(const void*, const void* const*, int, void*, int, int, int, long long, long long, long long, int, int, void*);
 int mdb_flash_fwd(const void*, const void* const*, const void* const*, void*, float*, int, int, int, int, const int*, long long,
                   long long, long long, long long, long long, long long, long long, long long, long long, long long, long long,
                   long long, float, const unsigned int*, unsigned int, const void*, void*);
@@ -232,6 +233,35 @@ PyObject* py_geglu_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int rc = mdb_gemm_geglu(x.data_ptr(), w.data_ptr(), out.data_ptr(), data(bias), static_cast<int>(M), static_cast<int>(N),
                                 static_cast<int>(K), lda, w.stride(0), N, stream());
   return done(rc, "mdb_gemm_geglu", out);
+  END_HANDLE_TH_ERRORS
+}
+
+// linear_group(x, w0, w1[, w2]): [..., K] x each [N, K]^T, side by side -> [..., n * N]
+PyObject* py_linear_group(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const int mats = static_cast<int>(n) - 1;
+  if (mats < 1 || mats > 3) return not_implemented();
+  for (Py_ssize_t i = 0; i < n; ++i)
+    if (!THPVariable_Check(a[i])) return not_implemented();
+  const Tensor &x = THPVariable_Unpack(a[0]), &w = THPVariable_Unpack(a[1]);
+  int64_t M, lda;
+  if (!bf16(x) || !rows_of(x, M, lda)) return not_implemented();
+  const void* ws[3] = {nullptr, nullptr, nullptr};
+  for (int i = 0; i < mats; ++i) {
+    const Tensor& t = THPVariable_Unpack(a[1 + i]);
+    if (!bf16(t) || t.dim() != 2 || t.sizes() != w.sizes() || t.stride(0) != w.stride(0) || t.stride(1) != 1) return not_implemented();
+    ws[i] = t.data_ptr();
+  }
+  const int64_t K = x.size(-1), N = w.size(0);
+  if (w.size(1) != K || (N & 7) || N <= 0 || K <= 0 || M > INT_MAX || N > INT_MAX / 3 || K > INT_MAX) return not_implemented();
+  std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
+  sizes.back() = mats * N;
+  const Tensor out = at::empty(sizes, x.options());
+  Plan plan;
+  if (!gemm_plan(M, mats * N, K, false, false, 0, 0, plan)) return nullptr;
+  const int rc = mdb_gemm_group(x.data_ptr(), ws, mats, out.data_ptr(), static_cast<int>(M), static_cast<int>(N),
+                                static_cast<int>(K), lda, w.stride(0), mats * N, plan.ctas, plan.bn, stream());
+  return done(rc, "mdb_gemm_group", out);
   END_HANDLE_TH_ERRORS
 }
 
@@ -452,7 +482,7 @@ PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches); }
 
 #define MDB_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
-PyMethodDef kMethods[] = {MDB_FAST(gemm), MDB_FAST(linear), MDB_FAST(geglu_linear), MDB_FAST(attention), MDB_FAST(layer_norm), MDB_FAST(geglu),
+PyMethodDef kMethods[] = {MDB_FAST(gemm), MDB_FAST(linear), MDB_FAST(geglu_linear), MDB_FAST(linear_group), MDB_FAST(attention), MDB_FAST(layer_norm), MDB_FAST(geglu),
                           MDB_FAST(rms_rope), MDB_FAST(group_norm_cl), MDB_FAST(conv), MDB_FAST(setup),
                           {"launches", py_launches, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

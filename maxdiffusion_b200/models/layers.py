@@ -29,6 +29,12 @@ class Linear(nn.Module):
     return f"in_features={self.in_features}, out_features={self.out_features}, bias={self.bias is not None}"
 
 
+def is_plain_linear(m: nn.Module) -> bool:
+  """Whether calling `m` is `OF.linear` and nothing else (no subclass, wrapper or hook), so that its product may run fused
+  with another."""
+  return type(m) is Linear and not m._forward_hooks and not m._forward_pre_hooks
+
+
 def project_gated_residual(proj: nn.Module, x, residual, gate):
   """residual + gate * proj(x). A plain `Linear` takes the fused GEMM-epilogue path; any other projection (e.g. a
   quantised one) runs as a module followed by the fused gated-residual kernel."""

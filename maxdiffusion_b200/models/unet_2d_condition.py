@@ -20,7 +20,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import functional as OF
-from .layers import Conv2d, GroupNorm, LayerNorm, Linear, sinusoidal_embedding
+from .layers import Conv2d, GroupNorm, LayerNorm, Linear, is_plain_linear, sinusoidal_embedding
 from .vae import ResnetBlock2D
 
 
@@ -87,9 +87,14 @@ class Attention(nn.Module):
   def forward(self, x, context=None, residual=None):
     ctx = x if context is None else context
     B, S, C = x.shape
-    q = self.to_q(x).view(B, S, self.heads, -1)
-    k = self.to_k(ctx).view(B, ctx.shape[1], self.heads, -1)
-    v = self.to_v(ctx).view(B, ctx.shape[1], self.heads, -1)
+    if is_plain_linear(self.to_q) and is_plain_linear(self.to_k) and is_plain_linear(self.to_v):
+      if context is None:
+        q, k, v = OF.linear_group(x, (self.to_q.weight, self.to_k.weight, self.to_v.weight))
+      else:
+        q, (k, v) = OF.linear(x, self.to_q.weight), OF.linear_group(ctx, (self.to_k.weight, self.to_v.weight))
+    else:
+      q, k, v = self.to_q(x), self.to_k(ctx), self.to_v(ctx)
+    q, k, v = (t.unflatten(-1, (self.heads, -1)) for t in (q, k, v))
     return self.to_out[0](OF.attention(q, k, v).reshape(B, S, C), residual=residual)
 
 
@@ -101,7 +106,7 @@ class GEGLU(nn.Module):
     self.proj = Linear(dim, 2 * inner)
 
   def forward(self, x):
-    if type(self.proj) is Linear and not self.proj._forward_hooks and not self.proj._forward_pre_hooks:
+    if is_plain_linear(self.proj):
       return OF.geglu_linear(x, self.proj.weight, self.proj.bias)
     return OF.geglu(self.proj(x))
 

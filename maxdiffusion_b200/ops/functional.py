@@ -184,6 +184,16 @@ def linear(x, weight, bias=None, activation: str | None = None, residual=None):
   return y if residual is None else residual + y
 
 
+def linear_group(x, weights):
+  """x @ w.T for up to three weights of one shape (the projections of an attention layer), as a tuple. Without autograd they
+  are one launch, and the results are slices of one buffer."""
+  if _fast(x) and x.shape[-1] % 8 == 0 and len(weights) <= 3 and _direct(x, *weights):
+    r = _lib.host_ops().linear_group(x, *weights)
+    if r is not NotImplemented:
+      return r.chunk(len(weights), dim=-1)
+  return tuple(linear(x, w) for w in weights)
+
+
 def linear_gated_residual(x, weight, bias, residual, gate):
   """residual + gate[:,None,:] * (x @ weightᵀ + bias), the output projection of an AdaLN-gated branch.
 

@@ -70,6 +70,22 @@ def test_geglu_linear(form, N):
   assert OF.geglu_linear(x, torch.nn.Parameter(w)).requires_grad
 
 
+@pytest.mark.parametrize("form", list(_FORMS))
+@pytest.mark.parametrize("n,N", [(2, 8), (3, 72), (3, 320), (2, 264)])
+def test_linear_group(form, n, N):
+  torch.manual_seed(5)
+  x, ws = _FORMS[form](), [_randn(N, 64) for _ in range(n)]
+  with torch.no_grad():
+    got = OF.linear_group(x, ws)
+    assert len(got) == n
+    for g, w in zip(got, ws):
+      want = x.double() @ w.double().t()
+      assert g.shape == want.shape and (g.double() - want).norm() < 4e-3 * want.norm()  # one rounding to bf16
+    odd = OF.linear_group(x, [ws[0], ws[1][:8]])
+    assert odd[1].shape[-1] == 8
+  assert OF.linear_group(x, [torch.nn.Parameter(w) for w in ws])[1].requires_grad
+
+
 @pytest.mark.parametrize("D", [8, 40, 64, 80, 128])
 def test_attention(monkeypatch, D):
   torch.manual_seed(1)
