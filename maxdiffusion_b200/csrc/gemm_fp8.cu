@@ -91,6 +91,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  allow_successor();
+  wait_for_predecessor();
 
   if (warp == 0) {
     if (elect_one()) {
@@ -323,8 +325,7 @@ static int gemm8_impl(const void* Aq, const void* Bq, void* out, const void* bia
   }
   const int num_tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int grid = num_tiles < sm_count() ? num_tiles : sm_count();
-  gemm_fp8_kernel<<<grid, NUM_THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream_ptr)>>>(ta, tb, p);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_overlapped(gemm_fp8_kernel, grid, NUM_THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream_ptr), ta, tb, p));
 }
 
 // x: bf16 [n] (n % 8 == 0); stats: device {sum x^2, max |x|} as produced by mdb_sumsq_maxabs.
