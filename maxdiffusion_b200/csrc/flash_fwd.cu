@@ -84,6 +84,9 @@ struct CopyPlan {
 
 struct Params {
   int B, H, q_len;
+  // Work items are two 128-row tiles of one (batch, head) up to item n_double; from there every tile is an item of its own:
+  // a last round that would leave most CTAs idle runs twice as many items of half the rows.
+  int n_double;
   int d;  // channels of a head, a multiple of 8 up to the built head_dim; TMA fills the rest of a tile with zeros
   int num_segments;
   int kv_len[MAX_SEGMENTS];
@@ -255,6 +258,21 @@ __device__ __forceinline__ uint64_t exp_half(const uint32_t (&s)[2][32], uint32_
   return rs;
 }
 
+struct Item {
+  int q0, n_tiles, head, batch;  // n_tiles 0: the second half of an item that has one tile only
+};
+__device__ __forceinline__ Item item_of(int work, int n_qb, const Params& p) {
+  const bool single = work >= p.n_double;
+  const int item = single ? p.n_double + ((work - p.n_double) >> 1) : work;
+  const int half = single ? (work - p.n_double) & 1 : 0;
+  Item t;
+  t.q0 = (item % n_qb) * 2 * BQ + half * BQ;
+  t.head = (item / n_qb) % p.H;
+  t.batch = item / (n_qb * p.H);
+  t.n_tiles = t.q0 >= p.q_len ? 0 : (single || p.q_len - t.q0 <= BQ) ? 1 : 2;
+  return t;
+}
+
 template <int HD, int KV_STAGES>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ KVMaps maps, const Params p,
@@ -293,7 +311,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int n_qb = (p.q_len + 2 * BQ - 1) / (2 * BQ);
-  const int total_work = n_qb * p.H * p.B;
+  const int total_work = p.n_double + 2 * (n_qb * p.H * p.B - p.n_double);
 
   int total_blocks = 0;
   for (int s = 0; s < p.num_segments; ++s) total_blocks += (p.kv_len[s] + BKV - 1) / BKV;
@@ -338,13 +356,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       unsigned long long seen = 0;  // (segment, head group) flags that have been observed
       bool ok = true;
       int it = 0;
-      for (int work = blockIdx.x; work < total_work && ok; work += n_compute, ++it) {
-        const int qb = work % n_qb;
-        const int head = (work / n_qb) % p.H;
-        const int batch = work / (n_qb * p.H);
-        const int q0 = qb * 2 * BQ;
-        const int n_tiles = (p.q_len - q0 > BQ) ? 2 : 1;
+      for (int work = blockIdx.x; work < total_work && ok; work += n_compute) {
+        const Item item = item_of(work, n_qb, p);
+        const int head = item.head, batch = item.batch, q0 = item.q0, n_tiles = item.n_tiles;
+        if (n_tiles == 0) continue;
         if (!mbar_wait(q_empty, (it & 1) ^ 1u, abort_flag, p.status, 43)) { ok = false; break; }
+        ++it;
         mbar_expect_tx(q_full, n_tiles * TILE_BYTES);
         for (int t = 0; t < n_tiles; ++t) {
           for (int c = 0; c < CH; ++c) {
@@ -393,10 +410,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       uint32_t n = 0;  // blocks of this tile so far, over all work items: buffer n & 1, use n >> 1
       bool ok = true;
       int it = 0;
-      for (int work = blockIdx.x; work < total_work && ok; work += n_compute, ++it) {
-        const int q0 = (work % n_qb) * 2 * BQ;
-        const bool active = t < ((p.q_len - q0 > BQ) ? 2 : 1);
+      for (int work = blockIdx.x; work < total_work && ok; work += n_compute) {
+        const int n_tiles = item_of(work, n_qb, p).n_tiles;
+        if (n_tiles == 0) continue;
+        const bool active = t < n_tiles;
         if (!mbar_wait(q_full, it & 1, abort_flag, p.status, 50)) { ok = false; break; }
+        ++it;
         for (int j = 0; j < total_blocks; ++j) {
           if (!mbar_wait(&k_full[stage], phase, abort_flag, p.status, 51)) { ok = false; break; }
           if (active) {
@@ -438,8 +457,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       uint32_t n = 0;
       bool ok = true;
       for (int work = blockIdx.x; work < total_work && ok; work += n_compute) {
-        const int q0 = (work % n_qb) * 2 * BQ;
-        const bool active = t < ((p.q_len - q0 > BQ) ? 2 : 1);
+        const int n_tiles = item_of(work, n_qb, p).n_tiles;
+        if (n_tiles == 0) continue;
+        const bool active = t < n_tiles;
         for (int j = 0; j < total_blocks; ++j) {
           if (!mbar_wait(&v_full[stage], phase, abort_flag, p.status, 52)) { ok = false; break; }
           if (active) {
@@ -472,12 +492,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     uint32_t n = 0, oc = 0;  // blocks of this tile so far; parity of o_final
     bool ok = total_blocks > 0;
     for (int work = blockIdx.x; work < total_work && ok; work += n_compute) {
-      const int qb = work % n_qb;
-      const int head = (work / n_qb) % p.H;
-      const int batch = work / (n_qb * p.H);
-      const int q0 = qb * 2 * BQ;
-      const int n_tiles = (p.q_len - q0 > BQ) ? 2 : 1;
-      if (t >= n_tiles) continue;
+      const Item item = item_of(work, n_qb, p);
+      const int head = item.head, batch = item.batch, q0 = item.q0;
+      if (t >= item.n_tiles) continue;
       const int q_row = q0 + t * BQ + row_in_tile;
       float m = -INFINITY, l = 0.0f;
       const bool fixed = p.m_fixed != nullptr && p.fixed_heads[head] != 0;  // uniform over the CTA
@@ -761,7 +778,14 @@ static int flash_fwd_launch(const void* q, const void* const* k_ptrs, const void
   }
   int n_compute = sm_count() - n_copy;
   if (n_compute < 1) return 3104;
-  if (total_work < n_compute) n_compute = static_cast<int>(total_work);
+  p.n_double = static_cast<int>(total_work);
+  if (n_copy == 0 && seg_flags == nullptr && total_work % n_compute * 2 <= n_compute) {
+    // the items of the last round as single tiles, when they all fit into it (1024^2 x 2 x 20 heads of 64: 38.4 us with
+    // whole items, 31.7 us so; 384^2 x 24 heads of 128: 14.5 / 9.7 us)
+    p.n_double = static_cast<int>(total_work - total_work % n_compute);
+  }
+  const long long n_items = p.n_double + 2 * (total_work - p.n_double);
+  if (n_items < n_compute) n_compute = static_cast<int>(n_items);
   if (n_copy > 0) {
     // Head groups. The compute CTAs take the work list in rounds of n_compute items and the list runs through the
     // q blocks of head 0, then head 1, ...: a round covers n_compute / n_qb heads. One group per round lets the first
@@ -787,7 +811,7 @@ static int flash_fwd_launch(const void* q, const void* const* k_ptrs, const void
     n_copy = g_tune_copy_ctas < sm_count() - 1 ? g_tune_copy_ctas : sm_count() - 1;
     cp.n_copy_ctas = n_copy;
     n_compute = sm_count() - n_copy;
-    if (total_work < n_compute) n_compute = static_cast<int>(total_work);
+    if (n_items < n_compute) n_compute = static_cast<int>(n_items);
   }
   const dim3 grid(n_compute + n_copy);
   cudaStream_t st = static_cast<cudaStream_t>(stream_ptr);
