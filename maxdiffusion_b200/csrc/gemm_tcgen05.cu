@@ -574,15 +574,9 @@ __global__ void splitk_fold_kernel(const __grid_constant__ Params p) {
     }
     const long long row = i / n_vec;
     const int col = static_cast<int>(i - row * n_vec) * 8;
-    if (p.bias) {
-      const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
-      const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+    if (p.bias) {  // single loads: a bias may start anywhere
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = unpack_bf16x2(bw[j]);
-        x[2 * j] += f.x;
-        x[2 * j + 1] += f.y;
-      }
+      for (int j = 0; j < 8; ++j) x[j] += __bfloat162float(p.bias[col + j]);
     }
     if (p.epi == kEpiGeluTanh) {
 #pragma unroll

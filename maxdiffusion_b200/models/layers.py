@@ -5,6 +5,7 @@ import math
 
 import torch
 import torch.nn as nn
+import torch.nn.modules.module as _hooks
 
 from ..ops import functional as OF
 
@@ -30,9 +31,10 @@ class Linear(nn.Module):
 
 
 def is_plain_linear(m: nn.Module) -> bool:
-  """Whether calling `m` is `OF.linear` and nothing else (no subclass, wrapper or hook), so that its product may run fused
-  with another."""
-  return type(m) is Linear and not m._forward_hooks and not m._forward_pre_hooks
+  """Whether calling `m` is `OF.linear` and nothing else (no subclass, wrapper, hook or replaced `forward`), so that its
+  product may run fused with another."""
+  return (type(m) is Linear and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__ and
+          not _hooks._global_forward_hooks and not _hooks._global_forward_pre_hooks)
 
 
 def project_gated_residual(proj: nn.Module, x, residual, gate):

@@ -66,6 +66,25 @@ def test_gemm_cut_contraction_with_epilogue(epi, M, N, Kd):
   assert _rel(got, want) < 4e-3
 
 
+def test_cut_contraction_takes_a_bias_that_starts_anywhere():
+  torch.manual_seed(4)
+  a, b, store = _randn(136, 4096), _randn(328, 4096, scale=0.05), _randn(400)
+  bias = store[3:331]  # 6 bytes into a 16-byte line
+  assert K.gemm_plan(136, 328, 4096)[2] > 1
+  assert _rel(K.gemm(a, b, bias=bias), a.double() @ b.double().t() + bias.double()) < 4e-3
+
+
+@pytest.mark.parametrize("Sq,B,H", [(256 * 37, 2, 2), (300, 7, 23), (1024, 2, 20), (129, 1, 1)])
+def test_attention_last_round_of_single_tiles(Sq, B, H):
+  """148 whole items, a last round of single tiles, and items whose second tile does not exist."""
+  torch.manual_seed(5)
+  q, k, v = _randn(B, Sq, H, 64), _randn(B, 200, H, 64), _randn(B, 200, H, 64)
+  out, lse = K.flash_fwd(q, [k], [v])
+  s = torch.einsum("bshd,bthd->bhst", q.double(), k.double()) / 8.0
+  assert _rel(out, torch.einsum("bhst,bthd->bshd", s.softmax(-1), v.double())) < 5e-3  # P is rounded to bf16 too
+  assert (lse.double() * 0.6931471805599453 - s.logsumexp(-1)).abs().max() < 1e-4
+
+
 @pytest.mark.parametrize("plan", [(1, 64, 3), (2, 256, 1), (2, 64, 2), (1, 256, 7), (2, 32, 1)])
 @pytest.mark.parametrize("B,H,W,Ci,Co", [(1, 8, 16, 64, 64), (2, 17, 23, 64, 328), (1, 33, 40, 96, 96), (3, 9, 70, 192, 24),
                                          (1, 5, 128, 64, 64), (1, 9, 250, 96, 96), (2, 3, 127, 320, 40)])
