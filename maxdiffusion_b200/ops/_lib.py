@@ -78,7 +78,11 @@ def host_ops():
 
         path = LIB_PATH.with_name("_host_ops.so")
         if not path.exists():
-          raise KernelError(f"{path} is missing; run `python -m maxdiffusion_b200.build`")
+          if os.environ.get("MDB200_NO_AUTOBUILD") == "1":
+            raise KernelError(f"{path} is missing; run `python -m maxdiffusion_b200.build`")
+          from maxdiffusion_b200 import build as _build
+
+          _build.build(verbose=False)
         spec = importlib.util.spec_from_file_location("_host_ops", path)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
