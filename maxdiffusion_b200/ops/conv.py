@@ -46,6 +46,8 @@ def _declare(L):
   L.mdb_conv_wgrad_boxed.restype = c_int
   L.mdb_softmax_rows.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_ll, c_int, c_void_p]
   L.mdb_softmax_rows.restype = c_int
+  L.mdb_softmax_split.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_ll, c_int, c_int, c_void_p]
+  L.mdb_softmax_split.restype = c_int
   L.mdb_gn_cl_sums.argtypes = [c_void_p] * 5 + [c_int] * 4 + [c_void_p]
   L.mdb_gn_cl_sums.restype = c_int
   L.mdb_gn_cl_apply.argtypes = [c_void_p] * 8 + [c_int] * 4 + [c_void_p]
@@ -655,12 +657,35 @@ def wide_head_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale
 
   T, D = q.shape
   scale = scale if scale is not None else D ** -0.5
+  if use_kernel(q) and T % 8 and D % 8 == 0 and T <= 32768 and not (torch.is_grad_enabled() and
+                                                                   (q.requires_grad or k.requires_grad or v.requires_grad)):
+    return _odd_head_attention(q, k, v, scale)
   if not use_kernel(q) or T % 8 or D % 8 or T > 32768:
     p = torch.softmax((q.float() @ k.float().t()) * scale, dim=-1)
     return (p @ v.float()).to(q.dtype)
   scores = K.gemm(q.contiguous(), k.contiguous(), alpha=scale)         # [T, T] = scale * Q K^T
   softmax_rows(scores)
   return K.gemm(scores, v.contiguous(), b_mn=True)                     # [T, D] = P V   (V is [K = T, N = D])
+
+
+def _odd_head_attention(q, k, v, scale):
+  """`wide_head_attention` for T that is no multiple of 8, with fp32 scores and probabilities (as the library products that
+  ran here before): the keys are padded with zero rows that the softmax leaves out, and the probabilities enter the second
+  product as three bf16 parts. 4500 positions of 384 channels: 752 us with library products, 133 us so, the same error
+  against float64 (1.653e-3, the rounding of the result)."""
+  from . import kernels as K
+
+  T, D = q.shape
+  pitch = _round_up(T, 8)
+  kp = torch.zeros((pitch, D), dtype=k.dtype, device=k.device)
+  kp[:T] = k
+  scores = K.gemm(q.contiguous(), kp, alpha=scale, out_dtype=torch.float32)  # [T, pitch]
+  parts = torch.empty((T, 3 * pitch), dtype=torch.bfloat16, device=q.device)
+  rc = _lib.lib().mdb_softmax_split(_lib.ptr(scores), scores.stride(0), _lib.ptr(parts), parts.stride(0), T, T, pitch, _lib.stream())
+  _lib.check(rc, "mdb_softmax_split")
+  v3 = torch.zeros((3, pitch, D), dtype=v.dtype, device=v.device)
+  v3[:, :T] = v
+  return K.gemm(parts, v3.view(3 * pitch, D), b_mn=True)
 
 
 # ---------------------------------------------------------------------------------------------

@@ -120,3 +120,14 @@ def test_attention_ragged_tails(D, Sq, Sk):
   s = torch.einsum("bshd,bthd->bhst", q.double(), k.double()) / D ** 0.5
   assert _rel(out, torch.einsum("bhst,bthd->bshd", s.softmax(-1), v.double())) < 5e-3  # P is rounded to bf16 too
   assert (lse.double() * 0.6931471805599453 - s.logsumexp(-1)).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("T,D", [(1, 384), (7, 64), (500, 384), (4500, 384), (9001, 16)])
+def test_wide_head_attention_of_odd_lengths(T, D):
+  """Scores and probabilities stay in 32 bits: the result is the float64 one rounded to bf16 once (2^-9 of a value; 1.7e-3 in
+  the 2-norm)."""
+  torch.manual_seed(6)
+  q, k, v = _randn(T, D, scale=2.0), _randn(T, D), _randn(T, D)
+  s = (q.double() @ k.double().t()) * D ** -0.5
+  with torch.no_grad():
+    assert _rel(C.wide_head_attention(q, k, v), s.softmax(-1) @ v.double()) < 2e-3
