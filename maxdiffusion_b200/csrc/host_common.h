@@ -21,10 +21,6 @@ int encode_tmap_bf16(CUtensorMap* map, const void* base, int rank, const uint64_
 int encode_tmap_u8(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
                    const uint64_t* strides_bytes, const uint32_t* box);
 
-// Same, for 4-byte elements (fp32), no swizzle unless box[0]*4 == 128.
-int encode_tmap_f32(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
-                    const uint64_t* strides_bytes, const uint32_t* box, int swizzle128);
-
 int sm_count();
 
 // Launch of a kernel that begins with `wait_for_predecessor()`: its set-up (barriers, TMEM, descriptor and instruction

@@ -87,12 +87,6 @@ int encode_tmap_u8(CUtensorMap* map, const void* base, int rank, const uint64_t*
                        CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-int encode_tmap_f32(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
-                    const uint64_t* strides_bytes, const uint32_t* box, int swizzle128) {
-  return encode_common(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, rank, dims, strides_bytes, box,
-                       swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
-}
-
 }  // namespace mdb
 
 // Reads the device status into `out` (4 uints) and optionally clears it. Synchronises the

@@ -42,7 +42,7 @@ def gemm_plan(M: int, N: int, K: int, b_mn: bool = False, splittable: bool = Tru
   long as its k-blocks or as the epilogue of a tile, whichever is longer; the last epilogue is exposed. Where the output has
   fewer tiles than the GPU has SMs (few tokens; weight gradients, whose contraction is the token count), cutting the
   contraction makes more work items at the price of fp32 partials and a second kernel (3 us + their traffic): 384 x 3072 x
-  15360 takes 51 us whole and 33 us in three parts. `tile_n` / `ctas` restrict the choice."""
+  15360 takes 51 us whole and 41 us in three parts. `tile_n` / `ctas` restrict the choice."""
   best, best_cost = (1, 256, 1), None
   num_kb = -(-K // 64)
   for (cg, bn), kb_us in _KB_US.items():
