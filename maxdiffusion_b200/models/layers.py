@@ -5,7 +5,7 @@ import math
 
 import torch
 import torch.nn as nn
-import torch.nn.modules.module as _hooks
+import torch.nn.modules.module as _module
 
 from ..ops import functional as OF
 
@@ -30,11 +30,18 @@ class Linear(nn.Module):
     return f"in_features={self.in_features}, out_features={self.out_features}, bias={self.bias is not None}"
 
 
+_LINEAR_FORWARD = Linear.forward
+
+
 def is_plain_linear(m: nn.Module) -> bool:
-  """Whether calling `m` is `OF.linear` and nothing else (no subclass, wrapper, hook or replaced `forward`), so that its
-  product may run fused with another."""
-  return (type(m) is Linear and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__ and
-          not _hooks._global_forward_hooks and not _hooks._global_forward_pre_hooks)
+  """Whether calling `m` is `OF.linear` and nothing else (no subclass, wrapper, replaced `forward` or hook of any kind that
+  `nn.Module.__call__` looks at), so that its product may run fused with another."""
+  if type(m) is not Linear or Linear.forward is not _LINEAR_FORWARD:
+    return False
+  d = m.__dict__
+  return not ("forward" in d or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or
+              _module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks or
+              _module._global_backward_pre_hooks)
 
 
 def project_gated_residual(proj: nn.Module, x, residual, gate):
