@@ -87,7 +87,7 @@ class Attention(nn.Module):
   def forward(self, x, context=None, residual=None):
     ctx = x if context is None else context
     B, S, C = x.shape
-    if is_plain_linear(self.to_q) and is_plain_linear(self.to_k) and is_plain_linear(self.to_v):
+    if all(is_plain_linear(m) and m.bias is None for m in (self.to_q, self.to_k, self.to_v)):  # `linear_group` adds no bias
       if context is None:
         q, k, v = OF.linear_group(x, (self.to_q.weight, self.to_k.weight, self.to_v.weight))
       else:

@@ -65,3 +65,16 @@ def test_a_replaced_forward_runs(monkeypatch):
   monkeypatch.setattr(layers.Linear, "forward", lambda self, *a, **k: (seen.append(self), forward(self, *a, **k))[1])
   ff(attn(x, ctx))
   assert {id(m) for m in seen} == {id(m) for m in _parts(attn, ff).values()}
+
+
+@pytest.mark.parametrize("which", ["to_q", "to_v"])  # a bias of the keys moves all scores of a row alike
+@pytest.mark.parametrize("cross", [False, True])
+def test_a_bias_put_on_a_projection_is_added(which, cross):
+  torch.manual_seed(1)
+  attn, x = U.Attention(16, 2), torch.randn(2, 5, 16)
+  ctx = torch.randn(2, 7, 16) if cross else None
+  getattr(attn, which).bias = torch.nn.Parameter(torch.randn(16))
+  src = x if ctx is None else ctx
+  q, k, v = (t.unflatten(-1, (2, 8)) for t in (attn.to_q(x), attn.to_k(src), attn.to_v(src)))
+  want = attn.to_out[0](U.OF.attention(q, k, v).reshape(2, 5, 16))
+  torch.testing.assert_close(attn(x, ctx), want, rtol=1e-6, atol=1e-6)  # the same fp32 products
