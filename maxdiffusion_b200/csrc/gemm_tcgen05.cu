@@ -658,7 +658,8 @@ extern "C" int mdb_gemm_epilogue_mode(int mode) {
 
 // C entry point. A is [M,K] with leading dimension lda (a_mn_major = 0) or [K,M] (a_mn_major = 1);
 // B is [N,K] (b_mn_major = 0) or [K,N] (b_mn_major = 1). All leading dimensions are in elements and
-// must be multiples of 8; N must be a multiple of 8. Returns 0 or a CUDA / encoder error code.
+// must be multiples of 8; N must be a multiple of 8; out, residual and gate start on 16-byte boundaries (they are moved 16
+// bytes at a time). Returns 0 or a CUDA / encoder error code.
 //
 // The launch shape is the caller's (`ops/kernels.py: gemm_plan`): `ctas` per tile (1 or 2), tile width `bn` (64, 128, 192
 // or 256; a transposed B needs a multiple of 64 columns per CTA), and `splits` of the contraction, which run as separate
@@ -675,6 +676,9 @@ extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void
   if ((N & 7) || (lda & 7) || (ldb & 7) || (ldo & 3) || (!out_f32 && (ldo & 7))) return 3001;
   if ((epi == kEpiGatedRes || epi == kEpiAddRes) && (!residual || (ldr & 7))) return 3002;
   if (epi == kEpiGatedRes && (!gate || (gate_ld & 3))) return 3003;
+  const auto misaligned = [](const void* t) { return (reinterpret_cast<uintptr_t>(t) & 15) != 0; };
+  if (misaligned(out) || misaligned(partial)) return 3006;
+  if ((epi == kEpiGatedRes || epi == kEpiAddRes) && (misaligned(residual) || (epi == kEpiGatedRes && misaligned(gate)))) return 3006;
   if ((ctas != 1 && ctas != 2) || (bn != 64 && bn != 128 && bn != 192 && bn != 256)) return 3004;
   if (splits < 1 || splits > 64 || (splits > 1 && partial == nullptr)) return 3005;
   const int bn_cta = bn / ctas;

@@ -83,6 +83,8 @@ bool bf16(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloa
 bool f32(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat; }
 const void* data(const Tensor* t) { return t ? t->data_ptr() : nullptr; }
 
+// What the kernels' 16-byte accesses need of a row-major bf16 matrix.
+bool aligned16(const Tensor& t, int64_t pitch) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 && (pitch & 7) == 0; }
 // All axes but the last as rows of one pitch. False: not that layout.
 bool rows_of(const Tensor& t, int64_t& rows, int64_t& pitch) {
   const int64_t n = t.dim();
@@ -162,7 +164,8 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t Kb = b_mn ? B.size(0) : B.size(1), N = b_mn ? B.size(1) : B.size(0);
   if (K != Kb || M <= 0 || N <= 0 || K <= 0 || M > INT_MAX || N > INT_MAX || K > INT_MAX) return not_implemented();
   if (bias && (!bf16(*bias) || !bias->is_contiguous())) return not_implemented();
-  if (residual && (!bf16(*residual) || residual->dim() != 2 || residual->stride(1) != 1)) return not_implemented();
+  if (residual && (!bf16(*residual) || residual->dim() != 2 || residual->stride(1) != 1 || !aligned16(*residual, residual->stride(0))))
+    return not_implemented();
   if (gate && (!f32(*gate) || gate->stride(-1) != 1)) return not_implemented();
   if (given && (!given->is_cuda() || given->dim() != 2 || given->size(0) != M || given->size(1) != N || given->stride(1) != 1))
     return not_implemented();
@@ -198,7 +201,8 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t K = x.size(-1), N = w.size(0);
   if (w.size(1) != K || N <= 0 || K <= 0 || M > INT_MAX || N > INT_MAX || K > INT_MAX) return not_implemented();
   if (bias && (!bf16(*bias) || !bias->is_contiguous() || bias->numel() != N)) return not_implemented();
-  if (residual && (!bf16(*residual) || !rows_of(*residual, Mr, ldr) || Mr != M || residual->size(-1) != N)) return not_implemented();
+  if (residual && (!bf16(*residual) || !rows_of(*residual, Mr, ldr) || Mr != M || residual->size(-1) != N || !aligned16(*residual, ldr)))
+    return not_implemented();
   std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = N;
   const Tensor out = at::empty(sizes, x.options());

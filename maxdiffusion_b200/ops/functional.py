@@ -106,6 +106,12 @@ class remat:
 # ---------------------------------------------------------------------------------------------
 # linear (+ bias, + GELU-tanh / SiLU), the GEMM family
 # ---------------------------------------------------------------------------------------------
+def _residual_rows(residual: torch.Tensor, n: int) -> torch.Tensor:
+  """The residual as a dense [rows, n] that the GEMM epilogue can read 16 bytes at a time: itself, or a copy."""
+  r2 = residual.reshape(-1, n)
+  return r2 if r2.is_contiguous() and r2.data_ptr() % 16 == 0 else r2.clone(memory_format=torch.contiguous_format)
+
+
 class _LinearFn(torch.autograd.Function):
 
   @staticmethod
@@ -117,8 +123,7 @@ class _LinearFn(torch.autograd.Function):
     ctx.has_bias = b is not None
     if residual is not None:
       # y = residual + x W^T + b: the add rides in the GEMM epilogue; its gradient is dy itself
-      r2 = residual.reshape(-1, w.shape[0])
-      y = K.gemm(x2, w, bias=b, epi="add_res", residual=r2 if r2.is_contiguous() else r2.contiguous())
+      y = K.gemm(x2, w, bias=b, epi="add_res", residual=_residual_rows(residual, w.shape[0]))
       ctx.save_for_backward(x2, w, None)
     elif act in ("gelu_tanh",) and need_grad:
       u = K.gemm(x2, w, bias=b)
@@ -168,8 +173,7 @@ def linear(x, weight, bias=None, activation: str | None = None, residual=None):
       if residual is None:
         y = K.gemm(x2, weight, bias=bias, epi=activation or "none")
       elif activation is None and residual.dtype == torch.bfloat16:
-        r2 = residual.reshape(-1, n)
-        y = K.gemm(x2, weight, bias=bias, epi="add_res", residual=r2 if r2.is_contiguous() else r2.contiguous())
+        y = K.gemm(x2, weight, bias=bias, epi="add_res", residual=_residual_rows(residual, n))
       else:
         return residual + K.gemm(x2, weight, bias=bias, epi=activation or "none").view(*x.shape[:-1], n)
       return y.view(*x.shape[:-1], n)

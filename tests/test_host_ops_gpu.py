@@ -45,6 +45,23 @@ def test_linear(monkeypatch, form, act):
   x, w, b = _FORMS[form](), _randn(72, 64), _randn(72)
   res = _randn(*x.shape[:-1], 72) if act == "residual" else None
   used = _both(monkeypatch, lambda: OF.linear(x, w, b, None if res is not None else act, residual=res))
+@pytest.mark.parametrize("name,cut", [("odd offset", lambda t: t[..., 4:76]), ("odd pitch", lambda t: t[..., :72]), ("misaligned", None),
+                                      ("in place", lambda t: t[..., 8:80])])
+def test_linear_residual_layouts(monkeypatch, name, cut):
+  """A residual that cannot be read 16 bytes at a time where it lies is copied, with and without the extension and autograd."""
+  torch.manual_seed(7)
+  x, w, b = _randn(3, 40, 64), _randn(72, 64), _randn(72)
+  if cut is None:  # dense, but it starts 8 bytes into its storage
+    res = _randn(3 * 40 * 72 + 4)[4:].view(3, 40, 72)
+  else:
+    res = cut(_randn(3, 40, {"odd offset": 80, "odd pitch": 76, "in place": 80}[name]))
+  want = OF.linear(x, w, b, residual=res.clone(memory_format=torch.contiguous_format))
+  _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res))
+  with torch.enable_grad():
+    got = OF.linear(x, torch.nn.Parameter(w), b, residual=res)
+    assert torch.equal(got, want)
+
+
   assert used or form in ("transposed", "part of a sequence", "expanded", "columns apart")
   _both(monkeypatch, lambda: OF.linear(x, w[::2], None))  # a strided weight
   if res is not None:
