@@ -152,13 +152,7 @@ class FluxDoubleBlock(nn.Module):
     qt, kt, vt = split_fused(self.add_qkv_proj(OF.layer_norm_mod(txt, scale=sc_t, shift=sh_t)), 3)
     q = OF.joint_norm_rope([(qt, self.norm_added_q, *rope_txt), (qi, self.norm_q, *rope_img)], H)
     k = OF.joint_norm_rope([(kt, self.norm_added_k, *rope_txt), (ki, self.norm_k, *rope_img)], H)
-    if torch.is_grad_enabled():
-      v = torch.cat([vt, vi], dim=1).unflatten(-1, (H, C // H))
-    else:  # two strided copies: a concatenation of slices runs at a fifth of the memory's rate
-      v = torch.empty((B, St + Si, C), device=vi.device, dtype=vi.dtype)
-      v[:, :St].copy_(vt)
-      v[:, St:].copy_(vi)
-      v = v.unflatten(-1, (H, C // H))
+    v = OF.joint_rows([vt, vi]).unflatten(-1, (H, C // H))
     o = OF.attention(q, k, v).reshape(B, St + Si, C)
     ot, oi = o[:, :St], o[:, St:]
     # projections are called as modules so that wrappers (run-time LoRA adapters, quantised layers) take effect; a

@@ -469,6 +469,20 @@ def joint_norm_rope(parts, heads: int, eps: float = 1e-6):
   return torch.cat([rms_norm_rope(x, w, cos, sin, heads=heads, per_head=True, eps=eps) for x, w, cos, sin in parts], dim=1)
 
 
+def joint_rows(parts):
+  """`torch.cat(parts, dim=1)` of [B, S_i, C]. Bf16 slices of wider buffers are copied one by one where nothing works through
+  autograd or a transform: the concatenation of slices runs at a fifth of the memory's rate."""
+  x0 = parts[0]
+  if all(_fast(t) and t.shape[0] == x0.shape[0] and t.shape[2] == x0.shape[2] for t in parts) and _direct(*parts):
+    out = torch.empty((x0.shape[0], sum(t.shape[1] for t in parts), x0.shape[2]), device=x0.device, dtype=x0.dtype)
+    at = 0
+    for t in parts:
+      out[:, at:at + t.shape[1]].copy_(t)
+      at += t.shape[1]
+    return out
+  return torch.cat(parts, dim=1)
+
+
 # ---------------------------------------------------------------------------------------------
 # elementwise
 # ---------------------------------------------------------------------------------------------
