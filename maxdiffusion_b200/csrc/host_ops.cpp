@@ -1,9 +1,10 @@
 // Host side of the ops that are launched hundreds of times per model call, as a CPython extension: shape checks, output
 // allocation, launch shape and the call of the C entry point, without ctypes (which converts 20 to 30 arguments per launch
 // one by one). Same kernels, same results and the same current stream as the Python wrappers in `ops/kernels.py` and
-// `ops/conv.py`, which remain the full interface: a function here returns NotImplemented for every input that it does not
-// handle (another layout, dtype or device), and the caller goes on with the Python wrapper, which then also raises what
-// there is to raise.
+// `ops/conv.py`, which take every call: a function here returns NotImplemented for every input that it does not handle
+// (another layout, dtype or device), and the caller goes on with the Python wrapper, which then also raises what there is to
+// raise. `linear_group` and `geglu_linear` have no wrapper of their own: without them the caller runs one product per matrix,
+// and the product and GEGLU as two kernels.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -82,9 +83,9 @@ bool opt_tensor(PyObject* o, const Tensor*& t) {
 bool bf16(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; }
 bool f32(const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat; }
 const void* data(const Tensor* t) { return t ? t->data_ptr() : nullptr; }
-
 // What the kernels' 16-byte accesses need of a row-major bf16 matrix.
 bool aligned16(const Tensor& t, int64_t pitch) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 && (pitch & 7) == 0; }
+
 // All axes but the last as rows of one pitch. False: not that layout.
 bool rows_of(const Tensor& t, int64_t& rows, int64_t& pitch) {
   const int64_t n = t.dim();

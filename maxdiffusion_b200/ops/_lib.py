@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+import warnings
 from pathlib import Path
 
 import torch
@@ -57,14 +58,44 @@ def lib() -> ctypes.CDLL:
           raise KernelError(f"{LIB_PATH} is missing; run `python -m maxdiffusion_b200.build`")
         from maxdiffusion_b200 import build as _build
 
-        _build.build(verbose=False)
+        _build.build_kernels(verbose=False)
       _LIB = ctypes.CDLL(str(LIB_PATH))
       _declare(_LIB)
   return _LIB
 
 
+class _NoHostOps:
+  """Stands where the host extension cannot be had: takes no call, so each goes on to the ctypes wrappers."""
+
+  def launches(self) -> int:
+    return 0
+
+  def __getattr__(self, name):
+    return lambda *args: NotImplemented
+
+
+def _load_host_ops():
+  import importlib.util
+
+  from . import kernels
+
+  path = LIB_PATH.with_name("_host_ops.so")
+  if not path.exists():
+    if os.environ.get("MDB200_NO_AUTOBUILD") == "1":
+      raise KernelError(f"{path} is missing; run `python -m maxdiffusion_b200.build`")
+    from maxdiffusion_b200 import build as _build
+
+    _build.build_host_ops(verbose=False)
+  spec = importlib.util.spec_from_file_location("_host_ops", path)
+  mod = importlib.util.module_from_spec(spec)
+  spec.loader.exec_module(mod)
+  mod.setup(KernelError, kernels.gemm_plan)
+  return mod
+
+
 def host_ops():
-  """The CPython extension over the kernel library (`csrc/host_ops.cpp`), or None where there is no GPU."""
+  """The CPython extension over the kernel library (`csrc/host_ops.cpp`), or None where there is no GPU. Where it is missing
+  and cannot be built, or does not load, the ops run on the same kernels through the ctypes wrappers, with one warning."""
   global _HOST
   if _HOST is None:
     if not torch.cuda.is_available():
@@ -72,22 +103,11 @@ def host_ops():
     lib()
     with _LOCK:
       if _HOST is None:
-        import importlib.util
-
-        from . import kernels
-
-        path = LIB_PATH.with_name("_host_ops.so")
-        if not path.exists():
-          if os.environ.get("MDB200_NO_AUTOBUILD") == "1":
-            raise KernelError(f"{path} is missing; run `python -m maxdiffusion_b200.build`")
-          from maxdiffusion_b200 import build as _build
-
-          _build.build(verbose=False)
-        spec = importlib.util.spec_from_file_location("_host_ops", path)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
-        mod.setup(KernelError, kernels.gemm_plan)
-        _HOST = mod
+        try:
+          _HOST = _load_host_ops()
+        except (RuntimeError, ImportError, OSError) as e:
+          warnings.warn(f"no host extension: calls of the kernel library take more host time ({e})", RuntimeWarning, stacklevel=2)
+          _HOST = _NoHostOps()
   return _HOST
 
 

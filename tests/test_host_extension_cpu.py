@@ -1,0 +1,53 @@
+"""Loading of the host extension: what happens where it cannot be had."""
+import warnings
+
+import pytest
+import torch
+
+from maxdiffusion_b200 import build
+from maxdiffusion_b200.ops import _lib
+
+
+@pytest.fixture
+def fresh(monkeypatch, tmp_path):
+  """A GPU machine, as far as the loader can see, with an empty folder in place of the package's."""
+  monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+  monkeypatch.setattr(_lib, "lib", lambda: None)
+  monkeypatch.setattr(_lib, "_HOST", None)
+  monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "_kernels.so")
+  monkeypatch.delenv("MDB200_NO_AUTOBUILD", raising=False)
+  return tmp_path
+
+
+def _takes_nothing():
+  with pytest.warns(RuntimeWarning, match="host extension"):
+    host = _lib.host_ops()
+  assert host.linear(1, 2) is NotImplemented and host.conv() is NotImplemented and host.launches() == 0
+  with warnings.catch_warnings():
+    warnings.simplefilter("error")
+    assert _lib.host_ops() is host  # said once
+  assert _lib.launch_count() == _lib._launches
+
+
+def test_missing_and_not_to_be_built(fresh, monkeypatch):
+  monkeypatch.setenv("MDB200_NO_AUTOBUILD", "1")
+  _takes_nothing()
+
+
+def test_a_machine_that_cannot_compile_it(fresh, monkeypatch):
+  def fail(*a, **k):
+    raise RuntimeError("host_ops.cpp: g++ failed")
+  monkeypatch.setattr(build, "build_host_ops", fail)
+  _takes_nothing()
+
+
+def test_no_compiler_at_all(fresh, monkeypatch):
+  def fail(*a, **k):
+    raise FileNotFoundError("g++")
+  monkeypatch.setattr(build, "build_host_ops", fail)
+  _takes_nothing()
+
+
+def test_an_object_that_does_not_load(fresh):
+  (fresh / "_host_ops.so").write_bytes(b"not a shared object")
+  _takes_nothing()

@@ -8,20 +8,13 @@ from maxdiffusion_b200.ops import _lib, conv as OC, functional as OF, kernels as
 pytestmark = pytest.mark.gpu
 
 
-class _Nothing:
-  """Takes nothing: every call goes on to the Python wrappers."""
-
-  def __getattr__(self, name):
-    return lambda *a: NotImplemented
-
-
 def _both(monkeypatch, fn):
   with torch.no_grad():
     before = _lib.host_ops().launches()
     got = fn()
     used = _lib.host_ops().launches() > before
     with monkeypatch.context() as m:
-      m.setattr(_lib, "host_ops", lambda: _Nothing())
+      m.setattr(_lib, "_HOST", _lib._NoHostOps())
       want = fn()
   assert torch.equal(got, want) and got.shape == want.shape and got.stride() == want.stride() and got.dtype == want.dtype
   return used
@@ -45,6 +38,13 @@ def test_linear(monkeypatch, form, act):
   x, w, b = _FORMS[form](), _randn(72, 64), _randn(72)
   res = _randn(*x.shape[:-1], 72) if act == "residual" else None
   used = _both(monkeypatch, lambda: OF.linear(x, w, b, None if res is not None else act, residual=res))
+  assert used or form in ("transposed", "part of a sequence", "expanded", "columns apart")
+  _both(monkeypatch, lambda: OF.linear(x, w[::2], None))  # a strided weight
+  if res is not None:
+    _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.transpose(0, 1).contiguous().transpose(0, 1)))
+    _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.float()))
+
+
 @pytest.mark.parametrize("name,cut", [("odd offset", lambda t: t[..., 4:76]), ("odd pitch", lambda t: t[..., :72]), ("misaligned", None),
                                       ("in place", lambda t: t[..., 8:80])])
 def test_linear_residual_layouts(monkeypatch, name, cut):
@@ -60,13 +60,6 @@ def test_linear_residual_layouts(monkeypatch, name, cut):
   with torch.enable_grad():
     got = OF.linear(x, torch.nn.Parameter(w), b, residual=res)
     assert torch.equal(got, want)
-
-
-  assert used or form in ("transposed", "part of a sequence", "expanded", "columns apart")
-  _both(monkeypatch, lambda: OF.linear(x, w[::2], None))  # a strided weight
-  if res is not None:
-    _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.transpose(0, 1).contiguous().transpose(0, 1)))
-    _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.float()))
 
 
 _FORMS["more than a tile"] = lambda: _randn(3, 87, 64)
@@ -169,3 +162,16 @@ def test_direct_calls_leave_autograd_alone():
   y = OF.checkpoint_block(lambda t: (store.append(OF._direct(t)), OF.linear(t, w))[1], x.requires_grad_())
   y.float().sum().backward()
   assert store == [False, False] and w.grad is not None
+
+
+def test_fused_calls_without_the_extension(monkeypatch):
+  torch.manual_seed(8)
+  x, w, b, ws = _randn(3, 87, 64), _randn(272, 64), _randn(272), [_randn(72, 64) for _ in range(3)]
+  monkeypatch.setattr(_lib, "_HOST", _lib._NoHostOps())
+  with torch.no_grad():
+    u = x.double() @ w.double().t() + b.double()
+    want = u[..., :136] * torch.nn.functional.gelu(u[..., 136:])
+    assert (OF.geglu_linear(x, w, b).double() - want).norm() < 8e-3 * want.norm()  # the product is rounded in between
+    for got, m in zip(OF.linear_group(x, ws), ws):
+      want = x.double() @ m.double().t()
+      assert (got.double() - want).norm() < 4e-3 * want.norm()
