@@ -21,6 +21,7 @@ SRC_DIR = PKG_DIR / "csrc"
 OBJ_DIR = PKG_DIR / "csrc" / "build"
 LIB_PATH = PKG_DIR / "_kernels.so"
 HOST_PATH = PKG_DIR / "_host_ops.so"  # CPython extension over the kernel library (csrc/host_ops.cpp)
+HOST_FOR = "_host_ops.for"  # beside it: what it was built for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -94,6 +95,13 @@ def build_kernels(verbose: bool = True, force: bool = False) -> Path:
   return LIB_PATH
 
 
+def host_ops_target() -> str:
+  """What the extension's binary interface depends on: the versions of PyTorch and of Python."""
+  import torch
+
+  return f"PyTorch {torch.__version__}, Python {sys.version.split()[0]}"
+
+
 def build_host_ops(verbose: bool = True, force: bool = False) -> None:
   """Compiles csrc/host_ops.cpp against the installed PyTorch and links it to `_kernels.so` beside it."""
   import sysconfig
@@ -105,7 +113,8 @@ def build_host_ops(verbose: bool = True, force: bool = False) -> None:
   src, obj, stamp = SRC_DIR / "host_ops.cpp", OBJ_DIR / "host_ops.o", OBJ_DIR / "host_ops.sha"
   flags = ["-std=c++17", "-O2", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
   digest = hashlib.sha256(" ".join([torch.__version__, sys.version, *flags]).encode() + src.read_bytes()).hexdigest()
-  if force or not HOST_PATH.exists() or not stamp.exists() or stamp.read_text() != digest:
+  target = HOST_PATH.with_name(HOST_FOR)
+  if force or not HOST_PATH.exists() or not target.exists() or not stamp.exists() or stamp.read_text() != digest:
     inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda / "include"]
     libs = ["-L", str(PKG_DIR), "-l:_kernels.so", "-Wl,-rpath,$ORIGIN", "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu",
             "-ltorch", "-lc10_cuda", "-lc10"]  # PyTorch's libraries are loaded before this one: no run path to them
@@ -115,6 +124,7 @@ def build_host_ops(verbose: bool = True, force: bool = False) -> None:
       if res.returncode != 0:
         raise RuntimeError(f"{src.name}: {' '.join(cmd[:2])} failed:\n{res.stdout}\n{res.stderr}")
     stamp.write_text(digest)
+    target.write_text(host_ops_target())
     if verbose:
       print(f"[build] linked {HOST_PATH}")
 

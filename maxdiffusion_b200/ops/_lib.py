@@ -77,14 +77,14 @@ class _NoHostOps:
 def _load_host_ops():
   import importlib.util
 
+  from maxdiffusion_b200 import build as _build
   from . import kernels
 
-  path = LIB_PATH.with_name("_host_ops.so")
-  if not path.exists():
+  path, target = LIB_PATH.with_name("_host_ops.so"), LIB_PATH.with_name(_build.HOST_FOR)
+  built_for = target.read_text() if path.exists() and target.exists() else None
+  if built_for != _build.host_ops_target():  # missing, or built against another PyTorch or Python: it must not be loaded
     if os.environ.get("MDB200_NO_AUTOBUILD") == "1":
-      raise KernelError(f"{path} is missing; run `python -m maxdiffusion_b200.build`")
-    from maxdiffusion_b200 import build as _build
-
+      raise KernelError(f"{path} is {'missing' if built_for is None else f'for {built_for}'}; run `python -m maxdiffusion_b200.build`")
     _build.build_host_ops(verbose=False)
   spec = importlib.util.spec_from_file_location("_host_ops", path)
   mod = importlib.util.module_from_spec(spec)

@@ -1,4 +1,5 @@
 """Loading of the host extension: what happens where it cannot be had."""
+import importlib.util
 import warnings
 
 import pytest
@@ -50,4 +51,29 @@ def test_no_compiler_at_all(fresh, monkeypatch):
 
 def test_an_object_that_does_not_load(fresh):
   (fresh / "_host_ops.so").write_bytes(b"not a shared object")
+  (fresh / build.HOST_FOR).write_text(build.host_ops_target())
   _takes_nothing()
+
+
+@pytest.mark.parametrize("built_for", [None, "PyTorch 2.0.0, Python 3.8.1"])
+def test_an_object_for_another_pytorch_is_rebuilt_and_not_loaded(fresh, monkeypatch, built_for):
+  (fresh / "_host_ops.so").write_bytes(b"an object")
+  if built_for is not None:
+    (fresh / build.HOST_FOR).write_text(built_for)
+  asked, load = [], importlib.util.spec_from_file_location
+
+  def refuse(name, *a, **k):
+    assert name != "_host_ops", "loaded"
+    return load(name, *a, **k)
+  monkeypatch.setattr(importlib.util, "spec_from_file_location", refuse)
+
+  def fail(*a, **k):
+    asked.append(1)
+    raise RuntimeError("no compiler")
+  monkeypatch.setattr(build, "build_host_ops", fail)
+  _takes_nothing()
+  assert asked == [1]
+  monkeypatch.setenv("MDB200_NO_AUTOBUILD", "1")
+  monkeypatch.setattr(_lib, "_HOST", None)
+  _takes_nothing()
+  assert asked == [1]
