@@ -28,6 +28,11 @@ NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo", "--use_fast_math",
     "-Xcompiler", "-fPIC", "-Xptxas", "-v",
 ]
+PRECISE = {"softmax_split.cu"}  # built without --use_fast_math
+
+
+def _flags(src: Path) -> list[str]:
+  return [f for f in NVCC_FLAGS if f != "--use_fast_math" or src.name not in PRECISE]
 
 
 def _nvcc() -> str:
@@ -39,7 +44,7 @@ def _nvcc() -> str:
 
 def _digest(path: Path) -> str:
   h = hashlib.sha256()
-  h.update(" ".join(NVCC_FLAGS).encode())
+  h.update(" ".join(_flags(path)).encode())
   h.update(path.read_bytes())
   for hdr in sorted(SRC_DIR.glob("*.cuh")) + sorted(SRC_DIR.glob("*.h")):
     h.update(hdr.read_bytes())
@@ -52,7 +57,7 @@ def _compile_one(src: Path, verbose: bool) -> Path:
   digest = _digest(src)
   if obj.exists() and stamp.exists() and stamp.read_text() == digest:
     return obj
-  cmd = [_nvcc(), *NVCC_FLAGS, "-I", str(SRC_DIR), "-c", str(src), "-o", str(obj)]
+  cmd = [_nvcc(), *_flags(src), "-I", str(SRC_DIR), "-c", str(src), "-o", str(obj)]
   res = subprocess.run(cmd, capture_output=True, text=True)
   log = OBJ_DIR / (src.stem + ".ptxas.log")
   log.write_text(res.stdout + res.stderr)

@@ -626,61 +626,8 @@ softmax_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_bfl
   }
 }
 
-// Row softmax of fp32 scores whose result keeps its 24 bits: y = p0 + p1 + p2, three bf16 planes of `pitch` columns side by
-// side, so that a bf16 product with a matrix stacked three times accumulates fp32 probabilities. Columns from `cols` to
-// `pitch` are zeros. The row waits in shared memory between the passes; memory bound (one read of 4 bytes, one write of 6).
-__global__ void __launch_bounds__(SM_THREADS)
-softmax_split_kernel(const float* __restrict__ x, long long ldx, __nv_bfloat16* __restrict__ y, long long ldy, int cols, int pitch) {
-  extern __shared__ float row_s[];
-  __shared__ float red[SM_THREADS / 32];
-  const float* src = x + static_cast<long long>(blockIdx.x) * ldx;
-  __nv_bfloat16* dst = y + static_cast<long long>(blockIdx.x) * ldy;
-  float mx = -INFINITY;
-  for (int c = threadIdx.x; c < cols; c += SM_THREADS) {
-    const float v = src[c];
-    row_s[c] = v;
-    mx = fmaxf(mx, v);
-  }
-  mx = block_reduce(mx, true, red);
-  float sum = 0.0f;
-  for (int c = threadIdx.x; c < cols; c += SM_THREADS) {
-    // exp(v) as 2^t (1 + e): t the rounded product with log2 e, e what the rounding left
-    const float v = row_s[c] - mx;
-    const float t = v * 1.4426950408889634f;
-    const float e = fmaf(v, 1.4426950408889634f, -t) + v * 1.9259629911e-8f;
-    const float p = fast_exp2(t) * fmaf(e, 0.6931471805599453f, 1.0f);
-    row_s[c] = p;
-    sum += p;
-  }
-  sum = block_reduce(sum, false, red);
-  const float inv = 1.0f / sum;
-  for (int c = threadIdx.x; c < pitch; c += SM_THREADS) {
-    const float p = c < cols ? row_s[c] * inv : 0.0f;
-    const __nv_bfloat16 p0 = __float2bfloat16(p);
-    const float r1 = p - __bfloat162float(p0);
-    const __nv_bfloat16 p1 = __float2bfloat16(r1);
-    dst[c] = p0;
-    dst[pitch + c] = p1;
-    dst[2 * pitch + c] = __float2bfloat16(r1 - __bfloat162float(p1));
-  }
-}
-
 }  // namespace cln
 }  // namespace mdb
-
-// x fp32 [rows, cols] (row pitch ldx) -> y bf16 [rows, 3 * pitch] (row pitch ldy): see softmax_split_kernel.
-extern "C" int mdb_softmax_split(const float* x, long long ldx, void* y, long long ldy, long long rows, int cols, int pitch,
-                                 void* stream) {
-  using namespace mdb::cln;
-  if (rows <= 0 || cols <= 0) return 0;
-  if (pitch < cols || cols > 32768 || ldy < 3ll * pitch || rows > 0x7fffffff) return 3705;
-  const size_t smem = static_cast<size_t>(cols) * sizeof(float);
-  if (smem > 40 * 1024)
-    MDB_CHECK_CUDA(cudaFuncSetAttribute(softmax_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
-  softmax_split_kernel<<<static_cast<unsigned int>(rows), SM_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(
-      x, ldx, static_cast<__nv_bfloat16*>(y), ldy, cols, pitch);
-  return static_cast<int>(cudaGetLastError());
-}
 
 // x, y: bf16 [rows, cols] with leading dimensions ldx / ldy (multiples of 8); cols a multiple of 8, at most 32768.
 extern "C" int mdb_softmax_rows(const void* x, long long ldx, void* y, long long ldy, long long rows, int cols, void* stream) {

@@ -649,6 +649,17 @@ def softmax_rows(x: torch.Tensor) -> torch.Tensor:
   return x
 
 
+def softmax_split(scores: torch.Tensor, cols: int) -> torch.Tensor:
+  """Row softmax over the first `cols` columns of fp32 scores [rows, pitch], as three bf16 planes [rows, 3 * pitch] that add up
+  to the fp32 probabilities; the columns from `cols` on are zeros."""
+  rows, pitch = scores.shape
+  assert scores.dtype == torch.float32 and scores.stride(1) == 1 and 0 < cols <= pitch
+  parts = torch.empty((rows, 3 * pitch), dtype=torch.bfloat16, device=scores.device)
+  rc = _lib.lib().mdb_softmax_split(_lib.ptr(scores), scores.stride(0), _lib.ptr(parts), parts.stride(0), rows, cols, pitch, _lib.stream())
+  _lib.check(rc, "mdb_softmax_split")
+  return parts
+
+
 def wide_head_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional[float] = None) -> torch.Tensor:
   """Single-head attention for head sizes the flash kernels are not built for (q, k, v: [T, D], D a multiple of 8):
   scores on the tcgen05 GEMM, row softmax, P V on the GEMM. The score matrix is materialised in bf16 ([T, T]), which
@@ -680,9 +691,7 @@ def _odd_head_attention(q, k, v, scale):
   kp = torch.zeros((pitch, D), dtype=k.dtype, device=k.device)
   kp[:T] = k
   scores = K.gemm(q.contiguous(), kp, alpha=scale, out_dtype=torch.float32)  # [T, pitch]
-  parts = torch.empty((T, 3 * pitch), dtype=torch.bfloat16, device=q.device)
-  rc = _lib.lib().mdb_softmax_split(_lib.ptr(scores), scores.stride(0), _lib.ptr(parts), parts.stride(0), T, T, pitch, _lib.stream())
-  _lib.check(rc, "mdb_softmax_split")
+  parts = softmax_split(scores, T)
   v3 = torch.zeros((3, pitch, D), dtype=v.dtype, device=v.device)
   v3[:, :T] = v
   return K.gemm(parts, v3.view(3 * pitch, D), b_mn=True)

@@ -131,3 +131,27 @@ def test_wide_head_attention_of_odd_lengths(T, D):
   s = (q.double() @ k.double().t()) * D ** -0.5
   with torch.no_grad():
     assert _rel(C.wide_head_attention(q, k, v), s.softmax(-1) @ v.double()) < 2e-3
+
+
+@pytest.mark.parametrize("cols,pitch", [(1, 8), (7, 8), (255, 256), (4500, 4504), (9001, 9008), (32767, 32768)])
+def test_softmax_in_three_planes(cols, pitch):
+  """Against float64, probability by probability: in units of 2^-24 the rounded difference to the maximum costs |v|,
+  expf (2 ulp) and the division 5, the additions of the sum one each (cols / 256 + 13) and the third plane's rounding 1."""
+  torch.manual_seed(7)
+  x = torch.randn(9, pitch, device="cuda") * 8
+  x[1, : cols // 2] = -float("inf")  # what an overflowing product of finite values leaves
+  x[2, : cols // 2] = -3e38
+  x[3, : cols // 2] = -3.4e38
+  x[3, cols - 1] = 3.4e38
+  x[4, 0] = float("nan")
+  x[5, cols - 1] = float("inf")
+  x[6] = -float("inf")
+  x[:, cols:] = float("nan")  # not read
+  got = C.softmax_split(x, cols).view(9, 3, pitch)
+  assert not got[:, :, cols:].any()
+  p, want = got[:, :, :cols].double().sum(1), x[:, :cols].double().softmax(-1)
+  assert torch.equal(p.isnan(), x[:, :cols].softmax(-1).isnan())
+  ok = [0, 1, 2, 3, 7, 8]
+  v = (x[ok, :cols].double() - x[ok, :cols].double().amax(-1, keepdim=True)).clamp(min=-100)
+  bound = (v.abs() + 24 + cols / 256) * 2.0 ** -24 * want[ok] + 2.0 ** -133  # below that bf16 has no values left
+  assert ((p[ok] - want[ok]).abs() <= bound).all()
