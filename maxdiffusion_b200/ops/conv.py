@@ -668,8 +668,7 @@ def wide_head_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale
 
   T, D = q.shape
   scale = scale if scale is not None else D ** -0.5
-  if use_kernel(q) and T % 8 and D % 8 == 0 and T <= 32768 and not (torch.is_grad_enabled() and
-                                                                   (q.requires_grad or k.requires_grad or v.requires_grad)):
+  if _odd_head_ok(q, k, v):
     return _odd_head_attention(q, k, v, scale)
   if not use_kernel(q) or T % 8 or D % 8 or T > 32768:
     p = torch.softmax((q.float() @ k.float().t()) * scale, dim=-1)
@@ -677,6 +676,22 @@ def wide_head_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale
   scores = K.gemm(q.contiguous(), k.contiguous(), alpha=scale)         # [T, T] = scale * Q K^T
   softmax_rows(scores)
   return K.gemm(scores, v.contiguous(), b_mn=True)                     # [T, D] = P V   (V is [K = T, N = D])
+
+
+def _odd_head_ok(q, k, v) -> bool:
+  """Whether `_odd_head_attention` serves this call: as many keys as queries, no multiple of 8 of them, bf16 throughout, and
+  nothing that works through PyTorch's own operations (autograd, forward mode, a function transform, a tracer)."""
+  from . import functional as OF
+
+  T, D = q.shape
+  if not (T % 8 and D % 8 == 0 and T <= 32768 and k.shape == q.shape and v.dim() == 2 and v.shape[0] == T and v.shape[1] % 8 == 0):
+    return False
+  if OF.library_mode() or not all(use_kernel(t) and t.device == q.device for t in (q, k, v)):
+    return False
+  if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
+    return False
+  with torch.no_grad():
+    return OF._direct(q, k, v)
 
 
 def _odd_head_attention(q, k, v, scale):
@@ -688,13 +703,18 @@ def _odd_head_attention(q, k, v, scale):
 
   T, D = q.shape
   pitch = _round_up(T, 8)
+  q = q.contiguous()
+  if q.data_ptr() % 16:
+    q = q.clone()
   kp = torch.zeros((pitch, D), dtype=k.dtype, device=k.device)
   kp[:T] = k
-  scores = K.gemm(q.contiguous(), kp, alpha=scale, out_dtype=torch.float32)  # [T, pitch]
+  scores = K.gemm(q, kp, alpha=scale, out_dtype=torch.float32)  # [T, pitch]
   parts = softmax_split(scores, T)
-  v3 = torch.zeros((3, pitch, D), dtype=v.dtype, device=v.device)
-  v3[:, :T] = v
-  return K.gemm(parts, v3.view(3 * pitch, D), b_mn=True)
+  # an infinite or NaN value meets the first part alone: the others may be zero or negative where the probability is not
+  v3 = torch.zeros((3, pitch, v.shape[1]), dtype=v.dtype, device=v.device)
+  v3[0, :T] = v
+  v3[1:, :T] = torch.nan_to_num(v, nan=0.0, posinf=0.0, neginf=0.0)
+  return K.gemm(parts, v3.view(3 * pitch, -1), b_mn=True)
 
 
 # ---------------------------------------------------------------------------------------------

@@ -155,3 +155,21 @@ def test_softmax_in_three_planes(cols, pitch):
   v = (x[ok, :cols].double() - x[ok, :cols].double().amax(-1, keepdim=True)).clamp(min=-100)
   bound = (v.abs() + 24 + cols / 256) * 2.0 ** -24 * want[ok] + 2.0 ** -133  # below that bf16 has no values left
   assert ((p[ok] - want[ok]).abs() <= bound).all()
+
+
+def test_wide_head_attention_forms():
+  """Other numbers of keys, other widths of values, fp32 values, misaligned queries and infinite values: as plain PyTorch has it."""
+  torch.manual_seed(8)
+  T, D = 77, 64
+  q, k, v = _randn(T, D), _randn(T, D), _randn(T, D)
+  off = torch.empty(T * D + 4, device="cuda", dtype=torch.bfloat16)[4:].view(T, D).copy_(q)
+  inf = v.clone()
+  inf[3, 5], inf[4, 6], inf[70, 7] = float("inf"), -float("inf"), float("nan")
+  with torch.no_grad():
+    for a, b, c in ((q, k[:50], v[:50]), (q, k, v[:, :24]), (q, k, v.float()), (off, k, v), (q[:, ::2][:, :16], k[:, :16], v), (q, k, inf)):
+      got = C.wide_head_attention(a, b, c)
+      want = ((a.double() @ b.double().t()) * a.shape[1] ** -0.5).softmax(-1) @ c.double()
+      assert got.shape == want.shape and got.dtype == torch.bfloat16
+      bad = ~want.isfinite()
+      assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[bad].double().nan_to_num(), want[bad].nan_to_num().to(torch.bfloat16).double().nan_to_num())
+      assert _rel(got[~bad], want[~bad]) < 4e-3  # one rounding to bf16
