@@ -99,6 +99,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     assert gate.dtype == torch.float32 and gate.stride(-1) == 1
   if bias is not None:
     assert bias.dtype == torch.bfloat16 and bias.is_contiguous()
+  if out.numel() == 0:
+    return out
+  if K == 0:
+    return _empty_contraction(out, bias, epi, residual, gate, rows_per_batch)
   plain = bias is None and epi == "none" and residual is None and gate is None
   ctas, bn, splits = gemm_plan(M, N, K, b_mn, split_k == 0, _SM_COUNT, _FORCE_TILE_N, _FORCE_CTAS)
   if split_k > 0:
@@ -111,6 +115,23 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
       int(out.dtype == torch.float32), float(alpha), ctas, bn, splits, _lib.ptr(partial), _lib.stream())
   _lib.check(rc, "mdb_gemm_bf16")
   return out
+
+
+def _empty_contraction(out, bias, epi, residual, gate, rows_per_batch):
+  """`gemm` over no terms: the epilogue of a zero product."""
+  y = torch.zeros(out.shape, device=out.device, dtype=torch.float32)
+  if bias is not None:
+    y += bias
+  if epi == "gelu_tanh":
+    y = torch.nn.functional.gelu(y, approximate="tanh")
+  elif epi == "silu":
+    y = torch.nn.functional.silu(y)
+  elif epi == "gated_res":
+    rows = torch.arange(out.shape[0], device=out.device) // rows_per_batch if rows_per_batch > 0 else 0
+    y = residual + (gate[rows] if gate.dim() == 2 else gate) * y
+  elif epi == "add_res":
+    y = residual + y
+  return out.copy_(y)
 
 
 def gemm_epilogue_mode(direct: bool = False) -> None:
