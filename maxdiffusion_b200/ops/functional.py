@@ -191,7 +191,7 @@ def linear(x, weight, bias=None, activation: str | None = None, residual=None):
 def linear_group(x, weights):
   """x @ w.T for up to three weights of one shape (the projections of an attention layer), as a tuple. Without autograd they
   are one launch, and the results are slices of one buffer."""
-  if _fast(x) and x.shape[-1] % 8 == 0 and len(weights) <= 3 and _direct(x, *weights):
+  if _fast(x) and x.shape[-1] % 8 == 0 and len(weights) <= 3 and _direct(x, *weights) and not K.gemm_pinned():
     r = _lib.host_ops().linear_group(x, *weights)
     if r is not NotImplemented:
       return r.chunk(len(weights), dim=-1)
@@ -408,7 +408,7 @@ def geglu(u: torch.Tensor) -> torch.Tensor:
 
 def geglu_linear(x, weight, bias=None):
   """`geglu` of `linear`. Without autograd one kernel does both and the projection is never written."""
-  if _fast(x) and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and _direct(x, weight, bias):
+  if _fast(x) and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and _direct(x, weight, bias) and not K.gemm_pinned():
     r = _lib.host_ops().geglu_linear(x, weight, bias)
     if r is not NotImplemented:
       return r

@@ -43,7 +43,7 @@ def gemm_plan(M: int, N: int, K: int, b_mn: bool = False, splittable: bool = Tru
   fewer tiles than the GPU has SMs (few tokens; weight gradients, whose contraction is the token count), cutting the
   contraction makes more work items at the price of fp32 partials and a second kernel (3 us + their traffic): 384 x 3072 x
   15360 takes 51 us whole and 41 us in three parts. `tile_n` / `ctas` restrict the choice."""
-  best, best_cost = (1, 256, 1), None
+  best, best_cost = None, None
   num_kb = -(-K // 64)
   for (cg, bn), kb_us in _KB_US.items():
     if (ctas and cg != ctas) or (tile_n and bn != tile_n) or (b_mn and (bn // cg) % 64) or (cg == 2 and M <= 128 and not ctas):
@@ -61,6 +61,8 @@ def gemm_plan(M: int, N: int, K: int, b_mn: bool = False, splittable: bool = Tru
         cost = cost * 1.05 + 3.0 + s_eff * M * N * 8 / 6e6
       if best_cost is None or cost < best_cost - 1e-9:
         best, best_cost = (cg, bn, s_eff), cost
+  if best is None:  # a transposed B is fetched in 64-column pieces per CTA
+    raise _lib.KernelError(f"no GEMM tile {tile_n or ''} wide over {ctas} CTAs reads a transposed B")
   return best
 
 
@@ -71,6 +73,12 @@ def split_k_for(M: int, N: int, K: int, sms: int = _SM_COUNT) -> int:
 
 _FORCE_TILE_N = 0
 _FORCE_CTAS = 0
+_DIRECT_EPILOGUE = False
+
+
+def gemm_pinned() -> bool:
+  """Whether a launch shape or the epilogue is pinned: only `gemm` follows the pins, so fused products then run through it."""
+  return bool(_FORCE_TILE_N or _FORCE_CTAS or _DIRECT_EPILOGUE)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, bias=None, epi: str = "none",
@@ -136,8 +144,10 @@ def _empty_contraction(out, bias, epi, residual, gate, rows_per_batch):
 
 def gemm_epilogue_mode(direct: bool = False) -> None:
   """True pins the direct-store epilogue (16-byte stores from one thread per row); False restores the default
-  (128-byte slabs staged in shared memory and written by TMA stores). For benchmarks and tests."""
+  (slabs of 32 rows x 128 bytes that pass through shared memory and leave as full lines). For benchmarks and tests."""
+  global _DIRECT_EPILOGUE
   _lib.check(_lib.lib().mdb_gemm_epilogue_mode(int(direct)), "mdb_gemm_epilogue_mode")
+  _DIRECT_EPILOGUE = bool(direct)
 
 
 def gemm_force_tile_n(bn: int = 0) -> None:
