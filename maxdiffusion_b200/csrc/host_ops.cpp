@@ -51,7 +51,7 @@ namespace {
 
 using at::Tensor;
 
-long long g_launches = 0;        // under the GIL, like everything here
+long long g_launches = 0;        // these three and g_plans: under the GIL
 PyObject* g_error = nullptr;     // ops._lib.KernelError
 PyObject* g_plan = nullptr;      // ops.kernels.gemm_plan
 
@@ -60,6 +60,25 @@ constexpr int kCtasTarget = 148 * 4;
 PyObject* not_implemented() { Py_RETURN_NOTIMPLEMENTED; }
 
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+// Other Python threads run while this object lives: around the allocations and the entry points, which may wait for the GPU
+// (a full launch queue, the allocator). Nothing of Python's is touched meanwhile, nor what the lock guards above; a tensor
+// that Python holds is not copied. The destructor takes the lock back, also when an exception passes.
+class WithoutGil {
+ public:
+  WithoutGil() : state_(PyEval_SaveThread()) {}
+  ~WithoutGil() { PyEval_RestoreThread(state_); }
+  WithoutGil(const WithoutGil&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
+
+template <typename F>
+int unlocked(F&& f) {
+  const WithoutGil lock;
+  return f();
+}
 
 // nullptr and a Python error when the launch was refused
 PyObject* done(int rc, const char* what, const Tensor& out, int launches = 1) {
@@ -170,19 +189,23 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (gate && (!f32(*gate) || gate->stride(-1) != 1)) return not_implemented();
   if (given && (!given->is_cuda() || given->dim() != 2 || given->size(0) != M || given->size(1) != N || given->stride(1) != 1))
     return not_implemented();
-  const Tensor out = given ? *given : at::empty({M, N}, A.options().dtype(out_f32 ? at::kFloat : at::kBFloat16));
-  const bool f32_out = out.scalar_type() == at::kFloat;
-  if (!f32_out && out.scalar_type() != at::kBFloat16) return not_implemented();
+  const bool f32_out = given ? given->scalar_type() == at::kFloat : out_f32;
+  if (given && !f32_out && given->scalar_type() != at::kBFloat16) return not_implemented();
   Plan plan;
   if (!gemm_plan(M, N, K, b_mn, split_k == 0, tile_n, force_ctas, plan)) return nullptr;
   if (split_k > 0) plan.splits = (!bias && epi == 0 && !residual && !gate) ? static_cast<int>(split_k) : 1;
-  Tensor partial;
-  if (plan.splits > 1) partial = at::empty({plan.splits, M, N}, A.options().dtype(at::kFloat));
-  const int rc = mdb_gemm_bf16(A.data_ptr(), B.data_ptr(), out.data_ptr(), data(bias), data(residual), data(gate),
-                               static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), A.stride(0), B.stride(0),
-                               out.stride(0), residual ? residual->stride(0) : 0, gate && gate->dim() == 2 ? gate->stride(0) : 0,
-                               rows_per_batch, a_mn, b_mn, epi, f32_out, static_cast<float>(alpha), plan.ctas, plan.bn,
-                               plan.splits, plan.splits > 1 ? partial.data_ptr() : nullptr, stream());
+  Tensor out;
+  if (given) out = *given;
+  const int rc = unlocked([&] {
+    if (!given) out = at::empty({M, N}, A.options().dtype(f32_out ? at::kFloat : at::kBFloat16));
+    Tensor partial;
+    if (plan.splits > 1) partial = at::empty({plan.splits, M, N}, A.options().dtype(at::kFloat));
+    return mdb_gemm_bf16(A.data_ptr(), B.data_ptr(), out.data_ptr(), data(bias), data(residual), data(gate), static_cast<int>(M),
+                         static_cast<int>(N), static_cast<int>(K), A.stride(0), B.stride(0), out.stride(0),
+                         residual ? residual->stride(0) : 0, gate && gate->dim() == 2 ? gate->stride(0) : 0, rows_per_batch, a_mn,
+                         b_mn, epi, f32_out, static_cast<float>(alpha), plan.ctas, plan.bn, plan.splits,
+                         plan.splits > 1 ? partial.data_ptr() : nullptr, stream());
+  });
   return done(rc, "mdb_gemm_bf16", out);
   END_HANDLE_TH_ERRORS
 }
@@ -206,15 +229,17 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return not_implemented();
   std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = N;
-  const Tensor out = at::empty(sizes, x.options());
   Plan plan;
   if (!gemm_plan(M, N, K, false, true, tile_n, force_ctas, plan)) return nullptr;
-  Tensor partial;
-  if (plan.splits > 1) partial = at::empty({plan.splits, M, N}, x.options().dtype(at::kFloat));
-  const int rc = mdb_gemm_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), data(bias), data(residual), nullptr,
-                               static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), lda, w.stride(0), N, ldr, 0, 0, 0, 0,
-                               epi, 0, 1.0f, plan.ctas, plan.bn, plan.splits, plan.splits > 1 ? partial.data_ptr() : nullptr,
-                               stream());
+  Tensor out;
+  const int rc = unlocked([&] {
+    out = at::empty(sizes, x.options());
+    Tensor partial;
+    if (plan.splits > 1) partial = at::empty({plan.splits, M, N}, x.options().dtype(at::kFloat));
+    return mdb_gemm_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), data(bias), data(residual), nullptr, static_cast<int>(M),
+                         static_cast<int>(N), static_cast<int>(K), lda, w.stride(0), N, ldr, 0, 0, 0, 0, epi, 0, 1.0f, plan.ctas,
+                         plan.bn, plan.splits, plan.splits > 1 ? partial.data_ptr() : nullptr, stream());
+  });
   return done(rc, "mdb_gemm_bf16", out);
   END_HANDLE_TH_ERRORS
 }
@@ -234,9 +259,12 @@ PyObject* py_geglu_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (bias && (!bf16(*bias) || !bias->is_contiguous() || bias->numel() != 2 * N)) return not_implemented();
   std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = N;
-  const Tensor out = at::empty(sizes, x.options());
-  const int rc = mdb_gemm_geglu(x.data_ptr(), w.data_ptr(), out.data_ptr(), data(bias), static_cast<int>(M), static_cast<int>(N),
-                                static_cast<int>(K), lda, w.stride(0), N, stream());
+  Tensor out;
+  const int rc = unlocked([&] {
+    out = at::empty(sizes, x.options());
+    return mdb_gemm_geglu(x.data_ptr(), w.data_ptr(), out.data_ptr(), data(bias), static_cast<int>(M), static_cast<int>(N),
+                          static_cast<int>(K), lda, w.stride(0), N, stream());
+  });
   return done(rc, "mdb_gemm_geglu", out);
   END_HANDLE_TH_ERRORS
 }
@@ -261,11 +289,14 @@ PyObject* py_linear_group(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (w.size(1) != K || (N & 7) || N <= 0 || K <= 0 || M > INT_MAX || N > INT_MAX / 3 || K > INT_MAX) return not_implemented();
   std::vector<int64_t> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = mats * N;
-  const Tensor out = at::empty(sizes, x.options());
   Plan plan;
   if (!gemm_plan(M, mats * N, K, false, false, 0, 0, plan)) return nullptr;
-  const int rc = mdb_gemm_group(x.data_ptr(), ws, mats, out.data_ptr(), static_cast<int>(M), static_cast<int>(N),
-                                static_cast<int>(K), lda, w.stride(0), mats * N, plan.ctas, plan.bn, stream());
+  Tensor out;
+  const int rc = unlocked([&] {
+    out = at::empty(sizes, x.options());
+    return mdb_gemm_group(x.data_ptr(), ws, mats, out.data_ptr(), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), lda,
+                          w.stride(0), mats * N, plan.ctas, plan.bn, stream());
+  });
   return done(rc, "mdb_gemm_group", out);
   END_HANDLE_TH_ERRORS
 }
@@ -288,21 +319,22 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (D > 128 || (D & 7) || k.size(0) != B || v.size(0) != B || k.size(2) != H || v.size(2) != H || k.size(3) != D ||
       v.size(3) != D || k.size(1) != v.size(1) || k.size(1) > INT_MAX || S > INT_MAX)
     return not_implemented();
-  const Tensor out = at::empty({B, S, H, D}, q.options());
   const void *kp = k.data_ptr(), *vp = v.data_ptr();
   const int len = static_cast<int>(k.size(1)), b = static_cast<int>(B), h = static_cast<int>(H), s = static_cast<int>(S);
-  int rc;
-  if (D == 128 || D == 64) {
-    rc = (D == 128 ? mdb_flash_fwd : mdb_flash_fwd_d64)(
-        q.data_ptr(), &kp, &vp, out.data_ptr(), nullptr, b, h, s, 1, &len, q.stride(0), q.stride(1), q.stride(2), k.stride(0),
-        k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2), out.stride(0), out.stride(1), out.stride(2),
-        static_cast<float>(scale), nullptr, 0, nullptr, stream());
-  } else {
-    rc = mdb_flash_fwd_narrow(q.data_ptr(), &kp, &vp, out.data_ptr(), nullptr, b, h, s, 1, &len, q.stride(0), q.stride(1),
-                              q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
-                              out.stride(0), out.stride(1), out.stride(2), static_cast<float>(scale), static_cast<int>(D),
-                              stream());
-  }
+  Tensor out;
+  const int rc = unlocked([&] {
+    out = at::empty({B, S, H, D}, q.options());
+    if (D == 128 || D == 64) {
+      return (D == 128 ? mdb_flash_fwd : mdb_flash_fwd_d64)(
+          q.data_ptr(), &kp, &vp, out.data_ptr(), nullptr, b, h, s, 1, &len, q.stride(0), q.stride(1), q.stride(2), k.stride(0),
+          k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2), out.stride(0), out.stride(1), out.stride(2),
+          static_cast<float>(scale), nullptr, 0, nullptr, stream());
+    }
+    return mdb_flash_fwd_narrow(q.data_ptr(), &kp, &vp, out.data_ptr(), nullptr, b, h, s, 1, &len, q.stride(0), q.stride(1),
+                                q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
+                                out.stride(0), out.stride(1), out.stride(2), static_cast<float>(scale), static_cast<int>(D),
+                                stream());
+  });
   return done(rc, "mdb_flash_fwd", out);
   END_HANDLE_TH_ERRORS
 }
@@ -332,11 +364,13 @@ PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
       if (!f32(*p) || p->dim() != 2 || p->size(0) != B || p->size(1) != C || p->stride(1) != 1) return not_implemented();
     if (scale->stride(0) != shift->stride(0)) return not_implemented();
   }
-  const Tensor y = at::empty_like(x);
-  const int rc = mdb_ln_fwd(x.data_ptr(), y.data_ptr(), data(gamma), data(beta), static_cast<const float*>(data(scale)),
-                            static_cast<const float*>(data(shift)), scale ? scale->stride(0) : 0, static_cast<int>(B),
-                            static_cast<int>(S), static_cast<int>(C), static_cast<float>(eps), nullptr, nullptr,
-                            ctas_per_batch(B, S), stream());
+  Tensor y;
+  const int rc = unlocked([&] {
+    y = at::empty_like(x);
+    return mdb_ln_fwd(x.data_ptr(), y.data_ptr(), data(gamma), data(beta), static_cast<const float*>(data(scale)),
+                      static_cast<const float*>(data(shift)), scale ? scale->stride(0) : 0, static_cast<int>(B), static_cast<int>(S),
+                      static_cast<int>(C), static_cast<float>(eps), nullptr, nullptr, ctas_per_batch(B, S), stream());
+  });
   return done(rc, "mdb_ln_fwd", y);
   END_HANDLE_TH_ERRORS
 }
@@ -350,9 +384,12 @@ PyObject* py_geglu(PyObject*, PyObject* const* a, Py_ssize_t n) {
   std::vector<int64_t> sizes(u.sizes().begin(), u.sizes().end());
   const int64_t inner = sizes.back() / 2;
   sizes.back() = inner;
-  const Tensor y = at::empty(sizes, u.options());
-  return done(mdb_geglu_fwd(u.data_ptr(), y.data_ptr(), u.numel() / (2 * inner), static_cast<int>(inner), stream()),
-              "mdb_geglu_fwd", y);
+  Tensor y;
+  const int rc = unlocked([&] {
+    y = at::empty(sizes, u.options());
+    return mdb_geglu_fwd(u.data_ptr(), y.data_ptr(), u.numel() / (2 * inner), static_cast<int>(inner), stream());
+  });
+  return done(rc, "mdb_geglu_fwd", y);
   END_HANDLE_TH_ERRORS
 }
 
@@ -376,11 +413,13 @@ PyObject* py_rms_rope(PyObject*, PyObject* const* a, Py_ssize_t n) {
     for (const Tensor* p : {cs, sn})
       if (!f32(*p) || p->dim() != 2 || p->size(0) != S || p->size(1) != 64 || !p->is_contiguous()) return not_implemented();
   }
-  const Tensor y = at::empty({B, S, heads, C / heads}, x.options());
-  const int rc = mdb_rms_rope_fwd(x.data_ptr(), x.stride(1), y.data_ptr(), C, S * C, data(w), per_head,
-                                  static_cast<const float*>(data(cs)), static_cast<const float*>(data(sn)), static_cast<int>(B),
-                                  static_cast<int>(S), static_cast<int>(C), static_cast<int>(per_head ? 128 : C),
-                                  static_cast<float>(eps), nullptr, ctas_per_batch(B, S), stream());
+  Tensor y;
+  const int rc = unlocked([&] {
+    y = at::empty({B, S, heads, C / heads}, x.options());
+    return mdb_rms_rope_fwd(x.data_ptr(), x.stride(1), y.data_ptr(), C, S * C, data(w), per_head, static_cast<const float*>(data(cs)),
+                            static_cast<const float*>(data(sn)), static_cast<int>(B), static_cast<int>(S), static_cast<int>(C),
+                            static_cast<int>(per_head ? 128 : C), static_cast<float>(eps), nullptr, ctas_per_batch(B, S), stream());
+  });
   return done(rc, "mdb_rms_rope_fwd", y);
   END_HANDLE_TH_ERRORS
 }
@@ -402,20 +441,25 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (const Tensor* p : {gamma, beta})
     if (p && (!bf16(*p) || !p->is_contiguous() || p->numel() != C)) return not_implemented();
   const int splits = static_cast<int>(std::max<int64_t>(1, std::min((kCtasTarget + N - 1) / N, (HW + 15) / 16)));
-  const auto f = x.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous);
-  // one buffer: the strips' sums, then a and b [N, C], mean and rstd [N, groups]
-  const int64_t sums = N * splits * C * 2;
-  const Tensor work = at::empty({sums + 2 * N * C + 2 * N * groups}, f);
-  float* partial = work.data_ptr<float>();
-  float *ca = partial + sums, *cb = ca + N * C, *mean = cb + N * C, *rstd = mean + N * groups;
-  const Tensor y = at::empty_like(x);
-  void* st = stream();
   const int in = static_cast<int>(N), ic = static_cast<int>(C), ihw = static_cast<int>(HW), ig = static_cast<int>(groups);
-  int rc = mdb_gn_cl_sums(x.data_ptr(), nullptr, nullptr, nullptr, partial, in, ihw, ic, splits, st);
-  if (rc == 0)
-    rc = mdb_gn_cl_fold_fwd(partial, in, splits, ic, ig, static_cast<float>(HW * (C / groups)), static_cast<float>(eps),
-                            data(gamma), data(beta), gamma || beta ? 1 : 0, ca, cb, mean, rstd, st);
-  if (rc == 0) rc = mdb_gn_cl_apply(x.data_ptr(), nullptr, y.data_ptr(), ca, cb, nullptr, nullptr, nullptr, in, ihw, ic, act, st);
+  Tensor y;
+  const int rc = unlocked([&] {
+    // one buffer: the strips' sums, then a and b [N, C], mean and rstd [N, groups]
+    const int64_t sums = N * splits * C * 2;
+    const auto f = x.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous);
+    const Tensor work = at::empty({sums + 2 * N * C + 2 * N * groups}, f);
+    float* partial = work.data_ptr<float>();
+    float *ca = partial + sums, *cb = ca + N * C, *mean = cb + N * C, *rstd = mean + N * groups;
+    y = at::empty_like(x);
+    void* st = stream();
+    int err = mdb_gn_cl_sums(x.data_ptr(), nullptr, nullptr, nullptr, partial, in, ihw, ic, splits, st);
+    if (err == 0)
+      err = mdb_gn_cl_fold_fwd(partial, in, splits, ic, ig, static_cast<float>(HW * (C / groups)), static_cast<float>(eps),
+                               data(gamma), data(beta), gamma || beta ? 1 : 0, ca, cb, mean, rstd, st);
+    if (err == 0)
+      err = mdb_gn_cl_apply(x.data_ptr(), nullptr, y.data_ptr(), ca, cb, nullptr, nullptr, nullptr, in, ihw, ic, act, st);
+    return err;
+  });
   return done(rc, "mdb_gn_cl", y, 3);
   END_HANDLE_TH_ERRORS
 }
@@ -460,12 +504,15 @@ PyObject* py_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t m_tiles = PyLong_AsLongLong(a[24]);
   const int group = static_cast<int>(PyLong_AsLong(a[25]));
   if (PyErr_Occurred()) return nullptr;
-  Tensor partial;
-  if (splits > 1) partial = at::empty({splits * static_cast<int64_t>(classes) * m_tiles * 128 * n_pad}, out.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous));
-  const int rc = mdb_conv_igemm(x.data_ptr(), data(alt), w.data_ptr(), out.data_ptr(), data(bias), data(residual), dims, strides,
-                                alt_dims, alt_strides, box, ext, c_in, n_pad, w.size(1), static_cast<int>(classes), begin, taps,
-                                alt_dim, alt_shift, os, class_off, silu, ctas, max_bn, splits,
-                                splits > 1 ? partial.data_ptr() : nullptr, group, stream());
+  const int rc = unlocked([&] {
+    Tensor partial;
+    if (splits > 1)
+      partial = at::empty({splits * static_cast<int64_t>(classes) * m_tiles * 128 * n_pad},
+                          out.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous));
+    return mdb_conv_igemm(x.data_ptr(), data(alt), w.data_ptr(), out.data_ptr(), data(bias), data(residual), dims, strides, alt_dims,
+                          alt_strides, box, ext, c_in, n_pad, w.size(1), static_cast<int>(classes), begin, taps, alt_dim, alt_shift,
+                          os, class_off, silu, ctas, max_bn, splits, splits > 1 ? partial.data_ptr() : nullptr, group, stream());
+  });
   return done(rc, "mdb_conv_igemm", out);
   END_HANDLE_TH_ERRORS
 }
