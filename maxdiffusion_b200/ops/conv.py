@@ -90,7 +90,13 @@ class PackedConv:
   kind: str
   src: tuple = ()                 # (weight, bias, stride, pad_top_left) as given: what the PyTorch reference path runs
 
-  _tap_cache: dict = field(default_factory=dict, repr=False)
+  _tap_cache: dict = field(default_factory=dict, init=False, repr=False, compare=False)  # ctypes arrays: never pickled
+
+  def __getstate__(self):
+    return {k: v for k, v in self.__dict__.items() if k != "_tap_cache"}
+
+  def __setstate__(self, state):
+    self.__dict__.update(state, _tap_cache={})
 
   def row_group(self) -> int:
     """How many consecutive taps step along the width by one position each (they can share a fetched row): 2, 3 or 1."""
