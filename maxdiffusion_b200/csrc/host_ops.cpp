@@ -312,8 +312,8 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (const Tensor* t : ts) {
     if (!bf16(*t) || t->dim() != 4 || t->stride(3) != 1 || t->numel() == 0) return not_implemented();
     if (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) return not_implemented();
-    for (int i = 0; i < 3; ++i)
-      if (t->stride(i) & 7) return not_implemented();
+    for (int i = 0; i < 3; ++i)  // a broadcast dimension of a narrow head is copied, as by the padded path
+      if ((t->stride(i) & 7) || (t->stride(i) == 0 && t->size(i) > 1 && t->size(3) != 64 && t->size(3) != 128)) return not_implemented();
   }
   const int64_t B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3);
   if (D > 128 || (D & 7) || k.size(0) != B || v.size(0) != B || k.size(2) != H || v.size(2) != H || k.size(3) != D ||

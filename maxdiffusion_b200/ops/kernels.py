@@ -264,9 +264,11 @@ def flash_fwd(q: torch.Tensor, k_list: Sequence[torch.Tensor], v_list: Sequence[
 
 def flash_narrow_ok(*tensors) -> bool:
   """Whether `flash_fwd_narrow` can read these [B,S,H,D] tensors where they are: D a multiple of 8 up to 128, unit inner
-  stride, 16-byte aligned start and strides (what a projection's output has)."""
+  stride, 16-byte aligned start and strides (what a projection's output has), no broadcast dimension."""
   for t in tensors:
-    if t.shape[-1] % 8 or t.shape[-1] > 128 or t.stride(-1) != 1 or t.data_ptr() % 16 or any(st % 8 for st in t.stride()[:-1]):
+    if t.shape[-1] % 8 or t.shape[-1] > 128 or t.stride(-1) != 1 or t.data_ptr() % 16:
+      return False
+    if any(st % 8 or (st == 0 and n > 1) for st, n in zip(t.stride()[:-1], t.shape)):
       return False
   return True
 

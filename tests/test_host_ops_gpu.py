@@ -115,6 +115,11 @@ def test_norms_and_gates(monkeypatch):
   for C in (64, 640, 1280, 3072):
     x, g, b = _randn(2, 33, C), _randn(C), _randn(C)
     s = torch.randn(2, 3 * C, device="cuda")
+  one = _randn(1, 70, 1, D)  # keys and values shared by all heads and samples
+  shared = one.expand(2, 70, 3, D)
+  with torch.no_grad():
+    assert torch.equal(OF.attention(q, shared, shared), OF.attention(q, shared.contiguous(), shared.contiguous()))
+    assert torch.equal(OF.attention(shared, k, v), OF.attention(shared.contiguous(), k, v))
     assert _both(monkeypatch, lambda: OF.layer_norm_mod(x, g, b))
     assert _both(monkeypatch, lambda: OF.layer_norm_mod(x, scale=s[:, :C], shift=s[:, C:2 * C]))
     _both(monkeypatch, lambda: OF.layer_norm_mod(x, scale=s[:, :C].to(torch.bfloat16), shift=s[:, C:2 * C]))
