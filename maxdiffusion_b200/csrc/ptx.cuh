@@ -113,10 +113,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 // Bounded wait. `abort_flag` lives in shared memory: once any role of the CTA gives up, every
-// other role leaves its loops at its next wait.
+// other role leaves its loops at its next wait. The clock is first read after a batch of failed tries, since most waits end
+// before; PAUSE reads it after the first one, which holds the next try back for as long as that read takes.
+template <bool PAUSE = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           DeviceStatus* st, unsigned int where) {
-  uint64_t t0 = 0;  // the clock is first read after a batch of failed tries: most waits end before
+  uint64_t t0 = 0;
+  if (PAUSE) {
+    if (mbar_try_wait(bar, parity)) return true;
+    t0 = global_timer_ns();
+  }
   uint32_t spins = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
