@@ -20,6 +20,11 @@ def _both(monkeypatch, fn):
   return used
 
 
+def _launches(fn):
+  before = _lib.launch_count()
+  return fn(), _lib.launch_count() - before
+
+
 def _randn(*shape):
   return torch.randn(shape, device="cuda").to(torch.bfloat16)
 
@@ -29,6 +34,7 @@ _FORMS = {"dense": lambda: _randn(3, 40, 64), "2d": lambda: _randn(17, 64), "4d"
           "transposed": lambda: _randn(40, 3, 64).transpose(0, 1), "every second row": lambda: _randn(3, 80, 64)[:, ::2],
           "expanded": lambda: _randn(1, 40, 64).expand(3, 40, 64), "one row": lambda: _randn(1, 1, 64),
           "columns apart": lambda: _randn(3, 40, 128)[..., ::2]}
+_COPIED = ("transposed", "part of a sequence", "expanded", "columns apart")  # not one pitch: the wrappers copy these
 
 
 @pytest.mark.parametrize("form", list(_FORMS))
@@ -38,7 +44,7 @@ def test_linear(monkeypatch, form, act):
   x, w, b = _FORMS[form](), _randn(72, 64), _randn(72)
   res = _randn(*x.shape[:-1], 72) if act == "residual" else None
   used = _both(monkeypatch, lambda: OF.linear(x, w, b, None if res is not None else act, residual=res))
-  assert used or form in ("transposed", "part of a sequence", "expanded", "columns apart")
+  assert used or form in _COPIED
   _both(monkeypatch, lambda: OF.linear(x, w[::2], None))  # a strided weight
   if res is not None:
     _both(monkeypatch, lambda: OF.linear(x, w, b, residual=res.transpose(0, 1).contiguous().transpose(0, 1)))
@@ -62,7 +68,9 @@ def test_linear_residual_layouts(monkeypatch, name, cut):
     assert torch.equal(got, want)
 
 
-_FORMS["more than a tile"] = lambda: _randn(3, 87, 64)
+_TALL = {"more than a tile": lambda: _randn(3, 87, 64), "slice of channels, tall": lambda: _randn(3, 87, 192)[..., 64:128],
+         "every second row, tall": lambda: _randn(3, 174, 64)[:, ::2]}
+_FORMS.update(_TALL)
 
 
 @pytest.mark.parametrize("form", list(_FORMS))
@@ -75,7 +83,8 @@ def test_geglu_linear(form, N):
     for bias in (b, None):
       u = x.double() @ w.double().t() + (0 if bias is None else bias.double())
       want = u[..., :N] * torch.nn.functional.gelu(u[..., N:])
-      got = OF.geglu_linear(x, w, bias)
+      got, n = _launches(lambda: OF.geglu_linear(x, w, bias))
+      assert n == (1 if form in _TALL else 2)  # one kernel from 129 rows on
       assert got.shape == want.shape and (got.double() - want).norm() < 4e-3 * want.norm()
   assert OF.geglu_linear(x, torch.nn.Parameter(w)).requires_grad
 
@@ -86,13 +95,13 @@ def test_linear_group(form, n, N):
   torch.manual_seed(5)
   x, ws = _FORMS[form](), [_randn(N, 64) for _ in range(n)]
   with torch.no_grad():
-    got = OF.linear_group(x, ws)
-    assert len(got) == n
+    got, launched = _launches(lambda: OF.linear_group(x, ws))
+    assert len(got) == n and launched == (n if form in _COPIED else 1)
     for g, w in zip(got, ws):
       want = x.double() @ w.double().t()
       assert g.shape == want.shape and (g.double() - want).norm() < 4e-3 * want.norm()  # one rounding to bf16
-    odd = OF.linear_group(x, [ws[0], ws[1][:8]])
-    assert odd[1].shape[-1] == 8
+    odd, launched = _launches(lambda: OF.linear_group(x, [ws[0], ws[1][:8]]))
+    assert odd[1].shape[-1] == 8 and launched == (1 if N == 8 and form not in _COPIED else 2)
   assert OF.linear_group(x, [torch.nn.Parameter(w) for w in ws])[1].requires_grad
 
 
@@ -106,6 +115,11 @@ def test_attention(monkeypatch, D):
   _both(monkeypatch, lambda: OF.attention(q.transpose(1, 2).contiguous().transpose(1, 2), [k, k], [v, v]))
   if D in K.FLASH_HEAD_DIMS:
     return  # there the kernel itself refuses strides that TMA cannot take
+  one = _randn(1, 70, 1, D)  # keys and values shared by all heads and samples
+  shared = one.expand(2, 70, 3, D)
+  with torch.no_grad():
+    assert torch.equal(OF.attention(q, shared, shared), OF.attention(q, shared.contiguous(), shared.contiguous()))
+    assert torch.equal(OF.attention(shared, k, v), OF.attention(shared.contiguous(), k, v))
   wide = _randn(2, 70, 3, D + 4)
   _both(monkeypatch, lambda: OF.attention(wide[..., :D], wide[..., :D], wide[..., :D]))  # copied
 
@@ -115,11 +129,6 @@ def test_norms_and_gates(monkeypatch):
   for C in (64, 640, 1280, 3072):
     x, g, b = _randn(2, 33, C), _randn(C), _randn(C)
     s = torch.randn(2, 3 * C, device="cuda")
-  one = _randn(1, 70, 1, D)  # keys and values shared by all heads and samples
-  shared = one.expand(2, 70, 3, D)
-  with torch.no_grad():
-    assert torch.equal(OF.attention(q, shared, shared), OF.attention(q, shared.contiguous(), shared.contiguous()))
-    assert torch.equal(OF.attention(shared, k, v), OF.attention(shared.contiguous(), k, v))
     assert _both(monkeypatch, lambda: OF.layer_norm_mod(x, g, b))
     assert _both(monkeypatch, lambda: OF.layer_norm_mod(x, scale=s[:, :C], shift=s[:, C:2 * C]))
     _both(monkeypatch, lambda: OF.layer_norm_mod(x, scale=s[:, :C].to(torch.bfloat16), shift=s[:, C:2 * C]))
@@ -142,13 +151,13 @@ def test_group_norm_and_conv(monkeypatch, shape):
   x = _randn(*shape).contiguous(memory_format=torch.channels_last)
   g, b, w, cb = _randn(C), _randn(C), _randn(48, C, 3, 3) * 0.05, _randn(48)
   for act in (False, True):
-    _both(monkeypatch, lambda: OF.group_norm(x, 32, g, b, 1e-5, act))
-    _both(monkeypatch, lambda: OF.group_norm(x, 32, g.float(), b.float(), 1e-5, act))
-  _both(monkeypatch, lambda: OF.conv2d(x, w, cb))
-  _both(monkeypatch, lambda: OF.conv2d(x.contiguous(), w, None, upsample=True))
+    assert _both(monkeypatch, lambda: OF.group_norm(x, 32, g, b, 1e-5, act))
+    assert not _both(monkeypatch, lambda: OF.group_norm(x, 32, g.float(), b.float(), 1e-5, act))
+  assert _both(monkeypatch, lambda: OF.conv2d(x, w, cb))
+  assert _both(monkeypatch, lambda: OF.conv2d(x.contiguous(), w, None, upsample=True))
   clip, hist = _randn(1, 3, 6, 10, C), _randn(1, 2, 6, 10, C)
   pk = OC.pack_conv3d(_randn(40, C, 3, 3, 3) * 0.05, _randn(40))
-  _both(monkeypatch, lambda: OC.conv3d_causal(clip, pk, hist))
+  assert _both(monkeypatch, lambda: OC.conv3d_causal(clip, pk, hist))
 
 
 def test_direct_calls_leave_autograd_alone():

@@ -509,8 +509,8 @@ def test_gemm_split_k_matches_fp32(a_mn, b_mn, M, N, Kd, splits):
 @pytest.mark.parametrize("M,N,Kd", [(300, 328, 192), (4095, 1280, 640), (129, 8, 64), (1024, 2560, 320)])
 @pytest.mark.parametrize("epi", ["none", "gelu_tanh", "add_res", "gated_res"])
 @pytest.mark.parametrize("f32", [False, True])
-def test_gemm_tma_store_epilogue_equals_direct_stores(M, N, Kd, epi, f32):
-  """The epilogue that stages 128-byte slabs in shared memory and writes them with TMA stores against the one that
+def test_gemm_staged_epilogue_equals_direct_stores(M, N, Kd, epi, f32):
+  """The epilogue that passes slabs of 32 rows x 128 bytes through shared memory and stores full lines against the one that
   stores from one thread per row: same values bit for bit, ragged edges in M and N, every epilogue, both output types."""
   g = torch.Generator(device="cuda").manual_seed(0)
   a = torch.randn((M, Kd), device="cuda", generator=g).to(torch.bfloat16)
