@@ -7,8 +7,8 @@
 // What bounds it is the operand feed from L2: every shape ran at about 57 bytes per clock and SM, which a 128 x 256 tile
 // of one CTA (48 KB per 512 tensor clocks) turns into 60 % of the tensor rate. So tiles of more than 128 rows are
 // computed by a PAIR of CTAs (`cta_group::2`): 256 x BN, each CTA fetching its own 128 rows of A and half of B (32 KB per
-// 512 clocks at BN = 256) and draining its own 128 accumulator rows. One CTA / a pair: 65520 x 5120 x 5120 2566 / 2278 us
-// (1508 TFLOP/s), 4608 x 12288 x 3072 285 / 230 us.
+// 512 clocks at BN = 256) and draining its own 128 accumulator rows. One CTA / a pair, in turn under the power cap: 32760 x
+// 5120 x 5120 1400 / 1239 us, 4608 x 9216 x 3072 202 / 172 us, 4096 x 3072 x 12288 239 / 213 us.
 //
 // Either operand may be "MN-major" (stored transposed, i.e. A as [K,M] or B as [K,N]); this is what
 // lets dgrad (dX = dY * W) and wgrad (dW = dY^T * X) run on the same kernel without transposes.
@@ -36,12 +36,15 @@ constexpr int ACC_COLS = 256;     // TMEM columns of one accumulator
 constexpr int SLAB_BYTES = 32 * 128;
 constexpr int STAGING_BYTES = EPI_WARPS * SLAB_BYTES;
 constexpr int BIAS_BYTES = 2 * 256 * 4;  // the tile's bias columns as fp32, for two tiles in turn
-constexpr int FIXED_BYTES = STAGING_BYTES + BIAS_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int FIXED_BYTES = STAGING_BYTES + BIAS_BYTES + 256 /*barriers*/;
 constexpr int SMEM_LIMIT = 227 * 1024;
 // One stage holds a k-block of A (128 rows) and of this CTA's share of B; a multiple of 1024 bytes.
 __host__ __device__ constexpr int stage_bytes(int bn, int cg) { return A_BYTES + bn / cg * BK * 2; }
-__host__ constexpr int stages_for(int bn, int cg) {
-  const int n = (SMEM_LIMIT - FIXED_BYTES) / stage_bytes(bn, cg);
+// As many stages as fit: one CTA's tile 256 columns wide takes four (4 x 48 KiB; 3 stages / 4: 4608 x 9216 x 3072 244 / 202 us,
+// 8192 x 5120 x 320 43.5 / 30.7 us). A cut contraction leaves room beside it: the CTAs of the fold that follows start, and wait,
+// while the products still run (each takes a reserved kilobyte). With every byte taken 320 x 320 x 16384 took 19.3 us, 13.0 so.
+__host__ constexpr int stages_for(int bn, int cg, bool cut) {
+  const int n = (SMEM_LIMIT - FIXED_BYTES - (cut ? 8192 : 0)) / stage_bytes(bn, cg);
   return n < MAX_STAGES ? n : MAX_STAGES;
 }
 
@@ -116,8 +119,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   constexpr int TMEM_COLS = 2 * ACC_COLS;   // two accumulators
   const int STAGES = p.stages, BN = p.bn, BN_CTA = BN / CG;
   const int STAGE_BYTES = A_BYTES + BN_CTA * BK * 2;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];  // the 128-byte swizzle repeats every 1024 bytes
   uint8_t* staging = smem + STAGES * STAGE_BYTES;  // 1024-byte aligned: every stage is a multiple of 1024 bytes
   float* bias_s = reinterpret_cast<float*>(staging + STAGING_BYTES);
   uint64_t* bars = reinterpret_cast<uint64_t*>(staging + STAGING_BYTES + BIAS_BYTES);
@@ -618,6 +620,8 @@ int launch(const CUtensorMap& ta, const BMaps& tb, const Params& p, cudaStream_t
   static bool configured = false;
   if (!configured) {
     MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT));
+    // all of the SM's memory as shared memory: what a CTA does not use is room for the successor's CTAs to start in
+    MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     configured = true;
   }
   const int out_n = EK == kGeglu ? p.bn / 2 : p.bn;
@@ -724,7 +728,6 @@ extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void
   p.alpha = alpha;
   p.mats = 1;
   p.bn = bn;
-  p.stages = stages_for(bn, ctas);
   p.status = status_buffer();
   {
     // every split gets at least one k-block: the count is recomputed from the rounded-up range
@@ -736,6 +739,7 @@ extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void
     p.partial = static_cast<float*>(partial);
     if (p.splits <= 1) { p.splits = 1; p.kb_per_split = num_kb; }
   }
+  p.stages = stages_for(bn, ctas, p.splits > 1);
   const bool f32 = out_f32 || p.splits > 1;
   const bool act = epi == kEpiGeluTanh || epi == kEpiSilu, res = epi == kEpiGatedRes || epi == kEpiAddRes;
   int kind = kDirect;
@@ -780,7 +784,7 @@ extern "C" int mdb_gemm_geglu(const void* A, const void* B, void* out, const voi
   p.splits = 1;
   p.kb_per_split = (K + BK - 1) / BK;
   p.bn = bn;
-  p.stages = stages_for(bn, ctas);
+  p.stages = stages_for(bn, ctas, false);
   p.status = status_buffer();
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   return launch<false, false, 2, kGeglu>(ta, tb, p, stream);
@@ -815,7 +819,7 @@ extern "C" int mdb_gemm_group(const void* A, const void* const* B, int mats, voi
   p.splits = 1;
   p.kb_per_split = (K + BK - 1) / BK;
   p.bn = bn;
-  p.stages = stages_for(bn, ctas);
+  p.stages = stages_for(bn, ctas, false);
   p.status = status_buffer();
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   return ctas == 2 ? launch<false, false, 2, kPlain>(ta, tb, p, stream) : launch<false, false, 1, kPlain>(ta, tb, p, stream);

@@ -67,7 +67,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 // their operands live in uniform registers, and only behind `elect.sync` does the compiler know that a single lane is
 // active and issue them directly instead of looping over the lanes that might be. Measured on a B200, lane == 0 against
 // elected: weight gradient 4 x 64 x 64 x 640 -> 640 142.7 -> 97.7 us, conv 2 x 64 x 64 x 640 -> 640 78.3 -> 57.2 us,
-// GEMM 65520 x 5120 x 5120 2515 -> 2358 us.
+// GEMM 65520 x 5120 x 5120 by tiles of one CTA 2515 -> 2358 us.
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(
