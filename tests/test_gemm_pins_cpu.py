@@ -38,3 +38,13 @@ def test_fused_products_give_way_to_a_pin(monkeypatch, pin):
   monkeypatch.setattr(K, {"tile": "_FORCE_TILE_N", "ctas": "_FORCE_CTAS", "epilogue": "_DIRECT_EPILOGUE"}[pin], 2)
   run()
   assert asked == ["linear_group", "geglu_linear"]
+
+
+@pytest.mark.parametrize("M,N,Kd,b_mn,avoid", [(7000, 2048, 8192, False, (2, 256)), (640, 640, 16384, True, (2, 256))])
+def test_a_nearly_empty_last_round_of_pairs_is_not_preferred(M, N, Kd, b_mn, avoid):
+  assert K.gemm_plan(M, N, Kd, b_mn)[:2] != avoid
+
+
+@pytest.mark.parametrize("M,N,Kd", [(4608, 9216, 3072), (65520, 5120, 5120), (32760, 5120, 13824)])
+def test_large_products_run_on_wide_pairs(M, N, Kd):
+  assert K.gemm_plan(M, N, Kd) == (2, 256, 1)
