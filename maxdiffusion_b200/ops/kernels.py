@@ -49,7 +49,7 @@ def gemm_plan(M: int, N: int, K: int, b_mn: bool = False, splittable: bool = Tru
   contraction makes more work items at the price of fp32 partials and a second kernel (3 us + their traffic): 384 x 3072 x
   15360 takes 51 us whole and 41 us in three parts. `tile_n` / `ctas` restrict the choice."""
   best, best_cost = None, None
-  num_kb = -(-K // 64)
+  num_kb = max(1, -(-K // 64))
   for (cg, bn), kb_us in _KB_US.items():
     if (ctas and cg != ctas) or (tile_n and bn != tile_n) or (b_mn and (bn // cg) % 64) or (cg == 2 and M <= 128 and not ctas):
       continue

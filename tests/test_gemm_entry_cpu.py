@@ -41,4 +41,5 @@ def test_an_empty_contraction_is_the_epilogue_of_zero(epi):
   if epi == "none":
     assert not K.gemm(a, b, out_dtype=torch.float32).any()
     assert torch.equal(K.gemm(a.t(), b.t(), a_mn=True, b_mn=True, bias=bias), want.to(torch.bfloat16))
+  assert K.split_k_for(6, 8, 0) == 1 and K.gemm_plan(6, 8, 0)[2] == 1
   assert K.gemm(bf(0, 16), bf(8, 16)).shape == (0, 8) and K.gemm(bf(6, 16), bf(0, 16)).shape == (6, 0)
