@@ -485,15 +485,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               *reinterpret_cast<float4*>(o + 4) = make_float4(x[4], x[5], x[6], x[7]);
               continue;
             }
-            if (p.bias) {
-              const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
-              const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+            if (p.bias) {  // single loads: a bias may start anywhere
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float2 f = unpack_bf16x2(bw[j]);
-                x[2 * j] += f.x;
-                x[2 * j + 1] += f.y;
-              }
+              for (int j = 0; j < 8; ++j) x[j] += __bfloat162float(p.bias[col + j]);
             }
             if (p.epi == kEpiGeluTanh) {
 #pragma unroll

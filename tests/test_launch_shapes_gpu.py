@@ -173,3 +173,24 @@ def test_wide_head_attention_forms():
       bad = ~want.isfinite()
       assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[bad].double().nan_to_num(), want[bad].nan_to_num().to(torch.bfloat16).double().nan_to_num())
       assert _rel(got[~bad], want[~bad]) < 4e-3  # one rounding to bf16
+
+
+@pytest.mark.parametrize("epi", ["none", "gelu_tanh", "silu", "add_res"])
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("direct", [False, True])
+def test_a_bias_may_start_anywhere(epi, f32, direct):
+  """Every epilogue in one part: fp32 results with an activation or a residual are stored straight from the accumulator."""
+  torch.manual_seed(9)
+  a, b, store, res = _randn(136, 64), _randn(328, 64, scale=0.1), _randn(400), _randn(136, 328)
+  bias = store[3:331]  # 6 bytes into a 16-byte line
+  kw = dict(epi=epi, residual=res if epi == "add_res" else None, out_dtype=torch.float32 if f32 else torch.bfloat16)
+  K.gemm_epilogue_mode(direct)
+  try:
+    got, want = K.gemm(a, b, bias=bias, **kw), K.gemm(a, b, bias=bias.clone(), **kw)
+  finally:
+    K.gemm_epilogue_mode(False)
+  assert torch.equal(got, want)
+  y = a.double() @ b.double().t() + bias.double()
+  y = {"none": lambda: y, "gelu_tanh": lambda: torch.nn.functional.gelu(y, approximate="tanh"),
+       "silu": lambda: torch.nn.functional.silu(y), "add_res": lambda: y + res.double()}[epi]()
+  assert _rel(got, y) < (1e-3 if f32 else 4e-3)  # the approximate tanh and exponential; one rounding to bf16
