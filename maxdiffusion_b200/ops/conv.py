@@ -712,13 +712,13 @@ def _odd_head_attention(q, k, v, scale):
   q = q.contiguous()
   if q.data_ptr() % 16:
     q = q.clone()
-  kp = torch.zeros((pitch, D), dtype=k.dtype, device=k.device)
-  kp[:T] = k
+  kp = torch.empty((pitch, D), dtype=k.dtype, device=k.device)
+  kp[:T], kp[T:] = k, 0
   scores = K.gemm(q, kp, alpha=scale, out_dtype=torch.float32)  # [T, pitch]
   parts = softmax_split(scores, T)
   # an infinite or NaN value meets the first part alone: the others may be zero or negative where the probability is not
-  v3 = torch.zeros((3, pitch, v.shape[1]), dtype=v.dtype, device=v.device)
-  v3[0, :T] = v
+  v3 = torch.empty((3, pitch, v.shape[1]), dtype=v.dtype, device=v.device)
+  v3[0, :T], v3[:, T:] = v, 0
   v3[1:, :T] = torch.nan_to_num(v, nan=0.0, posinf=0.0, neginf=0.0)
   return K.gemm(parts, v3.view(3 * pitch, -1), b_mn=True)
 
