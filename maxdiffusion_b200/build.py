@@ -11,6 +11,7 @@ from __future__ import annotations
 import concurrent.futures
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -21,7 +22,6 @@ SRC_DIR = PKG_DIR / "csrc"
 OBJ_DIR = PKG_DIR / "csrc" / "build"
 LIB_PATH = PKG_DIR / "_kernels.so"
 HOST_PATH = PKG_DIR / "_host_ops.so"  # CPython extension over the kernel library (csrc/host_ops.cpp)
-HOST_FOR = "_host_ops.for"  # beside it: what it was built for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -107,6 +107,14 @@ def host_ops_target() -> str:
   return f"PyTorch {torch.__version__}, Python {sys.version.split()[0]}"
 
 
+def host_ops_built_for(path: Path) -> str | None:
+  """The `host_ops_target` that an object was built for, as its text has it (the object is not loaded); None: no such object."""
+  if not path.exists():
+    return None
+  found = re.search(rb"mdb_host_ops built for ([^;\0]+);", path.read_bytes())
+  return found.group(1).decode() if found else "something unknown"
+
+
 def build_host_ops(verbose: bool = True, force: bool = False) -> None:
   """Compiles csrc/host_ops.cpp against the installed PyTorch and links it to `_kernels.so` beside it."""
   import sysconfig
@@ -116,10 +124,10 @@ def build_host_ops(verbose: bool = True, force: bool = False) -> None:
   root = Path(torch.__file__).resolve().parent
   cuda = Path(_nvcc()).resolve().parent.parent
   src, obj, stamp = SRC_DIR / "host_ops.cpp", OBJ_DIR / "host_ops.o", OBJ_DIR / "host_ops.sha"
-  flags = ["-std=c++17", "-O2", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+  flags = ["-std=c++17", "-O2", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DMDB_BUILT_FOR="{host_ops_target()}"']
   digest = hashlib.sha256(" ".join([torch.__version__, sys.version, *flags]).encode() + src.read_bytes()).hexdigest()
-  target = HOST_PATH.with_name(HOST_FOR)
-  if force or not HOST_PATH.exists() or not target.exists() or not stamp.exists() or stamp.read_text() != digest:
+  if force or host_ops_built_for(HOST_PATH) != host_ops_target() or not stamp.exists() or stamp.read_text() != digest:
     inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda / "include"]
     libs = ["-L", str(PKG_DIR), "-l:_kernels.so", "-Wl,-rpath,$ORIGIN", "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu",
             "-ltorch", "-lc10_cuda", "-lc10"]  # PyTorch's libraries are loaded before this one: no run path to them
@@ -129,7 +137,6 @@ def build_host_ops(verbose: bool = True, force: bool = False) -> None:
       if res.returncode != 0:
         raise RuntimeError(f"{src.name}: {' '.join(cmd[:2])} failed:\n{res.stdout}\n{res.stderr}")
     stamp.write_text(digest)
-    target.write_text(host_ops_target())
     if verbose:
       print(f"[build] linked {HOST_PATH}")
 

@@ -47,6 +47,9 @@ int mdb_conv_igemm(const void*, const void*, const void*, void*, const void*, co
                    int, int, const long long*, const long long*, int, int, int, int, void*, int, void*);
 }
 
+// Read from the file before it is loaded (`build.host_ops_built_for`).
+extern "C" __attribute__((used)) const char mdb_host_ops_built_for[] = "mdb_host_ops built for " MDB_BUILT_FOR ";";
+
 namespace {
 
 using at::Tensor;

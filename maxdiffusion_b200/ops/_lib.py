@@ -80,8 +80,8 @@ def _load_host_ops():
   from maxdiffusion_b200 import build as _build
   from . import kernels
 
-  path, target = LIB_PATH.with_name("_host_ops.so"), LIB_PATH.with_name(_build.HOST_FOR)
-  built_for = target.read_text() if path.exists() and target.exists() else None
+  path = LIB_PATH.with_name("_host_ops.so")
+  built_for = _build.host_ops_built_for(path)
   if built_for != _build.host_ops_target():  # missing, or built against another PyTorch or Python: it must not be loaded
     if os.environ.get("MDB200_NO_AUTOBUILD") == "1":
       raise KernelError(f"{path} is {'missing' if built_for is None else f'for {built_for}'}; run `python -m maxdiffusion_b200.build`")

@@ -20,6 +20,16 @@ def fresh(monkeypatch, tmp_path):
   return tmp_path
 
 
+def _object(built_for):
+  return b"not a shared object \0mdb_host_ops built for " + built_for.encode() + b";\0"
+
+
+def test_the_object_says_what_it_was_built_for(tmp_path):
+  if build.HOST_PATH.exists():
+    assert build.host_ops_built_for(build.HOST_PATH) == build.host_ops_target()
+  assert build.host_ops_built_for(tmp_path / "none.so") is None
+
+
 def _takes_nothing():
   with pytest.warns(RuntimeWarning, match="host extension"):
     host = _lib.host_ops()
@@ -50,16 +60,13 @@ def test_no_compiler_at_all(fresh, monkeypatch):
 
 
 def test_an_object_that_does_not_load(fresh):
-  (fresh / "_host_ops.so").write_bytes(b"not a shared object")
-  (fresh / build.HOST_FOR).write_text(build.host_ops_target())
+  (fresh / "_host_ops.so").write_bytes(_object(build.host_ops_target()))
   _takes_nothing()
 
 
 @pytest.mark.parametrize("built_for", [None, "PyTorch 2.0.0, Python 3.8.1"])
 def test_an_object_for_another_pytorch_is_rebuilt_and_not_loaded(fresh, monkeypatch, built_for):
-  (fresh / "_host_ops.so").write_bytes(b"an object")
-  if built_for is not None:
-    (fresh / build.HOST_FOR).write_text(built_for)
+  (fresh / "_host_ops.so").write_bytes(b"an object" if built_for is None else _object(built_for))
   asked, load = [], importlib.util.spec_from_file_location
 
   def refuse(name, *a, **k):

@@ -11,4 +11,4 @@ def test_the_package_holds_sources_and_objects():
   files = {p.relative_to(PKG).as_posix() for pattern in patterns for p in PKG.glob(pattern)}
   sources = {f"csrc/{p.name}" for p in (PKG / "csrc").iterdir() if p.suffix in (".cu", ".cuh", ".h", ".cpp")}
   assert "csrc/host_ops.cpp" in sources and sources <= files, sources - files
-  assert {"_kernels.so", "_host_ops.so", "_host_ops.for"} <= set(patterns)
+  assert {"_kernels.so", "_host_ops.so"} <= set(patterns)
