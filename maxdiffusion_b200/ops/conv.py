@@ -703,7 +703,7 @@ def _odd_head_ok(q, k, v) -> bool:
 def _odd_head_attention(q, k, v, scale):
   """`wide_head_attention` for T that is no multiple of 8, with fp32 scores and probabilities (as the library products that
   ran here before): the keys are padded with zero rows that the softmax leaves out, and the probabilities enter the second
-  product as three bf16 parts. 4500 positions of 384 channels: 752 us with library products, 133 us so, the same error
+  product as three bf16 parts. 4500 positions of 384 channels: 755 us with library products, 140 us so, the same error
   against float64 (1.653e-3, the rounding of the result)."""
   from . import kernels as K
 
