@@ -94,10 +94,13 @@ struct TileCoord {
   bool in_range;  // false: the second half of a pair that covers the class's odd last M-tile
 };
 
-// First (tap, channel block) unit of work item `split`: the units are cut into ranges that differ by at most one.
+// First (tap, channel block) unit of work item `split`: the units are cut into ranges that differ by at most one. A whole
+// contraction goes without the divisions here and in `split_of`, which a tile of few steps feels: three taps in time at
+// 2 x 240 x 416 x 96 35.9 us with 64-bit divisions, 34.6 so; 3x3 at 256 x 256, 128 -> 8 11.5 / 11.0 us.
 __device__ __forceinline__ int unit_cut(int split, int splits, int units) {
-  return static_cast<int>(static_cast<long long>(units) * split / splits);
+  return splits == 1 ? split * units : units * split / splits;  // at most 36 taps of 128 blocks times 64 parts
 }
+__device__ __forceinline__ int split_of(int work, int splits, int num_tiles) { return splits == 1 ? 0 : work / num_tiles; }
 
 // Epilogue of 8 channels of one output position: bias, SiLU, residual, store.
 __device__ __forceinline__ void finish8(float (&x)[8], const Params& p, long long off, int col) {
@@ -229,7 +232,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       int issued = 0;
       bool ok = true;
       for (int work = group_id; work < num_work && ok; work += num_groups) {
-        const int split = work / num_tiles;
+        const int split = split_of(work, p.splits, num_tiles);
         const TileCoord tc = decode_tile<CG>(work - split * num_tiles, rank, p, nt1, nt2, nt3, num_mt, num_n);
         const int n0 = tc.n_idx * p.BN + rank * (p.BN / CG);
         const int t0 = p.tap_begin[tc.cls];
@@ -292,7 +295,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
       int it = 0;
       bool ok = true;
       for (int work = group_id; work < num_work && ok; work += num_groups, ++it) {
-        const int split = work / num_tiles;
+        const int split = split_of(work, p.splits, num_tiles);
         const int cls = (work - split * num_tiles) / (num_tiles / p.n_classes);
         const int n_taps = (p.tap_begin[cls + 1] - p.tap_begin[cls]) / GROUP;
         const int acc = it & 1;
@@ -358,7 +361,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     int it = 0;
     bool ok = true;
     for (int work = group_id; work < num_work && ok; work += num_groups, ++it) {
-      const int split = work / num_tiles;
+      const int split = split_of(work, p.splits, num_tiles);
       const TileCoord tc = decode_tile<CG>(work - split * num_tiles, rank, p, nt1, nt2, nt3, num_mt, num_n);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
