@@ -32,12 +32,13 @@ _SM_COUNT = 148
 
 # Microseconds of one 64-deep k-block per (CTAs per tile, tile width): the larger of the operand feed into an SM (about 122
 # bytes a nanosecond) and the products. Fitted on a B200 to 33 shapes of 128 .. 65 520 rows x 4 widths x 1 / 2 CTAs. A chip
-# full of wide tiles draws the most power and runs them at a lower clock: `_KB_FULL_US` more, by the share of pairs at work.
-# Without that, 3.03 rounds of pairs were preferred to 2.97 of single CTAs (7000 x 2048 x 8192 200 / 176 us), and 72 pairs in
-# one round to 140 single CTAs (640 x 640 x 16384 22.2 / 20.6 us); over 148 shapes the plan's mean loss against the best shape
-# falls from 1.4 to 1.0 %, and none takes more than a percent longer than by one CTA and 256 columns throughout.
+# full of wide tiles draws the most power and runs them at a lower clock: `_KB_FULL_US` more, by the share of slots at work.
+# Without that, 3.03 rounds of pairs were preferred to 2.97 of single CTAs (7000 x 2048 x 8192 200 / 176 us), and 72 wide
+# pairs in one round to narrower ones (640 x 640 x 16384 22.2 / 20.3 us); over 148 shapes the plan's mean loss against the best
+# shape falls from 1.4 to 1.0 %, and none takes more than 2 % longer than by one CTA and 256 columns throughout.
 _KB_US = {(1, 64): 0.19, (1, 128): 0.25, (1, 192): 0.30, (1, 256): 0.39, (2, 64): 0.17, (2, 128): 0.20, (2, 192): 0.235, (2, 256): 0.27}
-_KB_FULL_US = {(1, 128): 0.02, (1, 192): 0.01, (2, 192): 0.02, (2, 256): 0.03}
+# {(CTAs, width): (whole, cut contraction)}
+_KB_FULL_US = {(1, 128): (0.02, 0.02), (1, 192): (0.01, 0.03), (1, 256): (0.0, 0.02), (2, 192): (0.02, 0.02), (2, 256): (0.03, 0.03)}
 
 
 @functools.lru_cache(maxsize=4096)
@@ -62,7 +63,7 @@ def gemm_plan(M: int, N: int, K: int, b_mn: bool = False, splittable: bool = Tru
         break
       s_eff = -(-num_kb // per)
       rounds = -(-tiles * s_eff // slots)
-      us = kb_us + _KB_FULL_US.get((cg, bn), 0.0) * tiles * s_eff / (rounds * slots)
+      us = kb_us + _KB_FULL_US.get((cg, bn), (0.0, 0.0))[s_eff > 1] * tiles * s_eff / (rounds * slots)
       cost = rounds * max(per * us, epi_us) + epi_us
       if s_eff > 1:
         cost = cost * 1.05 + 3.0 + s_eff * M * N * 8 / 6e6
