@@ -40,13 +40,13 @@ constexpr int FIXED_BYTES = STAGING_BYTES + BIAS_BYTES + 256 /*barriers*/;
 constexpr int SMEM_LIMIT = 227 * 1024;
 // One stage holds a k-block of A (128 rows) and of this CTA's share of B; a multiple of 1024 bytes.
 __host__ __device__ constexpr int stage_bytes(int bn, int cg) { return A_BYTES + bn / cg * BK * 2; }
-// As many stages as fit: one CTA's tile 256 columns wide takes four (4 x 48 KiB; 3 stages / 4: 4608 x 9216 x 3072 244 / 202 us,
-// 8192 x 5120 x 320 43.5 / 30.7 us). `room` leaves 8 KB, in which CTAs of the kernels before and after can be on the SM too (each
-// takes a reserved kilobyte) so that launches overlap: under a cut contraction, for its fold (320 x 320 x 16384 19.3 us with
-// every byte taken, 13.0 so), and in launches of at most two rounds, where it costs at most one stage of many (a Flux preview
-// step, 300 launches, 3.63 / 3.50 ms; steps of longer products are 0.7 % faster without).
-__host__ constexpr int stages_for(int bn, int cg, bool room) {
-  const int n = (SMEM_LIMIT - FIXED_BYTES - (room ? 8192 : 0)) / stage_bytes(bn, cg);
+// As many stages as fit beside 8 KB, in which CTAs of the kernels before and after (a cut contraction's fold) can be on the SM
+// too, each with a reserved kilobyte, so that launches overlap: with every byte taken 320 x 320 x 16384 took 19.3 us, 13.0 so, a
+// Flux preview step (300 launches) 3.63 and 3.50 ms, a Wan step of 2 x 32760 tokens 160.4 and 158.7 ms. One CTA's tile 256 columns
+// wide takes all for its fourth stage (3 / 4: 4608 x 9216 x 3072 244 / 202 us, 8192 x 5120 x 320 43.5 / 30.7 us) unless a fold follows.
+__host__ constexpr int stages_for(int bn, int cg, bool cut) {
+  const int room = (SMEM_LIMIT - 8192 - FIXED_BYTES) / stage_bytes(bn, cg), all = (SMEM_LIMIT - FIXED_BYTES) / stage_bytes(bn, cg);
+  const int n = cut || room > 3 ? room : all;
   return n < MAX_STAGES ? n : MAX_STAGES;
 }
 
@@ -103,12 +103,6 @@ constexpr int MAX_MATS = 3;
 struct BMaps {
   CUtensorMap m[MAX_MATS];
 };
-
-static int pick_stages(const Params& p, int cg, int out_n) {
-  const long long tiles = static_cast<long long>((p.M + cg * BM - 1) / (cg * BM)) * ((p.N + out_n - 1) / out_n) * p.mats;
-  const bool few = tiles <= 2ll * (sm_count() / cg) && stages_for(p.bn, cg, true) > 3;
-  return stages_for(p.bn, cg, p.splits > 1 || few);
-}
 
 template <int GROUP_M>
 __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int& m_idx, int& n_idx) {
@@ -748,7 +742,7 @@ extern "C" int mdb_gemm_bf16(const void* A, const void* B, void* out, const void
     p.partial = static_cast<float*>(partial);
     if (p.splits <= 1) { p.splits = 1; p.kb_per_split = num_kb; }
   }
-  p.stages = pick_stages(p, ctas, bn);
+  p.stages = stages_for(bn, ctas, p.splits > 1);
   const bool f32 = out_f32 || p.splits > 1;
   const bool act = epi == kEpiGeluTanh || epi == kEpiSilu, res = epi == kEpiGatedRes || epi == kEpiAddRes;
   int kind = kDirect;
@@ -793,7 +787,7 @@ extern "C" int mdb_gemm_geglu(const void* A, const void* B, void* out, const voi
   p.splits = 1;
   p.kb_per_split = (K + BK - 1) / BK;
   p.bn = bn;
-  p.stages = pick_stages(p, ctas, bn / 2);
+  p.stages = stages_for(bn, ctas, false);
   p.status = status_buffer();
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   return launch<false, false, 2, kGeglu>(ta, tb, p, stream);
@@ -828,7 +822,7 @@ extern "C" int mdb_gemm_group(const void* A, const void* const* B, int mats, voi
   p.splits = 1;
   p.kb_per_split = (K + BK - 1) / BK;
   p.bn = bn;
-  p.stages = pick_stages(p, ctas, bn);
+  p.stages = stages_for(bn, ctas, false);
   p.status = status_buffer();
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   return ctas == 2 ? launch<false, false, 2, kPlain>(ta, tb, p, stream) : launch<false, false, 1, kPlain>(ta, tb, p, stream);
