@@ -41,8 +41,8 @@ constexpr int SMEM_LIMIT = 227 * 1024;
 // One stage holds a k-block of A (128 rows) and of this CTA's share of B; a multiple of 1024 bytes.
 __host__ __device__ constexpr int stage_bytes(int bn, int cg) { return A_BYTES + bn / cg * BK * 2; }
 // As many stages as fit beside 8 KB, in which CTAs of the kernels before and after (a cut contraction's fold) can be on the SM
-// too, each with a reserved kilobyte, so that launches overlap: with every byte taken 320 x 320 x 16384 took 19.3 us, 13.0 so, a
-// Flux preview step (300 launches) 3.63 and 3.50 ms, a Wan step of 2 x 32760 tokens 160.4 and 158.7 ms. One CTA's tile 256 columns
+// too, each with a reserved kilobyte, so that launches overlap: with every byte taken 320 x 320 x 16384 took 19.3 us, 13.0 so, and
+// a Flux preview step (300 launches) 3.63 and 3.50 ms; steps of long products are the same either way. One CTA's tile 256 columns
 // wide takes all for its fourth stage (3 / 4: 4608 x 9216 x 3072 244 / 202 us, 8192 x 5120 x 320 43.5 / 30.7 us) unless a fold follows.
 __host__ constexpr int stages_for(int bn, int cg, bool cut) {
   const int room = (SMEM_LIMIT - 8192 - FIXED_BYTES) / stage_bytes(bn, cg), all = (SMEM_LIMIT - FIXED_BYTES) / stage_bytes(bn, cg);
