@@ -29,7 +29,7 @@ constexpr int X_CHUNK_BYTES = BX * 128;         // 16 KiB
 constexpr int Y_CHUNK_BYTES = BY * 128;         // 8 KiB
 constexpr int MAX_SEGMENTS = 8;
 constexpr int EW_GROUPS = 4;                    // elementwise warp groups, 16 of the 64 columns each
-// Waits pause before they poll on (`mbar_wait<true>`): four elementwise groups and four role warps share the issue slots, and
+// Waits pause before they poll on (`mbar_wait<1>`): four elementwise groups and four role warps share the issue slots, and
 // tries without a pause take them from the groups that work. dQ + dK/dV at once, without / with the pause: 2 x 4096^2 x 10
 // heads of 64 474 / 436 us, 4608^2 x 24 heads of 128 737 / 709 us, 7000^2 x 3 heads of 128 380 / 353 us.
 constexpr int NUM_THREADS = 128 + EW_GROUPS * 128;  // warp 0 TMA, warp 1 score MMAs, warp 2 accumulating MMAs, warps 4.. elementwise
@@ -176,7 +176,7 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
       for (int seg = 0; seg < p.num_segments && ok; ++seg) {
         const int nblk = (p.y_len[seg] + BY - 1) / BY;
         for (int jb = 0; jb < nblk; ++jb) {
-          if (!mbar_wait<true>(&y_empty[stage], phase ^ 1u, abort_flag, p.status, 70)) { ok = false; break; }
+          if (!mbar_wait<1>(&y_empty[stage], phase ^ 1u, abort_flag, p.status, 70)) { ok = false; break; }
           float* st = stat_s + stage * 128;
           const uint32_t stat_bytes = stat_bulk ? static_cast<uint32_t>(min(BY, p.q_len - jb * BY)) * 4u : 0u;
           if (DKV && !stat_bulk) {
@@ -214,7 +214,7 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
     if (total_steps > 0 && issuing_lane<HD>(lane)) {
       constexpr uint32_t idesc_t = make_idesc_bf16(128, BY, false, false);   // score tiles, N = 64
       const bool second = warp == 3;
-      bool ok = mbar_wait<true>(x_full, 0, abort_flag, p.status, 80);
+      bool ok = mbar_wait<1>(x_full, 0, abort_flag, p.status, 80);
       tc_fence_after_sync();
       // Shared-memory descriptors are built once: the address field (bits 0-13, units of 16 bytes) of a
       // descriptor advances by plain addition.
@@ -227,10 +227,10 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
       for (int i = 0; i < total_steps && ok; ++i) {
         const int b = i % NBUF, use = i / NBUF;
         const uint64_t yd = ys0 + stage * STAGE_STEP;
-        if (!mbar_wait<true>(&y_full[stage], phase, abort_flag, p.status, 81)) { ok = false; break; }
+        if (!mbar_wait<1>(&y_full[stage], phase, abort_flag, p.status, 81)) { ok = false; break; }
         // the buffer was last used by step i - NBUF: its reader (a product, or in the DQ pass the elementwise load of
         // the first tile) must be done
-        if (use > 0 && !mbar_wait<true>(second ? &t2_free[b] : &t1_free[b], (use - 1) & 1, abort_flag, p.status, 82)) { ok = false; break; }
+        if (use > 0 && !mbar_wait<1>(second ? &t2_free[b] : &t1_free[b], (use - 1) & 1, abort_flag, p.status, 82)) { ok = false; break; }
         tc_fence_after_sync();
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
@@ -255,14 +255,14 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
         const uint64_t y1d = ym0 + stage * STAGE_STEP, y2d = y1d + TILE_STEP;
         if (DKV) {
           // dV += P^T dO_i as soon as P^T is stored; the first score tile is free afterwards
-          if (!mbar_wait<true>(&p_ready[b], use & 1, abort_flag, p.status, 83)) { ok = false; break; }
+          if (!mbar_wait<1>(&p_ready[b], use & 1, abort_flag, p.status, 83)) { ok = false; break; }
           tc_fence_after_sync();
 #pragma unroll
           for (int k = 0; k < BY / 16; ++k)  // packed bf16 columns of K-step k were written by column group k
             umma_ts(tmem_base + ACC, tmem_base + b * 64 + k * 16, y2d + k * (2048 >> 4), idesc_acc, (i > 0 || k > 0) ? 1u : 0u);
           umma_commit(&t1_free[b]);
         }
-        if (!mbar_wait<true>(&ds_ready[b], use & 1, abort_flag, p.status, 84)) { ok = false; break; }
+        if (!mbar_wait<1>(&ds_ready[b], use & 1, abort_flag, p.status, 84)) { ok = false; break; }
         tc_fence_after_sync();
 #pragma unroll
         for (int k = 0; k < BY / 16; ++k)  // DKV: dK += dS^T Q_i;  DQ: dQ += dS K_j
@@ -299,15 +299,15 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
           const int ystage = i % Y_STAGES;
           const float* st = stat_s + ystage * 128;
           if (DKV) {
-            if (!mbar_wait<true>(&y_full[ystage], (i / Y_STAGES) & 1, abort_flag, p.status, 92)) { ok = false; break; }
+            if (!mbar_wait<1>(&y_full[ystage], (i / Y_STAGES) & 1, abort_flag, p.status, 92)) { ok = false; break; }
           }
           const bool full_tile = (valid == BY) && (x0 + BX <= x_len);  // uniform over the CTA
           const uint32_t t1a = tmem_base + lane_off + b * 64 + wg * 16;
           const uint32_t t2a = tmem_base + lane_off + T2C + b * 64 + wg * 16;
           // ---- phase 1: P of this thread's 16 columns from the first score tile
-          if (!mbar_wait<true>(&t1_full[b], use & 1, abort_flag, p.status, 90)) { ok = false; break; }
+          if (!mbar_wait<1>(&t1_full[b], use & 1, abort_flag, p.status, 90)) { ok = false; break; }
           if (!DKV) {  // the DQ pass has nothing to hand over between the tiles: one phase, both tiles loaded at once
-            if (!mbar_wait<true>(&t2_full[b], use & 1, abort_flag, p.status, 93)) { ok = false; break; }
+            if (!mbar_wait<1>(&t2_full[b], use & 1, abort_flag, p.status, 93)) { ok = false; break; }
           }
           tc_fence_after_sync();
           uint32_t t1[16], t2[16], ds[8];
@@ -357,7 +357,7 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
           }
           // ---- phase 2: dS = P * (dP - delta) over the second score tile
           if (DKV) {
-            if (!mbar_wait<true>(&t2_full[b], use & 1, abort_flag, p.status, 93)) { ok = false; break; }
+            if (!mbar_wait<1>(&t2_full[b], use & 1, abort_flag, p.status, 93)) { ok = false; break; }
             tc_fence_after_sync();
             tmem_ld_x16(t2a, t2);
             tmem_wait_ld();
@@ -396,7 +396,7 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
           if (lane == 0) mbar_arrive(&ds_ready[b]);
         }
       }
-      if (ok && mbar_wait<true>(acc_final, 0, abort_flag, p.status, 91)) {
+      if (ok && mbar_wait<1>(acc_final, 0, abort_flag, p.status, 91)) {
         tc_fence_after_sync();
         // each column group writes a quarter of the output columns of every accumulator, 16 at a time
         const int n_acc = DKV ? 2 : 1;

@@ -4,13 +4,21 @@
 //   S_t = Q_t K_j^T      SS-form UMMA, fp32 in TMEM (64 columns), two buffers per tile
 //   P_t = exp2(S_t*c - m) written back over S_t as packed bf16 (tcgen05.st)
 //   O_t += P_t V_j       TS-form UMMA (A from TMEM, V is an MN-major smem operand)
-// The softmax is bound by the exponential unit (16 results per clock and SM, as many cycles per tile as both
-// products together), so the layout keeps the softmax warps of both tiles busy all the time: S of block j+1 is
-// multiplied into the tile's second buffer while block j is exponentiated, and four lanes in different warps issue
-// the products (S and P V of either tile), because the waits, commits and MMA instructions of a block cost one
-// issuing lane more cycles than the products take to run. Every hand-over is an mbarrier.
-// The running row max is refreshed lazily (only when it moves by more than 2^8), so the
-// accumulator rescale is rare; it waits for the tile's previous P V product first. The KV sequence may consist of several segments (one per ring
+// Two units have about the same to do: the exponential unit (16 results per clock and SM: 1024 clocks per block of both tiles)
+// and, at head_dim 128, the tensor pipe (1280 clocks: S at 64 columns is held back by shared memory, 4 KB of Q and 2 KB of K
+// per step of 16 at 128 bytes a clock). What is lost is lost in the softmax warps, two to a scheduler, whose chain
+// S -> P must stay short and whose issue slots nobody else may take:
+//   - S of block j+1 is multiplied into the tile's second buffer while block j is exponentiated;
+//   - a block is exponentiated against the running maximum while its own is still being taken (see below): 270 clocks off
+//     the chain of 1850 per block;
+//   - one lane per tile issues both of its products, and every wait sleeps between tries. With a lane per product
+//     (two spinning warps on the first scheduler) the softmax warps there ran 1000 clocks per block behind the others.
+// Together, against four issuing lanes, maximum first, waits that spin: 1 x 4608^2 x 24 heads of 128 236 -> 213 us,
+// 75600^2 x 8 heads of 128 21.9 -> 19.1 ms (under the power cap), 4 x 4096^2 x 10 heads of 64 301 -> 268 us; the same bits.
+// 128-key S tiles in a single buffer feed the tensor pipe better but lengthen the chain by more: 3.7 ms where this kernel
+// takes 3.1 (32760^2 x 8 heads). Turns of the two tiles at the exponential unit cost more in hand-overs than they save.
+// The running row max is refreshed lazily (only when it moves by more than 2^8), so the accumulator rescale is rare; it
+// waits for the tile's previous P V product first, and the block is then exponentiated again. The KV sequence may consist of several segments (one per ring
 // hop / context shard); (O, m, l) stay on chip across segments and the merge costs nothing.
 // A segment can be guarded by a ready flag in global memory that the loader warp waits on
 // (bounded) before its first TMA load of that segment.
@@ -48,8 +56,10 @@ constexpr int DEFAULT_KV_STAGES = 4;  // K / V pipeline depth; 2..5 are built an
 constexpr int CHUNK_BYTES = 128 * 128;       // 16 KiB: one chunk of a 128-row Q tile
 constexpr int KV_CHUNK_BYTES = BKV * 128;    // 8 KiB: one chunk of a 64-key K / V tile
 constexpr int MAX_SEGMENTS = 8;
-constexpr int ROLE_WARPS = 5;            // warp 0 TMA, warps 1 / 3 issue S of tile 0 / 1, warps 2 / 4 issue P V of tile 0 / 1
-constexpr int NUM_THREADS = ROLE_WARPS * 32 + 256;  // + softmax warps 5-8 (tile 0), 9-12 (tile 1)
+constexpr int ROLE_WARPS = 4;            // warp 0 TMA, warps 1 / 2 issue the products of tile 0 / 1, warp 3 allocates TMEM
+constexpr int NUM_THREADS = ROLE_WARPS * 32 + 256;  // + softmax warps 4-7 (tile 0), 8-11 (tile 1)
+// Sleep between the tries of a wait, in ns. A warp that polls takes issue slots from the softmax warps of its scheduler.
+constexpr int LOAD_PAUSE = 100, PAUSE = 20;
 template <int HD, int KV_STAGES>
 constexpr int smem_bytes() { return 2 * (HD / 64) * CHUNK_BYTES + 2 * KV_STAGES * (HD / 64) * KV_CHUNK_BYTES + 1024 + 512; }
 constexpr float kRescaleThreshold = 8.0f;
@@ -234,16 +244,23 @@ __device__ __forceinline__ void copy_cta(const CopyPlan& cp, int ci, DeviceStatu
 
 // exp2(s * scale - m) of 64 scores of a row, packed as bf16; returns the fp32 sums over even and odd keys. A ragged
 // tail (FULL = false) is a function of its own: the tests on every score would cost the common case as much as the rest.
-template <bool FULL>
-__device__ __forceinline__ uint64_t exp_half(const uint32_t (&s)[2][32], uint32_t (&pk)[32], float scale, float m, int valid) {
+// MAX also takes the maximum of the scores, in the shadow of the exponential unit.
+template <bool FULL, bool MAX>
+__device__ __forceinline__ uint64_t exp_half(const uint32_t (&s)[2][32], uint32_t (&pk)[32], float scale, float m, int valid, float& mx) {
   const uint64_t scale2 = pack_f32x2(scale, scale), neg_m2 = pack_f32x2(-m, -m);
   uint64_t rs = 0;
+  float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       float p0, p1;
-      unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[c][2 * i]), __uint_as_float(s[c][2 * i + 1])), scale2, neg_m2), p0, p1);
+      const float s0 = __uint_as_float(s[c][2 * i]), s1 = __uint_as_float(s[c][2 * i + 1]);
+      if (MAX) {
+        if (i & 1) mx1 = max3(mx1, s0, s1);
+        else mx0 = max3(mx0, s0, s1);
+      }
+      unpack_f32x2(fma_f32x2(pack_f32x2(s0, s1), scale2, neg_m2), p0, p1);
       p0 = fast_exp2(p0);
       p1 = fast_exp2(p1);
       if (!FULL) {
@@ -255,6 +272,7 @@ __device__ __forceinline__ uint64_t exp_half(const uint32_t (&s)[2][32], uint32_
       pk[c * 16 + i] = pack_bf16x2(p0, p1);
     }
   }
+  if (MAX) mx = fmaxf(mx0, mx1);
   return rs;
 }
 
@@ -336,7 +354,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     fence_mbar_init();
     prefetch_tensormap(&tmap_q);
   }
-  if (warp == 1) {
+  if (warp == 3) {
     tmem_alloc(tmem_ptr_smem, 512);
     tmem_relinquish();
   }
@@ -360,7 +378,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const Item item = item_of(work, n_qb, p);
         const int head = item.head, batch = item.batch, q0 = item.q0, n_tiles = item.n_tiles;
         if (n_tiles == 0) continue;
-        if (!mbar_wait(q_empty, (it & 1) ^ 1u, abort_flag, p.status, 43)) { ok = false; break; }
+        if (!mbar_wait<LOAD_PAUSE>(q_empty, (it & 1) ^ 1u, abort_flag, p.status, 43)) { ok = false; break; }
         ++it;
         mbar_expect_tx(q_full, n_tiles * TILE_BYTES);
         for (int t = 0; t < n_tiles; ++t) {
@@ -379,13 +397,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             }
           }
           for (int jb = 0; jb < nblk; ++jb) {
-            if (!mbar_wait(&k_empty[stage], phase ^ 1u, abort_flag, p.status, 41)) { ok = false; break; }
+            if (!mbar_wait<LOAD_PAUSE>(&k_empty[stage], phase ^ 1u, abort_flag, p.status, 41)) { ok = false; break; }
             mbar_expect_tx(&k_full[stage], KV_TILE_BYTES);
             for (int c = 0; c < CH; ++c) {
               tma_load_4d(sk + stage * KV_TILE_BYTES + c * KV_CHUNK_BYTES, &maps.k[seg], &k_full[stage], c * 64, head,
                           jb * BKV, batch);
             }
-            if (!mbar_wait(&v_empty[stage], phase ^ 1u, abort_flag, p.status, 42)) { ok = false; break; }
+            if (!mbar_wait<LOAD_PAUSE>(&v_empty[stage], phase ^ 1u, abort_flag, p.status, 42)) { ok = false; break; }
             mbar_expect_tx(&v_full[stage], KV_TILE_BYTES);
             for (int c = 0; c < CH; ++c) {
               tma_load_4d(sv + stage * KV_TILE_BYTES + c * KV_CHUNK_BYTES, &maps.v[seg], &v_full[stage], c * 64, head,
@@ -396,17 +414,20 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
       }
     }
-  } else if (warp == 1 || warp == 3) {
-    // ------------------------------ issuing lanes: S_t = Q_t K_j^T --------------
+  } else if (warp == 1 || warp == 2) {
+    // ------------------------------ issuing lanes: S_t = Q_t K_j^T, O_t += P_t V_j --------------
     if (total_blocks > 0 && elect_one()) {
-      const int t = warp >> 1;  // warp 1 -> tile 0, warp 3 -> tile 1
+      const int t = warp - 1;
       constexpr uint32_t idesc_s = make_idesc_bf16(128, BKV, false, false);
+      constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, false, true);
       // descriptors are built once; the address field (units of 16 bytes) advances by addition
       const uint64_t qd = make_smem_desc(smem_u32(sq + t * TILE_BYTES), 16, 1024);
       const uint64_t kd0 = make_smem_desc(smem_u32(sk), 16, 1024);
+      const uint64_t vd0 = make_smem_desc(smem_u32(sv), KV_CHUNK_BYTES, 1024);
       constexpr uint32_t STAGE_STEP = KV_TILE_BYTES >> 4;
-      int stage = 0;
-      uint32_t phase = 0;
+      const uint32_t o_col = tmem_base + 256 + t * 128;
+      int k_stage = 0, v_stage = 0;
+      uint32_t k_phase = 0, v_phase = 0;
       uint32_t n = 0;  // blocks of this tile so far, over all work items: buffer n & 1, use n >> 1
       bool ok = true;
       int it = 0;
@@ -414,71 +435,54 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         const int n_tiles = item_of(work, n_qb, p).n_tiles;
         if (n_tiles == 0) continue;
         const bool active = t < n_tiles;
-        if (!mbar_wait(q_full, it & 1, abort_flag, p.status, 50)) { ok = false; break; }
+        if (!mbar_wait<PAUSE>(q_full, it & 1, abort_flag, p.status, 50)) { ok = false; break; }
         ++it;
-        for (int j = 0; j < total_blocks; ++j) {
-          if (!mbar_wait(&k_full[stage], phase, abort_flag, p.status, 51)) { ok = false; break; }
-          if (active) {
-            const uint32_t b = n & 1u;
-            // the buffer last held P of block n - 2: its P V product must have completed
-            if (n >= 2 && !mbar_wait(&s_free[t * 2 + b], ((n >> 1) - 1) & 1u, abort_flag, p.status, 55)) { ok = false; break; }
-            tc_fence_after_sync();
-            const uint64_t kd = kd0 + stage * STAGE_STEP;
-            const uint32_t s_col = tmem_base + t * 128 + b * 64;
+        // S of block j + 1 is issued ahead of P V of block j
+        for (int j = -1; j < total_blocks; ++j) {
+          if (j + 1 < total_blocks) {
+            if (!mbar_wait<PAUSE>(&k_full[k_stage], k_phase, abort_flag, p.status, 51)) { ok = false; break; }
+            if (active) {
+              const uint32_t g = n + (j < 0 ? 0u : 1u), b = g & 1u;
+              // the buffer last held P of block g - 2: its P V product must have completed
+              if (g >= 2 && !mbar_wait<PAUSE>(&s_free[t * 2 + b], ((g >> 1) - 1) & 1u, abort_flag, p.status, 55)) { ok = false; break; }
+              tc_fence_after_sync();
+              const uint64_t kd = kd0 + k_stage * STAGE_STEP;
+              const uint32_t s_col = tmem_base + t * 128 + b * 64;
 #pragma unroll
-            for (int k = 0; k < D / 16; ++k) {
-              const uint32_t qo = ((k >> 2) * CHUNK_BYTES + (k & 3) * 32) >> 4;
-              const uint32_t ko = ((k >> 2) * KV_CHUNK_BYTES + (k & 3) * 32) >> 4;
-              umma_ss(s_col, qd + qo, kd + ko, idesc_s, k > 0 ? 1u : 0u);
+              for (int k = 0; k < D / 16; ++k) {
+                const uint32_t qo = ((k >> 2) * CHUNK_BYTES + (k & 3) * 32) >> 4;
+                const uint32_t ko = ((k >> 2) * KV_CHUNK_BYTES + (k & 3) * 32) >> 4;
+                umma_ss(s_col, qd + qo, kd + ko, idesc_s, k > 0 ? 1u : 0u);
+              }
+              umma_commit(&s_full[t * 2 + b]);
+              umma_commit(&k_empty[k_stage]);  // this K block is free once the S MMAs have read it
+              // the S MMAs of the last block are the last readers of the Q tile: free it for the next work item
+              if (j + 2 == total_blocks) umma_commit(q_empty);
+            } else {
+              mbar_arrive(&k_empty[k_stage]);
+              if (j + 2 == total_blocks) mbar_arrive(q_empty);
             }
-            umma_commit(&s_full[t * 2 + b]);
-            umma_commit(&k_empty[stage]);  // this K block is free once the S MMAs have read it
-            // the S MMAs of the last block are the last readers of the Q tile: free it for the next work item
-            if (j + 1 == total_blocks) umma_commit(q_empty);
-            ++n;
-          } else {
-            mbar_arrive(&k_empty[stage]);
-            if (j + 1 == total_blocks) mbar_arrive(q_empty);
+            if (++k_stage == KV_STAGES) { k_stage = 0; k_phase ^= 1u; }
           }
-          if (++stage == KV_STAGES) { stage = 0; phase ^= 1u; }
-        }
-      }
-    }
-  } else if (warp == 2 || warp == 4) {
-    // ------------------------------ issuing lanes: O_t += P_t V_j ----------------
-    if (total_blocks > 0 && elect_one()) {
-      const int t = (warp >> 1) - 1;  // warp 2 -> tile 0, warp 4 -> tile 1
-      constexpr uint32_t idesc_pv = make_idesc_bf16(128, D, false, true);
-      const uint64_t vd0 = make_smem_desc(smem_u32(sv), KV_CHUNK_BYTES, 1024);
-      constexpr uint32_t STAGE_STEP = KV_TILE_BYTES >> 4;
-      const uint32_t o_col = tmem_base + 256 + t * 128;
-      int stage = 0;
-      uint32_t phase = 0;
-      uint32_t n = 0;
-      bool ok = true;
-      for (int work = blockIdx.x; work < total_work && ok; work += n_compute) {
-        const int n_tiles = item_of(work, n_qb, p).n_tiles;
-        if (n_tiles == 0) continue;
-        const bool active = t < n_tiles;
-        for (int j = 0; j < total_blocks; ++j) {
-          if (!mbar_wait(&v_full[stage], phase, abort_flag, p.status, 52)) { ok = false; break; }
+          if (j < 0) continue;
+          if (!mbar_wait<PAUSE>(&v_full[v_stage], v_phase, abort_flag, p.status, 52)) { ok = false; break; }
           if (active) {
             const uint32_t b = n & 1u;
-            if (!mbar_wait(&p_full[t * 2 + b], (n >> 1) & 1u, abort_flag, p.status, 53)) { ok = false; break; }
+            if (!mbar_wait<PAUSE>(&p_full[t * 2 + b], (n >> 1) & 1u, abort_flag, p.status, 53)) { ok = false; break; }
             tc_fence_after_sync();
-            const uint64_t vd = vd0 + stage * STAGE_STEP;
+            const uint64_t vd = vd0 + v_stage * STAGE_STEP;
             const uint32_t p_col = tmem_base + t * 128 + b * 64;
 #pragma unroll
             for (int k = 0; k < BKV / 16; ++k)
               umma_ts(o_col, p_col + k * 8, vd + k * (2048 >> 4), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
             umma_commit(&s_free[t * 2 + b]);
-            umma_commit(&v_empty[stage]);
+            umma_commit(&v_empty[v_stage]);
             if (j + 1 == total_blocks) umma_commit(&o_final[t]);
             ++n;
           } else {
-            mbar_arrive(&v_empty[stage]);
+            mbar_arrive(&v_empty[v_stage]);
           }
-          if (++stage == KV_STAGES) { stage = 0; phase ^= 1u; }
+          if (++v_stage == KV_STAGES) { v_stage = 0; v_phase ^= 1u; }
         }
       }
     }
@@ -508,36 +512,37 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           const int valid = min(BKV, p.kv_len[seg] - jb * BKV);
           const uint32_t b = n & 1u;
           const uint32_t s_addr = tmem_base + lane_off + t * 128 + b * 64;
-          if (!mbar_wait(&s_full[t * 2 + b], (n >> 1) & 1u, abort_flag, p.status, 60)) { ok = false; break; }
+          if (!mbar_wait<PAUSE>(&s_full[t * 2 + b], (n >> 1) & 1u, abort_flag, p.status, 60)) { ok = false; break; }
           tc_fence_after_sync();
           uint32_t sv2[2][32];
           tmem_ld_x32(s_addr, sv2[0]);
           tmem_ld_x32(s_addr + 32, sv2[1]);
           tmem_wait_ld();
-          if (!fixed) {
-            float mx0 = -INFINITY, mx1 = -INFINITY;  // two chains
-            if (valid == BKV) {
-#pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                mx0 = max3(mx0, __uint_as_float(sv2[0][i]), __uint_as_float(sv2[0][i + 1]));
-                mx1 = max3(mx1, __uint_as_float(sv2[1][i]), __uint_as_float(sv2[1][i + 1]));
-              }
-            } else {
+          // Probabilities, to be written over S as packed bf16 (32 columns). The maximum moves by more than the threshold
+          // in few blocks only, so a block is exponentiated against the running one while its own is still being taken,
+          // and again in the rare case: the maximum is off the chain from S to P.
+          uint32_t pk[32];
+          uint64_t rs = 0;
+          float mx = -INFINITY;
+          bool done = false;
+          if (!fixed && j > 0 && valid == BKV) {
+            rs = exp_half<true, true>(sv2, pk, p.scale_log2, m, valid, mx);
+            done = !__any_sync(0xffffffffu, mx * p.scale_log2 - m > kRescaleThreshold);
+          }
+          if (!done) {
+            if (!fixed) {
 #pragma unroll
               for (int c = 0; c < 2; ++c)
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
-                  if (c * 32 + i < valid) mx0 = fmaxf(mx0, __uint_as_float(sv2[c][i]));
+                  if (c * 32 + i < valid) mx = fmaxf(mx, __uint_as_float(sv2[c][i]));
                 }
-            }
-            const float m_new = fmaxf(m, fmaxf(mx0, mx1) * p.scale_log2);
-            if (j == 0) {
-              m = m_new;
-            } else {
-              const bool need = (m_new - m) > kRescaleThreshold;
-              if (__any_sync(0xffffffffu, need)) {
+              const float m_new = fmaxf(m, mx * p.scale_log2);
+              if (j == 0) {
+                m = m_new;
+              } else if (__any_sync(0xffffffffu, m_new - m > kRescaleThreshold)) {
                 // O must be at rest: the P V product of the previous block (the other buffer) has to be complete
-                if (!mbar_wait(&s_free[t * 2 + (b ^ 1u)], ((n - 1) >> 1) & 1u, abort_flag, p.status, 62)) { ok = false; break; }
+                if (!mbar_wait<PAUSE>(&s_free[t * 2 + (b ^ 1u)], ((n - 1) >> 1) & 1u, abort_flag, p.status, 62)) { ok = false; break; }
                 tc_fence_after_sync();
                 const float alpha = fast_exp2(m - m_new);
                 l *= alpha;
@@ -554,11 +559,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
                 tmem_wait_st();
               }
             }
+            rs = valid == BKV ? exp_half<true, false>(sv2, pk, p.scale_log2, m, valid, mx)
+                              : exp_half<false, false>(sv2, pk, p.scale_log2, m, valid, mx);
           }
-          // probabilities, written over S as packed bf16 (32 columns)
-          uint32_t pk[32];
-          const uint64_t rs = valid == BKV ? exp_half<true>(sv2, pk, p.scale_log2, m, valid)
-                                           : exp_half<false>(sv2, pk, p.scale_log2, m, valid);
           float rs0, rs1;
           unpack_f32x2(rs, rs0, rs1);
           tmem_st_x32(s_addr, pk);
@@ -570,7 +573,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         }
       }
       if (!ok) break;
-      if (!mbar_wait(&o_final[t], oc & 1u, abort_flag, p.status, 61)) { ok = false; break; }
+      if (!mbar_wait<PAUSE>(&o_final[t], oc & 1u, abort_flag, p.status, 61)) { ok = false; break; }
       ++oc;
       tc_fence_after_sync();
       const float inv = (l > 0.0f) ? 1.0f / l : 0.0f;
@@ -613,7 +616,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 3) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }

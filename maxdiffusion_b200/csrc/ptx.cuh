@@ -114,19 +114,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 // Bounded wait. `abort_flag` lives in shared memory: once any role of the CTA gives up, every
 // other role leaves its loops at its next wait. The clock is first read after a batch of failed tries, since most waits end
-// before; PAUSE reads it after the first one, which holds the next try back for as long as that read takes.
-template <bool PAUSE = false>
+// before; PAUSE = 1 reads it after the first one, which holds the next try back for as long as that read takes, and a larger
+// PAUSE sleeps for about that many nanoseconds after every failed try.
+template <int PAUSE = 0>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           DeviceStatus* st, unsigned int where) {
   uint64_t t0 = 0;
-  if (PAUSE) {
+  if (PAUSE == 1) {
     if (mbar_try_wait(bar, parity)) return true;
     t0 = global_timer_ns();
   }
   uint32_t spins = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((++spins & 0x3ffu) == 0u) {
+    if (PAUSE > 1) __nanosleep(PAUSE);
+    if ((++spins & (PAUSE > 1 ? 0x3fu : 0x3ffu)) == 0u) {
       if (*abort_flag) return false;
       if (status_failed(st)) {
         *abort_flag = 1;

@@ -194,3 +194,31 @@ def test_a_bias_may_start_anywhere(epi, f32, direct):
   y = {"none": lambda: y, "gelu_tanh": lambda: torch.nn.functional.gelu(y, approximate="tanh"),
        "silu": lambda: torch.nn.functional.silu(y), "add_res": lambda: y + res.double()}[epi]()
   assert _rel(got, y) < (1e-3 if f32 else 4e-3)  # the approximate tanh and exponential; one rounding to bf16
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,lens", [(128, [65]), (257, [128]), (300, [192]), (130, [577]), (384, [64, 129, 200])])
+def test_attention_when_the_maximum_moves(D, Sq, lens):
+  """A block is exponentiated against the running maximum and again when its own is far above it: scores that grow from
+  block to block for some rows, stay for others, over tails and segments. Probabilities and the output are rounded to bf16."""
+  torch.manual_seed(11)
+  q = _randn(2, Sq, 3, D)
+  k = [_randn(2, n, 3, D) for n in lens]
+  v = [_randn(2, n, 3, D) for n in lens]
+  q[:, ::5] *= 0.05  # rows whose maximum hardly moves beside rows whose maximum does
+  at = 0
+  for x in k:
+    x *= (1.0 + (torch.arange(x.shape[1], device="cuda") + at)[None, :, None, None] / 24).to(torch.bfloat16)
+    at += x.shape[1]
+  kk, vv = torch.cat(k, 1).double().transpose(1, 2), torch.cat(v, 1).double().transpose(1, 2)
+  s = q.double().transpose(1, 2) @ kk.transpose(-1, -2) * D ** -0.5
+  big = torch.zeros((2, at + max(lens), 3, D), device="cuda", dtype=torch.bfloat16)  # segments of one allocation share strides
+  kb, vb = [], []
+  for x, y in zip(k, v):
+    kb.append(big.clone()[:, :x.shape[1]].copy_(x))
+    vb.append(big.clone()[:, :y.shape[1]].copy_(y))
+  got, lse = K.flash_fwd(q, kb, vb)
+  assert _rel(got.transpose(1, 2), s.softmax(-1) @ vv) < 4e-3
+  want = torch.logsumexp(s, -1) / 0.6931471805599453
+  # sums of fp32 exponentials in the log2 domain, scores of up to a few hundred
+  assert (lse.double() - want).abs().max() < 1e-5 * want.abs().max() + 1e-4
