@@ -304,12 +304,15 @@ PyObject* py_linear_group(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// attention(q, k, v, scale): [B,S,H,D] without a log-sum-exp; D a multiple of 8 up to 128
+// attention(q, k, v, scale, out): [B,S,H,D] without a log-sum-exp; D a multiple of 8 up to 128. `out` may be None or a view
+// whose rows of D are dense (a part of a wider buffer).
 PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 4 || !THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2])) return not_implemented();
+  if (n != 5 || !THPVariable_Check(a[0]) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2])) return not_implemented();
   const Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
   const double scale = PyFloat_AsDouble(a[3]);
+  const Tensor* dst = nullptr;
+  if (!opt_tensor(a[4], dst)) return not_implemented();
   if (PyErr_Occurred()) return nullptr;
   const Tensor* ts[3] = {&q, &k, &v};
   for (const Tensor* t : ts) {
@@ -317,6 +320,12 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) return not_implemented();
     for (int i = 0; i < 3; ++i)  // a broadcast dimension of a narrow head is copied, as by the padded path
       if ((t->stride(i) & 7) || (t->stride(i) == 0 && t->size(i) > 1 && t->size(3) != 64 && t->size(3) != 128)) return not_implemented();
+  }
+  if (dst) {
+    if (!bf16(*dst) || dst->sizes() != q.sizes() || dst->stride(3) != 1 || (reinterpret_cast<uintptr_t>(dst->data_ptr()) & 15))
+      return not_implemented();
+    for (int i = 0; i < 3; ++i)
+      if (dst->stride(i) & 7) return not_implemented();
   }
   const int64_t B = q.size(0), S = q.size(1), H = q.size(2), D = q.size(3);
   if (D > 128 || (D & 7) || k.size(0) != B || v.size(0) != B || k.size(2) != H || v.size(2) != H || k.size(3) != D ||
@@ -326,7 +335,7 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int len = static_cast<int>(k.size(1)), b = static_cast<int>(B), h = static_cast<int>(H), s = static_cast<int>(S);
   Tensor out;
   const int rc = unlocked([&] {
-    out = at::empty({B, S, H, D}, q.options());
+    out = dst ? *dst : at::empty({B, S, H, D}, q.options());
     if (D == 128 || D == 64) {
       return (D == 128 ? mdb_flash_fwd : mdb_flash_fwd_d64)(
           q.data_ptr(), &kp, &vp, out.data_ptr(), nullptr, b, h, s, 1, &len, q.stride(0), q.stride(1), q.stride(2), k.stride(0),

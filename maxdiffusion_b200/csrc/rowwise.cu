@@ -12,6 +12,8 @@
 // row, so per-column partial sums live in registers for the whole strip and are written once per
 // CTA to a scratch buffer [gridDim.x * gridDim.y, n_sums, C]; a second kernel folds the partials
 // in a fixed order (bitwise reproducible).
+#include <limits.h>
+
 #include "host_common.h"
 
 namespace mdb {
@@ -582,6 +584,99 @@ rms_rope_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, __nv_bfl
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// The same norm and rotation per 128-wide head for the q and k columns of fused projections, and a copy of the v columns, for
+// up to two streams whose results are joined along the sequence: out[0..2] are [B, s_total, C], stream i's rows start at
+// position `at`. Bound by memory: every row is read once and written once. A warp takes one section (q, k or v) of a row, so
+// that cos, sin and the weight are loaded once for all its heads; short sequences still give three warps per row. One launch
+// instead of up to six (q, k and a copy of v per stream): 512 + 4096 rows of 9216 76.7 -> 29.8 us (5.7 TB/s), 128 + 256 rows
+// 15.0 -> 5.3 us; q and k of 4608 rows 34.6 -> 19.8 us.
+// ---------------------------------------------------------------------------------------
+struct QkvStream {
+  const __nv_bfloat16* x;          // q, k, v columns side by side, C each
+  long long ldx;                   // row pitch; a batch is `rows` rows on
+  const __nv_bfloat16 *wq, *wk;    // [128]
+  const float *cos_t, *sin_t;      // [rows, 64]
+  int rows, at;
+};
+struct QkvArgs {
+  QkvStream s[2];
+  __nv_bfloat16* out[3];
+  int s_total, C, sections;        // sections 2: v stays where it is
+  long long tasks;                 // B * s_total * sections
+  float eps;
+};
+
+__global__ void __launch_bounds__(THREADS) qkv_rope_kernel(const __grid_constant__ QkvArgs p) {
+  allow_successor();
+  wait_for_predecessor();
+  const long long task = (blockIdx.x * static_cast<long long>(THREADS) + threadIdx.x) >> 5;
+  if (task >= p.tasks) return;
+  const int lane = threadIdx.x & 31;
+  const long long row = task / p.sections;  // of the joint sequence
+  const int section = static_cast<int>(task - row * p.sections);
+  const long long batch = row / p.s_total;
+  const int joint_pos = static_cast<int>(row - batch * p.s_total);
+  const QkvStream& st = p.s[joint_pos >= p.s[1].at ? 1 : 0];
+  const int pos = joint_pos - st.at;
+  const __nv_bfloat16* x = st.x + (batch * st.rows + pos) * st.ldx + static_cast<long long>(section) * p.C;
+  __nv_bfloat16* y = p.out[section] + row * p.C;
+  const int nvec = p.C >> 3;  // a multiple of 16: half a warp per head
+  if (section == 2) {
+    for (int v0 = lane; v0 < nvec; v0 += 128) {
+      uint4 r[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (v0 + 32 * u < nvec) r[u] = reinterpret_cast<const uint4*>(x)[v0 + 32 * u];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (v0 + 32 * u < nvec) reinterpret_cast<uint4*>(y)[v0 + 32 * u] = r[u];
+    }
+    return;
+  }
+  float wv[8];
+  load8((section == 0 ? st.wq : st.wk) + (lane & 15) * 8, wv);
+  const int pair0 = (lane & 15) * 4;
+  const float4 cv = *reinterpret_cast<const float4*>(st.cos_t + static_cast<long long>(pos) * 64 + pair0);
+  const float4 sv = *reinterpret_cast<const float4*>(st.sin_t + static_cast<long long>(pos) * 64 + pair0);
+  const float c4[4] = {cv.x, cv.y, cv.z, cv.w};
+  const float s4[4] = {sv.x, sv.y, sv.z, sv.w};
+  for (int b0 = 0; b0 < nvec; b0 += 128) {  // uniform over the warp: the shuffles below need every lane
+    uint4 r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int vi = b0 + 32 * u + lane;
+      r[u] = vi < nvec ? reinterpret_cast<const uint4*>(x)[vi] : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int vi = b0 + 32 * u + lane;
+      if (b0 + 32 * u >= nvec) break;
+      float v[8], sq = 0.0f;
+      const uint32_t w4[4] = {r[u].x, r[u].y, r[u].z, r[u].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = unpack_bf16x2(w4[j]);
+        v[2 * j] = f.x;
+        v[2 * j + 1] = f.y;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sq += v[j] * v[j];
+      const float rstd = rsqrtf(half_warp_sum(sq) / 128.0f + p.eps);
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = v[j] * rstd * wv[j];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = o[2 * j], b = o[2 * j + 1];
+        o[2 * j] = a * c4[j] - b * s4[j];
+        o[2 * j + 1] = a * s4[j] + b * c4[j];
+      }
+      if (vi < nvec) store8(y + vi * 8, o);
+    }
+  }
+}
+
 // Backward: dy is the gradient w.r.t. the rotated output. partial[cta][0][c] = sum_rows dyn*xhat
 // (gradient of w before folding heads when w_per_head).
 template <int NV>
@@ -978,6 +1073,42 @@ extern "C" int mdb_rms_rope_fwd(const void* x, long long ldx, void* y, long long
   if ((ldy | y_batch) & 7) return 3204;
   return launch_rms_rope_fwd(x, ldx, y, ldy, y_batch, w, w_per_head, cos_t, sin_t, num_batches, rows_per_batch, C, group, eps, rstd_out,
                              sc, ctas_per_batch, stream);
+}
+
+// q, k (and v when out_v is not null) of up to two fused projections, joined along the sequence: x[i] is [B, rows[i], >= 2C or
+// 3C] with row pitch ldx[i]; out_* are [B, rows[0] + rows[1], C].
+extern "C" int mdb_qkv_rope_fwd(int n, const void* const* x, const long long* ldx, const int* rows, const void* const* wq,
+                                const void* const* wk, const float* const* cos_t, const float* const* sin_t, int num_batches, int C,
+                                float eps, void* out_q, void* out_k, void* out_v, void* stream) {
+  using namespace mdb::rw;
+  if (n < 1 || n > 2 || C <= 0 || (C & 127)) return 3202;
+  QkvArgs a;
+  a.s_total = 0;
+  for (int i = 0; i < n; ++i) {
+    if (rows[i] < 0 || (ldx[i] & 7) || (reinterpret_cast<uintptr_t>(x[i]) & 15) || (reinterpret_cast<uintptr_t>(wq[i]) & 15) ||
+        (reinterpret_cast<uintptr_t>(wk[i]) & 15) || (reinterpret_cast<uintptr_t>(cos_t[i]) & 15) ||
+        (reinterpret_cast<uintptr_t>(sin_t[i]) & 15))
+      return 3204;
+    a.s[i] = {static_cast<const __nv_bfloat16*>(x[i]), ldx[i], static_cast<const __nv_bfloat16*>(wq[i]),
+              static_cast<const __nv_bfloat16*>(wk[i]), cos_t[i], sin_t[i], rows[i], a.s_total};
+    a.s_total += rows[i];
+  }
+  if (n == 1) {
+    a.s[1] = a.s[0];
+    a.s[1].at = INT_MAX;
+  }
+  a.out[0] = static_cast<__nv_bfloat16*>(out_q);
+  a.out[1] = static_cast<__nv_bfloat16*>(out_k);
+  a.out[2] = static_cast<__nv_bfloat16*>(out_v);
+  a.C = C;
+  a.sections = out_v ? 3 : 2;
+  a.eps = eps;
+  a.tasks = static_cast<long long>(num_batches) * a.s_total * a.sections;
+  if (a.tasks <= 0) return 0;
+  const long long ctas = (a.tasks * 32 + THREADS - 1) / THREADS;
+  if (ctas > INT_MAX) return 3204;
+  launch_overlapped(qkv_rope_kernel, dim3(static_cast<unsigned int>(ctas)), THREADS, 0, static_cast<cudaStream_t>(stream), a);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // The same kernel with the Ulysses head <-> sequence exchange folded into its stores: nothing is written locally; head

@@ -148,11 +148,16 @@ class FluxDoubleBlock(nn.Module):
     H = self.heads
     sh_i, sc_i, g_i, sh2_i, sc2_i, g2_i = _modulation(self.norm1, temb, 6)
     sh_t, sc_t, g_t, sh2_t, sc2_t, g2_t = _modulation(self.norm1_context, temb, 6)
-    qi, ki, vi = split_fused(self.to_qkv(OF.layer_norm_mod(img, scale=sc_i, shift=sh_i)), 3)
-    qt, kt, vt = split_fused(self.add_qkv_proj(OF.layer_norm_mod(txt, scale=sc_t, shift=sh_t)), 3)
-    q = OF.joint_norm_rope([(qt, self.norm_added_q, *rope_txt), (qi, self.norm_q, *rope_img)], H)
-    k = OF.joint_norm_rope([(kt, self.norm_added_k, *rope_txt), (ki, self.norm_k, *rope_img)], H)
-    v = OF.joint_rows([vt, vi]).unflatten(-1, (H, C // H))
+    fi = self.to_qkv(OF.layer_norm_mod(img, scale=sc_i, shift=sh_i))
+    ft = self.add_qkv_proj(OF.layer_norm_mod(txt, scale=sc_t, shift=sh_t))
+    joint = OF.fused_qkv([(ft, self.norm_added_q, self.norm_added_k, *rope_txt), (fi, self.norm_q, self.norm_k, *rope_img)], H)
+    if joint is not None:
+      q, k, v = joint
+    else:
+      (qi, ki, vi), (qt, kt, vt) = split_fused(fi, 3), split_fused(ft, 3)
+      q = OF.joint_norm_rope([(qt, self.norm_added_q, *rope_txt), (qi, self.norm_q, *rope_img)], H)
+      k = OF.joint_norm_rope([(kt, self.norm_added_k, *rope_txt), (ki, self.norm_k, *rope_img)], H)
+      v = OF.joint_rows([vt, vi]).unflatten(-1, (H, C // H))
     o = OF.attention(q, k, v).reshape(B, St + Si, C)
     ot, oi = o[:, :St], o[:, St:]
     # projections are called as modules so that wrappers (run-time LoRA adapters, quantised layers) take effect; a
@@ -177,6 +182,16 @@ class FluxSingleBlock(nn.Module):
     self.norm_q, self.norm_k = nn.Parameter(torch.ones(128)), nn.Parameter(torch.ones(128))
     self.proj_out = Linear(dim + hidden, dim)
 
+  def _qkv(self, f, rope):
+    """q, k, v [B, S, H, 128] of the fused projection's first 3 * dim columns."""
+    C, H = self.dim, self.heads
+    joint = OF.fused_qkv([(f, self.norm_q, self.norm_k, *rope)], H, copy_v=False)
+    if joint is not None:
+      return joint
+    q = OF.rms_norm_rope(f[..., :C], self.norm_q, *rope, heads=H, per_head=True)
+    k = OF.rms_norm_rope(f[..., C:2 * C], self.norm_k, *rope, heads=H, per_head=True)
+    return q, k, f[..., 2 * C:3 * C].unflatten(-1, (H, C // H))
+
   def forward(self, x, temb, rope, pctx=None):
     B, S, C = x.shape
     H = self.heads
@@ -195,15 +210,12 @@ class FluxSingleBlock(nn.Module):
       f = K.gemm(h2, w[:3 * C], bias=None if b is None else b[:3 * C].contiguous()).view(B, S, 3 * C)
       cat = torch.empty((B, S, C + self.hidden), device=h.device, dtype=h.dtype)
       K.gemm(h2, w[3 * C:], bias=None if b is None else b[3 * C:].contiguous(), epi="gelu_tanh", out=cat.view(B * S, -1)[:, C:])
-      q = OF.rms_norm_rope(f[..., :C], self.norm_q, *rope, heads=H, per_head=True)
-      k = OF.rms_norm_rope(f[..., C:2 * C], self.norm_k, *rope, heads=H, per_head=True)
-      cat[..., :C] = OF.attention(q, k, f[..., 2 * C:].unflatten(-1, (H, C // H))).reshape(B, S, C)
+      q, k, v = self._qkv(f, rope)
+      OF.attention_into(cat[..., :C].unflatten(-1, (H, C // H)), q, k, v)
       return _clip(project_gated_residual(self.proj_out, cat, x, gate))
     f = self.qkv_mlp(h)
-    q, k, v, mlp = f[..., :C], f[..., C:2 * C], f[..., 2 * C:3 * C], f[..., 3 * C:]
-    q = OF.rms_norm_rope(q, self.norm_q, *rope, heads=H, per_head=True)
-    k = OF.rms_norm_rope(k, self.norm_k, *rope, heads=H, per_head=True)
-    o = OF.attention(q, k, v.unflatten(-1, (H, C // H))).reshape(B, S, C)
+    mlp = f[..., 3 * C:]
+    o = OF.attention(*self._qkv(f, rope)).reshape(B, S, C)
     cat = torch.cat([o, F.gelu(mlp, approximate="tanh")], dim=-1)
     return _clip(project_gated_residual(self.proj_out, cat, x, gate))
 

@@ -204,6 +204,8 @@ def _declare(L: ctypes.CDLL) -> None:
   L.mdb_rms_rope_fwd.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
                                  c_int, c_int, c_float, c_void_p, c_int, c_void_p]
   L.mdb_rms_rope_fwd.restype = c_int
+  L.mdb_qkv_rope_fwd.argtypes = [c_int] + [c_void_p] * 7 + [c_int, c_int, c_float] + [c_void_p] * 4
+  L.mdb_qkv_rope_fwd.restype = c_int
   L.mdb_rms_rope_bwd.argtypes = [c_void_p, c_ll, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                  c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_void_p]
   L.mdb_rms_rope_bwd.restype = c_int

@@ -489,6 +489,27 @@ def rms_rope_fwd(x, w=None, cos=None, sin=None, heads=1, per_head=False, eps=1e-
   return (y, rstd) if save_stats else y
 
 
+def qkv_rope_fwd(streams, heads: int, eps: float = 1e-6, copy_v: bool = True):
+  """Per-head RMSNorm + RoPE of the q and k columns of one or two fused projections, joined along the sequence, and the v
+  columns copied beside them: streams = [(x [B,S_i,>=3C], wq, wk, cos, sin), ...] -> q, k, v [B, sum S_i, heads, 128]. Without
+  `copy_v` (one stream) v is a view of x."""
+  B, C = streams[0][0].shape[0], heads * 128
+  n, S = len(streams), sum(x.shape[1] for x, *_ in streams)
+  for x, wq, wk, cos, sin in streams:
+    assert x.dtype == torch.bfloat16 and x.shape[0] == B and x.shape[2] >= 3 * C and x.stride(2) == 1 and x.stride(0) == x.shape[1] * x.stride(1)
+    assert all(w.dtype == torch.bfloat16 and w.shape == (128,) and w.is_contiguous() for w in (wq, wk))
+    assert all(t.dtype == torch.float32 and t.shape == (x.shape[1], 64) and t.is_contiguous() for t in (cos, sin))
+  assert copy_v or n == 1
+  out = torch.empty((3 if copy_v else 2, B, S, C), device=streams[0][0].device, dtype=torch.bfloat16)
+  ptrs = lambda i: (ctypes.c_void_p * n)(*[s[i].data_ptr() for s in streams])
+  rc = _lib.lib().mdb_qkv_rope_fwd(n, ptrs(0), (ctypes.c_longlong * n)(*[s[0].stride(1) for s in streams]),
+                                   (ctypes.c_int * n)(*[s[0].shape[1] for s in streams]), ptrs(1), ptrs(2), ptrs(3), ptrs(4), B, C,
+                                   float(eps), out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr() if copy_v else None, _lib.stream())
+  _lib.check(rc, "mdb_qkv_rope_fwd")
+  q, k = out[0].view(B, S, heads, 128), out[1].view(B, S, heads, 128)
+  return q, k, out[2].view(B, S, heads, 128) if copy_v else streams[0][0][..., 2 * C:3 * C].unflatten(-1, (heads, 128))
+
+
 def rms_rope_bwd(dy, x, rstd, w=None, cos=None, sin=None, per_head=False, need_dw=True):
   """dy: [B,S,H,D] (any strides with unit inner stride over [H*D]); returns dx [B,S,C] and dw fp32 [C]."""
   B, S, C = x.shape

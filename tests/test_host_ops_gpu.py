@@ -189,3 +189,30 @@ def test_fused_calls_without_the_extension(monkeypatch):
     for got, m in zip(OF.linear_group(x, ws), ws):
       want = x.double() @ m.double().t()
       assert (got.double() - want).norm() < 4e-3 * want.norm()
+
+
+@pytest.mark.parametrize("B,rows,heads", [(1, (1, 1), 1), (2, (7, 33), 3), (1, (128, 256), 24), (2, (40,), 2), (1, (5,), 9)])
+def test_fused_qkv_and_attention_into(B, rows, heads):
+  """One launch for the norm, rotation and joining of q, k, v against one launch per stream and matrix: the same bits; attention
+  stored into a part of a wider buffer against a copy of its result."""
+  torch.manual_seed(6)
+  C, extra = heads * 128, 0 if len(rows) == 2 else 72
+  parts = [(_randn(B, s, 3 * C + extra), _randn(128), _randn(128), torch.randn(s, 64, device="cuda"), torch.randn(s, 64, device="cuda"))
+           for s in rows]
+  one = lambda x, w, c, s: OF.rms_norm_rope(x, w, c, s, heads=heads, per_head=True)
+  with torch.no_grad():
+    q, k, v = OF.fused_qkv(parts, heads, copy_v=len(rows) == 2)
+    assert torch.equal(q, torch.cat([one(x[..., :C], wq, c, s) for x, wq, wk, c, s in parts], dim=1))
+    assert torch.equal(k, torch.cat([one(x[..., C:2 * C], wk, c, s) for x, wq, wk, c, s in parts], dim=1))
+    assert torch.equal(v, torch.cat([x[..., 2 * C:3 * C].unflatten(-1, (heads, 128)) for x, *_ in parts], dim=1))
+    wide = torch.zeros((B, sum(rows), C + 264), device="cuda", dtype=torch.bfloat16)
+    OF.attention_into(wide[..., 8:8 + C].unflatten(-1, (heads, 128)), q, k, v)
+    assert torch.equal(wide[..., 8:8 + C], OF.attention(q, k, v).flatten(2)) and wide[..., :8].eq(0).all() and wide[..., 8 + C:].eq(0).all()
+    off = torch.zeros((B, sum(rows), C + 3), device="cuda", dtype=torch.bfloat16)  # rows of no 16-byte pitch: copied
+    OF.attention_into(off[..., 1:1 + C].unflatten(-1, (heads, 128)), q, k, v)
+    assert torch.equal(off[..., 1:1 + C], wide[..., 8:8 + C])
+  x, wq, wk, c, s = parts[0]
+  assert OF.fused_qkv([(x, wq.requires_grad_(), wk, c, s)], heads, copy_v=False) is None  # autograd: the differentiable ops
+  with torch.no_grad():
+    for bad in ((x.float(), wq, wk, c, s), (x, wq.float(), wk, c, s), (x, wq, wk, c.double(), s), (x[..., 4:], wq, wk, c, s)):
+      assert OF.fused_qkv([bad], heads, copy_v=False) is None
