@@ -36,6 +36,7 @@ struct Params {
   const float* scale_a;  // device scalars
   const float* scale_b;
   int a_e5m2, b_e5m2;
+  int gelu;  // 1: GELU (tanh form) of the result as bf16 holds it
   int int8;  // 1: operands are signed 8-bit integers (tcgen05 kind::i8, int32 accumulators)
   DeviceStatus* status;
 };
@@ -48,6 +49,15 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
   const int local = tile - group * tiles_per_group;
   m_idx = first_m + local % rows;
   n_idx = local / rows;
+}
+
+// x sigmoid(2 sqrt(2/pi) (x + 0.044715 x^3)) = GELU in its tanh form, of x rounded to bf16: what a pass of its own over the
+// stored product computes (4608 x 12288: 31 us, of a slice of a wider product 150 us). The product's 24 steps of 128 hide it.
+// Exponential and division to a few units of fp32, not the hardware's tanh of 11 bits: the next layer's quantiser sees the
+// same values as behind PyTorch's GELU.
+__device__ __forceinline__ float gelu_of_bf16(float x) {
+  x = __bfloat162float(__float2bfloat16(x));
+  return x / (1.0f + __expf(-1.5957691216057308f * (x + 0.044715f * x * x * x)));
 }
 
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -194,6 +204,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
                 x[2 * j + 1] += f.y;
               }
             }
+            if (p.gelu) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) x[j] = gelu_of_bf16(x[j]);
+            }
             uint4 ov;
             ov.x = pack_bf16x2(x[0], x[1]);
             ov.y = pack_bf16x2(x[2], x[3]);
@@ -272,12 +286,12 @@ quantize_int8_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ q
 // scale_a / scale_b: device floats. a_e5m2 / b_e5m2 select the 8-bit format of each operand.
 static int gemm8_impl(const void* Aq, const void* Bq, void* out, const void* bias, const float* scale_a,
                       const float* scale_b, int M, int N, int K, long long lda, long long ldb, long long ldo, int a_e5m2,
-                      int b_e5m2, int int8, void* stream_ptr);
+                      int b_e5m2, int int8, int gelu, void* stream_ptr);
 
 extern "C" int mdb_gemm_fp8(const void* Aq, const void* Bq, void* out, const void* bias, const float* scale_a,
                             const float* scale_b, int M, int N, int K, long long lda, long long ldb, long long ldo,
                             int a_e5m2, int b_e5m2, void* stream_ptr) {
-  return gemm8_impl(Aq, Bq, out, bias, scale_a, scale_b, M, N, K, lda, ldb, ldo, a_e5m2, b_e5m2, 0, stream_ptr);
+  return gemm8_impl(Aq, Bq, out, bias, scale_a, scale_b, M, N, K, lda, ldb, ldo, a_e5m2, b_e5m2, 0, 0, stream_ptr);
 }
 
 // The same kernel on signed 8-bit integers (tcgen05 kind::i8, exact int32 accumulation): Aq [M, K], Bq [N, K] int8,
@@ -286,16 +300,23 @@ extern "C" int mdb_gemm_fp8(const void* Aq, const void* Bq, void* out, const voi
 extern "C" int mdb_gemm_int8(const void* Aq, const void* Bq, void* out, const void* bias, const float* scale_a,
                              const float* scale_b, int M, int N, int K, long long lda, long long ldb, long long ldo,
                              void* stream_ptr) {
-  return gemm8_impl(Aq, Bq, out, bias, scale_a, scale_b, M, N, K, lda, ldb, ldo, 0, 0, 1, stream_ptr);
+  return gemm8_impl(Aq, Bq, out, bias, scale_a, scale_b, M, N, K, lda, ldb, ldo, 0, 0, 1, 0, stream_ptr);
+}
+
+// Either product (e4m3 or int8 operands) with GELU in its tanh form behind it.
+extern "C" int mdb_gemm8_gelu(const void* Aq, const void* Bq, void* out, const void* bias, const float* scale_a, const float* scale_b,
+                              int M, int N, int K, long long lda, long long ldb, long long ldo, int int8, void* stream_ptr) {
+  return gemm8_impl(Aq, Bq, out, bias, scale_a, scale_b, M, N, K, lda, ldb, ldo, 0, 0, int8, 1, stream_ptr);
 }
 
 static int gemm8_impl(const void* Aq, const void* Bq, void* out, const void* bias, const float* scale_a,
                       const float* scale_b, int M, int N, int K, long long lda, long long ldb, long long ldo, int a_e5m2,
-                      int b_e5m2, int int8, void* stream_ptr) {
+                      int b_e5m2, int int8, int gelu, void* stream_ptr) {
   using namespace mdb;
   using namespace mdb::gemm8;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((N & 7) || (lda & 15) || (ldb & 15) || (ldo & 7) || !scale_a || !scale_b) return 3101;
+  if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(bias)) & 15) return 3101;  // 16-byte stores and loads
   CUtensorMap ta, tb;
   uint64_t dims_a[2] = {static_cast<uint64_t>(K), static_cast<uint64_t>(M)};
   uint64_t str_a[1] = {static_cast<uint64_t>(lda)};
@@ -317,6 +338,7 @@ static int gemm8_impl(const void* Aq, const void* Bq, void* out, const void* bia
   p.a_e5m2 = a_e5m2;
   p.b_e5m2 = b_e5m2;
   p.int8 = int8;
+  p.gelu = gelu;
   p.status = status_buffer();
   static bool configured = false;
   if (!configured) {

@@ -24,6 +24,7 @@ import torch.nn.functional as F
 
 from ...ops import functional as OF
 from ..layers import Linear, project_gated_residual, sinusoidal_embedding
+from ..quantizations import is_plain_quantized
 
 
 @dataclass
@@ -213,6 +214,12 @@ class FluxSingleBlock(nn.Module):
       q, k, v = self._qkv(f, rope)
       OF.attention_into(cat[..., :C].unflatten(-1, (H, C // H)), q, k, v)
       return _clip(project_gated_residual(self.proj_out, cat, x, gate))
+    if h.is_cuda and is_plain_quantized(self.qkv_mlp):  # the same on 8-bit operands
+      cat = torch.empty((B, S, C + self.hidden), device=h.device, dtype=h.dtype)
+      f = self.qkv_mlp.split_gelu(h, 3 * C, cat[..., C:])
+      if f is not None:
+        OF.attention_into(cat[..., :C].unflatten(-1, (H, C // H)), *self._qkv(f, rope))
+        return _clip(project_gated_residual(self.proj_out, cat, x, gate))
     f = self.qkv_mlp(h)
     mlp = f[..., 3 * C:]
     o = OF.attention(*self._qkv(f, rope)).reshape(B, S, C)

@@ -36,8 +36,11 @@ _LINEAR_FORWARD = Linear.forward
 def is_plain_linear(m: nn.Module) -> bool:
   """Whether calling `m` is `OF.linear` and nothing else (no subclass, wrapper, replaced `forward` or hook of any kind that
   `nn.Module.__call__` looks at), so that its product may run fused with another."""
-  if type(m) is not Linear or Linear.forward is not _LINEAR_FORWARD:
-    return False
+  return type(m) is Linear and Linear.forward is _LINEAR_FORWARD and calls_forward_only(m)
+
+
+def calls_forward_only(m: nn.Module) -> bool:
+  """Whether calling `m` runs the `forward` of its class and nothing else."""
   d = m.__dict__
   return not ("forward" in d or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or
               _module._global_forward_hooks or _module._global_forward_pre_hooks or _module._global_backward_hooks or

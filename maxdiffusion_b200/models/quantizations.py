@@ -23,8 +23,9 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops import functional as OF
 from ..ops import kernels as K
-from .layers import Linear
+from .layers import Linear, calls_forward_only
 
 FP8_MAX = {False: 448.0, True: 57344.0}
 
@@ -110,9 +111,41 @@ class Fp8Linear(nn.Module):
     self._wq, self._w_scale = (K.quantize_int8 if self.int8 else K.quantize_fp8)(w.contiguous())
     self._version = self.weight._version
 
+  def _takes(self, x) -> bool:
+    return (x.is_cuda and x.dtype == torch.bfloat16 and self.in_features % 16 == 0 and self.out_features % 8 == 0
+            and (x.numel() // self.in_features) % 8 == 0)
+
+  def _operands(self, x):
+    """(x as 8-bit rows, its scale, bias) for products without autograd; the weight's copy is fresh afterwards."""
+    if self._wq is None or self._version != self.weight._version:
+      self.requantize()
+    x2 = x.reshape(-1, self.in_features)
+    xq, scale = (K.quantize_int8 if self.int8 else K.quantize_fp8)(x2 if x2.is_contiguous() else x2.contiguous())
+    return xq, scale, None if self.bias is None else self.bias.to(torch.bfloat16).contiguous()
+
+  def split_gelu(self, x, cut: int, out):
+    """The first `cut` columns of the product; GELU (tanh form) of the others goes to `out` [..., out_features - cut] (unit inner
+    stride, rows of one pitch). None where autograd or a transform is at work, or where the kernel does not take these
+    tensors: the caller then uses `forward`."""
+    rows = out.view(-1, out.shape[-1]) if out.is_contiguous() else out.flatten(0, -2)
+    if not (self._takes(x) and x.numel() > 0 and 0 < cut < self.out_features and cut % 8 == 0 and not OF.library_mode() and
+            OF._direct(x, self.weight, self.bias, out) and rows.data_ptr() == out.data_ptr() and rows.stride(-1) == 1 and
+            rows.stride(0) % 8 == 0 and rows.data_ptr() % 16 == 0):
+      return None
+    xq, scale, bias = self._operands(x)
+    lo, hi = (None, None) if bias is None else (bias[:cut], bias[cut:])
+    if bias is not None and (lo.data_ptr() | hi.data_ptr()) % 16:
+      lo, hi = lo.clone(), hi.clone()
+    K.gemm8(xq, scale, self._wq[cut:], self._w_scale, hi, gelu=True, out=rows)
+    return K.gemm8(xq, scale, self._wq[:cut], self._w_scale, lo).view(*x.shape[:-1], cut)
+
   def forward(self, x, activation: Optional[str] = None):
-    ok = (x.is_cuda and x.dtype == torch.bfloat16 and self.in_features % 16 == 0 and self.out_features % 8 == 0
-          and (x.numel() // self.in_features) % 8 == 0)
+    ok = self._takes(x)
+    if ok and activation == "gelu_tanh" and x.numel() > 0 and not OF.library_mode() and OF._direct(x, self.weight, self.bias):
+      xq, scale, bias = self._operands(x)
+      if bias is not None and bias.data_ptr() % 16:
+        bias = bias.clone()
+      return K.gemm8(xq, scale, self._wq, self._w_scale, bias, gelu=True).view(*x.shape[:-1], self.out_features)
     if not ok:
       fq = fake_quantize_int8 if self.int8 else fake_quantize
       y = F.linear(x, fq(self.weight.to(x.dtype)), None if self.bias is None else self.bias.to(x.dtype)) \
@@ -138,6 +171,11 @@ class Fp8Linear(nn.Module):
 class Int8Linear(Fp8Linear):
   """Drop-in for `layers.Linear` with the product on the int8 tensor-core path (per-tensor symmetric scales)."""
   int8 = True
+
+
+def is_plain_quantized(m: nn.Module) -> bool:
+  """Whether calling `m` is the quantised product and nothing else, so that it may run in parts."""
+  return type(m) in (Fp8Linear, Int8Linear) and calls_forward_only(m)
 
 
 def get_quantization_mode(config) -> Optional[str]:

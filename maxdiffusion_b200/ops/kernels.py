@@ -818,6 +818,8 @@ def _declare_fp8(L):
   L.mdb_quantize_fp8.restype = c_int
   L.mdb_gemm_int8.argtypes = [c_void_p] * 6 + [c_int] * 3 + [c_ll] * 3 + [c_void_p]
   L.mdb_gemm_int8.restype = c_int
+  L.mdb_gemm8_gelu.argtypes = [c_void_p] * 6 + [c_int] * 3 + [c_ll] * 3 + [c_int, c_void_p]
+  L.mdb_gemm8_gelu.restype = c_int
   L.mdb_quantize_int8.argtypes = [c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_void_p]
   L.mdb_quantize_int8.restype = c_int
 
@@ -849,6 +851,29 @@ def gemm_fp8(aq, a_scale, bq, b_scale, bias=None, a_e5m2: bool = False, b_e5m2: 
                                _lib.ptr(b_scale), M, N, K, aq.stride(0), bq.stride(0), out.stride(0), int(a_e5m2),
                                int(b_e5m2), _lib.stream())
   _lib.check(rc, "mdb_gemm_fp8")
+  return out
+
+
+def gemm8(aq, a_scale, bq, b_scale, bias=None, gelu: bool = False, out=None):
+  """`gemm_fp8` (uint8 operands holding e4m3) or `gemm_int8` (int8 operands), optionally with GELU (tanh form) of the bf16 result
+  in the epilogue, into `out` [M,N] (rows of any pitch that is a multiple of 8) if given."""
+  assert aq.dtype == bq.dtype and aq.dtype in (torch.uint8, torch.int8) and aq.dim() == 2 and bq.dim() == 2
+  assert aq.stride(-1) == 1 and bq.stride(-1) == 1 and aq.shape[1] == bq.shape[1]
+  M, K = aq.shape
+  N = bq.shape[0]
+  if out is None:
+    out = torch.empty((M, N), device=aq.device, dtype=torch.bfloat16)
+  assert out.shape == (M, N) and out.dtype == torch.bfloat16 and out.stride(-1) == 1
+  args = (_lib.ptr(aq), _lib.ptr(bq), _lib.ptr(out), _lib.ptr(bias), _lib.ptr(a_scale), _lib.ptr(b_scale), M, N, K, aq.stride(0),
+          bq.stride(0), out.stride(0))
+  int8 = aq.dtype == torch.int8
+  if gelu:
+    rc = _lib.lib().mdb_gemm8_gelu(*args, int(int8), _lib.stream())
+  elif int8:
+    rc = _lib.lib().mdb_gemm_int8(*args, _lib.stream())
+  else:
+    rc = _lib.lib().mdb_gemm_fp8(*args, 0, 0, _lib.stream())
+  _lib.check(rc, "mdb_gemm8")
   return out
 
 

@@ -222,3 +222,40 @@ def test_attention_when_the_maximum_moves(D, Sq, lens):
   want = torch.logsumexp(s, -1) / 0.6931471805599453
   # sums of fp32 exponentials in the log2 domain, scores of up to a few hundred
   assert (lse.double() - want).abs().max() < 1e-5 * want.abs().max() + 1e-4
+
+
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("M,N,Kd", [(8, 8, 16), (136, 264, 144), (256, 640, 3072)])
+def test_gelu_behind_an_8_bit_product(int8, M, N, Kd):
+  """GELU in the epilogue is the GELU of the stored product: one rounding of the same value, so at most one unit of bf16 off
+  where the two forms of tanh fall on different sides of a tie."""
+  torch.manual_seed(12)
+  quant = K.quantize_int8 if int8 else K.quantize_fp8
+  (aq, sa), (bq, sb), bias = quant(_randn(M, Kd)), quant(_randn(N, Kd, scale=0.05)), _randn(N)
+  y = (K.gemm_int8 if int8 else K.gemm_fp8)(aq, sa, bq, sb, bias)
+  want = torch.nn.functional.gelu(y.double(), approximate="tanh")
+  wide = torch.zeros((M, N + 72), device="cuda", dtype=torch.bfloat16)
+  got = K.gemm8(aq, sa, bq, sb, bias, gelu=True, out=wide[:, 64:64 + N])
+  assert ((got.double() - want).abs() <= want.abs() / 256 + 1e-6).all() and wide[:, :64].eq(0).all() and wide[:, 64 + N:].eq(0).all()
+  assert torch.equal(K.gemm8(aq, sa, bq, sb, bias), y)
+
+
+@pytest.mark.parametrize("mode", ["fp8", "int8"])
+def test_quantised_linear_in_parts(mode):
+  from maxdiffusion_b200.models.layers import Linear
+  from maxdiffusion_b200.models.quantizations import Fp8Linear, Int8Linear, is_plain_quantized
+
+  torch.manual_seed(13)
+  m = (Int8Linear if mode == "int8" else Fp8Linear)(Linear(128, 400).to("cuda", torch.bfloat16))
+  x = _randn(2, 12, 128)
+  whole = m(x.detach().requires_grad_()).detach()  # through autograd
+  with torch.no_grad():
+    assert torch.equal(m(x), whole)
+    cat = torch.zeros((2, 12, 80 + 160), device="cuda", dtype=torch.bfloat16)
+    assert torch.equal(m.split_gelu(x, 240, cat[..., 80:]), whole[..., :240]) and cat[..., :80].eq(0).all()
+    assert torch.equal(cat[..., 80:], m(x, "gelu_tanh")[..., 240:])
+    assert m.split_gelu(x, 241, cat[..., 81:]) is None and m.split_gelu(x[:, :3, :], 240, cat[:, :3, 80:]) is None
+  assert m.split_gelu(x, 240, cat[..., 80:]) is None  # the weight wants a gradient
+  assert is_plain_quantized(m)
+  m.register_forward_hook(lambda *a: None)
+  assert not is_plain_quantized(m)
