@@ -447,21 +447,31 @@ __device__ __forceinline__ float2 cta_sum2(float2 v, float2* red) {
   return t;
 }
 
-// forward: a = rstd * gamma, b = beta - mean * a; also mean / rstd [N, G] for the backward
+// forward: a = rstd * gamma, b = beta - mean * a; also mean / rstd [N, G] for the backward. `shift` (null: none) holds a value
+// per sample and channel that is to be added to x first: the sums of x + t follow from those of x, and act((x + t) a + b) is
+// act(x a + (t a + b)), so neither pass over x changes and no pass of its own adds it (an SDXL step at 1024^2: 17 passes of 16 us).
 __global__ void __launch_bounds__(256)
 gn_cl_fold_fwd_kernel(const float2* __restrict__ partial, int splits, int C, int groups, float count, float eps,
                       const void* gamma, const void* beta, int params_bf16, float* __restrict__ a, float* __restrict__ b,
-                      float* __restrict__ mean_out, float* __restrict__ rstd_out) {
+                      float* __restrict__ mean_out, float* __restrict__ rstd_out, const __nv_bfloat16* __restrict__ shift,
+                      long long shift_pitch) {
   allow_successor();
   wait_for_predecessor();
   __shared__ float2 red[256];
   extern __shared__ float2 ch[];  // [cg] channel sums
   const int g = blockIdx.x, n = blockIdx.y, cg = C / groups;
   group_channel_sums(partial + static_cast<long long>(n) * splits * C + g * cg, splits, C, cg, red, ch);
+  const __nv_bfloat16* sh = shift != nullptr ? shift + n * shift_pitch + g * cg : nullptr;
   float2 t = make_float2(0.0f, 0.0f);
   for (int j = threadIdx.x; j < cg; j += 256) {
-    t.x += ch[j].x;
-    t.y += ch[j].y;
+    if (sh != nullptr) {
+      const float v = __bfloat162float(sh[j]), hw = count / cg;
+      t.x += ch[j].x + hw * v;
+      t.y += ch[j].y + v * (2.0f * ch[j].x + hw * v);
+    } else {
+      t.x += ch[j].x;
+      t.y += ch[j].y;
+    }
   }
   t = cta_sum2(t, red);
   const float mean = t.x / count;
@@ -474,7 +484,8 @@ gn_cl_fold_fwd_kernel(const float2* __restrict__ partial, int splits, int C, int
     const int c = g * cg + j;
     const float av = rstd * param_at(gamma, params_bf16, c);
     a[static_cast<long long>(n) * C + c] = av;
-    b[static_cast<long long>(n) * C + c] = (beta != nullptr ? param_at(beta, params_bf16, c) : 0.0f) - mean * av;
+    const float at = sh != nullptr ? __bfloat162float(sh[j]) - mean : -mean;
+    b[static_cast<long long>(n) * C + c] = (beta != nullptr ? param_at(beta, params_bf16, c) : 0.0f) + at * av;
   }
 }
 
@@ -515,10 +526,10 @@ gn_cl_fold_bwd_kernel(const float2* __restrict__ partial, int splits, int C, int
 }  // namespace mdb
 
 // partial: fp32 [N, splits, C, 2] from mdb_gn_cl_sums; gamma / beta: [C] bf16 (params_bf16 = 1) or fp32, may be null;
-// a, b: fp32 [N, C]; mean, rstd: fp32 [N, groups]. count = pixels * channels per group.
+// a, b: fp32 [N, C]; mean, rstd: fp32 [N, groups]. count = pixels * channels per group. shift: bf16 [N, C] or null.
 extern "C" int mdb_gn_cl_fold_fwd(const float* partial, int N, int splits, int C, int groups, float count, float eps,
                                   const void* gamma, const void* beta, int params_bf16, float* a, float* b, float* mean,
-                                  float* rstd, void* stream) {
+                                  float* rstd, const void* shift, long long shift_pitch, void* stream) {
   if (N <= 0) return 0;
   if (groups <= 0 || C % groups || splits < 1 || C > 8192) return 3704;
   if (N > 65535) return 3704;
@@ -526,7 +537,8 @@ extern "C" int mdb_gn_cl_fold_fwd(const float* partial, int N, int splits, int C
   if (smem > 40 * 1024)
     MDB_CHECK_CUDA(cudaFuncSetAttribute(mdb::cln::gn_cl_fold_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
   mdb::launch_overlapped(mdb::cln::gn_cl_fold_fwd_kernel, dim3(groups, N), 256, smem, static_cast<cudaStream_t>(stream),
-      reinterpret_cast<const float2*>(partial), splits, C, groups, count, eps, gamma, beta, params_bf16, a, b, mean, rstd);
+      reinterpret_cast<const float2*>(partial), splits, C, groups, count, eps, gamma, beta, params_bf16, a, b, mean, rstd,
+      static_cast<const __nv_bfloat16*>(shift), shift_pitch);
   return static_cast<int>(cudaGetLastError());
 }
 

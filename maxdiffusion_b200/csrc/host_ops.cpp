@@ -39,7 +39,7 @@ int mdb_rms_rope_fwd(const void*, long long, void*, long long, long long, const 
                      int, int, float, float*, int, void*);
 int mdb_gn_cl_sums(const void*, const void*, const float*, const float*, float*, int, int, int, int, void*);
 int mdb_gn_cl_fold_fwd(const float*, int, int, int, int, float, float, const void*, const void*, int, float*, float*, float*,
-                       float*, void*);
+                       float*, const void*, long long, void*);
 int mdb_gn_cl_apply(const void*, const void*, void*, const float*, const float*, const float*, const float*, const float*, int,
                     int, int, int, void*);
 int mdb_conv_igemm(const void*, const void*, const void*, void*, const void*, const void*, const long long*, const long long*,
@@ -436,14 +436,14 @@ PyObject* py_rms_rope(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// group_norm_cl(x, groups, gamma, beta, eps, act): x [N,C,H,W] in channels-last memory
+// group_norm_cl(x, groups, gamma, beta, eps, act, shift): x [N,C,H,W] in channels-last memory, shift [N,C] or None
 PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 6 || !THPVariable_Check(a[0])) return not_implemented();
+  if (n != 7 || !THPVariable_Check(a[0])) return not_implemented();
   const Tensor& x = THPVariable_Unpack(a[0]);
-  const Tensor *gamma, *beta;
+  const Tensor *gamma, *beta, *shift;
   const int64_t groups = PyLong_AsLong(a[1]);
-  if (!opt_tensor(a[2], gamma) || !opt_tensor(a[3], beta)) return not_implemented();
+  if (!opt_tensor(a[2], gamma) || !opt_tensor(a[3], beta) || !opt_tensor(a[6], shift)) return not_implemented();
   const double eps = PyFloat_AsDouble(a[4]);
   const bool act = a[5] == Py_True;
   if (PyErr_Occurred()) return nullptr;
@@ -452,6 +452,8 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (groups <= 0 || C % groups || (C & 7) || C > 2048 || N > 65535 || HW > INT_MAX) return not_implemented();
   for (const Tensor* p : {gamma, beta})
     if (p && (!bf16(*p) || !p->is_contiguous() || p->numel() != C)) return not_implemented();
+  if (shift && (!bf16(*shift) || shift->dim() != 2 || shift->size(0) != N || shift->size(1) != C || shift->stride(1) != 1))
+    return not_implemented();
   const int splits = static_cast<int>(std::max<int64_t>(1, std::min((kCtasTarget + N - 1) / N, (HW + 15) / 16)));
   const int in = static_cast<int>(N), ic = static_cast<int>(C), ihw = static_cast<int>(HW), ig = static_cast<int>(groups);
   Tensor y;
@@ -467,7 +469,8 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
     int err = mdb_gn_cl_sums(x.data_ptr(), nullptr, nullptr, nullptr, partial, in, ihw, ic, splits, st);
     if (err == 0)
       err = mdb_gn_cl_fold_fwd(partial, in, splits, ic, ig, static_cast<float>(HW * (C / groups)), static_cast<float>(eps),
-                               data(gamma), data(beta), gamma || beta ? 1 : 0, ca, cb, mean, rstd, st);
+                               data(gamma), data(beta), gamma || beta ? 1 : 0, ca, cb, mean, rstd, data(shift),
+                               shift ? shift->stride(0) : 0, st);
     if (err == 0)
       err = mdb_gn_cl_apply(x.data_ptr(), nullptr, y.data_ptr(), ca, cb, nullptr, nullptr, nullptr, in, ihw, ic, act, st);
     return err;

@@ -53,7 +53,7 @@ def _declare(L):
   L.mdb_gn_cl_apply.argtypes = [c_void_p] * 8 + [c_int] * 4 + [c_void_p]
   L.mdb_gn_cl_apply.restype = c_int
   c_float = ctypes.c_float
-  L.mdb_gn_cl_fold_fwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_int] + [c_void_p] * 5
+  L.mdb_gn_cl_fold_fwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_int] + [c_void_p] * 5 + [c_ll, c_void_p]
   L.mdb_gn_cl_fold_fwd.restype = c_int
   L.mdb_gn_cl_fold_bwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int] + [c_void_p] * 8
   L.mdb_gn_cl_fold_bwd.restype = c_int
@@ -762,8 +762,9 @@ def _gn_params(gamma, beta):
   return (None if gamma is None else conv(gamma)), (None if beta is None else conv(beta)), int(bf16)
 
 
-def group_norm_cl_fwd(x3: torch.Tensor, groups: int, gamma, beta, eps: float, act: bool):
-  """x3 [N, HW, C] bf16 contiguous -> (y, a, b, mean, rstd): y = act(x * a + b) with a, b fp32 [N, C]. Three launches:
+def group_norm_cl_fwd(x3: torch.Tensor, groups: int, gamma, beta, eps: float, act: bool, shift=None):
+  """x3 [N, HW, C] bf16 contiguous -> (y, a, b, mean, rstd): y = act(x * a + b) with a, b fp32 [N, C]. `shift` (bf16 [N, C]) is
+  added to x first (the statistics and b are those of the sum). Three launches:
   per-channel sums, the fold to coefficients (one CTA per sample), the apply pass."""
   N, HW, C = x3.shape
   partial = _gn_partial(x3)
@@ -774,7 +775,7 @@ def group_norm_cl_fwd(x3: torch.Tensor, groups: int, gamma, beta, eps: float, ac
   g, bt, bf16 = _gn_params(gamma, beta)
   rc = _lib.lib().mdb_gn_cl_fold_fwd(_lib.ptr(partial), N, partial.shape[1], C, groups, float(HW * (C // groups)), float(eps),
                                      _lib.ptr(g), _lib.ptr(bt), bf16, _lib.ptr(a), _lib.ptr(b), _lib.ptr(mean), _lib.ptr(rstd),
-                                     _lib.stream())
+                                     _lib.ptr(shift), shift.stride(0) if shift is not None else 0, _lib.stream())
   _lib.check(rc, "mdb_gn_cl_fold_fwd")
   return _gn_apply(x3, None, a, b, None, None, None, act), a, b, mean, rstd
 

@@ -710,18 +710,25 @@ def _is_channels_last(x: torch.Tensor) -> bool:
   return x.dim() == 4 and x.shape[1] > 1 and x.is_contiguous(memory_format=torch.channels_last) and not x.is_contiguous()
 
 
-def group_norm(x, groups: int, gamma=None, beta=None, eps: float = 1e-6, act: bool = False):
+def group_norm(x, groups: int, gamma=None, beta=None, eps: float = 1e-6, act: bool = False, shift=None):
   """GroupNorm over a channels-first tensor [N, C, *spatial] with optional fused SiLU. A 4-D bf16 tensor in
-  channels-last memory (what `conv2d` produces) stays in that layout."""
+  channels-last memory (what `conv2d` produces) stays in that layout. `shift` [N, C] is added to x first: without autograd in
+  the fold of the sums, where it costs no pass over x."""
   if _fast(x) and _is_channels_last(x) and x.shape[1] % 8 == 0 and x.shape[1] <= 2048:
-    if _direct(x, gamma, beta):
-      r = _lib.host_ops().group_norm_cl(x, groups, gamma, beta, eps, act)
+    if _direct(x, gamma, beta, shift):
+      if shift is not None and (shift.dtype != torch.bfloat16 or shift.shape != x.shape[:2] or shift.stride(1) != 1):
+        return group_norm(x + shift[:, :, None, None], groups, gamma, beta, eps, act)
+      r = _lib.host_ops().group_norm_cl(x, groups, gamma, beta, eps, act, shift)
       if r is not NotImplemented:
         return r
       N, C, H, W = x.shape
-      y3 = OC.group_norm_cl_fwd(x.permute(0, 2, 3, 1).view(N, H * W, C), groups, gamma, beta, eps, act)[0]
+      y3 = OC.group_norm_cl_fwd(x.permute(0, 2, 3, 1).view(N, H * W, C), groups, gamma, beta, eps, act, shift)[0]
       return y3.view(N, H, W, C).permute(0, 3, 1, 2)
+    if shift is not None:
+      return group_norm(x + shift[:, :, None, None], groups, gamma, beta, eps, act)
     return _GroupNormCLFn.apply(x, gamma, beta, groups, eps, act)
+  if shift is not None:
+    x = x + shift.reshape(*shift.shape, *(1,) * (x.dim() - 2))
   if x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and not _LIBRARY_MODE:
     x = x if x.is_contiguous() else x.contiguous()
     return _GroupNormFn.apply(x, gamma, beta, groups, eps, act)
@@ -749,7 +756,7 @@ def _packed(weight: torch.Tensor, bias, kind: str, make):
   return hit[1]
 
 
-def _conv2d_fwd(x, weight, bias, stride, pad, upsample):
+def _conv2d_fwd(x, weight, bias, stride, pad, upsample, residual=None):
   """(output NCHW in channels-last memory, the input as a dense [N, H, W, C])."""
   xc = x.contiguous(memory_format=torch.channels_last).permute(0, 2, 3, 1)
   if upsample:
@@ -758,7 +765,7 @@ def _conv2d_fwd(x, weight, bias, stride, pad, upsample):
   else:
     pk = _packed(weight, bias, f"s{stride}p{pad}", lambda: OC.pack_conv2d(weight.detach(), None if bias is None else bias.detach(),
                                                                          stride=stride, pad_top_left=pad))
-    y = OC.conv2d(OC.pad_channels(xc, pk.c_in), pk)
+    y = OC.conv2d(OC.pad_channels(xc, pk.c_in), pk, residual=residual)
   return y.permute(0, 3, 1, 2), xc
 
 
@@ -801,9 +808,10 @@ class _Conv2dFn(torch.autograd.Function):
     return dx, dw, db, None, None, None
 
 
-def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = False):
+def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = False, residual=None):
   """2-D convolution of an NCHW tensor. `padding` is an int (all sides) or "far" (zero rows / columns after the image
-  only: the VAE's stride-2 down-sampling). With `upsample` the input is nearest-2x up-sampled first (fused).
+  only: the VAE's stride-2 down-sampling). With `upsample` the input is nearest-2x up-sampled first (fused). `residual`, of the
+  result's shape, is added to it, where it can be in the kernel's epilogue.
 
   CUDA bf16 3x3 convolutions run on the implicit-GEMM kernels and return channels-last memory; 1x1 convolutions are
   GEMMs over the pixel rows; everything else is `torch.nn.functional.conv2d`."""
@@ -813,21 +821,32 @@ def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = Fa
   if _fast(x) and k == 1 and stride == 1 and pad_tl == 0 and not upsample and ci % 8 == 0 and co % 8 == 0:
     n, c, h, w = x.shape
     rows = x.contiguous(memory_format=torch.channels_last).permute(0, 2, 3, 1).reshape(n, h * w, c)
-    y = linear(rows, weight.reshape(co, ci), bias)
-    return y.view(n, h, w, co).permute(0, 3, 1, 2)
+    res = None
+    if residual is not None and residual.shape == (n, co, h, w) and residual.dtype == x.dtype:
+      res = residual.permute(0, 2, 3, 1).reshape(n, h * w, co)
+    y = linear(rows, weight.reshape(co, ci), bias, residual=res).view(n, h, w, co).permute(0, 3, 1, 2)
+    return y if res is not None or residual is None else residual + y
   even = x.shape[2] % 2 == 0 and x.shape[3] % 2 == 0
   if (_fast(x) and k == 3 and stride in (1, 2) and (stride == 1 or even) and
       ((stride == 1 and pad_tl == 1) or (stride == 2 and pad_tl in (0, 1)))):
     if weight.dtype != torch.bfloat16:
       weight = weight.to(torch.bfloat16)
-    if _direct(x, weight, bias):
-      return _conv2d_fwd(x, weight, bias, stride, pad_tl, upsample)[0]
-    return _Conv2dFn.apply(x, weight, bias, stride, pad_tl, upsample)
+    if _direct(x, weight, bias, residual):
+      if residual is not None and not upsample and co % 8 == 0 and _fast(residual) and residual.shape == (
+          x.shape[0], co, x.shape[2] // stride, x.shape[3] // stride):
+        rows = residual.permute(0, 2, 3, 1)
+        if rows.is_contiguous() and rows.data_ptr() % 16 == 0:
+          return _conv2d_fwd(x, weight, bias, stride, pad_tl, False, rows)[0]
+      y = _conv2d_fwd(x, weight, bias, stride, pad_tl, upsample)[0]
+    else:
+      y = _Conv2dFn.apply(x, weight, bias, stride, pad_tl, upsample)
+    return y if residual is None else residual + y
   if upsample:
     x = F.interpolate(x, scale_factor=2.0, mode="nearest")
   if padding == "far":
     x = F.pad(x, (0, 1, 0, 1))
-  return F.conv2d(x, weight.to(x.dtype), None if bias is None else bias.to(x.dtype), stride=stride, padding=pad_tl)
+  y = F.conv2d(x, weight.to(x.dtype), None if bias is None else bias.to(x.dtype), stride=stride, padding=pad_tl)
+  return y if residual is None else residual + y
 
 
 def lincomb(xs, coefs, out_dtype=None):

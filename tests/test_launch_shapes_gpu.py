@@ -259,3 +259,38 @@ def test_quantised_linear_in_parts(mode):
   assert is_plain_quantized(m)
   m.register_forward_hook(lambda *a: None)
   assert not is_plain_quantized(m)
+
+
+@pytest.mark.parametrize("shape,groups", [((2, 64, 8, 8), 32), ((1, 320, 17, 5), 32), ((3, 96, 1, 9), 3)])
+def test_norm_of_sum_and_conv_with_a_residual(shape, groups):
+  """The value per sample and channel enters the fold of GroupNorm's sums, the residual the convolution's epilogue; wrappers,
+  hooks and other layouts take the separate additions. Oracle: float64."""
+  from maxdiffusion_b200.models.layers import Conv2d, GroupNorm, conv_plus, norm_of_sum
+
+  torch.manual_seed(14)
+  N, C, H, W = shape
+  cl = dict(memory_format=torch.channels_last)
+  x, t = _randn(*shape).contiguous(**cl), _randn(N, C) * 3
+  rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+  norm, conv = GroupNorm(groups, C, eps=1e-5).to("cuda", torch.bfloat16), Conv2d(C, 48, 3, padding=1).to("cuda", torch.bfloat16)
+  one = Conv2d(C, 48, 1).to("cuda", torch.bfloat16)
+  norm.weight.data.normal_(), norm.bias.data.normal_()
+  res = _randn(N, 48, H, W).contiguous(**cl)
+  F = torch.nn.functional
+  with torch.no_grad():
+    want = F.silu(F.group_norm(x.double() + t.double()[:, :, None, None], groups, norm.weight.double(), norm.bias.double(), 1e-5))
+    assert rel(norm_of_sum(norm, x, t), want) < 4e-3  # one rounding to bf16
+    assert rel(norm_of_sum(norm, x, t.t().contiguous().t()), want) < 8e-3  # another stride: x + t is rounded as well
+    for m in (conv, one):
+      y = F.conv2d(x.double(), m.weight.double(), m.bias.double(), padding=m.padding) + res.double()
+      fused = conv_plus(m, x, res)
+      assert rel(fused, y) < 4e-3 and fused.shape == y.shape
+      assert rel(conv_plus(m, x, res.contiguous()), y) < 6e-3 and rel(conv_plus(m, x, res.float()), y) < 6e-3
+      h = m.register_forward_hook(lambda mod, a, out: out * 0)
+      assert torch.equal(conv_plus(m, x, res), res)  # a hook on the module sees the convolution alone
+      h.remove()
+  a, b = x.detach().requires_grad_(), t.detach().requires_grad_()
+  norm_of_sum(norm, a, b).float().square().sum().backward()
+  a64, b64 = x.double().requires_grad_(), t.double().requires_grad_()
+  F.silu(F.group_norm(a64 + b64[:, :, None, None], groups, norm.weight.double(), norm.bias.double(), 1e-5)).square().sum().backward()
+  assert rel(a.grad, a64.grad) < 3e-2 and rel(b.grad, b64.grad) < 3e-2  # bf16 gradients of a bf16 sum
