@@ -91,12 +91,13 @@ class PackedConv:
   src: tuple = ()                 # (weight, bias, stride, pad_top_left) as given: what the PyTorch reference path runs
 
   _tap_cache: dict = field(default_factory=dict, init=False, repr=False, compare=False)  # ctypes arrays: never pickled
+  _launches: dict = field(default_factory=dict, init=False, repr=False, compare=False)  # `conv2d_nchw`: arguments by input size
 
   def __getstate__(self):
-    return {k: v for k, v in self.__dict__.items() if k != "_tap_cache"}
+    return {k: v for k, v in self.__dict__.items() if k not in ("_tap_cache", "_launches")}
 
   def __setstate__(self, state):
-    self.__dict__.update(state, _tap_cache={})
+    self.__dict__.update(state, _tap_cache={}, _launches={})
 
   def row_group(self) -> int:
     """How many consecutive taps step along the width by one position each (they can share a fetched row): 2, 3 or 1."""
@@ -438,6 +439,49 @@ def conv2d(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = N
     assert residual.shape == out.shape and residual.is_contiguous()
   _launch(x, None, pk, dims, strides, None, None, box, ext, out, os_, [0], residual, silu)
   return out if pk.n_pad == pk.n_out else out[..., :pk.n_out]
+
+
+def _conv2d_launch(pk: PackedConv, B: int, H: int, W: int):
+  """(arguments of the host extension's `conv` behind the residual, output height, output width) of a dense [B, H, W, c_in]."""
+  C, n = pk.c_in, pk.n_pad
+  if pk.kind == "conv2d_s2":
+    Ho, Wo = H // 2, W // 2
+    b1, b3, _ = _pick_box(Wo, Ho, 1, False)
+    box, dims, strides = (b1, 1, b3), (2 * C, Wo, 2, Ho, B), (2 * C, W * C, 2 * W * C, H * W * C)
+    ext, os_ = (Wo, 1, Ho, B), (n, 0, Wo * n, Ho * Wo * n)
+  else:
+    Ho, Wo = H, W
+    box, dims, strides = tuple(_tile_box(pk, W, H, B, True)), (C, W, H, B, 1), (C, W * C, H * W * C, B * H * W * C)
+    ext, os_ = (W, H, B, 1), (n, W * n, H * W * n, B * H * W * n)
+  taps, begin, n_classes = pk.tap_arrays()
+  group = pk.row_group() if box[0] == 128 else 1
+  m_tiles = ext[3]
+  for e, b in zip(ext[:3], box):
+    m_tiles *= -(-e // b)
+  ctas, max_bn, splits = conv_plan(m_tiles, n_classes, n, -(-C // 64) * min(len(c) for c in pk.taps), group)
+  return (dims, strides, dims, strides, box, ext, C, n, ctypes.addressof(taps), ctypes.addressof(begin), -1, 0, os_, (0,), 0, ctas, max_bn,
+          splits, m_tiles, group), Ho, Wo
+
+
+def conv2d_nchw(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = None):
+  """`conv2d` of an NCHW tensor in channels-last memory, with a residual like the result, as NCHW in channels-last memory, with
+  little host work: what the launch needs is kept with the packed weights for up to 32 input sizes. None where the host
+  extension or these tensors do not fit: the caller then uses `conv2d`."""
+  host = _lib.host_ops()
+  if (host is None or _PLAN is not None or not _ROWS or pk.kind not in ("conv2d", "conv2d_s2") or x.shape[1] != pk.c_in or
+      pk.n_pad != pk.n_out or not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 or x.numel() == 0):
+    return None
+  B, _, H, W = x.shape
+  if pk.kind == "conv2d_s2" and (H | W) & 1:
+    return None
+  hit = pk._launches.get((B, H, W))
+  if hit is None:
+    if len(pk._launches) >= 32:
+      pk._launches.clear()
+    hit = pk._launches[(B, H, W)] = _conv2d_launch(pk, B, H, W)
+  args, Ho, Wo = hit
+  out = torch.empty((B, pk.n_out, Ho, Wo), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
+  return None if host.conv(x, None, pk.w, out, pk.bias, residual, *args) is NotImplemented else out
 
 
 def _parity_conv(x, pk, silu=False, halo: int = 0):

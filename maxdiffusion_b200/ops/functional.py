@@ -756,6 +756,14 @@ def _packed(weight: torch.Tensor, bias, kind: str, make):
   return hit[1]
 
 
+def _packed_conv2d(weight, bias, stride, pad):
+  return _packed(weight, bias, _CONV_KINDS[(stride, pad)], lambda: OC.pack_conv2d(
+      weight.detach(), None if bias is None else bias.detach(), stride=stride, pad_top_left=pad))
+
+
+_CONV_KINDS = {(s, p): f"s{s}p{p}" for s in (1, 2) for p in (0, 1)}
+
+
 def _conv2d_fwd(x, weight, bias, stride, pad, upsample, residual=None):
   """(output NCHW in channels-last memory, the input as a dense [N, H, W, C])."""
   xc = x.contiguous(memory_format=torch.channels_last).permute(0, 2, 3, 1)
@@ -763,8 +771,7 @@ def _conv2d_fwd(x, weight, bias, stride, pad, upsample, residual=None):
     pk = _packed(weight, bias, "up", lambda: OC.pack_upsample_conv2d(weight.detach(), None if bias is None else bias.detach()))
     y = OC.upsample2x_conv2d(OC.pad_channels(xc, pk.c_in), pk)
   else:
-    pk = _packed(weight, bias, f"s{stride}p{pad}", lambda: OC.pack_conv2d(weight.detach(), None if bias is None else bias.detach(),
-                                                                         stride=stride, pad_top_left=pad))
+    pk = _packed_conv2d(weight, bias, stride, pad)
     y = OC.conv2d(OC.pad_channels(xc, pk.c_in), pk, residual=residual)
   return y.permute(0, 3, 1, 2), xc
 
@@ -832,11 +839,17 @@ def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = Fa
     if weight.dtype != torch.bfloat16:
       weight = weight.to(torch.bfloat16)
     if _direct(x, weight, bias, residual):
+      rows = None
       if residual is not None and not upsample and co % 8 == 0 and _fast(residual) and residual.shape == (
-          x.shape[0], co, x.shape[2] // stride, x.shape[3] // stride):
+          x.shape[0], co, x.shape[2] // stride, x.shape[3] // stride) and residual.data_ptr() % 16 == 0:
         rows = residual.permute(0, 2, 3, 1)
-        if rows.is_contiguous() and rows.data_ptr() % 16 == 0:
-          return _conv2d_fwd(x, weight, bias, stride, pad_tl, False, rows)[0]
+        rows = rows if rows.is_contiguous() else None
+      if not upsample and (rows is not None or residual is None):
+        y = OC.conv2d_nchw(x, _packed_conv2d(weight, bias, stride, pad_tl), rows)
+        if y is not None:
+          return y
+      if rows is not None:
+        return _conv2d_fwd(x, weight, bias, stride, pad_tl, False, rows)[0]
       y = _conv2d_fwd(x, weight, bias, stride, pad_tl, upsample)[0]
     else:
       y = _Conv2dFn.apply(x, weight, bias, stride, pad_tl, upsample)

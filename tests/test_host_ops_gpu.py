@@ -216,3 +216,26 @@ def test_fused_qkv_and_attention_into(B, rows, heads):
   with torch.no_grad():
     for bad in ((x.float(), wq, wk, c, s), (x, wq.float(), wk, c, s), (x, wq, wk, c.double(), s), (x[..., 4:], wq, wk, c, s)):
       assert OF.fused_qkv([bad], heads, copy_v=False) is None
+
+
+@pytest.mark.parametrize("stride,shape", [(1, (2, 32, 8, 8)), (1, (1, 48, 17, 5)), (2, (2, 32, 6, 10)), (1, (3, 32, 1, 1))])
+def test_conv2d_nchw_launches_what_conv2d_does(stride, shape):
+  """The kept launch arguments against those of `conv2d`: the same bits over several sizes, with and without a residual, and
+  again after a change of the weights."""
+  torch.manual_seed(7)
+  cl = dict(memory_format=torch.channels_last)
+  w, b = _randn(40, shape[1], 3, 3) * 0.05, _randn(40)
+  with torch.no_grad():
+    for pad in (0, 1) if stride == 2 else (1,):
+      pk = OC.pack_conv2d(w, b, stride=stride, pad_top_left=pad)
+      for B in (shape[0], shape[0] + 1, shape[0]):
+        x = _randn(B, *shape[1:]).contiguous(**cl)
+        res = _randn(B, 40, shape[2] // stride, shape[3] // stride).contiguous(**cl)
+        for r in (None, res):
+          rows = None if r is None else r.permute(0, 2, 3, 1)
+          got = OC.conv2d_nchw(x, pk, rows)
+          assert torch.equal(got.permute(0, 2, 3, 1), OC.conv2d(x.permute(0, 2, 3, 1), pk, residual=rows))
+      assert OC.conv2d_nchw(_randn(1, shape[1], 6, 6), pk) is None  # not channels-last
+    x = _randn(*shape).contiguous(**cl)
+    first = OF.conv2d(x, w, b, stride=stride)
+    assert torch.equal(OF.conv2d(x, w.mul_(2), b * 2, stride=stride), (first.float() * 2).to(torch.bfloat16))
