@@ -6,7 +6,10 @@
 //   DQ  pass : a CTA keeps one 128-row block (Q_i, dO_i) resident and streams 64-key blocks of
 //              (K_j, V_j) over every KV segment:  S = Q K^T, dP = dO V^T -> dS -> dQ += dS K
 //
-// with P = exp2(S*c - lse2) and dS = P * (dP - delta), delta = rowsum(dO * O). No atomics and no
+// With one KV segment the DKV pass also writes dS, and dQ is one product over it (`flash_dq_kernel`); the DQ pass serves several
+// segments and sequences whose dS does not fit.
+//
+// Here P = exp2(S*c - lse2) and dS = P * (dP - delta), delta = rowsum(dO * O). No atomics and no
 // cross-CTA reduction are needed, so results are bitwise reproducible. The two score tiles of a
 // step are double buffered in TMEM so the elementwise warps (16 warps, each warp group owns 16 of
 // the 64 columns) overlap with the tensor core. The streamed tile is used twice from the same
@@ -42,6 +45,8 @@ __device__ __forceinline__ bool issuing_lane(int lane) {
   if (HD == 128) return elect_one();
   return lane == 0;
 }
+// dS of 128 keys x 64 queries as bf16: [half of the keys][16 queries][64 keys][32 bytes], 32-byte swizzle
+constexpr int DS_TILE_BYTES = BX * BY * 2;
 template <int HD>
 constexpr int smem_bytes() {
   return 2 * (HD / 64) * X_CHUNK_BYTES + Y_STAGES * 2 * (HD / 64) * Y_CHUNK_BYTES + Y_STAGES * 128 * 4 + 1024 + 256;
@@ -72,6 +77,9 @@ struct Params {
   int seg_batches, n_seg, out_rot, out_step;
   int x_len_seg[MAX_SEGMENTS];
   long long o_seg_stride;
+  // DKV pass of one segment: dS is also written out (null: not), see `flash_dq_kernel`
+  uint8_t* ds;
+  int ds_blocks;  // blocks of 64 queries per tile row
   DeviceStatus* status;
 };
 
@@ -394,6 +402,16 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ds_ready[b]);
+          if (DKV && p.ds != nullptr) {
+            // the warp's 32 rows of 32 bytes in line, eight full lines a store: with rows of 128 bytes (the 128-byte swizzle) every
+            // lane met a line of its own, and the stores held the operand reads up (dK, dV at 32760^2 x 4 heads 3.2 -> 4.6 ms)
+            uint8_t* dst = p.ds + (((static_cast<long long>(batch) * p.H + head) * gridDim.x + blockIdx.x) * p.ds_blocks + jb) * DS_TILE_BYTES +
+                           (quarter >> 1) * 8192 + wg * 2048 + ((quarter & 1) * 32 + lane) * 32;
+            uint32_t o[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) o[c] = (lane & 4) ? ds[c ^ 4] : ds[c];  // 32-byte swizzle: rows 4-7 of 8 swap their halves
+            store_32b(dst, o);
+          }
         }
       }
       if (ok && mbar_wait<1>(acc_final, 0, abort_flag, p.status, 91)) {
@@ -445,6 +463,133 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// dQ = scale * dS K from the dS that the DKV pass wrote (tiles of 128 keys x 64 queries, in the order the DKV pass made them:
+// [batch, head, key block, query block]), instead of a pass that multiplies S and dP again: five products instead of seven per
+// pair of tiles, for dS once through memory in each direction. A tile is copied into shared memory as it is, where it is an
+// MN-major A operand; K is the MN-major B operand. One CTA per 128 queries of a head, 64 keys per stage, two CTAs on an SM so
+// that one's loads go on while the other starts or stores. Bound by reading dS: 6.1 to 6.5 TB/s from 4096^2 up (32760^2 x 4 heads
+// 1.40 ms, where the pass that multiplies again takes 2.74), 1.7 to 4.3 TB/s where dS stays in L2 and a launch is 12 to 40 us.
+constexpr int DQ_THREADS = 192;  // warp 0 copies, warp 1 products, warps 2-5 results
+template <int HD>
+__host__ __device__ constexpr int dq_stages() { return HD == 128 ? 3 : 4; }
+template <int HD>
+__host__ __device__ constexpr int dq_smem_bytes() { return dq_stages<HD>() * (16384 + HD * 128) + 1024 + 256; }
+
+struct DqParams {
+  const uint8_t* ds;
+  int H, q_len, kv_len, ds_blocks, key_blocks;
+  void* out;
+  long long o_sb, o_ss, o_sh;
+  float scale;
+  DeviceStatus* status;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(DQ_THREADS, 2) flash_dq_kernel(const __grid_constant__ CUtensorMap tmap_k, const DqParams p) {
+  constexpr int STAGES = dq_stages<HD>();
+  constexpr int A_BYTES = 16384, STAGE_BYTES = A_BYTES + HD * 128;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* done = empty + STAGES;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
+  const int steps = (p.kv_len + 63) / 64;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+    prefetch_tensormap(&tmap_k);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_ptr_smem, HD);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+  if (warp == 0) {
+    if (elect_one()) {
+      const int chunks = min(2, p.ds_blocks - 2 * m);  // the last 64 queries may have no second block: its rows are not stored
+      const uint8_t* src = p.ds + ((static_cast<long long>(batch) * p.H + head) * p.key_blocks * p.ds_blocks + 2 * m) * DS_TILE_BYTES;
+      int stage = 0, issued = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int s = 0; s < steps; ++s) {
+        if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 100)) { ok = false; break; }
+        uint8_t* sa = smem + stage * STAGE_BYTES;
+        mbar_expect_tx(&full[stage], chunks * 8192 + HD * 128);
+        for (int c = 0; c < chunks; ++c)
+          bulk_load_1d(sa + c * 8192, src + (static_cast<long long>(s >> 1) * p.ds_blocks + c) * DS_TILE_BYTES + (s & 1) * 8192, 8192,
+                       &full[stage]);
+        for (int c = 0; c < HD / 64; ++c) tma_load_4d(sa + A_BYTES + c * 8192, &tmap_k, &full[stage], c * 64, head, s * 64, batch);
+        ++issued;
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (!ok) {  // its own copies in flight end before the CTA leaves
+        for (int i = 0; i < min(issued, STAGES); ++i) {
+          const int s = (stage - 1 - i + 2 * STAGES) % STAGES;
+          const uint32_t ph = i < stage ? phase : phase ^ 1u;
+          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(&full[s], ph); ++spin) {}
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(128, HD, true, true);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int s = 0; s < steps; ++s) {
+        if (!mbar_wait(&full[stage], phase, abort_flag, p.status, 101)) { ok = false; break; }
+        tc_fence_after_sync();
+        const uint64_t ad = make_smem_desc_sw32(smem_u32(smem + stage * STAGE_BYTES), 2048, 256);
+        const uint64_t bd = make_smem_desc(smem_u32(smem + stage * STAGE_BYTES + A_BYTES), 8192, 1024);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) umma_ss(tmem_base, ad + k * (512 >> 4), bd + k * (2048 >> 4), idesc, (s > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&empty[stage]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+      }
+      if (ok) umma_commit(done);
+    }
+  } else if (mbar_wait<100>(done, 0, abort_flag, p.status, 102)) {
+    tc_fence_after_sync();
+    const int quarter = warp & 3;
+    const int row = m * 128 + quarter * 32 + lane;
+    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + batch * p.o_sb + static_cast<long long>(row) * p.o_ss + head * p.o_sh;
+#pragma unroll 1
+    for (int c = 0; c < HD / 32; ++c) {
+      uint32_t r[32];
+      tmem_ld_x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c * 32, r);
+      tmem_wait_ld();
+      if (row < p.q_len) {
+        float x[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(r[i]) * p.scale;
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          *reinterpret_cast<uint4*>(o + c * 32 + v * 8) =
+              make_uint4(pack_bf16x2(x[v * 8], x[v * 8 + 1]), pack_bf16x2(x[v * 8 + 2], x[v * 8 + 3]),
+                         pack_bf16x2(x[v * 8 + 4], x[v * 8 + 5]), pack_bf16x2(x[v * 8 + 6], x[v * 8 + 7]));
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, HD);
   }
 }
 
@@ -522,7 +667,7 @@ static int flash_bwd_dkv_launch(const void* q, const void* d_o, const void* k, c
                                 const long long* qs, const long long* gs, const long long* ks, const long long* vs,
                                 const long long* dks, const long long* dvs, float softmax_scale, int out_f32,
                                 void* stream, int n_seg = 0, const int* seg_lens = nullptr, int out_rot = 0,
-                                int out_step = 1, long long o_seg_stride = 0) {
+                                int out_step = 1, long long o_seg_stride = 0, void* ds = nullptr) {
   if (B <= 0 || H <= 0 || q_len <= 0 || kv_len <= 0) return 0;
   if (n_seg < 0 || n_seg > MAX_SEGMENTS || (n_seg > 0 && seg_lens == nullptr)) return 3250;
   // stacked form: K and V are [n_seg * B, kv_len, H, D] with one batch stride across segments
@@ -553,6 +698,9 @@ static int flash_bwd_dkv_launch(const void* q, const void* d_o, const void* k, c
   p.out_rot = n_seg > 0 ? ((out_rot % n_seg) + n_seg) % n_seg : 0;
   p.out_step = n_seg > 0 ? ((out_step % n_seg) + n_seg) % n_seg : 0;
   p.o_seg_stride = o_seg_stride;
+  if (ds != nullptr && (n_seg > 0 || (reinterpret_cast<uintptr_t>(ds) & 127))) return 3251;
+  p.ds = static_cast<uint8_t*>(ds);
+  p.ds_blocks = (q_len + BY - 1) / BY;
   for (int s = 0; s < MAX_SEGMENTS; ++s) {
     const int len = (s < n_seg) ? seg_lens[s] : 0;
     if (len < 0 || len > kv_len) return 3250;
@@ -595,6 +743,8 @@ static int flash_bwd_dq_launch(const void* q, const void* d_o, const void* const
   }
   p.B = B; p.H = H; p.x_len = q_len; p.num_segments = num_segments;
   p.seg_batches = 0; p.n_seg = 1; p.out_rot = 0; p.out_step = 0; p.o_seg_stride = 0;
+  p.ds = nullptr;
+  p.ds_blocks = 0;
   for (int s = 0; s < MAX_SEGMENTS; ++s) p.x_len_seg[s] = 0;
   p.lse = lse; p.delta = delta; p.q_len = q_len;
   p.out0 = dq; p.out1 = nullptr;
@@ -614,6 +764,33 @@ static int flash_bwd_dq_launch(const void* q, const void* d_o, const void* const
   return static_cast<int>(cudaGetLastError());
 }
 
+// bf16 dQ from the dS that mdb_flash_bwd_dkv_ds wrote; one KV segment, kv_len > 0.
+template <int HD>
+static int flash_dq_launch(const void* ds, const void* k, void* dq, int B, int H, int q_len, int kv_len, const long long* ks,
+                           const long long* dqs, float softmax_scale, void* stream) {
+  if (B <= 0 || H <= 0 || q_len <= 0) return 0;
+  if (kv_len <= 0 || ds == nullptr || (reinterpret_cast<uintptr_t>(ds) & 127)) return 3251;
+  CUtensorMap tk;
+  int rc = make_map_d<HD>(&tk, k, B, kv_len, H, ks[0], ks[1], ks[2], 64);
+  if (rc) return rc;
+  DqParams p;
+  p.ds = static_cast<const uint8_t*>(ds);
+  p.H = H; p.q_len = q_len; p.kv_len = kv_len;
+  p.ds_blocks = (q_len + BY - 1) / BY;
+  p.key_blocks = (kv_len + BX - 1) / BX;
+  p.out = dq;
+  p.o_sb = dqs[0]; p.o_ss = dqs[1]; p.o_sh = dqs[2];
+  p.scale = softmax_scale;
+  p.status = status_buffer();
+  static bool configured = false;
+  if (!configured) {
+    MDB_CHECK_CUDA(cudaFuncSetAttribute(flash_dq_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, dq_smem_bytes<HD>()));
+    configured = true;
+  }
+  flash_dq_kernel<HD><<<dim3((q_len + 127) / 128, H, B), DQ_THREADS, dq_smem_bytes<HD>(), static_cast<cudaStream_t>(stream)>>>(tk, p);
+  return static_cast<int>(cudaGetLastError());
+}
+
 // C entry points: head_dim 128, and `_d64` for head_dim 64 (Stable Diffusion / SDXL / LTX-Video heads).
 #define MDB_FAB_ENTRY(SUFFIX, HD)                                                                                        \
   extern "C" int mdb_flash_delta##SUFFIX(const void* o, const void* d_o, float* delta, int B, int S, int H,               \
@@ -628,6 +805,21 @@ static int flash_bwd_dq_launch(const void* q, const void* d_o, const void* const
                                            const long long* dvs, float softmax_scale, int out_f32, void* stream) {        \
     return flash_bwd_dkv_launch<HD>(q, d_o, k, v, lse, delta, dk, dv, B, H, q_len, kv_len, qs, gs, ks, vs, dks, dvs,      \
                                     softmax_scale, out_f32, stream);                                                      \
+  }                                                                                                                       \
+  /* the same, and dS [B, H, ceil(kv_len / 128), ceil(q_len / 64)] tiles of 16 KiB for mdb_flash_dq_from_ds */              \
+  extern "C" int mdb_flash_bwd_dkv_ds##SUFFIX(const void* q, const void* d_o, const void* k, const void* v,               \
+                                              const float* lse, const float* delta, void* dk, void* dv, int B, int H,     \
+                                              int q_len, int kv_len, const long long* qs, const long long* gs,            \
+                                              const long long* ks, const long long* vs, const long long* dks,             \
+                                              const long long* dvs, float softmax_scale, int out_f32, void* stream,       \
+                                              void* ds) {                                                                 \
+    return flash_bwd_dkv_launch<HD>(q, d_o, k, v, lse, delta, dk, dv, B, H, q_len, kv_len, qs, gs, ks, vs, dks, dvs,      \
+                                    softmax_scale, out_f32, stream, 0, nullptr, 0, 1, 0, ds);                             \
+  }                                                                                                                       \
+  extern "C" int mdb_flash_dq_from_ds##SUFFIX(const void* ds, const void* k, void* dq, int B, int H, int q_len,           \
+                                              int kv_len, const long long* ks, const long long* dqs, float softmax_scale, \
+                                              void* stream) {                                                             \
+    return flash_dq_launch<HD>(ds, k, dq, B, H, q_len, kv_len, ks, dqs, softmax_scale, stream);                           \
   }                                                                                                                       \
   extern "C" int mdb_flash_bwd_dkv_stacked##SUFFIX(                                                                      \
       const void* q, const void* d_o, const void* k, const void* v, const float* lse, const float* delta, void* dk,       \

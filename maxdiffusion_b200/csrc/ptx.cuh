@@ -159,6 +159,12 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
                "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// 32 bytes of one thread (a whole sector), 32-byte aligned.
+__device__ __forceinline__ void store_32b(void* gdst, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(gdst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* desc, uint64_t* bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -404,6 +410,13 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   d |= 1ull << 46;
   d |= 2ull << 61;
   return d;
+}
+
+// The same with the 32-byte swizzle (layout 6), for an MN-major operand: K rows of 16 contiguous MN elements (32 bytes); SBO = 256 B
+//   between groups of 8 K rows, LBO = byte distance between consecutive 16-element MN chunks. One UMMA K-step (16 rows) advances
+//   the start address by 512 B.
+__device__ __forceinline__ uint64_t make_smem_desc_sw32(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return (make_smem_desc(smem_addr, lbo_bytes, sbo_bytes) & ~(7ull << 61)) | (6ull << 61);
 }
 
 // Instruction descriptor for kind::f16 with bf16 inputs and fp32 accumulation.

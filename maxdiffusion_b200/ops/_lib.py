@@ -233,13 +233,18 @@ def _declare(L: ctypes.CDLL) -> None:
   L.mdb_flash_delta.restype = c_int
   L.mdb_flash_bwd_dkv.argtypes = [c_void_p] * 8 + [c_int] * 4 + [c_llp] * 6 + [c_float, c_int, c_void_p]
   L.mdb_flash_bwd_dkv.restype = c_int
+  L.mdb_flash_bwd_dkv_ds.argtypes = L.mdb_flash_bwd_dkv.argtypes + [c_void_p]
+  L.mdb_flash_bwd_dkv_ds.restype = c_int
+  L.mdb_flash_dq_from_ds.argtypes = [c_void_p] * 3 + [c_int] * 4 + [c_llp] * 2 + [c_float, c_void_p]
+  L.mdb_flash_dq_from_ds.restype = c_int
   L.mdb_flash_bwd_dq.argtypes = ([c_void_p, c_void_p, ctypes.POINTER(c_void_p), ctypes.POINTER(c_void_p), c_void_p,
                                   c_void_p, c_void_p] + [c_int] * 4 + [ctypes.POINTER(c_int)] + [c_llp] * 5 +
                                  [c_float, c_int, c_void_p])
   L.mdb_flash_bwd_dq.restype = c_int
   L.mdb_flash_bwd_dkv_stacked.argtypes = L.mdb_flash_bwd_dkv.argtypes + [c_int, ctypes.POINTER(c_int), c_int, c_int, c_ll]
   L.mdb_flash_bwd_dkv_stacked.restype = c_int
-  for name in ("mdb_flash_delta", "mdb_flash_bwd_dkv", "mdb_flash_bwd_dkv_stacked", "mdb_flash_bwd_dq"):  # head_dim 64 variants: same signatures
+  for name in ("mdb_flash_delta", "mdb_flash_bwd_dkv", "mdb_flash_bwd_dkv_ds", "mdb_flash_dq_from_ds", "mdb_flash_bwd_dkv_stacked",
+               "mdb_flash_bwd_dq"):  # head_dim 64 variants: same signatures
     getattr(L, name + "_d64").argtypes = getattr(L, name).argtypes
     getattr(L, name + "_d64").restype = c_int
   for fn in _EXTRA:

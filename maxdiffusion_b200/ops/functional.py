@@ -247,6 +247,9 @@ class _AttentionFn(torch.autograd.Function):
     if d_o.stride(-1) != 1:
       d_o = d_o.contiguous()
     delta = K.flash_delta(out, d_o)
+    if n == 1:
+      dq, dk, dv = K.flash_bwd(q, d_o, ks[0], vs[0], lse, delta, ctx.scale)
+      return dq, None, None, None, dk, dv
     dq = K.flash_bwd_dq(q, d_o, ks, vs, lse, delta, ctx.scale)
     dks, dvs = [], []
     for k, v in zip(ks, vs):

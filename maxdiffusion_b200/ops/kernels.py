@@ -380,6 +380,57 @@ def flash_bwd_dkv(q, d_o, k, v, lse, delta, scale=None, out_dtype=torch.bfloat16
   return dk, dv
 
 
+_DS_BYTES = 9 << 30  # most of dS that is held at a time: four heads of 32760^2
+
+
+def flash_ds_chunk(B: int, H: int, Sq: int, Skv: int, limit: int | None = None) -> int:
+  """(batch, head) pairs whose dS `flash_bwd` holds at a time; 0: none, dQ multiplies S and dP again. All that fit, or of the
+  numbers that do the one that leaves least of the GPU idle in the rounds of its CTAs (one per 128 keys)."""
+  per = -(-Skv // 128) * -(-Sq // 64) * 16384
+  most = min(B * H, (_DS_BYTES if limit is None else limit) // per) if per else 0
+  if most == B * H or most < 1:
+    return most
+  most = min(most, H)  # parts of one sample: a part of the heads is one stride of the tensors
+  blocks = -(-Skv // 128)
+  rounds = lambda pairs: -(-pairs * blocks // _SM_COUNT)
+  cost = lambda n: (H // n) * rounds(n) + (rounds(H % n) if H % n else 0)
+  return min(range(1, most + 1), key=lambda n: (cost(n), -n))
+
+
+def flash_bwd(q, d_o, k, v, lse, delta, scale=None):
+  """dQ, dK, dV of attention over one KV segment (bf16): the pass over keys also writes dS, from which dQ is one product. Where
+  dS of a head is too large, or the memory for it is not there, dQ is a pass of its own (`flash_bwd_dq`).
+
+  Both, two passes / dS kept, on a B200: 4 x 1024^2 x 20 heads of 64 147 / 142 us, 4 x 4096^2 x 10 830 / 745, 4 x 4096 x 77 keys x 10
+  135 / 109; 4608^2 x 24 heads of 128 719 / 649 us, 32760 x 512 keys x 40 1972 / 1336, 32760^2 x 4 6.02 / 5.25 ms."""
+  B, Sq, H, D = q.shape
+  Skv = k.shape[1]
+  assert D in FLASH_HEAD_DIMS and all(t.stride(-1) == 1 for t in (q, d_o, k, v))
+  n = flash_ds_chunk(B, H, Sq, Skv)
+  ds = None
+  if n:
+    try:
+      ds = torch.empty(n * -(-Skv // 128) * -(-Sq // 64) * 16384, device=q.device, dtype=torch.uint8)
+    except torch.OutOfMemoryError:
+      pass
+  if ds is None:
+    return (flash_bwd_dq(q, d_o, [k], [v], lse, delta, scale), *flash_bwd_dkv(q, d_o, k, v, lse, delta, scale))
+  dq, dk, dv = (torch.empty(t.shape, device=q.device, dtype=torch.bfloat16) for t in (q, k, k))
+  scale = float(scale if scale is not None else 1.0 / math.sqrt(D))
+  dkv, from_ds = _flash_entry("mdb_flash_bwd_dkv_ds", D), _flash_entry("mdb_flash_dq_from_ds", D)
+  qs, gs, ks, vs, dqs, dks = (_strides3(t) for t in (q, d_o, k, v, dq, dk))
+  stream = _lib.stream()
+  parts = [(0, B, 0, H)] if n == B * H else [(b, 1, h, min(n, H - h)) for b in range(B) for h in range(0, H, n)]
+  for b, nb, h, nh in parts:
+    at = lambda t: t.data_ptr() + (b * t.stride(0) + h * t.stride(2)) * 2
+    row = (b * H + h) * Sq * 4
+    rc = dkv(at(q), at(d_o), at(k), at(v), lse.data_ptr() + row, delta.data_ptr() + row, at(dk), at(dv), nb, nh, Sq, Skv, qs, gs, ks, vs,
+             dks, dks, scale, 0, stream, ds.data_ptr())
+    _lib.check(rc, "mdb_flash_bwd_dkv_ds")
+    _lib.check(from_ds(ds.data_ptr(), at(k), at(dq), nb, nh, Sq, Skv, ks, dqs, scale, stream), "mdb_flash_dq_from_ds")
+  return dq, dk, dv
+
+
 def flash_bwd_dkv_stacked(q, d_o, kg, vg, lens, lse, delta, scale=None, dk=None, dv=None, out_rot: int = 0,
                           out_step: int = 1, out_dtype=torch.bfloat16):
   """dK, dV of ALL stacked KV segments kg / vg [n, B, Skv, H, D] from the local queries in ONE launch (the segments

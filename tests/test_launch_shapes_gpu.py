@@ -294,3 +294,27 @@ def test_norm_of_sum_and_conv_with_a_residual(shape, groups):
   a64, b64 = x.double().requires_grad_(), t.double().requires_grad_()
   F.silu(F.group_norm(a64 + b64[:, :, None, None], groups, norm.weight.double(), norm.bias.double(), 1e-5)).square().sum().backward()
   assert rel(a.grad, a64.grad) < 3e-2 and rel(b.grad, b64.grad) < 3e-2  # bf16 gradients of a bf16 sum
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Sq,Skv,H", [(1, 1, 1, 1), (2, 64, 65, 3), (1, 129, 128, 2), (2, 300, 77, 2), (1, 577, 450, 4)])
+def test_attention_backward_with_ds_kept(D, B, Sq, Skv, H, monkeypatch):
+  """dQ from the dS that the pass over keys wrote, whole and a head at a time, against float64 and against the two passes."""
+  torch.manual_seed(15)
+  q, k, v, g = _randn(B, Sq, H, D), _randn(B, Skv, 2 * H, D)[:, :, ::2], _randn(B, Skv, H, D), _randn(B, H, Sq, D).transpose(1, 2)
+  out, lse = K.flash_fwd(q, [k], [v])
+  delta = K.flash_delta(out, g)
+  dq, dk, dv = K.flash_bwd(q, g, k, v, lse, delta)
+  monkeypatch.setattr(K, "_DS_BYTES", -(-Skv // 128) * -(-Sq // 64) * 16384)
+  assert K.flash_ds_chunk(B, H, Sq, Skv) == 1
+  assert all(torch.equal(a, b) for a, b in zip(K.flash_bwd(q, g, k, v, lse, delta), (dq, dk, dv)))
+  monkeypatch.setattr(K, "_DS_BYTES", 0)  # no room: the two passes
+  old = K.flash_bwd(q, g, k, v, lse, delta)
+  assert torch.equal(old[1], dk) and torch.equal(old[2], dv) and torch.equal(old[0], K.flash_bwd_dq(q, g, [k], [v], lse, delta))
+  qd, kd, vd = (t.double().transpose(1, 2).requires_grad_() for t in (q, k, v))
+  y = ((qd @ kd.transpose(-1, -2)) * D ** -0.5).softmax(-1) @ vd
+  y.backward(g.double().transpose(1, 2))
+  if Skv > 1:  # one key: its probability is 1 and dS is rounding alone
+    assert _rel(dq.transpose(1, 2), qd.grad) < 1.05 * _rel(old[0].transpose(1, 2), qd.grad) + 1e-4
+    assert _rel(dk.transpose(1, 2), kd.grad) < 2e-2
+  assert _rel(dv.transpose(1, 2), vd.grad) < 2e-2
