@@ -525,6 +525,133 @@ gn_cl_fold_bwd_kernel(const float2* __restrict__ partial, int splits, int C, int
 }  // namespace cln
 }  // namespace mdb
 
+// ---------------------------------------------------------------------------------------------------------------
+// GroupNorm of few pixels in one launch: a CTA per sample and group holds the group's values in shared memory (each thread its
+// own), so x is read once, the variance is that of the centred values, and two launches and their gaps go. V: channels per load.
+// One CTA reads a group in pieces of 2 to 16 bytes per thread, so it wins where launches and latency count, three launches / one:
+// 2 x 8^2 x 1280 7.8 / 3.7 us, 2 x 16^2 x 1280 9.1 / 6.7, 2 x 32^2 x 640 (40 KB a group) 10.4 / 8.2; with 60 to 80 KB a group it loses
+// (2 x 32^2 x 960 10.0 / 13.0, x 1280 13.1 / 18.8, 2 x 64^2 x 320 11.8 / 24.0).
+// ---------------------------------------------------------------------------------------------------------------
+namespace mdb {
+namespace cln {
+
+constexpr int GN_SMALL_THREADS = 512;
+
+__device__ __forceinline__ float cta_sum(float v, float* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.0f;
+#pragma unroll
+  for (int w = 0; w < GN_SMALL_THREADS / 32; ++w) t += red[w];
+  __syncthreads();
+  return t;
+}
+
+template <int V>
+struct alignas(V * 2) BfVec {
+  __nv_bfloat16 v[V];
+};
+
+template <int V>
+__global__ void __launch_bounds__(GN_SMALL_THREADS)
+gn_cl_small_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int HW, int C, int cg, float eps, const void* gamma,
+                   const void* beta, int params_bf16, const __nv_bfloat16* __restrict__ shift, long long shift_pitch, int act) {
+  allow_successor();
+  wait_for_predecessor();
+  extern __shared__ __align__(16) uint8_t gn_smem[];
+  __shared__ float red[GN_SMALL_THREADS / 32];
+  BfVec<V>* held = reinterpret_cast<BfVec<V>*>(gn_smem);
+  const int g = blockIdx.x, n = blockIdx.y, nv = cg / V, total = HW * nv;
+  const __nv_bfloat16* sh = shift != nullptr ? shift + n * shift_pitch + g * cg : nullptr;
+  const long long base = static_cast<long long>(n) * HW * C + g * cg;
+  // vector i is number i % nv of pixel i / nv; a thread walks i in steps of the block without a division per step
+  const int step_pix = GN_SMALL_THREADS / nv, step_v = GN_SMALL_THREADS % nv;
+  const int pix0 = threadIdx.x / nv, v0 = threadIdx.x % nv;
+  float s = 0.0f;
+  {
+    int pix = pix0, v = v0;
+    for (int i = threadIdx.x; i < total; i += 4 * GN_SMALL_THREADS) {
+      BfVec<V> r[4];
+      int vv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        vv[u] = v;
+        if (i + u * GN_SMALL_THREADS < total) r[u] = *reinterpret_cast<const BfVec<V>*>(x + base + static_cast<long long>(pix) * C + v * V);
+        pix += step_pix;
+        v += step_v;
+        if (v >= nv) { v -= nv; ++pix; }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (i + u * GN_SMALL_THREADS < total) {
+          held[i + u * GN_SMALL_THREADS] = r[u];
+#pragma unroll
+          for (int j = 0; j < V; ++j) s += __bfloat162float(r[u].v[j]) + (sh != nullptr ? __bfloat162float(sh[vv[u] * V + j]) : 0.0f);
+        }
+      }
+    }
+  }
+  const float count = static_cast<float>(HW) * cg;
+  const float mean = cta_sum(s, red) / count;
+  s = 0.0f;
+  int v = v0;
+  for (int i = threadIdx.x; i < total; i += GN_SMALL_THREADS) {
+    const BfVec<V> r = held[i];
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const float d = __bfloat162float(r.v[j]) + (sh != nullptr ? __bfloat162float(sh[v * V + j]) : 0.0f) - mean;
+      s += d * d;
+    }
+    v += step_v;
+    if (v >= nv) v -= nv;
+  }
+  const float rstd = rsqrtf(cta_sum(s, red) / count + eps);
+  int pix = pix0;
+  v = v0;
+  for (int i = threadIdx.x; i < total; i += GN_SMALL_THREADS) {
+    const BfVec<V> r = held[i];
+    BfVec<V> o;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int c = g * cg + v * V + j;
+      const float a = rstd * param_at(gamma, params_bf16, c);
+      const float d = __bfloat162float(r.v[j]) + (sh != nullptr ? __bfloat162float(sh[v * V + j]) : 0.0f) - mean;
+      const float z = d * a + (beta != nullptr ? param_at(beta, params_bf16, c) : 0.0f);
+      o.v[j] = __float2bfloat16(act ? z / (1.0f + __expf(-z)) : z);
+    }
+    *reinterpret_cast<BfVec<V>*>(y + base + static_cast<long long>(pix) * C + v * V) = o;
+    pix += step_pix;
+    v += step_v;
+    if (v >= nv) { v -= nv; ++pix; }
+  }
+}
+
+}  // namespace cln
+}  // namespace mdb
+
+// x, y: bf16 [N, HW, C] contiguous, C / groups even; gamma / beta: [C] bf16 (params_bf16 = 1) or fp32, may be null; shift: bf16 [N, C] or
+// null, added to x first. The values of a group (HW * C / groups) must fit into 200 KB: error 3705 otherwise.
+extern "C" int mdb_gn_cl_small(const void* x, void* y, int N, int HW, int C, int groups, float eps, const void* gamma, const void* beta,
+                               int params_bf16, const void* shift, long long shift_pitch, int act, void* stream) {
+  using namespace mdb::cln;
+  if (N <= 0 || HW <= 0) return 0;
+  if (groups <= 0 || C % groups || N > 65535) return 3704;
+  const int cg = C / groups;
+  if ((cg & 1) || static_cast<long long>(HW) * cg * 2 > 200 * 1024 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15))
+    return 3705;
+  const size_t smem = static_cast<size_t>(HW) * cg * 2;
+  const auto launch = [&](auto kern) {
+    if (smem > 40 * 1024) MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    return static_cast<int>(mdb::launch_overlapped(kern, dim3(groups, N), GN_SMALL_THREADS, smem, static_cast<cudaStream_t>(stream),
+        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), HW, C, cg, eps, gamma, beta, params_bf16,
+        static_cast<const __nv_bfloat16*>(shift), shift_pitch, act));
+  };
+  // a group starts at a multiple of cg channels of rows that are multiples of cg: the load is as wide as cg allows
+  return cg % 8 == 0 ? launch(gn_cl_small_kernel<8>) : cg % 4 == 0 ? launch(gn_cl_small_kernel<4>) : launch(gn_cl_small_kernel<2>);
+}
+
 // partial: fp32 [N, splits, C, 2] from mdb_gn_cl_sums; gamma / beta: [C] bf16 (params_bf16 = 1) or fp32, may be null;
 // a, b: fp32 [N, C]; mean, rstd: fp32 [N, groups]. count = pixels * channels per group. shift: bf16 [N, C] or null.
 extern "C" int mdb_gn_cl_fold_fwd(const float* partial, int N, int splits, int C, int groups, float count, float eps,

@@ -38,6 +38,7 @@ int mdb_geglu_fwd(const void*, void*, long long, int, void*);
 int mdb_rms_rope_fwd(const void*, long long, void*, long long, long long, const void*, int, const float*, const float*, int, int,
                      int, int, float, float*, int, void*);
 int mdb_gn_cl_sums(const void*, const void*, const float*, const float*, float*, int, int, int, int, void*);
+int mdb_gn_cl_small(const void*, void*, int, int, int, int, float, const void*, const void*, int, const void*, long long, int, void*);
 int mdb_gn_cl_fold_fwd(const float*, int, int, int, int, float, float, const void*, const void*, int, float*, float*, float*,
                        float*, const void*, long long, void*);
 int mdb_gn_cl_apply(const void*, const void*, void*, const float*, const float*, const float*, const float*, const float*, int,
@@ -59,6 +60,7 @@ PyObject* g_error = nullptr;     // ops._lib.KernelError
 PyObject* g_plan = nullptr;      // ops.kernels.gemm_plan
 
 constexpr int kCtasTarget = 148 * 4;
+constexpr int64_t kGnSmallBytes = 40 * 1024, kGnSmallMost = 200 * 1024;
 
 PyObject* not_implemented() { Py_RETURN_NOTIMPLEMENTED; }
 
@@ -447,9 +449,11 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const double eps = PyFloat_AsDouble(a[4]);
   const bool act = a[5] == Py_True;
   if (PyErr_Occurred()) return nullptr;
-  if (!bf16(x) || x.dim() != 4 || x.numel() == 0 || !x.is_contiguous(at::MemoryFormat::ChannelsLast)) return not_implemented();
+  if (!bf16(x) || x.dim() != 4 || x.numel() == 0 || !x.is_contiguous(at::MemoryFormat::ChannelsLast) ||
+      (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15))
+    return not_implemented();
   const int64_t N = x.size(0), C = x.size(1), HW = x.size(2) * x.size(3);
-  if (groups <= 0 || C % groups || (C & 7) || C > 2048 || N > 65535 || HW > INT_MAX) return not_implemented();
+  if (groups <= 0 || C % groups || (C & 7) || N > 65535 || HW > INT_MAX) return not_implemented();
   for (const Tensor* p : {gamma, beta})
     if (p && (!bf16(*p) || !p->is_contiguous() || p->numel() != C)) return not_implemented();
   if (shift && (!bf16(*shift) || shift->dim() != 2 || shift->size(0) != N || shift->size(1) != C || shift->stride(1) != 1))
@@ -457,6 +461,17 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int splits = static_cast<int>(std::max<int64_t>(1, std::min((kCtasTarget + N - 1) / N, (HW + 15) / 16)));
   const int in = static_cast<int>(N), ic = static_cast<int>(C), ihw = static_cast<int>(HW), ig = static_cast<int>(groups);
   Tensor y;
+  // `ops.conv.gn_small`: up to 40 KB a group one launch is faster than three; beyond 2048 channels the three do not take x
+  const int64_t cg = C / groups;
+  if (cg % 2 == 0 && HW * cg * 2 <= (C > 2048 ? kGnSmallMost : kGnSmallBytes)) {
+    const int rc = unlocked([&] {
+      y = at::empty_like(x);
+      return mdb_gn_cl_small(x.data_ptr(), y.data_ptr(), in, ihw, ic, ig, static_cast<float>(eps), data(gamma), data(beta),
+                             gamma || beta ? 1 : 0, data(shift), shift ? shift->stride(0) : 0, act, stream());
+    });
+    return done(rc, "mdb_gn_cl_small", y);
+  }
+  if (C > 2048) return not_implemented();
   const int rc = unlocked([&] {
     // one buffer: the strips' sums, then a and b [N, C], mean and rstd [N, groups]
     const int64_t sums = N * splits * C * 2;

@@ -717,7 +717,7 @@ def group_norm(x, groups: int, gamma=None, beta=None, eps: float = 1e-6, act: bo
   """GroupNorm over a channels-first tensor [N, C, *spatial] with optional fused SiLU. A 4-D bf16 tensor in
   channels-last memory (what `conv2d` produces) stays in that layout. `shift` [N, C] is added to x first: without autograd in
   the fold of the sums, where it costs no pass over x."""
-  if _fast(x) and _is_channels_last(x) and x.shape[1] % 8 == 0 and x.shape[1] <= 2048:
+  if _fast(x) and _is_channels_last(x) and x.shape[1] % 8 == 0:
     if _direct(x, gamma, beta, shift):
       if shift is not None and (shift.dtype != torch.bfloat16 or shift.shape != x.shape[:2] or shift.stride(1) != 1):
         return group_norm(x + shift[:, :, None, None], groups, gamma, beta, eps, act)
@@ -725,11 +725,18 @@ def group_norm(x, groups: int, gamma=None, beta=None, eps: float = 1e-6, act: bo
       if r is not NotImplemented:
         return r
       N, C, H, W = x.shape
-      y3 = OC.group_norm_cl_fwd(x.permute(0, 2, 3, 1).view(N, H * W, C), groups, gamma, beta, eps, act, shift)[0]
-      return y3.view(N, H, W, C).permute(0, 3, 1, 2)
-    if shift is not None:
-      return group_norm(x + shift[:, :, None, None], groups, gamma, beta, eps, act)
-    return _GroupNormCLFn.apply(x, gamma, beta, groups, eps, act)
+      small = OC.gn_small(C, H * W, groups) and x.numel() > 0
+      if small or C <= 2048:
+        x3 = x.permute(0, 2, 3, 1).view(N, H * W, C)
+        x3 = x3.clone() if x.data_ptr() % 16 else x3  # 16-byte loads
+        y3 = (OC.group_norm_cl_small(x3, groups, gamma, beta, eps, act, shift) if small else
+              OC.group_norm_cl_fwd(x3, groups, gamma, beta, eps, act, shift)[0])
+        return y3.view(N, H, W, C).permute(0, 3, 1, 2)
+    elif x.shape[1] <= 2048:
+      if shift is not None:
+        x = x + shift[:, :, None, None]
+        return group_norm(x, groups, gamma, beta, eps, act)
+      return _GroupNormCLFn.apply(x, gamma, beta, groups, eps, act)
   if shift is not None:
     x = x + shift.reshape(*shift.shape, *(1,) * (x.dim() - 2))
   if x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and not _LIBRARY_MODE:

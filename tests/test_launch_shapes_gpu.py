@@ -318,3 +318,29 @@ def test_attention_backward_with_ds_kept(D, B, Sq, Skv, H, monkeypatch):
     assert _rel(dq.transpose(1, 2), qd.grad) < 1.05 * _rel(old[0].transpose(1, 2), qd.grad) + 1e-4
     assert _rel(dk.transpose(1, 2), kd.grad) < 2e-2
   assert _rel(dv.transpose(1, 2), vd.grad) < 2e-2
+
+
+@pytest.mark.parametrize("shape,groups", [((2, 64, 8, 8), 32), ((1, 320, 17, 5), 32), ((3, 96, 1, 9), 3), ((2, 640, 32, 32), 32), ((1, 1280, 31, 33), 32), ((2, 16, 1, 1), 8), ((2, 2560, 8, 8), 32), ((1, 2560, 32, 32), 32)])
+@pytest.mark.parametrize("act,affine,shifted", [(True, True, True), (False, False, False)])
+def test_group_norm_of_few_pixels(shape, groups, act, affine, shifted):
+  """One launch with the group's values in shared memory (2, 4 or 8 channels a load), against float64 and the three launches."""
+  from maxdiffusion_b200.ops import functional as OF
+
+  torch.manual_seed(17)
+  N, Ch, H, W = shape
+  x = (_randn(*shape) * 2 + 30).contiguous(memory_format=torch.channels_last)  # a mean far above the deviation
+  gamma, beta = (_randn(Ch), _randn(Ch)) if affine else (None, None)
+  t = _randn(N, 2 * Ch)[:, Ch:] if shifted else None
+  xs = x.double() + (t.double()[:, :, None, None] if shifted else 0.0)
+  want = torch.nn.functional.group_norm(xs, groups, None if gamma is None else gamma.double(), None if beta is None else beta.double(), 1e-5)
+  want = torch.nn.functional.silu(want) if act else want
+  with torch.no_grad():
+    got = OF.group_norm(x, groups, gamma, beta, 1e-5, act, t)
+    rows = None if Ch > 2048 else C.group_norm_cl_fwd(x.permute(0, 2, 3, 1).reshape(N, H * W, Ch), groups, gamma, beta, 1e-5, act, t)[0]
+  assert got.is_contiguous(memory_format=torch.channels_last)
+  assert got.shape == x.shape
+  if rows is None:
+    assert _rel(got, want) < 4e-3
+  elif H * W * Ch // groups > 2:  # two values: the deviation is rounding alone
+    three = _rel(rows.view(N, H, W, Ch).permute(0, 3, 1, 2), want)
+    assert _rel(got, want) < 4e-3 and _rel(got, want) < three + 1e-4
