@@ -38,7 +38,8 @@ int mdb_geglu_fwd(const void*, void*, long long, int, void*);
 int mdb_rms_rope_fwd(const void*, long long, void*, long long, long long, const void*, int, const float*, const float*, int, int,
                      int, int, float, float*, int, void*);
 int mdb_gn_cl_sums(const void*, const void*, const float*, const float*, float*, int, int, int, int, void*);
-int mdb_gn_cl_small(const void*, void*, int, int, int, int, float, const void*, const void*, int, const void*, long long, int, void*);
+// weak: over a kernel library without it the norm takes the three launches
+__attribute__((weak)) int mdb_gn_cl_small(const void*, void*, int, int, int, int, float, const void*, const void*, int, const void*, long long, int, void*);
 int mdb_gn_cl_fold_fwd(const float*, int, int, int, int, float, float, const void*, const void*, int, float*, float*, float*,
                        float*, const void*, long long, void*);
 int mdb_gn_cl_apply(const void*, const void*, void*, const float*, const float*, const float*, const float*, const float*, int,
@@ -463,7 +464,7 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor y;
   // `ops.conv.gn_small`: up to 40 KB a group one launch is faster than three; beyond 2048 channels the three do not take x
   const int64_t cg = C / groups;
-  if (cg % 2 == 0 && HW * cg * 2 <= (C > 2048 ? kGnSmallMost : kGnSmallBytes)) {
+  if (mdb_gn_cl_small != nullptr && cg % 2 == 0 && HW * cg * 2 <= (C > 2048 ? kGnSmallMost : kGnSmallBytes)) {
     const int rc = unlocked([&] {
       y = at::empty_like(x);
       return mdb_gn_cl_small(x.data_ptr(), y.data_ptr(), in, ihw, ic, ig, static_cast<float>(eps), data(gamma), data(beta),
