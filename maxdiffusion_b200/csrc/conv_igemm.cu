@@ -59,7 +59,7 @@ struct Tap {
   int koff;            // first K index of this tap in the weight matrix
 };
 
-enum Epilogue : int { kEpiNone = 0, kEpiSilu = 1 };
+enum Epilogue : int { kEpiNone = 0, kEpiSilu = 1, kEpiRoundFirst = 2 };  // flags; the last: a residual is added to the result as bf16 holds it
 
 struct Params {
   int n_classes;
@@ -102,7 +102,8 @@ __device__ __forceinline__ int unit_cut(int split, int splits, int units) {
 }
 __device__ __forceinline__ int split_of(int work, int splits, int num_tiles) { return splits == 1 ? 0 : work / num_tiles; }
 
-// Epilogue of 8 channels of one output position: bias, SiLU, residual, store.
+// Epilogue of 8 channels of one output position: bias, SiLU, residual, store. With kEpiRoundFirst the bits are those of a
+// convolution whose result is stored and added in a pass of its own.
 __device__ __forceinline__ void finish8(float (&x)[8], const Params& p, long long off, int col) {
   if (p.bias) {
     const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
@@ -114,11 +115,15 @@ __device__ __forceinline__ void finish8(float (&x)[8], const Params& p, long lon
       x[2 * j + 1] += f.y;
     }
   }
-  if (p.epi == kEpiSilu) {
+  if (p.epi & kEpiSilu) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = x[j] / (1.0f + __expf(-x[j]));
   }
   if (p.residual) {
+    if (p.epi & kEpiRoundFirst) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = __bfloat162float(__float2bfloat16(x[j]));
+    }
     const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + off + col);
     const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
 #pragma unroll
@@ -485,6 +490,7 @@ extern "C" int mdb_conv_igemm_tune(int ups, int stages, int ctas_per_sm) {
 //   box       : tile extents along dims 1..3 (product 128);  ext: output positions along dims 1..4
 //   taps      : n_taps_total x 6 ints (o0, o1, o2, o3, o4, koff);  tap_begin: n_classes + 1 ints
 //   out_strides (dims 1..4, elements), class_off (n_classes): where output position (p1..p4) of a class goes
+//   epi: flags of `Epilogue`
 //   group: taps that share a fetched row (consecutive in the table, one step along dim 1 apart; box[0] = 128)
 //   ctas_per_tile (1 / 2), max_bn (widest tile), splits: the launch shape (`ops/conv.py: conv_plan`); with splits > 1
 //   `partial` holds splits * n_classes * M-tiles * 128 * N fp32 values

@@ -511,7 +511,7 @@ bool ints(PyObject* o, T* out, Py_ssize_t n) {
 }
 
 // conv(x, x_alt, w, out, bias, residual, dims, strides, alt_dims, alt_strides, box, ext, c_in, n_pad, taps, begin, alt_dim,
-//      alt_shift, out_strides, class_off, silu, ctas, max_bn, splits, m_tiles, group): the arguments of `ops.conv._launch`, shapes as
+//      alt_shift, out_strides, class_off, epi, ctas, max_bn, splits, m_tiles, group): the arguments of `ops.conv._launch`, shapes as
 // tuples, taps and begin as the addresses of int arrays. Returns `out`.
 PyObject* py_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -530,7 +530,7 @@ PyObject* py_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int* taps = static_cast<const int*>(PyLong_AsVoidPtr(a[14]));
   const int* begin = static_cast<const int*>(PyLong_AsVoidPtr(a[15]));
   const int alt_dim = static_cast<int>(PyLong_AsLong(a[16])), alt_shift = static_cast<int>(PyLong_AsLong(a[17]));
-  const int silu = static_cast<int>(PyLong_AsLong(a[20])), ctas = static_cast<int>(PyLong_AsLong(a[21]));
+  const int epi = static_cast<int>(PyLong_AsLong(a[20])), ctas = static_cast<int>(PyLong_AsLong(a[21]));
   const int max_bn = static_cast<int>(PyLong_AsLong(a[22])), splits = static_cast<int>(PyLong_AsLong(a[23]));
   const int64_t m_tiles = PyLong_AsLongLong(a[24]);
   const int group = static_cast<int>(PyLong_AsLong(a[25]));
@@ -542,7 +542,7 @@ PyObject* py_conv(PyObject*, PyObject* const* a, Py_ssize_t n) {
                           out.options().dtype(at::kFloat).memory_format(at::MemoryFormat::Contiguous));
     return mdb_conv_igemm(x.data_ptr(), data(alt), w.data_ptr(), out.data_ptr(), data(bias), data(residual), dims, strides, alt_dims,
                           alt_strides, box, ext, c_in, n_pad, w.size(1), static_cast<int>(classes), begin, taps, alt_dim, alt_shift,
-                          os, class_off, silu, ctas, max_bn, splits, splits > 1 ? partial.data_ptr() : nullptr, group, stream());
+                          os, class_off, epi, ctas, max_bn, splits, splits > 1 ? partial.data_ptr() : nullptr, group, stream());
   });
   return done(rc, "mdb_conv_igemm", out);
   END_HANDLE_TH_ERRORS

@@ -332,7 +332,7 @@ _ROWS = True  # False: never share fetched rows (benchmarks, tests)
 
 
 def _launch(x, x_alt, pk: PackedConv, dims, strides, alt_dims, alt_strides, box, ext, out, out_strides, class_off,
-            residual, silu, alt_dim=-1, alt_shift=0, tap_shift1=0):
+            residual, epi, alt_dim=-1, alt_shift=0, tap_shift1=0):
   taps, begin, n_classes = pk.tap_arrays(tap_shift1)
   LL, I = ctypes.c_longlong, ctypes.c_int
   arr = lambda T, v: _carray(T, tuple(v))
@@ -346,7 +346,7 @@ def _launch(x, x_alt, pk: PackedConv, dims, strides, alt_dims, alt_strides, box,
     dims, strides, box, ext = tuple(dims), tuple(strides), tuple(box), tuple(ext)
     r = host.conv(x, x_alt, pk.w, out, pk.bias, residual, dims, strides, tuple(alt_dims) if alt_dims else dims,
                   tuple(alt_strides) if alt_strides else strides, box, ext, pk.c_in, pk.n_pad, ctypes.addressof(taps),
-                  ctypes.addressof(begin), alt_dim, alt_shift, tuple(out_strides), tuple(class_off), 1 if silu else 0, ctas,
+                  ctypes.addressof(begin), alt_dim, alt_shift, tuple(out_strides), tuple(class_off), int(epi), ctas,
                   max_bn, splits, m_tiles, group)
     if r is not NotImplemented:
       return out
@@ -357,7 +357,7 @@ def _launch(x, x_alt, pk: PackedConv, dims, strides, alt_dims, alt_strides, box,
       _lib.ptr(x), _lib.ptr(x_alt), _lib.ptr(pk.w), _lib.ptr(out), _lib.ptr(pk.bias), _lib.ptr(residual),
       arr(LL, dims), arr(LL, strides), arr(LL, alt_dims if alt_dims else dims), arr(LL, alt_strides if alt_strides else strides),
       arr(I, box), arr(I, ext), pk.c_in, pk.n_pad, pk.w.shape[1], n_classes, begin, taps, alt_dim, alt_shift,
-      arr(LL, out_strides), arr(LL, class_off), 1 if silu else 0, ctas, max_bn, splits, _lib.ptr(partial), group, _lib.stream())
+      arr(LL, out_strides), arr(LL, class_off), int(epi), ctas, max_bn, splits, _lib.ptr(partial), group, _lib.stream())
   _lib.check(rc, "mdb_conv_igemm")
   return out
 
@@ -414,11 +414,17 @@ def conv3d_causal(x: torch.Tensor, pk: PackedConv, hist: Optional[torch.Tensor] 
   return out if pk.n_pad == pk.n_out else out[..., :pk.n_out]
 
 
-def conv2d(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = None, silu: bool = False) -> torch.Tensor:
-  """x [B, H, W, C] -> [B, Ho, Wo, N] (Ho = H for stride 1, H / 2 for stride 2)."""
+_ROUND_FIRST = 2  # epilogue flag: a residual is added to the result as bf16 holds it (`csrc/conv_igemm.cu`)
+
+
+def conv2d(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = None, silu: bool = False,
+           round_first: bool = False) -> torch.Tensor:
+  """x [B, H, W, C] -> [B, Ho, Wo, N] (Ho = H for stride 1, H / 2 for stride 2). A residual is added in fp32, or with
+  `round_first` to the rounded result: the bits of a convolution and an addition one after the other."""
   if not use_kernel(x):
     w, b, stride, p = pk.src
-    return ref_conv2d(x[..., :w.shape[1]], w, b, stride=stride, pad_top_left=p, residual=residual, silu=silu).to(x.dtype)
+    y = ref_conv2d(x[..., :w.shape[1]], w, b, stride=stride, pad_top_left=p, residual=None if round_first else residual, silu=silu).to(x.dtype)
+    return residual + y if round_first and residual is not None else y
   _check_cl(x, pk.c_in)
   B, H, W, C = x.shape
   n = pk.n_pad
@@ -439,12 +445,14 @@ def conv2d(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = N
     raise ValueError(f"conv2d cannot run weights packed as {pk.kind}")
   if residual is not None:
     assert residual.shape == out.shape and residual.is_contiguous()
-  _launch(x, None, pk, dims, strides, None, None, box, ext, out, os_, [0], residual, silu)
+  _launch(x, None, pk, dims, strides, None, None, box, ext, out, os_, [0], residual,
+          int(silu) | (_ROUND_FIRST if round_first else 0))
   return out if pk.n_pad == pk.n_out else out[..., :pk.n_out]
 
 
 def _conv2d_launch(pk: PackedConv, B: int, H: int, W: int):
-  """(arguments of the host extension's `conv` behind the residual, output height, output width) of a dense [B, H, W, c_in]."""
+  """(arguments of the host extension's `conv` between the residual and the epilogue, those behind it, output height, output
+  width) of a dense [B, H, W, c_in]."""
   C, n = pk.c_in, pk.n_pad
   if pk.kind == "conv2d_s2":
     Ho, Wo = H // 2, W // 2
@@ -461,11 +469,11 @@ def _conv2d_launch(pk: PackedConv, B: int, H: int, W: int):
   for e, b in zip(ext[:3], box):
     m_tiles *= -(-e // b)
   ctas, max_bn, splits = conv_plan(m_tiles, n_classes, n, -(-C // 64) * min(len(c) for c in pk.taps), group)
-  return (dims, strides, dims, strides, box, ext, C, n, ctypes.addressof(taps), ctypes.addressof(begin), -1, 0, os_, (0,), 0, ctas, max_bn,
-          splits, m_tiles, group), Ho, Wo
+  return ((dims, strides, dims, strides, box, ext, C, n, ctypes.addressof(taps), ctypes.addressof(begin), -1, 0, os_, (0,)),
+          (ctas, max_bn, splits, m_tiles, group), Ho, Wo)
 
 
-def conv2d_nchw(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = None):
+def conv2d_nchw(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor] = None, round_first: bool = False):
   """`conv2d` of an NCHW tensor in channels-last memory, with a residual like the result, as NCHW in channels-last memory, with
   little host work: what the launch needs is kept with the packed weights for up to 32 input sizes. None where the host
   extension or these tensors do not fit: the caller then uses `conv2d`."""
@@ -481,9 +489,9 @@ def conv2d_nchw(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor
     if len(pk._launches) >= 32:
       pk._launches.clear()
     hit = pk._launches[(B, H, W)] = _conv2d_launch(pk, B, H, W)
-  args, Ho, Wo = hit
+  shapes, plan, Ho, Wo = hit
   out = torch.empty((B, pk.n_out, Ho, Wo), dtype=x.dtype, device=x.device, memory_format=torch.channels_last)
-  return None if host.conv(x, None, pk.w, out, pk.bias, residual, *args) is NotImplemented else out
+  return None if host.conv(x, None, pk.w, out, pk.bias, residual, *shapes, _ROUND_FIRST if round_first else 0, *plan) is NotImplemented else out
 
 
 def _parity_conv(x, pk, silu=False, halo: int = 0):

@@ -782,7 +782,7 @@ def _conv2d_fwd(x, weight, bias, stride, pad, upsample, residual=None):
     y = OC.upsample2x_conv2d(OC.pad_channels(xc, pk.c_in), pk)
   else:
     pk = _packed_conv2d(weight, bias, stride, pad)
-    y = OC.conv2d(OC.pad_channels(xc, pk.c_in), pk, residual=residual)
+    y = OC.conv2d(OC.pad_channels(xc, pk.c_in), pk, residual=residual, round_first=True)
   return y.permute(0, 3, 1, 2), xc
 
 
@@ -827,8 +827,8 @@ class _Conv2dFn(torch.autograd.Function):
 
 def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = False, residual=None):
   """2-D convolution of an NCHW tensor. `padding` is an int (all sides) or "far" (zero rows / columns after the image
-  only: the VAE's stride-2 down-sampling). With `upsample` the input is nearest-2x up-sampled first (fused). `residual`, of the
-  result's shape, is added to it, where it can be in the kernel's epilogue.
+  only: the VAE's stride-2 down-sampling). With `upsample` the input is nearest-2x up-sampled first (fused). `residual + y` with
+  a residual of the result's shape is formed in the kernel's epilogue where it can be, with the bits of the two operations.
 
   CUDA bf16 3x3 convolutions run on the implicit-GEMM kernels and return channels-last memory; 1x1 convolutions are
   GEMMs over the pixel rows; everything else is `torch.nn.functional.conv2d`."""
@@ -855,7 +855,7 @@ def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = Fa
         rows = residual.permute(0, 2, 3, 1)
         rows = rows if rows.is_contiguous() else None
       if not upsample and (rows is not None or residual is None):
-        y = OC.conv2d_nchw(x, _packed_conv2d(weight, bias, stride, pad_tl), rows)
+        y = OC.conv2d_nchw(x, _packed_conv2d(weight, bias, stride, pad_tl), rows, round_first=True)
         if y is not None:
           return y
       if rows is not None:
