@@ -20,7 +20,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import functional as OF
-from .layers import Conv2d, GroupNorm, LayerNorm, Linear, is_plain_linear, sinusoidal_embedding, conv_plus
+from .layers import Conv2d, GroupNorm, LayerNorm, Linear, is_plain_linear, sinusoidal_embedding
 from .vae import ResnetBlock2D
 
 
@@ -156,11 +156,11 @@ class Transformer2DModel(nn.Module):
       y = self.proj_in(y).permute(0, 2, 3, 1).reshape(b, h * w, c)
     for blk in self.transformer_blocks:
       y = blk(y, context)
-    if not self.linear_proj:
-      return conv_plus(self.proj_out, y.reshape(b, h, w, c).permute(0, 3, 1, 2), res)
-    if is_plain_linear(self.proj_out) and y.is_cuda and y.dtype == res.dtype:  # the add rides in the product's epilogue
-      return self.proj_out(y, residual=res.permute(0, 2, 3, 1).reshape(b, h * w, c)).reshape(b, h, w, c).permute(0, 3, 1, 2)
-    return self.proj_out(y).reshape(b, h, w, c).permute(0, 3, 1, 2) + res
+    if self.linear_proj:
+      y = self.proj_out(y).reshape(b, h, w, c).permute(0, 3, 1, 2)
+    else:
+      y = self.proj_out(y.reshape(b, h, w, c).permute(0, 3, 1, 2))
+    return y + res
 
 
 class Downsample2D(nn.Module):

@@ -838,11 +838,8 @@ def conv2d(x, weight, bias=None, stride: int = 1, padding=1, upsample: bool = Fa
   if _fast(x) and k == 1 and stride == 1 and pad_tl == 0 and not upsample and ci % 8 == 0 and co % 8 == 0:
     n, c, h, w = x.shape
     rows = x.contiguous(memory_format=torch.channels_last).permute(0, 2, 3, 1).reshape(n, h * w, c)
-    res = None
-    if residual is not None and residual.shape == (n, co, h, w) and residual.dtype == x.dtype:
-      res = residual.permute(0, 2, 3, 1).reshape(n, h * w, co)
-    y = linear(rows, weight.reshape(co, ci), bias, residual=res).view(n, h, w, co).permute(0, 3, 1, 2)
-    return y if res is not None or residual is None else residual + y
+    y = linear(rows, weight.reshape(co, ci), bias).view(n, h, w, co).permute(0, 3, 1, 2)
+    return y if residual is None else residual + y
   even = x.shape[2] % 2 == 0 and x.shape[3] % 2 == 0
   if (_fast(x) and k == 3 and stride in (1, 2) and (stride == 1 or even) and
       ((stride == 1 and pad_tl == 1) or (stride == 2 and pad_tl in (0, 1)))):

@@ -13,7 +13,7 @@ def _cl(*shape, scale=1.0):
 
 
 @pytest.mark.parametrize("shape,co,k,stride", [((2, 32, 8, 8), 40, 3, 1), ((1, 48, 17, 5), 64, 3, 1), ((2, 1280, 8, 8), 1280, 3, 1),
-                                               ((1, 64, 40, 24), 320, 3, 1), ((2, 32, 6, 10), 32, 3, 2)])
+                                               ((1, 64, 40, 24), 320, 3, 1), ((2, 32, 6, 10), 32, 3, 2), ((2, 64, 9, 8), 40, 1, 1)])
 @pytest.mark.parametrize("grad", [False, True])
 def test_a_convolution_and_its_residual(shape, co, k, stride, grad):
   """A residual in the epilogue is added to the rounded result, over whole and cut contractions."""
@@ -23,3 +23,21 @@ def test_a_convolution_and_its_residual(shape, co, k, stride, grad):
   with torch.set_grad_enabled(grad):
     assert torch.equal(conv_plus(m, x, res), res + m(x))
     assert torch.equal(conv_plus(m, x, res.contiguous()), res.contiguous() + m(x))
+
+
+@pytest.mark.parametrize("linear_proj", [True, False])
+@pytest.mark.parametrize("grad", [False, True])
+def test_a_transformer_and_its_residual(linear_proj, grad):
+  """The output projection's result is rounded before the input is added, as a hook that does nothing leaves it."""
+  from maxdiffusion_b200.models.unet_2d_condition import Transformer2DModel
+
+  torch.manual_seed(2)
+  m = Transformer2DModel(128, 2, 1, 64, 32, linear_proj).to("cuda", torch.bfloat16)
+  x, context = _cl(2, 128, 8, 12, scale=30.0), torch.randn(2, 7, 64, device="cuda").to(torch.bfloat16)
+  with torch.set_grad_enabled(grad):
+    out = m(x, context)
+    seen = []
+    m.proj_out.register_forward_hook(lambda mod, args, y: seen.append(y))
+    assert torch.equal(m(x, context), out)
+  y = seen[0].unflatten(1, (8, 12)).permute(0, 3, 1, 2) if linear_proj else seen[0]
+  assert torch.equal(out, y + x)
