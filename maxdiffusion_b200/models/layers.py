@@ -111,26 +111,18 @@ class GroupNorm(nn.GroupNorm):
 _CONV_FORWARD, _GROUP_NORM_FORWARD = Conv2d.forward, GroupNorm.forward
 
 
-_NN_LINEAR_FORWARD = nn.Linear.forward
-
-
-def row_linear(m: nn.Module, x):
-  """m(x) of a plain `nn.Linear` and a few rows; without autograd through `OF.linear`, a third of the library call's host time."""
-  if type(m) is nn.Linear and nn.Linear.forward is _NN_LINEAR_FORWARD and calls_forward_only(m) and x.dtype == m.weight.dtype:
-    if OF._fast(x) and OF._direct(x, m.weight, m.bias):
-      return OF.linear(x, m.weight, m.bias)
-  return m(x)
-
-
 def conv_plus(m: nn.Module, x, residual):
-  """residual + m(x); in one kernel where calling `m` is `OF.conv2d` and nothing else (no wrapper, replaced `forward` or hook)."""
+  """residual + m(x), the same bits; in one kernel where calling `m` is `OF.conv2d` and nothing else (no wrapper, replaced `forward`
+  or hook)."""
   if type(m) is Conv2d and Conv2d.forward is _CONV_FORWARD and calls_forward_only(m):
     return m(x, residual=residual)
   return residual + m(x)
 
 
 def norm_of_sum(m: nn.Module, x, shift, act: bool = True):
-  """m(x + shift[:, :, None, None], act); x is not written again where calling `m` is `OF.group_norm` and nothing else."""
+  """m(x + shift[:, :, None, None], act); where calling `m` is `OF.group_norm` and nothing else, x is not written again and the sum
+  is not rounded, so the result is closer to the exact one but not the bits of the two operations (a UNet step moves by 1 %:
+  its blocks add in bf16)."""
   if type(m) is GroupNorm and GroupNorm.forward is _GROUP_NORM_FORWARD and calls_forward_only(m):
     return m(x, act=act, shift=shift)
   return m(x + shift[:, :, None, None], act=act)

@@ -15,7 +15,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import functional as OF
-from .layers import Conv2d, GroupNorm, conv_plus, norm_of_sum, row_linear
+from .layers import Conv2d, GroupNorm, conv_plus
 
 
 @dataclass
@@ -59,9 +59,8 @@ class ResnetBlock2D(nn.Module):
   def forward(self, x, temb=None):
     h = self.conv1(self.norm1(x, act=True))
     if self.time_emb_proj is not None and temb is not None:
-      h = norm_of_sum(self.norm2, h, row_linear(self.time_emb_proj, F.silu(temb)))
-    else:
-      h = self.norm2(h, act=True)
+      h = h + self.time_emb_proj(F.silu(temb))[:, :, None, None]
+    h = self.norm2(h, act=True)
     return conv_plus(self.conv2, h, self.conv_shortcut(x) if self.conv_shortcut is not None else x)
 
 

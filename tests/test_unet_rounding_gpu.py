@@ -4,6 +4,7 @@ import torch
 import torch.nn.functional as F
 
 from maxdiffusion_b200.models.layers import Conv2d, conv_plus
+from maxdiffusion_b200.models.vae import ResnetBlock2D
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +42,17 @@ def test_a_transformer_and_its_residual(linear_proj, grad):
     assert torch.equal(m(x, context), out)
   y = seen[0].unflatten(1, (8, 12)).permute(0, 3, 1, 2) if linear_proj else seen[0]
   assert torch.equal(out, y + x)
+
+
+@pytest.mark.parametrize("cin,cout,size,rows", [(64, 64, (16, 16), 2), (96, 64, (17, 5), 2), (320, 640, (40, 40), 1)])
+@pytest.mark.parametrize("grad", [False, True])
+def test_a_resnet_block_and_its_time_embedding(cin, cout, size, rows, grad):
+  """The embedding is added in bf16 in front of the norm, its projection is the module's own product."""
+  torch.manual_seed(3)
+  m = ResnetBlock2D(cin, cout, temb_channels=128, eps=1e-5).to("cuda", torch.bfloat16)
+  x, temb = _cl(2, cin, *size), torch.randn(rows, 128, device="cuda").to(torch.bfloat16)
+  with torch.set_grad_enabled(grad):
+    h = m.conv1(m.norm1(x, act=True))
+    h = h + F.linear(F.silu(temb), m.time_emb_proj.weight, m.time_emb_proj.bias)[:, :, None, None]
+    h = m.conv2(m.norm2(h, act=True))
+    assert torch.equal(m(x, temb), (x if m.conv_shortcut is None else m.conv_shortcut(x)) + h)
