@@ -447,6 +447,34 @@ __device__ __forceinline__ float2 cta_sum2(float2 v, float2* red) {
   return t;
 }
 
+// (mean, rstd) of a group from its channel sums; every thread gets them, the first 256 add.
+__device__ __forceinline__ float2 group_stats(const float2* ch, int cg, const __nv_bfloat16* sh, float count, float eps, float2* red) {
+  float2 t = make_float2(0.0f, 0.0f);
+  if (threadIdx.x < 256) {
+    for (int j = threadIdx.x; j < cg; j += 256) {
+      if (sh != nullptr) {
+        const float v = __bfloat162float(sh[j]), hw = count / cg;
+        t.x += ch[j].x + hw * v;
+        t.y += ch[j].y + v * (2.0f * ch[j].x + hw * v);
+      } else {
+        t.x += ch[j].x;
+        t.y += ch[j].y;
+      }
+    }
+  }
+  t = cta_sum2(t, red);
+  const float mean = t.x / count;
+  return make_float2(mean, rsqrtf(fmaxf(t.y / count - mean * mean, 0.0f) + eps));
+}
+
+// (a, b) of channel c, the group's j-th
+__device__ __forceinline__ float2 group_coef(float2 mr, const void* gamma, const void* beta, int params_bf16, int c, const __nv_bfloat16* sh,
+                                             int j) {
+  const float av = mr.y * param_at(gamma, params_bf16, c);
+  const float at = sh != nullptr ? __bfloat162float(sh[j]) - mr.x : -mr.x;
+  return make_float2(av, (beta != nullptr ? param_at(beta, params_bf16, c) : 0.0f) + at * av);
+}
+
 // forward: a = rstd * gamma, b = beta - mean * a; also mean / rstd [N, G] for the backward. `shift` (null: none) holds a value
 // per sample and channel that is to be added to x first: the sums of x + t follow from those of x, and act((x + t) a + b) is
 // act(x a + (t a + b)), so neither pass over x changes and no pass of its own adds it (an SDXL step at 1024^2: 17 passes of 16 us).
@@ -462,30 +490,16 @@ gn_cl_fold_fwd_kernel(const float2* __restrict__ partial, int splits, int C, int
   const int g = blockIdx.x, n = blockIdx.y, cg = C / groups;
   group_channel_sums(partial + static_cast<long long>(n) * splits * C + g * cg, splits, C, cg, red, ch);
   const __nv_bfloat16* sh = shift != nullptr ? shift + n * shift_pitch + g * cg : nullptr;
-  float2 t = make_float2(0.0f, 0.0f);
-  for (int j = threadIdx.x; j < cg; j += 256) {
-    if (sh != nullptr) {
-      const float v = __bfloat162float(sh[j]), hw = count / cg;
-      t.x += ch[j].x + hw * v;
-      t.y += ch[j].y + v * (2.0f * ch[j].x + hw * v);
-    } else {
-      t.x += ch[j].x;
-      t.y += ch[j].y;
-    }
-  }
-  t = cta_sum2(t, red);
-  const float mean = t.x / count;
-  const float rstd = rsqrtf(fmaxf(t.y / count - mean * mean, 0.0f) + eps);
+  const float2 mr = group_stats(ch, cg, sh, count, eps, red);
   if (threadIdx.x == 0) {
-    mean_out[n * groups + g] = mean;
-    rstd_out[n * groups + g] = rstd;
+    mean_out[n * groups + g] = mr.x;
+    rstd_out[n * groups + g] = mr.y;
   }
   for (int j = threadIdx.x; j < cg; j += 256) {
     const int c = g * cg + j;
-    const float av = rstd * param_at(gamma, params_bf16, c);
-    a[static_cast<long long>(n) * C + c] = av;
-    const float at = sh != nullptr ? __bfloat162float(sh[j]) - mean : -mean;
-    b[static_cast<long long>(n) * C + c] = (beta != nullptr ? param_at(beta, params_bf16, c) : 0.0f) + at * av;
+    const float2 ab = group_coef(mr, gamma, beta, params_bf16, c, sh, j);
+    a[static_cast<long long>(n) * C + c] = ab.x;
+    b[static_cast<long long>(n) * C + c] = ab.y;
   }
 }
 
@@ -526,130 +540,221 @@ gn_cl_fold_bwd_kernel(const float2* __restrict__ partial, int splits, int C, int
 }  // namespace mdb
 
 // ---------------------------------------------------------------------------------------------------------------
-// GroupNorm of few pixels in one launch: a CTA per sample and group holds the group's values in shared memory (each thread its
-// own), so x is read once, the variance is that of the centred values, and two launches and their gaps go. V: channels per load.
-// One CTA reads a group in pieces of 2 to 16 bytes per thread, so it wins where launches and latency count, three launches / one:
-// 2 x 8^2 x 1280 7.8 / 3.7 us, 2 x 16^2 x 1280 9.1 / 6.7, 2 x 32^2 x 640 (40 KB a group) 10.4 / 8.2; with 60 to 80 KB a group it loses
-// (2 x 32^2 x 960 10.0 / 13.0, x 1280 13.1 / 18.8, 2 x 64^2 x 320 11.8 / 24.0).
+// GroupNorm of few pixels in one launch: a CTA per sample and group holds the group's values in shared memory, so x is read once
+// and two launches and their gaps go. Every sum is taken in the order of the kernels it stands for, so the bits are theirs:
+//   CF = false: up to 2048 channels, the three launches above (strips, rows of a pass, lanes of the fold);
+//   CF = true:  beyond, where they do not go, the channels-first kernels (`groupnorm.cu`: leaves of 8 pixels or of one, the
+//               butterfly of a warp, the one over eight warps, channels in order) without the copies to and from their layout.
+// Bound by the latency of one CTA's loads and passes over shared memory (4 us and 0.12 us per KB of a group), so it wins where the
+// launches of the others cost more. Microseconds, the other kernels / this one: 2 x 8^2 x 1280 7.9 / 4.4, 2 x 16^2 x 1280 9.4 / 6.1,
+// 1 x 16^2 x 1920 9.7 / 6.7; channels-first with its copies 2 x 8^2 x 2560 48.5 / 6.6, 2 x 32^2 x 2560 90.2 / 23.7.
 // ---------------------------------------------------------------------------------------------------------------
 namespace mdb {
 namespace cln {
 
-constexpr int GN_SMALL_THREADS = 512;
+constexpr int GN_GROUP_THREADS = 512;
+constexpr int GN_GROUP_SMEM = 226 * 1024;
+constexpr int GN_LEAF_CHANNELS = GN_GROUP_THREADS / 32;  // a warp per channel adds the leaves
 
-__device__ __forceinline__ float cta_sum(float v, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float t = 0.0f;
-#pragma unroll
-  for (int w = 0; w < GN_SMALL_THREADS / 32; ++w) t += red[w];
-  __syncthreads();
-  return t;
+// Shared memory: float2 [512] (sums across warps), [cg] coefficients, [cg] channel sums, [part] strip sums or leaves, then the values
+// as pairs of channels, a pixel's in an odd number of words: threads of neighbouring pixels and channels meet other banks.
+struct GroupLayout {
+  int part, pitch;
+  long long bytes;
+};
+__host__ __device__ inline GroupLayout group_layout(bool cf, int HW, int cg, int splits) {
+  GroupLayout l;
+  const int leaves = HW % 8 == 0 ? HW / 8 : HW;
+  l.part = cf ? GN_LEAF_CHANNELS * ((leaves < 256 ? leaves : 256) | 1) : splits * cg;
+  l.pitch = (cg / 2) | 1;
+  l.bytes = (GN_GROUP_THREADS + 2ll * cg + l.part) * 8 + 4ll * HW * l.pitch;
+  return l;
 }
 
-template <int V>
-struct alignas(V * 2) BfVec {
-  __nv_bfloat16 v[V];
-};
+__device__ __forceinline__ float2 warp_sum2(float2 v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  return v;
+}
 
-template <int V>
-__global__ void __launch_bounds__(GN_SMALL_THREADS)
-gn_cl_small_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int HW, int C, int cg, float eps, const void* gamma,
-                   const void* beta, int params_bf16, const __nv_bfloat16* __restrict__ shift, long long shift_pitch, int act) {
+template <bool CF>
+__global__ void __launch_bounds__(GN_GROUP_THREADS)
+gn_cl_group_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, int HW, int C, int cg, int splits, float eps,
+                   const void* gamma, const void* beta, int params_bf16, const __nv_bfloat16* __restrict__ shift, long long shift_pitch,
+                   int act) {
   allow_successor();
   wait_for_predecessor();
-  extern __shared__ __align__(16) uint8_t gn_smem[];
-  __shared__ float red[GN_SMALL_THREADS / 32];
-  BfVec<V>* held = reinterpret_cast<BfVec<V>*>(gn_smem);
-  const int g = blockIdx.x, n = blockIdx.y, nv = cg / V, total = HW * nv;
+  extern __shared__ __align__(16) float2 gn_smem[];
+  constexpr int T = GN_GROUP_THREADS;
+  const GroupLayout lay = group_layout(CF, HW, cg, splits);
+  const int W = cg >> 1, P = lay.pitch, total = HW * W;
+  float2 *red = gn_smem, *ab = red + T, *ch = ab + cg, *part = ch + cg;
+  uint32_t* held = reinterpret_cast<uint32_t*>(part + lay.part);
+  const int g = blockIdx.x, n = blockIdx.y, tid = threadIdx.x;
   const __nv_bfloat16* sh = shift != nullptr ? shift + n * shift_pitch + g * cg : nullptr;
-  const long long base = static_cast<long long>(n) * HW * C + g * cg;
-  // vector i is number i % nv of pixel i / nv; a thread walks i in steps of the block without a division per step
-  const int step_pix = GN_SMALL_THREADS / nv, step_v = GN_SMALL_THREADS % nv;
-  const int pix0 = threadIdx.x / nv, v0 = threadIdx.x % nv;
-  float s = 0.0f;
+  const long long base = (static_cast<long long>(n) * HW * C + g * cg) >> 1, row_words = C >> 1;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(x) + base;
+  uint32_t* dst = reinterpret_cast<uint32_t*>(y) + base;
+  // word i is number i % W of pixel i / W; a thread walks i in steps of the block without a division per step
+  const int step_pix = T / W, step_w = T % W;
+  const int pix0 = tid / W, w0 = tid % W;
   {
-    int pix = pix0, v = v0;
-    for (int i = threadIdx.x; i < total; i += 4 * GN_SMALL_THREADS) {
-      BfVec<V> r[4];
-      int vv[4];
+    int pix = pix0, w = w0;
+    for (int i = tid; i < total; i += 8 * T) {
+      uint32_t r[8];
+      int at[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        vv[u] = v;
-        if (i + u * GN_SMALL_THREADS < total) r[u] = *reinterpret_cast<const BfVec<V>*>(x + base + static_cast<long long>(pix) * C + v * V);
+      for (int u = 0; u < 8; ++u) {
+        at[u] = pix * P + w;
+        if (i + u * T < total) r[u] = src[pix * row_words + w];
         pix += step_pix;
-        v += step_v;
-        if (v >= nv) { v -= nv; ++pix; }
+        w += step_w;
+        if (w >= W) { w -= W; ++pix; }
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (i + u * GN_SMALL_THREADS < total) {
-          held[i + u * GN_SMALL_THREADS] = r[u];
-#pragma unroll
-          for (int j = 0; j < V; ++j) s += __bfloat162float(r[u].v[j]) + (sh != nullptr ? __bfloat162float(sh[vv[u] * V + j]) : 0.0f);
+      for (int u = 0; u < 8; ++u)
+        if (i + u * T < total) held[at[u]] = r[u];
+    }
+  }
+  __syncthreads();
+  const float count = static_cast<float>(cg) * static_cast<float>(HW);
+  if (!CF) {
+    const int rows_per_pass = 256 / (C >> 3), per = (HW + splits - 1) / splits;
+    for (int task = tid; task < splits * W; task += T) {
+      const int s = task / W, cw = task - s * W;
+      const int row0 = s * per, row1 = min(HW, row0 + per);
+      float2 t0 = make_float2(0.0f, 0.0f), t1 = t0;
+      for (int r = 0; r < min(rows_per_pass, per); ++r) {
+        float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+        for (int row = row0 + r; row < row1; row += rows_per_pass) {
+          const float2 f = unpack_bf16x2(held[row * P + cw]);
+          s0.x += f.x;
+          s1.x += f.y;
+          s0.y += f.x * f.x;
+          s1.y += f.y * f.y;
         }
+        t0.x += s0.x;
+        t0.y += s0.y;
+        t1.x += s1.x;
+        t1.y += s1.y;
       }
+      part[s * cg + 2 * cw] = t0;
+      part[s * cg + 2 * cw + 1] = t1;
+    }
+    __syncthreads();
+    group_channel_sums(part, splits, cg, cg, red, ch);
+    const float2 mr = group_stats(ch, cg, sh, count, eps, red);
+    for (int j = tid; j < cg; j += T) ab[j] = group_coef(mr, gamma, beta, params_bf16, g * cg + j, sh, j);
+  } else {
+    const int vec = HW % 8 == 0 ? 8 : 1, leaves = min(256, HW / vec), LP = leaves | 1;
+    const int warp = tid >> 5, lane = tid & 31;
+    for (int c0 = 0; c0 < cg; c0 += GN_LEAF_CHANNELS) {
+      for (int task = tid; task < leaves * (GN_LEAF_CHANNELS / 2); task += T) {
+        const int k = task % (GN_LEAF_CHANNELS / 2), t = task / (GN_LEAF_CHANNELS / 2), cw = (c0 >> 1) + k;
+        if (cw >= W) continue;
+        float2 s0 = make_float2(0.0f, 0.0f), s1 = s0, add = s0;
+        if (sh != nullptr) add = make_float2(__bfloat162float(sh[2 * cw]), __bfloat162float(sh[2 * cw + 1]));
+        for (int i = t * vec; i < HW; i += 256 * vec) {
+#pragma unroll 8
+          for (int j = 0; j < vec; ++j) {
+            float2 f = unpack_bf16x2(held[(i + j) * P + cw]);
+            if (sh != nullptr) f = make_float2(f.x + add.x, f.y + add.y);
+            s0.x += f.x;
+            s0.y = fmaf(f.x, f.x, s0.y);
+            s1.x += f.y;
+            s1.y = fmaf(f.y, f.y, s1.y);
+          }
+        }
+        part[2 * k * LP + t] = s0;
+        part[(2 * k + 1) * LP + t] = s1;
+      }
+      __syncthreads();
+      if (c0 + warp < cg) {
+        float2 keep = make_float2(0.0f, 0.0f);
+        for (int v = 0; v * 32 < leaves; ++v) {
+          const int t = v * 32 + lane;
+          const float2 sum = warp_sum2(t < leaves ? part[warp * LP + t] : make_float2(0.0f, 0.0f));
+          if (lane == v) keep = sum;
+        }
+        keep = warp_sum2(keep);
+        if (lane == 0) ch[c0 + warp] = keep;
+      }
+      __syncthreads();
+    }
+    if (tid == 0) {
+      float2 t = make_float2(0.0f, 0.0f);
+      for (int j = 0; j < cg; ++j) {
+        t.x += ch[j].x;
+        t.y += ch[j].y;
+      }
+      red[0] = t;
+    }
+    __syncthreads();
+    const float2 t = red[0];
+    const float mean = t.x / count;
+    const float var = fmaxf(t.y / count - mean * mean, 0.0f);
+    const float rstd = rsqrtf(var + eps);
+    for (int j = tid; j < cg; j += T) {
+      const int c = g * cg + j;
+      const float ga = gamma != nullptr ? param_at(gamma, params_bf16, c) : 1.0f, be = beta != nullptr ? param_at(beta, params_bf16, c) : 0.0f;
+      const float a = rstd * ga, b = be - mean * rstd * ga;
+      ab[j] = make_float2(a, sh != nullptr ? fmaf(__bfloat162float(sh[j]), a, b) : b);
     }
   }
-  const float count = static_cast<float>(HW) * cg;
-  const float mean = cta_sum(s, red) / count;
-  s = 0.0f;
-  int v = v0;
-  for (int i = threadIdx.x; i < total; i += GN_SMALL_THREADS) {
-    const BfVec<V> r = held[i];
-#pragma unroll
-    for (int j = 0; j < V; ++j) {
-      const float d = __bfloat162float(r.v[j]) + (sh != nullptr ? __bfloat162float(sh[v * V + j]) : 0.0f) - mean;
-      s += d * d;
+  __syncthreads();
+  int pix = pix0, w = w0;
+  for (int i = tid; i < total; i += T) {
+    const float2 f = unpack_bf16x2(held[pix * P + w]);
+    const float4 k = *reinterpret_cast<const float4*>(ab + 2 * w);
+    float z0 = fmaf(f.x, k.x, k.y), z1 = fmaf(f.y, k.z, k.w);
+    if (act) {
+      z0 = z0 / (1.0f + __expf(-z0));
+      z1 = z1 / (1.0f + __expf(-z1));
     }
-    v += step_v;
-    if (v >= nv) v -= nv;
-  }
-  const float rstd = rsqrtf(cta_sum(s, red) / count + eps);
-  int pix = pix0;
-  v = v0;
-  for (int i = threadIdx.x; i < total; i += GN_SMALL_THREADS) {
-    const BfVec<V> r = held[i];
-    BfVec<V> o;
-#pragma unroll
-    for (int j = 0; j < V; ++j) {
-      const int c = g * cg + v * V + j;
-      const float a = rstd * param_at(gamma, params_bf16, c);
-      const float d = __bfloat162float(r.v[j]) + (sh != nullptr ? __bfloat162float(sh[v * V + j]) : 0.0f) - mean;
-      const float z = d * a + (beta != nullptr ? param_at(beta, params_bf16, c) : 0.0f);
-      o.v[j] = __float2bfloat16(act ? z / (1.0f + __expf(-z)) : z);
-    }
-    *reinterpret_cast<BfVec<V>*>(y + base + static_cast<long long>(pix) * C + v * V) = o;
+    dst[pix * row_words + w] = pack_bf16x2(z0, z1);
     pix += step_pix;
-    v += step_v;
-    if (v >= nv) { v -= nv; ++pix; }
+    w += step_w;
+    if (w >= W) { w -= W; ++pix; }
   }
 }
 
 }  // namespace cln
 }  // namespace mdb
 
-// x, y: bf16 [N, HW, C] contiguous, C / groups even; gamma / beta: [C] bf16 (params_bf16 = 1) or fp32, may be null; shift: bf16 [N, C] or
-// null, added to x first. The values of a group (HW * C / groups) must fit into 200 KB: error 3705 otherwise.
-extern "C" int mdb_gn_cl_small(const void* x, void* y, int N, int HW, int C, int groups, float eps, const void* gamma, const void* beta,
-                               int params_bf16, const void* shift, long long shift_pitch, int act, void* stream) {
+constexpr int kGnGroupElsewhere = 3705;  // `mdb_gn_cl_group`: another path is the faster one, or the only one
+
+// x, y: bf16 [N, HW, C] contiguous; gamma / beta: [C] bf16 (params_bf16 = 1) or fp32, may be null; shift: bf16 [N, C] or null, added to x
+// first; splits: the strips of `mdb_gn_cl_sums` for this size. Code 3705 (nothing was launched) where the kernel does not take the
+// call; this is the only place where that is decided.
+extern "C" int mdb_gn_cl_group(const void* x, void* y, int N, int HW, int C, int groups, int splits, float eps, const void* gamma,
+                               const void* beta, int params_bf16, const void* shift, long long shift_pitch, int act, void* stream) {
   using namespace mdb::cln;
   if (N <= 0 || HW <= 0) return 0;
-  if (groups <= 0 || C % groups || N > 65535) return 3704;
+  if (groups <= 0 || C % groups || (C & 7) || splits < 1) return 3704;
   const int cg = C / groups;
-  if ((cg & 1) || static_cast<long long>(HW) * cg * 2 > 200 * 1024 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15))
-    return 3705;
-  const size_t smem = static_cast<size_t>(HW) * cg * 2;
-  const auto launch = [&](auto kern) {
-    if (smem > 40 * 1024) MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    return static_cast<int>(mdb::launch_overlapped(kern, dim3(groups, N), GN_SMALL_THREADS, smem, static_cast<cudaStream_t>(stream),
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), HW, C, cg, eps, gamma, beta, params_bf16,
-        static_cast<const __nv_bfloat16*>(shift), shift_pitch, act));
-  };
-  // a group starts at a multiple of cg channels of rows that are multiples of cg: the load is as wide as cg allows
-  return cg % 8 == 0 ? launch(gn_cl_small_kernel<8>) : cg % 4 == 0 ? launch(gn_cl_small_kernel<4>) : launch(gn_cl_small_kernel<2>);
+  if ((cg & 1) || N > 65535 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15)) return kGnGroupElsewhere;
+  const bool cf = C > 2048;
+  if (cf) {
+    // whatever fits is 2.2 to 18 times as fast (1 to 8 samples of 4^2 to 32^2 x 2560); from 4096 pixels on the channels-first kernels
+    // may cut a channel into several sums
+    if (HW >= 4096) return kGnGroupElsewhere;
+  } else {
+    // Three launches / one, 320 to 1920 channels in 32 groups, 4^2 to 40^2 pixels: up to 30 KB a group 1.05 to 1.8 at 32 and 64 CTAs, from 31 KB
+    // on 0.91 to 1.07; up to 16 KB 0.99 to 1.5 at 128 and 256 CTAs, from 20 KB on 0.67 to 1.04; one CTA of 40 KB 0.76, 2048 of 20 KB 0.83.
+    const long long ctas = static_cast<long long>(groups) * N, most = ctas >= 32 && ctas <= 74 ? 30 * 1024 : ctas <= 256 ? 16 * 1024 : 0;
+    if (static_cast<long long>(HW) * cg * 2 > most) return kGnGroupElsewhere;
+  }
+  const GroupLayout lay = group_layout(cf, HW, cg, splits);
+  if (lay.bytes > GN_GROUP_SMEM) return kGnGroupElsewhere;
+  auto kern = cf ? gn_cl_group_kernel<true> : gn_cl_group_kernel<false>;
+  const int smem = static_cast<int>(lay.bytes);
+  if (smem > 40 * 1024) MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GN_GROUP_SMEM));
+  return static_cast<int>(mdb::launch_overlapped(kern, dim3(groups, N), GN_GROUP_THREADS, static_cast<size_t>(smem),
+      static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), HW, C, cg, splits, eps, gamma,
+      beta, params_bf16, static_cast<const __nv_bfloat16*>(shift), shift_pitch, act));
 }
 
 // partial: fp32 [N, splits, C, 2] from mdb_gn_cl_sums; gamma / beta: [C] bf16 (params_bf16 = 1) or fp32, may be null;

@@ -39,7 +39,7 @@ int mdb_rms_rope_fwd(const void*, long long, void*, long long, long long, const 
                      int, int, float, float*, int, void*);
 int mdb_gn_cl_sums(const void*, const void*, const float*, const float*, float*, int, int, int, int, void*);
 // weak: over a kernel library without it the norm takes the three launches
-__attribute__((weak)) int mdb_gn_cl_small(const void*, void*, int, int, int, int, float, const void*, const void*, int, const void*, long long, int, void*);
+__attribute__((weak)) int mdb_gn_cl_group(const void*, void*, int, int, int, int, int, float, const void*, const void*, int, const void*, long long, int, void*);
 int mdb_gn_cl_fold_fwd(const float*, int, int, int, int, float, float, const void*, const void*, int, float*, float*, float*,
                        float*, const void*, long long, void*);
 int mdb_gn_cl_apply(const void*, const void*, void*, const float*, const float*, const float*, const float*, const float*, int,
@@ -61,7 +61,7 @@ PyObject* g_error = nullptr;     // ops._lib.KernelError
 PyObject* g_plan = nullptr;      // ops.kernels.gemm_plan
 
 constexpr int kCtasTarget = 148 * 4;
-constexpr int64_t kGnSmallBytes = 40 * 1024, kGnSmallMost = 200 * 1024;
+constexpr int kGnGroupElsewhere = 3705;
 
 PyObject* not_implemented() { Py_RETURN_NOTIMPLEMENTED; }
 
@@ -462,15 +462,13 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int splits = static_cast<int>(std::max<int64_t>(1, std::min((kCtasTarget + N - 1) / N, (HW + 15) / 16)));
   const int in = static_cast<int>(N), ic = static_cast<int>(C), ihw = static_cast<int>(HW), ig = static_cast<int>(groups);
   Tensor y;
-  // `ops.conv.gn_small`: up to 40 KB a group one launch is faster than three; beyond 2048 channels the three do not take x
-  const int64_t cg = C / groups;
-  if (mdb_gn_cl_small != nullptr && cg % 2 == 0 && HW * cg * 2 <= (C > 2048 ? kGnSmallMost : kGnSmallBytes)) {
+  if (mdb_gn_cl_group != nullptr) {
     const int rc = unlocked([&] {
       y = at::empty_like(x);
-      return mdb_gn_cl_small(x.data_ptr(), y.data_ptr(), in, ihw, ic, ig, static_cast<float>(eps), data(gamma), data(beta),
+      return mdb_gn_cl_group(x.data_ptr(), y.data_ptr(), in, ihw, ic, ig, splits, static_cast<float>(eps), data(gamma), data(beta),
                              gamma || beta ? 1 : 0, data(shift), shift ? shift->stride(0) : 0, act, stream());
     });
-    return done(rc, "mdb_gn_cl_small", y);
+    if (rc != kGnGroupElsewhere) return done(rc, "mdb_gn_cl_group", y);
   }
   if (C > 2048) return not_implemented();
   const int rc = unlocked([&] {

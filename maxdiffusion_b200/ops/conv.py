@@ -55,8 +55,8 @@ def _declare(L):
   c_float = ctypes.c_float
   L.mdb_gn_cl_fold_fwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_int] + [c_void_p] * 5 + [c_ll, c_void_p]
   L.mdb_gn_cl_fold_fwd.restype = c_int
-  L.mdb_gn_cl_small.argtypes = [c_void_p, c_void_p] + [c_int] * 4 + [c_float, c_void_p, c_void_p, c_int, c_void_p, c_ll, c_int, c_void_p]
-  L.mdb_gn_cl_small.restype = c_int
+  L.mdb_gn_cl_group.argtypes = [c_void_p, c_void_p] + [c_int] * 5 + [c_float, c_void_p, c_void_p, c_int, c_void_p, c_ll, c_int, c_void_p]
+  L.mdb_gn_cl_group.restype = c_int
   L.mdb_gn_cl_fold_bwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int] + [c_void_p] * 8
   L.mdb_gn_cl_fold_bwd.restype = c_int
 
@@ -816,22 +816,20 @@ def _gn_params(gamma, beta):
   return (None if gamma is None else conv(gamma)), (None if beta is None else conv(beta)), int(bf16)
 
 
-def gn_small(C: int, HW: int, groups: int) -> bool:
-  """Whether GroupNorm without a backward takes the kernel that holds a group's values in shared memory: where that is faster than
-  the three launches (`csrc/cl_norm.cu`), and up to 200 KB a group beyond their 2048 channels, where the alternative is a copy to
-  channels-first memory (2 x 8^2 x 2560 44 / 4.7 us, 2 x 16^2 x 2560 50 / 10.4)."""
-  cg = C // groups
-  return C % groups == 0 and cg % 2 == 0 and HW * cg * 2 <= (200 if C > 2048 else 40) * 1024
+_GN_ELSEWHERE = 3705  # `mdb_gn_cl_group`: not a call for this kernel, nothing was launched
 
 
-def group_norm_cl_small(x3: torch.Tensor, groups: int, gamma, beta, eps: float, act: bool, shift=None):
-  """act(GroupNorm(x + shift)) of x3 [N, HW, C] bf16 contiguous in one launch; sizes for which `gn_small` holds."""
+def group_norm_cl_group(x3: torch.Tensor, groups: int, gamma, beta, eps: float, act: bool, shift=None):
+  """act(GroupNorm(x + shift)) of x3 [N, HW, C] bf16 contiguous in one launch, with the bits of `group_norm_cl_fwd` (up to 2048
+  channels) or of the channels-first kernels (beyond). None where the kernel does not take the call (`csrc/cl_norm.cu`)."""
   N, HW, C = x3.shape
   y = torch.empty_like(x3)
   g, bt, bf16 = _gn_params(gamma, beta)
-  rc = _lib.lib().mdb_gn_cl_small(_lib.ptr(x3), _lib.ptr(y), N, HW, C, groups, float(eps), _lib.ptr(g), _lib.ptr(bt), bf16, _lib.ptr(shift),
-                                  shift.stride(0) if shift is not None else 0, int(act), _lib.stream())
-  _lib.check(rc, "mdb_gn_cl_small")
+  rc = _lib.lib().mdb_gn_cl_group(_lib.ptr(x3), _lib.ptr(y), N, HW, C, groups, _gn_splits(N, HW), float(eps), _lib.ptr(g), _lib.ptr(bt), bf16,
+                                  _lib.ptr(shift), shift.stride(0) if shift is not None else 0, int(act), _lib.stream())
+  if rc == _GN_ELSEWHERE:
+    return None
+  _lib.check(rc, "mdb_gn_cl_group")
   return y
 
 

@@ -725,12 +725,12 @@ def group_norm(x, groups: int, gamma=None, beta=None, eps: float = 1e-6, act: bo
       if r is not NotImplemented:
         return r
       N, C, H, W = x.shape
-      small = OC.gn_small(C, H * W, groups) and x.numel() > 0
-      if small or C <= 2048:
-        x3 = x.permute(0, 2, 3, 1).view(N, H * W, C)
-        x3 = x3.clone() if x.data_ptr() % 16 else x3  # 16-byte loads
-        y3 = (OC.group_norm_cl_small(x3, groups, gamma, beta, eps, act, shift) if small else
-              OC.group_norm_cl_fwd(x3, groups, gamma, beta, eps, act, shift)[0])
+      x3 = x.permute(0, 2, 3, 1).view(N, H * W, C)
+      x3 = x3.clone() if x.data_ptr() % 16 else x3  # 16-byte loads
+      y3 = OC.group_norm_cl_group(x3, groups, gamma, beta, eps, act, shift) if x.numel() > 0 else None
+      if y3 is None and C <= 2048:
+        y3 = OC.group_norm_cl_fwd(x3, groups, gamma, beta, eps, act, shift)[0]
+      if y3 is not None:
         return y3.view(N, H, W, C).permute(0, 3, 1, 2)
     elif x.shape[1] <= 2048:
       if shift is not None:
