@@ -758,10 +758,10 @@ extern "C" int mdb_gn_cl_group(const void* x, void* y, int N, int HW, int C, int
 }
 
 // partial: fp32 [N, splits, C, 2] from mdb_gn_cl_sums; gamma / beta: [C] bf16 (params_bf16 = 1) or fp32, may be null;
-// a, b: fp32 [N, C]; mean, rstd: fp32 [N, groups]. count = pixels * channels per group. shift: bf16 [N, C] or null.
-extern "C" int mdb_gn_cl_fold_fwd(const float* partial, int N, int splits, int C, int groups, float count, float eps,
-                                  const void* gamma, const void* beta, int params_bf16, float* a, float* b, float* mean,
-                                  float* rstd, const void* shift, long long shift_pitch, void* stream) {
+// a, b: fp32 [N, C]; mean, rstd: fp32 [N, groups]. count = pixels * channels per group. shift: bf16 [N, C] or null, added to x.
+extern "C" int mdb_gn_cl_fold_shift_fwd(const float* partial, int N, int splits, int C, int groups, float count, float eps,
+                                        const void* gamma, const void* beta, int params_bf16, float* a, float* b, float* mean,
+                                        float* rstd, const void* shift, long long shift_pitch, void* stream) {
   if (N <= 0) return 0;
   if (groups <= 0 || C % groups || splits < 1 || C > 8192) return 3704;
   if (N > 65535) return 3704;
@@ -772,6 +772,12 @@ extern "C" int mdb_gn_cl_fold_fwd(const float* partial, int N, int splits, int C
       reinterpret_cast<const float2*>(partial), splits, C, groups, count, eps, gamma, beta, params_bf16, a, b, mean, rstd,
       static_cast<const __nv_bfloat16*>(shift), shift_pitch);
   return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int mdb_gn_cl_fold_fwd(const float* partial, int N, int splits, int C, int groups, float count, float eps,
+                                  const void* gamma, const void* beta, int params_bf16, float* a, float* b, float* mean,
+                                  float* rstd, void* stream) {
+  return mdb_gn_cl_fold_shift_fwd(partial, N, splits, C, groups, count, eps, gamma, beta, params_bf16, a, b, mean, rstd, nullptr, 0, stream);
 }
 
 // ca, cb, cc, dgamma_n, dbeta_n: fp32 [N, C] (the caller sums the last two over N).

@@ -38,10 +38,11 @@ int mdb_geglu_fwd(const void*, void*, long long, int, void*);
 int mdb_rms_rope_fwd(const void*, long long, void*, long long, long long, const void*, int, const float*, const float*, int, int,
                      int, int, float, float*, int, void*);
 int mdb_gn_cl_sums(const void*, const void*, const float*, const float*, float*, int, int, int, int, void*);
-// weak: over a kernel library without it the norm takes the three launches
+// Weak: over a kernel library without it the norm takes the three launches, whose entry points have kept their arguments. An entry
+// point whose arguments change gets another name, so that an object of one kind never calls a library of another.
 __attribute__((weak)) int mdb_gn_cl_group(const void*, void*, int, int, int, int, int, float, const void*, const void*, int, const void*, long long, int, void*);
 int mdb_gn_cl_fold_fwd(const float*, int, int, int, int, float, float, const void*, const void*, int, float*, float*, float*,
-                       float*, const void*, long long, void*);
+                       float*, void*);
 int mdb_gn_cl_apply(const void*, const void*, void*, const float*, const float*, const float*, const float*, const float*, int,
                     int, int, int, void*);
 int mdb_conv_igemm(const void*, const void*, const void*, void*, const void*, const void*, const long long*, const long long*,
@@ -439,14 +440,14 @@ PyObject* py_rms_rope(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// group_norm_cl(x, groups, gamma, beta, eps, act, shift): x [N,C,H,W] in channels-last memory, shift [N,C] or None
+// group_norm_cl(x, groups, gamma, beta, eps, act): x [N,C,H,W] in channels-last memory
 PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 7 || !THPVariable_Check(a[0])) return not_implemented();
+  if (n != 6 || !THPVariable_Check(a[0])) return not_implemented();
   const Tensor& x = THPVariable_Unpack(a[0]);
-  const Tensor *gamma, *beta, *shift;
+  const Tensor *gamma, *beta;
   const int64_t groups = PyLong_AsLong(a[1]);
-  if (!opt_tensor(a[2], gamma) || !opt_tensor(a[3], beta) || !opt_tensor(a[6], shift)) return not_implemented();
+  if (!opt_tensor(a[2], gamma) || !opt_tensor(a[3], beta)) return not_implemented();
   const double eps = PyFloat_AsDouble(a[4]);
   const bool act = a[5] == Py_True;
   if (PyErr_Occurred()) return nullptr;
@@ -457,8 +458,6 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (groups <= 0 || C % groups || (C & 7) || N > 65535 || HW > INT_MAX) return not_implemented();
   for (const Tensor* p : {gamma, beta})
     if (p && (!bf16(*p) || !p->is_contiguous() || p->numel() != C)) return not_implemented();
-  if (shift && (!bf16(*shift) || shift->dim() != 2 || shift->size(0) != N || shift->size(1) != C || shift->stride(1) != 1))
-    return not_implemented();
   const int splits = static_cast<int>(std::max<int64_t>(1, std::min((kCtasTarget + N - 1) / N, (HW + 15) / 16)));
   const int in = static_cast<int>(N), ic = static_cast<int>(C), ihw = static_cast<int>(HW), ig = static_cast<int>(groups);
   Tensor y;
@@ -466,7 +465,7 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int rc = unlocked([&] {
       y = at::empty_like(x);
       return mdb_gn_cl_group(x.data_ptr(), y.data_ptr(), in, ihw, ic, ig, splits, static_cast<float>(eps), data(gamma), data(beta),
-                             gamma || beta ? 1 : 0, data(shift), shift ? shift->stride(0) : 0, act, stream());
+                             gamma || beta ? 1 : 0, nullptr, 0, act, stream());
     });
     if (rc != kGnGroupElsewhere) return done(rc, "mdb_gn_cl_group", y);
   }
@@ -478,13 +477,12 @@ PyObject* py_group_norm_cl(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor work = at::empty({sums + 2 * N * C + 2 * N * groups}, f);
     float* partial = work.data_ptr<float>();
     float *ca = partial + sums, *cb = ca + N * C, *mean = cb + N * C, *rstd = mean + N * groups;
-    y = at::empty_like(x);
+    if (!y.defined()) y = at::empty_like(x);
     void* st = stream();
     int err = mdb_gn_cl_sums(x.data_ptr(), nullptr, nullptr, nullptr, partial, in, ihw, ic, splits, st);
     if (err == 0)
       err = mdb_gn_cl_fold_fwd(partial, in, splits, ic, ig, static_cast<float>(HW * (C / groups)), static_cast<float>(eps),
-                               data(gamma), data(beta), gamma || beta ? 1 : 0, ca, cb, mean, rstd, data(shift),
-                               shift ? shift->stride(0) : 0, st);
+                               data(gamma), data(beta), gamma || beta ? 1 : 0, ca, cb, mean, rstd, st);
     if (err == 0)
       err = mdb_gn_cl_apply(x.data_ptr(), nullptr, y.data_ptr(), ca, cb, nullptr, nullptr, nullptr, in, ihw, ic, act, st);
     return err;

@@ -53,8 +53,10 @@ def _declare(L):
   L.mdb_gn_cl_apply.argtypes = [c_void_p] * 8 + [c_int] * 4 + [c_void_p]
   L.mdb_gn_cl_apply.restype = c_int
   c_float = ctypes.c_float
-  L.mdb_gn_cl_fold_fwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_int] + [c_void_p] * 5 + [c_ll, c_void_p]
+  L.mdb_gn_cl_fold_fwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p, c_int] + [c_void_p] * 5
   L.mdb_gn_cl_fold_fwd.restype = c_int
+  L.mdb_gn_cl_fold_shift_fwd.argtypes = L.mdb_gn_cl_fold_fwd.argtypes + [c_ll, c_void_p]
+  L.mdb_gn_cl_fold_shift_fwd.restype = c_int
   L.mdb_gn_cl_group.argtypes = [c_void_p, c_void_p] + [c_int] * 5 + [c_float, c_void_p, c_void_p, c_int, c_void_p, c_ll, c_int, c_void_p]
   L.mdb_gn_cl_group.restype = c_int
   L.mdb_gn_cl_fold_bwd.argtypes = [c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int] + [c_void_p] * 8
@@ -844,10 +846,13 @@ def group_norm_cl_fwd(x3: torch.Tensor, groups: int, gamma, beta, eps: float, ac
   mean = torch.empty((N, groups), device=x3.device, dtype=torch.float32)
   rstd = torch.empty_like(mean)
   g, bt, bf16 = _gn_params(gamma, beta)
-  rc = _lib.lib().mdb_gn_cl_fold_fwd(_lib.ptr(partial), N, partial.shape[1], C, groups, float(HW * (C // groups)), float(eps),
-                                     _lib.ptr(g), _lib.ptr(bt), bf16, _lib.ptr(a), _lib.ptr(b), _lib.ptr(mean), _lib.ptr(rstd),
-                                     _lib.ptr(shift), shift.stride(0) if shift is not None else 0, _lib.stream())
-  _lib.check(rc, "mdb_gn_cl_fold_fwd")
+  args = (_lib.ptr(partial), N, partial.shape[1], C, groups, float(HW * (C // groups)), float(eps), _lib.ptr(g), _lib.ptr(bt), bf16,
+          _lib.ptr(a), _lib.ptr(b), _lib.ptr(mean), _lib.ptr(rstd))
+  if shift is None:
+    _lib.check(_lib.lib().mdb_gn_cl_fold_fwd(*args, _lib.stream()), "mdb_gn_cl_fold_fwd")
+  else:
+    rc = _lib.lib().mdb_gn_cl_fold_shift_fwd(*args, _lib.ptr(shift), shift.stride(0), _lib.stream())
+    _lib.check(rc, "mdb_gn_cl_fold_shift_fwd")
   return _gn_apply(x3, None, a, b, None, None, None, act), a, b, mean, rstd
 
 

@@ -721,7 +721,7 @@ def group_norm(x, groups: int, gamma=None, beta=None, eps: float = 1e-6, act: bo
     if _direct(x, gamma, beta, shift):
       if shift is not None and (shift.dtype != torch.bfloat16 or shift.shape != x.shape[:2] or shift.stride(1) != 1):
         return group_norm(x + shift[:, :, None, None], groups, gamma, beta, eps, act)
-      r = _lib.host_ops().group_norm_cl(x, groups, gamma, beta, eps, act, shift)
+      r = _lib.host_ops().group_norm_cl(x, groups, gamma, beta, eps, act) if shift is None else NotImplemented
       if r is not NotImplemented:
         return r
       N, C, H, W = x.shape
