@@ -94,7 +94,8 @@ class Attention(nn.Module):
         q, (k, v) = OF.linear(x, self.to_q.weight), OF.linear_group(ctx, (self.to_k.weight, self.to_v.weight))
     else:
       q, k, v = self.to_q(x), self.to_k(ctx), self.to_v(ctx)
-    q, k, v = (t.view(B, t.shape[1], self.heads, t.shape[2] // self.heads) for t in (q, k, v))
+    # the batch of each: a context of one sample broadcasts over x's where attention does
+    q, k, v = (t.view(*t.shape[:-1], self.heads, t.shape[-1] // self.heads) for t in (q, k, v))
     return self.to_out[0](OF.attention(q, k, v).reshape(B, S, C), residual=residual)
 
 
