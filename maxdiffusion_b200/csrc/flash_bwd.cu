@@ -77,13 +77,15 @@ struct Params {
   int seg_batches, n_seg, out_rot, out_step;
   int x_len_seg[MAX_SEGMENTS];
   long long o_seg_stride;
-  // DKV pass of one segment: dS is also written out (null: not), see `flash_dq_kernel`
+  // DKV pass of one segment (template DS): dS is also written out, see `flash_dq_kernel`
   uint8_t* ds;
   int ds_blocks;  // blocks of 64 queries per tile row
   DeviceStatus* status;
 };
 
-template <bool DKV, int HD>
+// DS: the DKV pass of one segment that also writes dS. A kernel of its own: as a run-time branch of the DKV pass the addresses and
+// the second life of ds[] put 16 bytes of every DKV launch into local memory (96 registers are all that 640 threads leave).
+template <bool DKV, int HD, bool DS = false>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
   constexpr int D = HD;                        // head_dim: 64 or 128
@@ -297,9 +299,13 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
         lse_r = p.lse[stat_base + x_row];
         delta_r = p.delta[stat_base + x_row];
       }
+      uint8_t* ds_row = nullptr;  // this thread's 32 bytes of the next tile
+      if (DS)
+        ds_row = p.ds + ((static_cast<long long>(batch) * p.H + head) * gridDim.x + blockIdx.x) * p.ds_blocks * DS_TILE_BYTES +
+                 (quarter >> 1) * 8192 + wg * 2048 + ((quarter & 1) * 32 + lane) * 32;
       bool ok = true;
       int i = 0;
-      for (int seg = 0; seg < p.num_segments && ok; ++seg) {
+      for (int seg = 0; seg < (DS ? 1 : p.num_segments) && ok; ++seg) {
         const int nblk = (p.y_len[seg] + BY - 1) / BY;
         for (int jb = 0; jb < nblk; ++jb, ++i) {
           const int b = i % NBUF, use = i / NBUF;
@@ -402,15 +408,14 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ds_ready[b]);
-          if (DKV && p.ds != nullptr) {
+          if (DS) {
             // the warp's 32 rows of 32 bytes in line, eight full lines a store: with rows of 128 bytes (the 128-byte swizzle) every
             // lane met a line of its own, and the stores held the operand reads up (dK, dV at 32760^2 x 4 heads 3.2 -> 4.6 ms)
-            uint8_t* dst = p.ds + (((static_cast<long long>(batch) * p.H + head) * gridDim.x + blockIdx.x) * p.ds_blocks + jb) * DS_TILE_BYTES +
-                           (quarter >> 1) * 8192 + wg * 2048 + ((quarter & 1) * 32 + lane) * 32;
             uint32_t o[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) o[c] = (lane & 4) ? ds[c ^ 4] : ds[c];  // 32-byte swizzle: rows 4-7 of 8 swap their halves
-            store_32b(dst, o);
+            store_32b(ds_row, o);
+            ds_row += DS_TILE_BYTES;
           }
         }
       }
@@ -709,11 +714,13 @@ static int flash_bwd_dkv_launch(const void* q, const void* d_o, const void* k, c
   p.status = status_buffer();
   static bool configured = false;
   if (!configured) {
-    MDB_CHECK_CUDA(cudaFuncSetAttribute(flash_bwd_kernel<true, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<HD>()));
+    for (auto kern : {flash_bwd_kernel<true, HD, false>, flash_bwd_kernel<true, HD, true>})
+      MDB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<HD>()));
     configured = true;
   }
   dim3 grid((kv_len + BX - 1) / BX, H, x_batches);
-  flash_bwd_kernel<true, HD><<<grid, NUM_THREADS, smem_bytes<HD>(), static_cast<cudaStream_t>(stream)>>>(maps, p);
+  const auto kern = p.ds != nullptr ? flash_bwd_kernel<true, HD, true> : flash_bwd_kernel<true, HD, false>;
+  kern<<<grid, NUM_THREADS, smem_bytes<HD>(), static_cast<cudaStream_t>(stream)>>>(maps, p);
   return static_cast<int>(cudaGetLastError());
 }
 
