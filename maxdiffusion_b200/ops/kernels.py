@@ -380,7 +380,11 @@ def flash_bwd_dkv(q, d_o, k, v, lse, delta, scale=None, out_dtype=torch.bfloat16
   return dk, dv
 
 
-_DS_BYTES = 9 << 30  # most of dS that is held at a time: four heads of 32760^2
+_DS_BYTES = 9 << 30      # most of dS that is held at a time: four heads of 32760^2
+_DS_CAPTURED = 1 << 30   # ... inside a captured graph, whose pool keeps it for as long as the graph lives
+_DS_TEMPORARY = 256 << 20  # up to here dS is asked for like any other temporary tensor
+_DS_MARGIN = 1 << 30     # memory that a request for more leaves to others
+_ds_refused: dict = {}   # device -> (bytes, memory in reach) of the last request that was refused or made the allocator flush
 
 
 def flash_ds_chunk(B: int, H: int, Sq: int, Skv: int, limit: int | None = None) -> int:
@@ -397,25 +401,64 @@ def flash_ds_chunk(B: int, H: int, Sq: int, Skv: int, limit: int | None = None) 
   return min(range(1, most + 1), key=lambda n: (cost(n), -n))
 
 
+def _ds_memory(device):
+  """(bytes in reach of a new tensor, how often the allocator had to give back its blocks and try again)."""
+  free = torch.cuda.mem_get_info(device)[0]
+  try:
+    stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
+    return free + stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"], stats["num_alloc_retries"]
+  except (RuntimeError, KeyError):  # an allocator that keeps no such figures
+    return free, 0
+
+
+def _ds_buffer(B: int, H: int, Sq: int, Skv: int, device):
+  """(pairs, buffer for their dS), or (0, None) where dQ is to be a pass of its own. A large buffer is asked for only where the
+  memory is there: a request that the allocator cannot serve makes it give back all its blocks and wait for the device, and one
+  backward per layer would ask. One that was refused, or served that way, is not repeated until there is more memory by its size."""
+  per = -(-Skv // 128) * -(-Sq // 64) * 16384
+  limit, room = _DS_BYTES, None
+  captured = device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+  if captured:
+    limit = min(limit, _DS_CAPTURED)  # the driver is not asked during a capture
+  elif device.index in _ds_refused or flash_ds_chunk(B, H, Sq, Skv) * per > _DS_TEMPORARY:
+    room, retries = _ds_memory(device)
+    limit = min(limit, room - _DS_MARGIN)
+    if device.index in _ds_refused:
+      size, was = _ds_refused[device.index]
+      if room < was + size:
+        limit = min(limit, size - 1)
+      else:
+        _ds_refused.pop(device.index, None)
+  while True:
+    n = flash_ds_chunk(B, H, Sq, Skv, max(limit, 0))
+    if n == 0:
+      return 0, None
+    try:
+      ds = torch.empty(n * per, device=device, dtype=torch.uint8)
+    except torch.OutOfMemoryError:
+      if not captured:
+        _ds_refused[device.index] = (n * per, room if room is not None else _ds_memory(device)[0])
+      limit = n * per // 2
+      continue
+    if room is not None and _ds_memory(device)[1] != retries:
+      _ds_refused[device.index] = (n * per, room)
+    return n, ds
+
+
 def flash_bwd(q, d_o, k, v, lse, delta, scale=None):
   """dQ, dK, dV of attention over one KV segment (bf16): the pass over keys also writes dS, from which dQ is one product. Where
-  dS of a head is too large, or the memory for it is not there, dQ is a pass of its own (`flash_bwd_dq`).
+  dS of a head is too large, or the memory for it is not there, dQ is a pass of its own (`flash_bwd_dq`); the bits are the same.
 
   Both, two passes / dS kept, on a B200: 4 x 1024^2 x 20 heads of 64 147 / 142 us, 4 x 4096^2 x 10 830 / 745, 4 x 4096 x 77 keys x 10
   135 / 109; 4608^2 x 24 heads of 128 719 / 649 us, 32760 x 512 keys x 40 1972 / 1336, 32760^2 x 4 6.02 / 5.25 ms."""
   B, Sq, H, D = q.shape
   Skv = k.shape[1]
   assert D in FLASH_HEAD_DIMS and all(t.stride(-1) == 1 for t in (q, d_o, k, v))
-  n = flash_ds_chunk(B, H, Sq, Skv)
-  ds = None
-  if n:
-    try:
-      ds = torch.empty(n * -(-Skv // 128) * -(-Sq // 64) * 16384, device=q.device, dtype=torch.uint8)
-    except torch.OutOfMemoryError:
-      pass
+  dq, dk, dv = (torch.empty(t.shape, device=q.device, dtype=torch.bfloat16) for t in (q, k, k))  # the results come before dS
+  n, ds = _ds_buffer(B, H, Sq, Skv, q.device)
   if ds is None:
-    return (flash_bwd_dq(q, d_o, [k], [v], lse, delta, scale), *flash_bwd_dkv(q, d_o, k, v, lse, delta, scale))
-  dq, dk, dv = (torch.empty(t.shape, device=q.device, dtype=torch.bfloat16) for t in (q, k, k))
+    flash_bwd_dq(q, d_o, [k], [v], lse, delta, scale, dq=dq)
+    return (dq, *flash_bwd_dkv(q, d_o, k, v, lse, delta, scale, dk=dk, dv=dv))
   scale = float(scale if scale is not None else 1.0 / math.sqrt(D))
   dkv, from_ds = _flash_entry("mdb_flash_bwd_dkv_ds", D), _flash_entry("mdb_flash_dq_from_ds", D)
   qs, gs, ks, vs, dqs, dks = (_strides3(t) for t in (q, d_o, k, v, dq, dk))
@@ -461,8 +504,8 @@ def flash_bwd_dkv_stacked(q, d_o, kg, vg, lens, lse, delta, scale=None, dk=None,
   return dk, dv
 
 
-def flash_bwd_dq(q, d_o, k_list, v_list, lse, delta, scale=None, out_dtype=torch.bfloat16):
-  """dQ of the local queries over every KV segment."""
+def flash_bwd_dq(q, d_o, k_list, v_list, lse, delta, scale=None, out_dtype=torch.bfloat16, dq=None):
+  """dQ of the local queries over every KV segment, into `dq` [B,Sq,H,D] (unit head_dim stride) if given."""
   if isinstance(k_list, torch.Tensor):
     k_list, v_list = [k_list], [v_list]
   B, Sq, H, D = q.shape
@@ -470,7 +513,9 @@ def flash_bwd_dq(q, d_o, k_list, v_list, lse, delta, scale=None, out_dtype=torch
   for k, v in zip(k_list, v_list):
     assert k.stride() == k0.stride() and v.stride() == v0.stride() and k.stride(-1) == 1 and v.stride(-1) == 1
   n = len(k_list)
-  dq = torch.empty((B, Sq, H, D), device=q.device, dtype=out_dtype)
+  if dq is None:
+    dq = torch.empty((B, Sq, H, D), device=q.device, dtype=out_dtype)
+  assert dq.shape == (B, Sq, H, D) and dq.dtype == out_dtype and dq.stride(-1) == 1
   kp = (ctypes.c_void_p * n)(*[k.data_ptr() for k in k_list])
   vp = (ctypes.c_void_p * n)(*[v.data_ptr() for v in v_list])
   lens = (ctypes.c_int * n)(*[k.shape[1] for k in k_list])
