@@ -177,9 +177,21 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
       }
       const long long stat_base = (static_cast<long long>(ybatch) * p.H + head) * p.q_len;
       // lse / delta of the streamed query rows ride in the stage. When the rows start on 16-byte boundaries they are
-      // fetched by bulk copies that complete on the stage's barrier; otherwise the lanes copy them by hand.
+      // fetched by bulk copies that complete on the stage's barrier; otherwise the lanes copy them by hand, one block ahead: loads
+      // that the stage waits for cost it a memory latency, and behind the stores of dS a long one. dK, dV, dQ with dS kept, loads in the
+      // stage / ahead: 4097^2 x 40 heads 1539 / 861 us, 14625^2 x 40 17.9 / 10.4 ms (two passes 14.6 / 13.1; 14624^2 10.0).
       const bool stat_bulk = DKV && (p.q_len % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.lse) & 15) == 0) &&
                              ((reinterpret_cast<uintptr_t>(p.delta) & 15) == 0);
+      float next_lse[2] = {0.0f, 0.0f}, next_delta[2] = {0.0f, 0.0f};  // of rows lane and lane + 32 of the next block
+      const auto fetch_stat = [&](int jb) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int q = jb * BY + lane + 32 * h;
+          next_lse[h] = q < p.q_len ? p.lse[stat_base + q] : 0.0f;
+          next_delta[h] = q < p.q_len ? p.delta[stat_base + q] : 0.0f;
+        }
+      };
+      if (DKV && !stat_bulk) fetch_stat(0);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -192,12 +204,11 @@ flash_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
           if (DKV && !stat_bulk) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              const int qi = lane + 32 * h;
-              const int q = jb * BY + qi;
-              st[qi] = (q < p.q_len) ? p.lse[stat_base + q] : 0.0f;
-              st[64 + qi] = (q < p.q_len) ? p.delta[stat_base + q] : 0.0f;
+              st[lane + 32 * h] = next_lse[h];
+              st[64 + lane + 32 * h] = next_delta[h];
             }
             __syncwarp();
+            fetch_stat(jb + 1);
           }
           if (lane == 0) {
             uint8_t* d1 = sy + stage * 2 * Y_TILE_BYTES;
