@@ -382,9 +382,9 @@ def flash_bwd_dkv(q, d_o, k, v, lse, delta, scale=None, out_dtype=torch.bfloat16
 
 _DS_BYTES = 9 << 30      # most of dS that is held at a time: four heads of 32760^2
 _DS_CAPTURED = 1 << 30   # ... inside a captured graph, whose pool keeps it for as long as the graph lives
-_DS_TEMPORARY = 256 << 20  # up to here dS is asked for like any other temporary tensor
+_DS_TEMPORARY = 2 << 30  # up to here dS is asked for like any other temporary tensor
 _DS_MARGIN = 1 << 30     # memory that a request for more leaves to others
-_ds_refused: dict = {}   # device -> (bytes, memory in reach) of the last request that was refused or made the allocator flush
+_ds_refused: dict = {}   # device -> (bytes, memory in reach) at the last request that was refused or made the allocator flush
 
 
 def flash_ds_chunk(B: int, H: int, Sq: int, Skv: int, limit: int | None = None) -> int:
@@ -401,56 +401,78 @@ def flash_ds_chunk(B: int, H: int, Sq: int, Skv: int, limit: int | None = None) 
   return min(range(1, most + 1), key=lambda n: (cost(n), -n))
 
 
-def _ds_memory(device):
-  """(bytes in reach of a new tensor, how often the allocator had to give back its blocks and try again)."""
-  free = torch.cuda.mem_get_info(device)[0]
+def _ds_pays(n: int, B: int, H: int, Sq: int, Skv: int) -> bool:
+  """Whether dS of `n` (batch, head) pairs at a time is faster than a dQ pass. All pairs at once always are: 1.02 to 1.43 times for 1
+  to 4 x 256 to 32760 queries x 77 to 32760 keys x 10 to 40 heads of 64 and 128 (1.02 at 4096^2 x 12 heads, 1.10 at 4096^2 x 40). Parts
+  leave SMs idle at the end of each, and a dK/dV pass that writes dS takes 1.17 times as long: in rounds of CTAs (a row of queries
+  each) the passes over keys cost 1 and 1.17, the dQ pass 0.83, the product over dS 0.43 of the work, a part about 1100 rows. Times as
+  fast, this model / measured: 32760^2 x 40 heads by 4 1.14 / 1.22, 28500^2 x 12 by 5 1.11 / 1.18, 16000^2 x 24 by 4 1.03 / 1.09, 10000^2 x 12
+  by 5 1.03 / 0.97, 22000^2 x 40 by 2 0.94 / 0.83, 8 x 4096^2 x 10 heads of 64 by 10 0.88 / 0.84."""
+  if n == B * H:
+    return True
+  keys, queries = -(-Skv // 128), -(-Sq // 128)
+  rounds = lambda blocks: -(-blocks // _SM_COUNT)
+  two = Sq * rounds(B * H * keys) + 0.83 * Skv * rounds(B * H * queries)
+  part = lambda pairs: Sq * (1.17 * rounds(pairs * keys) + 0.43 * pairs * keys / _SM_COUNT) + 1100 if pairs else 0
+  return 1.03 * B * (H // n * part(n) + part(H % n)) < two
+
+
+def _ds_stats(device) -> tuple[int, int]:
+  """(bytes that the allocator holds and nobody uses, how often it had to give back its blocks and try again)."""
   try:
     stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
-    return free + stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"], stats["num_alloc_retries"]
+    return stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"], stats["num_alloc_retries"]
   except (RuntimeError, KeyError):  # an allocator that keeps no such figures
-    return free, 0
+    return 0, 0
+
+
+def _ds_room(device, enough: int) -> int:
+  """Bytes in reach of a new tensor; where the allocator has `enough` by itself, the driver is not asked (70 us, and milliseconds
+  while the GPU is busy)."""
+  unused = _ds_stats(device)[0]
+  return unused if unused >= enough else unused + torch.cuda.mem_get_info(device)[0]
 
 
 def _ds_buffer(B: int, H: int, Sq: int, Skv: int, device):
   """(pairs, buffer for their dS), or (0, None) where dQ is to be a pass of its own. A large buffer is asked for only where the
   memory is there: a request that the allocator cannot serve makes it give back all its blocks and wait for the device, and one
-  backward per layer would ask. One that was refused, or served that way, is not repeated until there is more memory by its size."""
+  backward per layer would ask. After one that was refused, or served that way, no more than half of it is asked for until there is
+  more memory by its size."""
   per = -(-Skv // 128) * -(-Sq // 64) * 16384
-  limit, room = _DS_BYTES, None
+  limit, room, retries = _DS_BYTES, None, 0
   captured = device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+  size, was = _ds_refused.get(device.index, (1 << 62, 0))
   if captured:
     limit = min(limit, _DS_CAPTURED)  # the driver is not asked during a capture
-  elif device.index in _ds_refused or flash_ds_chunk(B, H, Sq, Skv) * per > _DS_TEMPORARY:
-    room, retries = _ds_memory(device)
-    limit = min(limit, room - _DS_MARGIN)
-    if device.index in _ds_refused:
-      size, was = _ds_refused[device.index]
-      if room < was + size:
-        limit = min(limit, size - 1)
-      else:
-        _ds_refused.pop(device.index, None)
+  elif (want := flash_ds_chunk(B, H, Sq, Skv) * per) > _DS_TEMPORARY or 2 * want >= size:
+    room, retries = _ds_room(device, want + _DS_MARGIN), _ds_stats(device)[1]
+    limit = min(limit, room - _DS_MARGIN if want > _DS_TEMPORARY else limit, size // 2 if room < was + size else limit)
   while True:
     n = flash_ds_chunk(B, H, Sq, Skv, max(limit, 0))
-    if n == 0:
+    if n == 0 or not _ds_pays(n, B, H, Sq, Skv):
       return 0, None
     try:
       ds = torch.empty(n * per, device=device, dtype=torch.uint8)
     except torch.OutOfMemoryError:
       if not captured:
-        _ds_refused[device.index] = (n * per, room if room is not None else _ds_memory(device)[0])
+        _ds_refused[device.index] = (n * per, _ds_room(device, 1 << 62) if room is None else room)
       limit = n * per // 2
       continue
-    if room is not None and _ds_memory(device)[1] != retries:
-      _ds_refused[device.index] = (n * per, room)
+    if room is not None:
+      if _ds_stats(device)[1] != retries:
+        _ds_refused[device.index] = (n * per, room)
+      elif n * per >= size:
+        _ds_refused.pop(device.index, None)
     return n, ds
 
 
 def flash_bwd(q, d_o, k, v, lse, delta, scale=None):
   """dQ, dK, dV of attention over one KV segment (bf16): the pass over keys also writes dS, from which dQ is one product. Where
-  dS of a head is too large, or the memory for it is not there, dQ is a pass of its own (`flash_bwd_dq`); the bits are the same.
+  dS of a head is too large, the memory for it is not there or its parts are too small, dQ is a pass of its own (`flash_bwd_dq`);
+  the bits are the same.
 
-  Both, two passes / dS kept, on a B200: 4 x 1024^2 x 20 heads of 64 147 / 142 us, 4 x 4096^2 x 10 830 / 745, 4 x 4096 x 77 keys x 10
-  135 / 109; 4608^2 x 24 heads of 128 719 / 649 us, 32760 x 512 keys x 40 1972 / 1336, 32760^2 x 4 6.02 / 5.25 ms."""
+  Both, two passes / dS kept, on a B200: 4 x 1024^2 x 20 heads of 64 139 / 131 us, 4 x 4096^2 x 10 835 / 755, 4 x 4096 x 77 keys x 10
+  112 / 93; 4608^2 x 24 heads of 128 720 / 647, 32760 x 512 keys x 40 1546 / 1288 us, 32760^2 x 40 64.9 / 53.3 ms."""
   B, Sq, H, D = q.shape
   Skv = k.shape[1]
   assert D in FLASH_HEAD_DIMS and all(t.stride(-1) == 1 for t in (q, d_o, k, v))

@@ -11,7 +11,7 @@ PER = -(-S // 128) * -(-S // 64) * 16384  # dS of a head
 
 @pytest.fixture
 def world(monkeypatch):
-  """Records requests for memory and launches. `most`: bytes that a request may have; `room`: what `_ds_memory` says."""
+  """Records requests for memory and launches. `most`: bytes that a request may have; `room`: what `_ds_room` says."""
 
   class World:
     most, room, retries, asked, launched = 1 << 60, 1 << 60, 0, [], []
@@ -30,7 +30,9 @@ def world(monkeypatch):
   monkeypatch.setattr(torch, "empty", limited)
   monkeypatch.setattr(K, "_flash_entry", lambda name, d: lambda *args: w.launched.append(name) or 0)
   monkeypatch.setattr(_lib, "stream", lambda: 0)
-  monkeypatch.setattr(K, "_ds_memory", lambda device: (w.room, w.retries), raising=False)
+  monkeypatch.setattr(K, "_ds_room", lambda device, enough: w.room, raising=False)
+  monkeypatch.setattr(K, "_ds_stats", lambda device: (0, w.retries), raising=False)
+  monkeypatch.setattr(K, "_ds_pays", lambda *a: True, raising=False)
   monkeypatch.setattr(K, "_ds_refused", {}, raising=False)
   return w
 
@@ -80,13 +82,13 @@ def test_a_large_buffer_is_asked_for_only_where_the_memory_is(world, monkeypatch
 
 def test_a_request_that_made_the_allocator_flush_is_not_repeated(world, monkeypatch):
   monkeypatch.setattr(K, "_DS_TEMPORARY", 0, raising=False)
-  calls = []
+  world.room = 100 << 30
 
-  def memory(device):  # every other look finds one more flush: the one of the request in between
-    calls.append(device)
-    return 100 << 30, len(calls) // 2
+  def stats(device):  # looked at before a request and after it: it has made the allocator flush
+    world.retries += 1
+    return 0, world.retries
 
-  monkeypatch.setattr(K, "_ds_memory", memory, raising=False)
+  monkeypatch.setattr(K, "_ds_stats", stats, raising=False)
   _backward()
   _backward()
   assert _ds(world)[0] == H * PER and max(_ds(world)[1:], default=0) < H * PER

@@ -17,6 +17,7 @@ def _inputs(B, S, H, D):
 def test_memory_that_does_not_hold_ds(monkeypatch):
   """The process may take 300 MiB more; the results take 35 and dS of all heads 282: refused once, then what fits."""
   monkeypatch.setattr(K, "_ds_refused", {})
+  monkeypatch.setattr(K, "_ds_pays", lambda *a: True)
   args = _inputs(1, 3000, 16, 128)
   want = K.flash_bwd(*args)
   torch.cuda.empty_cache()
@@ -61,4 +62,5 @@ def test_whole_and_in_parts_are_the_same_bits(monkeypatch):
   want = (K.flash_bwd_dq(args[0], args[1], [args[2]], [args[3]], args[4], args[5]), *K.flash_bwd_dkv(*args))
   for pairs in (8, 4, 3, 1):
     monkeypatch.setattr(K, "flash_ds_chunk", lambda *a, n=pairs: n)
+    monkeypatch.setattr(K, "_ds_pays", lambda *a: True)
     assert all(torch.equal(a, b) for a, b in zip(K.flash_bwd(*args), want))

@@ -19,7 +19,7 @@ def test_too_few_heads_at_a_time_are_not_asked_for(monkeypatch):
   monkeypatch.setattr(torch, "empty", lambda n, **kw: asked.append(n))
   monkeypatch.setattr(K, "_ds_refused", {})
   monkeypatch.setattr(K, "_ds_stats", lambda device: (0, 0))
-  monkeypatch.setattr(K, "_ds_room", lambda device: 4 << 30)  # 3 GB for dS: three heads of 22000^2
+  monkeypatch.setattr(K, "_ds_room", lambda device, enough: 4 << 30)  # 3 GB for dS: three heads of 22000^2
   assert K._ds_buffer(1, 40, 22000, 22000, torch.device("cpu")) == (0, None) and asked == []
-  monkeypatch.setattr(K, "_ds_room", lambda device: 5 << 30)  # 4 GB: four
+  monkeypatch.setattr(K, "_ds_room", lambda device, enough: 5 << 30)  # 4 GB: four
   assert K._ds_buffer(1, 40, 22000, 22000, torch.device("cpu"))[0] == 4 and len(asked) == 1
