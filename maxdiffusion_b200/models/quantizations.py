@@ -173,9 +173,13 @@ class Int8Linear(Fp8Linear):
   int8 = True
 
 
+_QUANTIZED_FORWARD = Fp8Linear.forward
+
+
 def is_plain_quantized(m: nn.Module) -> bool:
-  """Whether calling `m` is the quantised product and nothing else, so that it may run in parts."""
-  return type(m) in (Fp8Linear, Int8Linear) and calls_forward_only(m)
+  """Whether calling `m` is the quantised product and nothing else (no subclass, wrapper, hook, or `forward` replaced on the object
+  or its class), so that it may run in parts."""
+  return type(m) in (Fp8Linear, Int8Linear) and type(m).forward is _QUANTIZED_FORWARD and calls_forward_only(m)
 
 
 def get_quantization_mode(config) -> Optional[str]:
