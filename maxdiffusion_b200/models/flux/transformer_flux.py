@@ -214,12 +214,13 @@ class FluxSingleBlock(nn.Module):
       q, k, v = self._qkv(f, rope)
       OF.attention_into(cat[..., :C].unflatten(-1, (H, C // H)), q, k, v)
       return _clip(project_gated_residual(self.proj_out, cat, x, gate))
-    if h.is_cuda and is_plain_quantized(self.qkv_mlp):  # the same on 8-bit operands
+    if h.is_cuda and is_plain_quantized(self.qkv_mlp) and self.qkv_mlp.may_split(h, 3 * C):  # the same on 8-bit operands
       cat = torch.empty((B, S, C + self.hidden), device=h.device, dtype=h.dtype)
       f = self.qkv_mlp.split_gelu(h, 3 * C, cat[..., C:])
       if f is not None:
         OF.attention_into(cat[..., :C].unflatten(-1, (H, C // H)), *self._qkv(f, rope))
         return _clip(project_gated_residual(self.proj_out, cat, x, gate))
+      del cat
     f = self.qkv_mlp(h)
     mlp = f[..., 3 * C:]
     o = OF.attention(*self._qkv(f, rope)).reshape(B, S, C)

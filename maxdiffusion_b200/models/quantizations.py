@@ -123,13 +123,17 @@ class Fp8Linear(nn.Module):
     xq, scale = (K.quantize_int8 if self.int8 else K.quantize_fp8)(x2 if x2.is_contiguous() else x2.contiguous())
     return xq, scale, None if self.bias is None else self.bias.to(torch.bfloat16).contiguous()
 
+  def may_split(self, x, cut: int) -> bool:
+    """Whether `split_gelu` takes these sizes here and now: asked before there is a buffer for its result."""
+    return (self._takes(x) and x.numel() > 0 and 0 < cut < self.out_features and cut % 8 == 0 and not OF.library_mode() and
+            OF._direct(x, self.weight, self.bias))
+
   def split_gelu(self, x, cut: int, out):
     """The first `cut` columns of the product; GELU (tanh form) of the others goes to `out` [..., out_features - cut] (unit inner
     stride, rows of one pitch). None where autograd or a transform is at work, or where the kernel does not take these
     tensors: the caller then uses `forward`."""
     rows = out.view(-1, out.shape[-1]) if out.is_contiguous() else out.flatten(0, -2)
-    if not (self._takes(x) and x.numel() > 0 and 0 < cut < self.out_features and cut % 8 == 0 and not OF.library_mode() and
-            OF._direct(x, self.weight, self.bias, out) and rows.data_ptr() == out.data_ptr() and rows.stride(-1) == 1 and
+    if not (self.may_split(x, cut) and OF._direct(out) and rows.data_ptr() == out.data_ptr() and rows.stride(-1) == 1 and
             rows.stride(0) % 8 == 0 and rows.data_ptr() % 16 == 0):
       return None
     xq, scale, bias = self._operands(x)
