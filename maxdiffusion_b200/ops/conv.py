@@ -484,7 +484,7 @@ def conv2d_nchw(x: torch.Tensor, pk: PackedConv, residual: Optional[torch.Tensor
       pk.n_pad != pk.n_out or not x.is_contiguous(memory_format=torch.channels_last) or x.data_ptr() % 16 or x.numel() == 0):
     return None
   B, _, H, W = x.shape
-  if pk.kind == "conv2d_s2" and (H | W) & 1:
+  if pk.kind == "conv2d_s2" and (H | W) & 1 or (x.stride(0) | x.stride(2) | x.stride(3)) % 8:  # 1 x 1 images may have any strides
     return None
   hit = pk._launches.get((B, H, W))
   if hit is None:
