@@ -14,9 +14,13 @@
 //   - one lane per tile issues both of its products, and every wait sleeps between tries. With a lane per product
 //     (two spinning warps on the first scheduler) the softmax warps there ran 1000 clocks per block behind the others.
 // Together, against four issuing lanes, maximum first, waits that spin: 1 x 4608^2 x 24 heads of 128 236 -> 213 us,
-// 75600^2 x 8 heads of 128 21.9 -> 19.1 ms (under the power cap), 4 x 4096^2 x 10 heads of 64 301 -> 268 us; the same bits.
+// 75600^2 x 8 heads of 128 21.9 -> 19.1 ms (under the power cap), 4 x 4096^2 x 10 heads of 64 301 -> 268 us; the same bits. A lane that
+// issues P V of an item's last block before S of the next item's first costs where an item has two or three blocks: 2 x 4096 x 77 keys
+// 14.7 -> 14.9 us, 4 x 4096 x 77 23.9 -> 24.6, 768^2 x 24 heads of 128 14.4 -> 14.8.
 // 128-key S tiles in a single buffer feed the tensor pipe better but lengthen the chain by more: 3.7 ms where this kernel
-// takes 3.1 (32760^2 x 8 heads). Turns of the two tiles at the exponential unit cost more in hand-overs than they save.
+// takes 3.1 (32760^2 x 8 heads, single launches at full clocks; 3.6 in a loop under the power cap). Turns of the two tiles at
+// the exponential unit cost more in hand-overs than they save. At 8192^2 x 24 heads the tensor pipe and the exponential unit
+// are each busy for 0.67 of the active clocks, issue slots for 0.45.
 // The running row max is refreshed lazily (only when it moves by more than 2^8), so the accumulator rescale is rare; it
 // waits for the tile's previous P V product first, and the block is then exponentiated again. The KV sequence may consist of several segments (one per ring
 // hop / context shard); (O, m, l) stay on chip across segments and the merge costs nothing.
@@ -314,11 +318,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint8_t* sv = sk + KV_STAGES * KV_TILE_BYTES;        // [KV_STAGES] tiles
   uint64_t* bars = reinterpret_cast<uint64_t*>(sv + KV_STAGES * KV_TILE_BYTES);
   uint64_t* q_full = bars;                        // [1]
-  uint64_t* q_empty = bars + 1;                   // [1] both S lanes
+  uint64_t* q_empty = bars + 1;                   // [1] the issuing lanes of both tiles (S)
   uint64_t* k_full = bars + 2;                    // [KV_STAGES]
-  uint64_t* k_empty = k_full + KV_STAGES;         // [KV_STAGES] both S lanes
+  uint64_t* k_empty = k_full + KV_STAGES;         // [KV_STAGES] the issuing lanes of both tiles (S)
   uint64_t* v_full = k_empty + KV_STAGES;         // [KV_STAGES]
-  uint64_t* v_empty = v_full + KV_STAGES;         // [KV_STAGES] both P V lanes
+  uint64_t* v_empty = v_full + KV_STAGES;         // [KV_STAGES] the issuing lanes of both tiles (P V)
   uint64_t* s_full = v_empty + KV_STAGES;         // [2 tiles][2 buffers] S written
   uint64_t* p_full = s_full + 4;                  // [2][2] P stored over S
   uint64_t* s_free = p_full + 4;                  // [2][2] P V product that reads the buffer (and adds into O) completed
