@@ -384,7 +384,8 @@ _DS_BYTES = 9 << 30      # most of dS that is held at a time: four heads of 3276
 _DS_CAPTURED = 1 << 30   # ... inside a captured graph, whose pool keeps it for as long as the graph lives
 _DS_TEMPORARY = 2 << 30  # up to here dS is asked for like any other temporary tensor
 _DS_MARGIN = 1 << 30     # memory that a request for more leaves to others
-_ds_refused: dict = {}   # device -> (bytes, memory in reach) at the last request that was refused or made the allocator flush
+_ds_refused: dict = {}   # device -> (bytes, memory in reach) at the last request that was refused, or flushed the allocator twice
+_ds_flushed: dict = {}   # device -> bytes of the last request that the allocator served after giving back its blocks
 
 
 def flash_ds_chunk(B: int, H: int, Sq: int, Skv: int, limit: int | None = None) -> int:
@@ -436,8 +437,8 @@ def _ds_room(device, enough: int) -> int:
 def _ds_buffer(B: int, H: int, Sq: int, Skv: int, device):
   """(pairs, buffer for their dS), or (0, None) where dQ is to be a pass of its own. A large buffer is asked for only where the
   memory is there: a request that the allocator cannot serve makes it give back all its blocks and wait for the device, and one
-  backward per layer would ask. After one that was refused, or served that way, no more than half of it is asked for until there is
-  more memory by its size."""
+  backward per layer would ask. After one that was refused, or served that way for the second time (the first leaves a block that
+  later ones can have), no more than half of it is asked for until there is more memory by its size."""
   per = -(-Skv // 128) * -(-Sq // 64) * 16384
   limit, room, retries = _DS_BYTES, None, 0
   captured = device.type == "cuda" and torch.cuda.is_current_stream_capturing()
@@ -460,7 +461,9 @@ def _ds_buffer(B: int, H: int, Sq: int, Skv: int, device):
       continue
     if room is not None:
       if _ds_stats(device)[1] != retries:
-        _ds_refused[device.index] = (n * per, room)
+        if _ds_flushed.get(device.index) == n * per:
+          _ds_refused[device.index] = (n * per, room)
+        _ds_flushed[device.index] = n * per
       elif n * per >= size:
         _ds_refused.pop(device.index, None)
     return n, ds
