@@ -59,7 +59,8 @@ struct Tap {
   int koff;            // first K index of this tap in the weight matrix
 };
 
-enum Epilogue : int { kEpiNone = 0, kEpiSilu = 1, kEpiRoundFirst = 2 };  // flags; the last: a residual is added to the result as bf16 holds it
+// Flags; kEpiRoundFirst: a residual is added to the result as bf16 holds it.
+enum Epilogue : int { kEpiNone = 0, kEpiSilu = 1, kEpiRoundFirst = 2 };
 
 struct Params {
   int n_classes;

@@ -474,8 +474,9 @@ def flash_bwd(q, d_o, k, v, lse, delta, scale=None):
   dS of a head is too large, the memory for it is not there or its parts are too small, dQ is a pass of its own (`flash_bwd_dq`);
   the bits are the same.
 
-  Both, two passes / dS kept, on a B200 in CUDA graphs (the last in a loop under the power cap): 4 x 1024^2 x 20 heads of 64 139 / 131 us, 4 x 4096^2 x 10 835 / 755, 4 x 4096 x 77 keys x 10
-  112 / 93; 4608^2 x 24 heads of 128 720 / 647, 32760 x 512 keys x 40 1546 / 1288 us, 32760^2 x 40 64.9 / 53.3 ms."""
+  Both, two passes / dS kept, on a B200 in CUDA graphs (the last in a loop under the power cap): 4 x 1024^2 x 20 heads of 64 139 / 131
+  us, 4 x 4096^2 x 10 835 / 755, 4 x 4096 x 77 keys x 10 112 / 93; 4608^2 x 24 heads of 128 720 / 647, 32760 x 512 keys x 40 1546 /
+  1288 us, 32760^2 x 40 64.9 / 53.3 ms."""
   B, Sq, H, D = q.shape
   Skv = k.shape[1]
   assert D in FLASH_HEAD_DIMS and all(t.stride(-1) == 1 for t in (q, d_o, k, v))
